@@ -183,7 +183,15 @@ typedef struct ocnn_conv_epilogue {
   const float* bias_dev;      /* [Cout] or NULL (= 0)  */
   const void* residual_dev;   /* same dtype/layout/shape as y, or NULL */
   int32_t relu;
+  /* read only when relu is OCNN_EPILOGUE_BATCHNORM or OCNN_EPILOGUE_BATCHNORM | 1 (with ReLU): the
+   * layer is followed by a BatchNorm on its running statistics, given as it stands: scale_dev and
+   * bias_dev are its weight and bias, and the kernel applies
+   *   scale = weight / sqrt(var + eps),   bias - mean * scale. */
+  const float* bn_mean_dev;
+  const float* bn_var_dev;
+  float bn_eps;
 } ocnn_conv_epilogue;
+#define OCNN_EPILOGUE_BATCHNORM 0x4f424e00
 
 int ocnn_octree_conv(const void* x_dev, const float* weights_dev, void* y_dev,
                      const int32_t* neigh_dev, int h_in, int h_out, int cin, int cout,

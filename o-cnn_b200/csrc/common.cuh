@@ -127,6 +127,46 @@ __device__ __forceinline__ uint32_t pack2(float a, float b, bool half) {
   return w;
 }
 
+// ---- per-channel affine map of a convolution's epilogue ------------------------------------------
+// Either a ready scale and bias, or an inference BatchNorm as the layer holds it (scale and bias
+// are then its weight and bias): folding it where the kernel stages its columns costs one square
+// root and division per column and CTA, and spares a network the launches that would compute the
+// folded vectors before every layer (five per layer as tensor operations: 105 of the 162 launches
+// of a small batch's ResNet forward).
+struct ChannelAffine {
+  const float* scale;
+  const float* bias;
+  const float* mean;
+  const float* var;
+  float eps;
+  __host__ __device__ bool any() const { return scale != nullptr || bias != nullptr || var != nullptr; }
+};
+inline ChannelAffine channel_affine_of(const ocnn_conv_epilogue* ep) {
+  ChannelAffine p = {nullptr, nullptr, nullptr, nullptr, 0.f};
+  if (ep == nullptr) return p;
+  p.scale = ep->scale_dev;
+  p.bias = ep->bias_dev;
+  if ((ep->relu & ~1) == OCNN_EPILOGUE_BATCHNORM) {
+    p.mean = ep->bn_mean_dev;
+    p.var = ep->bn_var_dev;
+    p.eps = ep->bn_eps;
+  }
+  return p;
+}
+inline int epilogue_relu(const ocnn_conv_epilogue* ep) {
+  if (ep == nullptr) return 0;
+  return (ep->relu & ~1) == OCNN_EPILOGUE_BATCHNORM ? (ep->relu & 1) : (ep->relu != 0);
+}
+// (scale, bias) of channel c
+__device__ __forceinline__ float2 channel_affine(const ChannelAffine& p, int c) {
+  float s = p.scale ? p.scale[c] : 1.f, b = p.bias ? p.bias[c] : 0.f;
+  if (p.var) {
+    s = s / sqrtf(p.var[c] + p.eps);
+    if (p.mean) b -= p.mean[c] * s;
+  }
+  return make_float2(s, b);
+}
+
 // ---- neighbour index arithmetic ---------------------------------------------------------------
 // Position, inside the 4x4x4 neighbour block of a sibling group, of the cell at offset
 // (tx-1, ty-1, tz-1) from octant o of that group, tap = tx*9 + ty*3 + tz.  This is the closed

@@ -17,8 +17,7 @@ struct PwArgs {
   int h, cin;
   int y_stride;            // output channels of the whole layer (row stride of y / residual)
   int co_base;             // first output channel this launch produces
-  const float* scale;
-  const float* bias;
+  ChannelAffine aff;
   const __nv_bfloat16* residual;
   int relu;
   int f16;                 // the 16-bit elements are fp16 instead of bf16
@@ -31,8 +30,7 @@ struct PwArgs {
   // rows this one has just produced, while they are still in registers: y2 = act(scale2 * (w2 * y)
   // + bias2), w2 fp32 [C2, COUT]
   const float* w2;
-  const float* scale2;
-  const float* bias2;
+  ChannelAffine aff2;
   __nv_bfloat16* y2;
   int relu2;
 };
@@ -44,8 +42,10 @@ struct PwArgs {
 template <int CIN, int COUT, int ROWS, bool HALF>
 __global__ void __launch_bounds__(256) conv_pw_kernel(const PwArgs a) {
   extern __shared__ float ws[];                      // [cin][COUT]
+  __shared__ float2 saff[COUT];
   grid_dependency_trigger();
   grid_dependency_wait();
+  for (int i = threadIdx.x; i < COUT; i += blockDim.x) saff[i] = channel_affine(a.aff, a.co_base + i);
   for (int i = threadIdx.x; i < a.cin * COUT; i += blockDim.x) {
     const int co = i / a.cin, ci = i % a.cin;        // coalesced read of w[co][ci], transposed store
     ws[ci * COUT + co] = a.w[(long long)a.co_base * a.cin + i];
@@ -157,8 +157,7 @@ __global__ void __launch_bounds__(256) conv_pw_kernel(const PwArgs a) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           f[j] = acc[r][8 * q + j];
-          if (a.scale) f[j] *= a.scale[a.co_base + 8 * q + j];
-          if (a.bias) f[j] += a.bias[a.co_base + 8 * q + j];
+          f[j] = fmaf(f[j], saff[8 * q + j].x, saff[8 * q + j].y);
         }
         if (a.residual) {
           const uint32_t* rp = reinterpret_cast<const uint32_t*>(&rres[r][q]);
@@ -350,8 +349,9 @@ __global__ void __launch_bounds__(256) conv_pw_mma_kernel(const PwArgs a) {
   for (int j = 0; j < NT; ++j)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      sc[j][e] = a.scale ? a.scale[q * CQ + 2 * j + e] : 1.f;
-      bi[j][e] = a.bias ? a.bias[q * CQ + 2 * j + e] : 0.f;
+      const float2 sb = channel_affine(a.aff, q * CQ + 2 * j + e);
+      sc[j][e] = sb.x;
+      bi[j][e] = sb.y;
     }
   // The second layer's A operand is this layer's packed output: the pair (2q, 2q + 1) of
   // accumulator tile 2s is K pair 2q of slice s, that of tile 2s + 1 is K pair 2q + 8, i.e. logical
@@ -376,8 +376,9 @@ __global__ void __launch_bounds__(256) conv_pw_mma_kernel(const PwArgs a) {
     for (int j = 0; j < NT2; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        sc2[j][e] = a.scale2 ? a.scale2[q * CQ2 + 2 * j + e] : 1.f;
-        bi2[j][e] = a.bias2 ? a.bias2[q * CQ2 + 2 * j + e] : 0.f;
+        const float2 sb = channel_affine(a.aff2, q * CQ2 + 2 * j + e);
+        sc2[j][e] = sb.x;
+        bi2[j][e] = sb.y;
       }
   }
   const long long tiles = ((long long)a.h + 15) >> 4;
@@ -478,8 +479,7 @@ struct PwPairArgs {
   const uint16_t* packed;
   __nv_bfloat16* y;
   int h, npad;
-  const float* scale;
-  const float* bias;
+  ChannelAffine aff;
   const __nv_bfloat16* residual;
   int relu;
 };
@@ -519,8 +519,9 @@ __global__ void __launch_bounds__(256) conv_pw_pair_kernel(const PwPairArgs a) {
   for (int j = 0; j < NT; ++j)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      sc[j][e] = a.scale ? a.scale[q * CQ + 2 * j + e] : 1.f;
-      bi[j][e] = a.bias ? a.bias[q * CQ + 2 * j + e] : 0.f;
+      const float2 sb = channel_affine(a.aff, q * CQ + 2 * j + e);
+      sc[j][e] = sb.x;
+      bi[j][e] = sb.y;
     }
   const long long tiles = ((long long)a.h + 15) >> 4;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -639,8 +640,9 @@ __global__ void __launch_bounds__(256) conv_pw_mma_pool_kernel(const PwArgs a) {
   for (int j = 0; j < NT; ++j)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      sc[j][e] = a.scale ? a.scale[q * CQ + 2 * j + e] : 1.f;
-      bi[j][e] = a.bias ? a.bias[q * CQ + 2 * j + e] : 0.f;
+      const float2 sb = channel_affine(a.aff, q * CQ + 2 * j + e);
+      sc[j][e] = sb.x;
+      bi[j][e] = sb.y;
     }
   const long long groups = (long long)a.h >> 3;
   const long long supers = (groups + 15) >> 4;
@@ -788,13 +790,12 @@ int conv_pointwise_bf16(const void* x, const float* w, void* y, int h, int cin, 
   a.y = static_cast<__nv_bfloat16*>(y);
   a.h = h; a.cin = cin;
   a.y_stride = cout; a.co_base = 0;
-  a.scale = ep ? ep->scale_dev : nullptr;
-  a.bias = ep ? ep->bias_dev : nullptr;
+  a.aff = channel_affine_of(ep);
   a.residual = ep ? static_cast<const __nv_bfloat16*>(ep->residual_dev) : nullptr;
-  a.relu = ep ? ep->relu : 0;
+  a.relu = epilogue_relu(ep);
   a.f16 = f16 ? 1 : 0;
   a.pool_inv = nullptr;
-  a.w2 = nullptr; a.scale2 = nullptr; a.bias2 = nullptr; a.y2 = nullptr; a.relu2 = 0;
+  a.w2 = nullptr; a.aff2 = channel_affine_of(nullptr); a.y2 = nullptr; a.relu2 = 0;
   a.wide = (((uintptr_t)x % 32) == 0 && ((uintptr_t)y % 32) == 0 &&
             (!(ep && ep->residual_dev) || ((uintptr_t)ep->residual_dev % 32) == 0)) ? 1 : 0;
   {
@@ -834,14 +835,13 @@ int conv_pointwise_pool_bf16(const void* x, const float* w, void* top, const int
   a.y = static_cast<__nv_bfloat16*>(top);
   a.h = h; a.cin = cin;
   a.y_stride = cout; a.co_base = 0;
-  a.scale = ep ? ep->scale_dev : nullptr;
-  a.bias = ep ? ep->bias_dev : nullptr;
+  a.aff = channel_affine_of(ep);
   a.residual = ep ? static_cast<const __nv_bfloat16*>(ep->residual_dev) : nullptr;
-  a.relu = ep ? ep->relu : 0;
+  a.relu = epilogue_relu(ep);
   a.f16 = f16 ? 1 : 0;
   a.wide = 0;
   a.pool_inv = inv;
-  a.w2 = nullptr; a.scale2 = nullptr; a.bias2 = nullptr; a.y2 = nullptr; a.relu2 = 0;
+  a.w2 = nullptr; a.aff2 = channel_affine_of(nullptr); a.y2 = nullptr; a.relu2 = 0;
   // is it a shape of the mma kernel?  (decided before anything is launched)
   bool known = false;
   for (int ci : {8, 16, 32, 64})
@@ -870,18 +870,16 @@ int conv_pointwise_chain_bf16(const void* x, const float* w1, void* y1, int h, i
   a.y = static_cast<__nv_bfloat16*>(y1);
   a.h = h; a.cin = cin;
   a.y_stride = cmid; a.co_base = 0;
-  a.scale = ep1 ? ep1->scale_dev : nullptr;
-  a.bias = ep1 ? ep1->bias_dev : nullptr;
+  a.aff = channel_affine_of(ep1);
   a.residual = ep1 ? static_cast<const __nv_bfloat16*>(ep1->residual_dev) : nullptr;
-  a.relu = ep1 ? ep1->relu : 0;
+  a.relu = epilogue_relu(ep1);
   a.f16 = f16 ? 1 : 0;
   a.wide = 0;
   a.pool_inv = nullptr;
   a.w2 = w2;
-  a.scale2 = ep2 ? ep2->scale_dev : nullptr;
-  a.bias2 = ep2 ? ep2->bias_dev : nullptr;
+  a.aff2 = channel_affine_of(ep2);
   a.y2 = static_cast<__nv_bfloat16*>(y2);
-  a.relu2 = ep2 ? ep2->relu : 0;
+  a.relu2 = epilogue_relu(ep2);
   const long long warps = ((long long)h + 15) / 16;
   const long long want = (warps + 47) / 48;
   const long long cap = (long long)sm_count() * 8;
@@ -918,10 +916,9 @@ int conv_pointwise_pair_packed(const void* xa, int ca, const void* xb, int cb, c
   a.packed = static_cast<const uint16_t*>(packed);
   a.y = static_cast<__nv_bfloat16*>(y);
   a.h = h; a.npad = npad;
-  a.scale = ep ? ep->scale_dev : nullptr;
-  a.bias = ep ? ep->bias_dev : nullptr;
+  a.aff = channel_affine_of(ep);
   a.residual = ep ? static_cast<const __nv_bfloat16*>(ep->residual_dev) : nullptr;
-  a.relu = ep ? ep->relu : 0;
+  a.relu = epilogue_relu(ep);
   const long long warps = ((long long)h + 15) / 16;
   const long long want = (warps + 47) / 48;
   const long long cap = (long long)sm_count() * 8;

@@ -39,8 +39,7 @@ struct ConvArgs {
   int transposed;      // deconvolution: weights are [Cin, Cout*K], element (ci, co*K + t)
   int up;              // stride-2 deconvolution: rows are nodes of the finer level, x rows are
                        // their parents' ranks among the non-empty nodes (= sibling-group indices)
-  const float* scale;
-  const float* bias;
+  ChannelAffine aff;
   const void* residual;
   int relu;
   signed char tap[27];
@@ -206,8 +205,8 @@ __global__ void __launch_bounds__(BM* BN / 16) conv_simt_kernel(const ConvArgs a
   for (int j = 0; j < 4; ++j) {
     const int co = n0 + tn * 4 + j;
     if (co >= a.cout) continue;
-    const float sc = a.scale ? a.scale[co] : 1.f;
-    const float bi = a.bias ? a.bias[co] : 0.f;
+    const float2 sb = channel_affine(a.aff, co);
+    const float sc = sb.x, bi = sb.y;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int h = h0 + tm * 4 + i;
@@ -246,10 +245,9 @@ int conv_simt_launch(const void* x, const float* w, void* y, const int32_t* neig
   a.K = tl.count; a.stride = stride; a.identity = identity ? 1 : 0;
   a.transposed = transposed ? 1 : 0;
   a.up = (transposed && stride == 2) ? 1 : 0;
-  a.scale = ep ? ep->scale_dev : nullptr;
-  a.bias = ep ? ep->bias_dev : nullptr;
+  a.aff = channel_affine_of(ep);
   a.residual = ep ? ep->residual_dev : nullptr;
-  a.relu = ep ? ep->relu : 0;
+  a.relu = epilogue_relu(ep);
   // a stride-1 deconvolution gathers from the mirrored offsets: node p receives from the node h
   // with p = h + offset(t), i.e. h = p - offset(t)
   for (int i = 0; i < 27; ++i)

@@ -85,8 +85,7 @@ struct TcArgs {
                     // node n / fold_cout of the row
   const int* scatter_child;   // with expand_cout: Child block of the finer level; octant o of tile
                               // row h is written to row scatter_child[8h + o] (skipped when < 0)
-  const float* scale;
-  const float* bias;
+  ChannelAffine aff;
   const __nv_bfloat16* residual;
   int relu;
   int* status;
@@ -311,8 +310,9 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
     if (a.fold_cout) co = n % a.fold_cout;
     if (GENERAL && a.expand_cout) co = (co_base + n) % a.expand_cout;
     const bool live = n < a.row_elems;
-    s_scale[n] = (live && a.scale) ? a.scale[co] : 1.f;
-    s_bias[n] = (live && a.bias) ? a.bias[co] : 0.f;
+    const float2 sb = live ? channel_affine(a.aff, co) : make_float2(1.f, 0.f);
+    s_scale[n] = sb.x;
+    s_bias[n] = sb.y;
   }
   if (tid < kTileM) {
     const int h = h0 + tid;          // node, or sibling group in group mode
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
     const uint32_t lane_base = tmem_base + ((uint32_t)(warp * 32) << 16);
     if (alive) {
       __nv_bfloat16* y_row = a.y + (long long)h * a.y_stride + co_base;
-      const bool has_sb = a.scale != nullptr || a.bias != nullptr;
+      const bool has_sb = a.aff.any();
       const bool scatter = GENERAL && a.scatter_child != nullptr;
       for (int c0 = 0; c0 < a.npad; c0 += 32) {
         uint4 res_cur[4];
@@ -820,8 +820,9 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
   for (int n = tid; n < a.npad; n += kThreadsP) {
     const bool live = n < a.row_elems;
     const int co = a.group ? (n & (a.cout - 1)) : (a.fold_cout ? n % a.fold_cout : co_base + n);
-    s_scale[n] = (live && a.scale) ? a.scale[co] : 1.f;
-    s_bias[n] = (live && a.bias) ? a.bias[co] : 0.f;
+    const float2 sb = live ? channel_affine(a.aff, co) : make_float2(1.f, 0.f);
+    s_scale[n] = sb.x;
+    s_bias[n] = sb.y;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1102,7 +1103,7 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
     constexpr bool f16 = HALF;
     bool alive = true;
-    const bool has_sb = a.scale != nullptr || a.bias != nullptr;
+    const bool has_sb = a.aff.any();
     int it = 0;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
       const int b = it % acc_bufs;
@@ -1329,7 +1330,7 @@ __global__ void pack_weights_group_kernel(const float* __restrict__ w, uint16_t*
 template <bool HALF>
 __global__ void fold_tail_kernel(const __nv_bfloat16* __restrict__ x, const uint16_t* __restrict__ packed,
                                  __nv_bfloat16* __restrict__ y, long long first, int count, int cin,
-                                 int cout, const float* __restrict__ scale, const float* __restrict__ bias,
+                                 int cout, const ChannelAffine aff,
                                  const __nv_bfloat16* __restrict__ residual, int relu) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count * cout) return;
@@ -1341,8 +1342,10 @@ __global__ void fold_tail_kernel(const __nv_bfloat16* __restrict__ x, const uint
     const float2 xf = unpack2((uint32_t)xr[ci], HALF), wf = unpack2((uint32_t)wv, HALF);
     acc = fmaf(xf.x, wf.x, acc);
   }
-  if (scale) acc *= scale[co];
-  if (bias) acc += bias[co];
+  if (aff.any()) {
+    const float2 sb = channel_affine(aff, co);
+    acc = fmaf(acc, sb.x, sb.y);
+  }
   const long long at = (first + node) * cout + co;
   if (residual) acc += unpack2((uint32_t)reinterpret_cast<const uint16_t*>(residual)[at], HALF).x;
   if (relu) acc = fmaxf(acc, 0.f);
@@ -1623,15 +1626,15 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
     if (dtype == OCNN_F16)
       fold_tail_kernel<true><<<ceil_div(threads, 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
           static_cast<const __nv_bfloat16*>(x), static_cast<const uint16_t*>(packed),
-          static_cast<__nv_bfloat16*>(y), first, fold_tail, cin, cout, ep ? ep->scale_dev : nullptr,
-          ep ? ep->bias_dev : nullptr, ep ? static_cast<const __nv_bfloat16*>(ep->residual_dev) : nullptr,
-          ep ? ep->relu : 0);
+          static_cast<__nv_bfloat16*>(y), first, fold_tail, cin, cout, channel_affine_of(ep),
+          ep ? static_cast<const __nv_bfloat16*>(ep->residual_dev) : nullptr,
+          epilogue_relu(ep));
     else
       fold_tail_kernel<false><<<ceil_div(threads, 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
           static_cast<const __nv_bfloat16*>(x), static_cast<const uint16_t*>(packed),
-          static_cast<__nv_bfloat16*>(y), first, fold_tail, cin, cout, ep ? ep->scale_dev : nullptr,
-          ep ? ep->bias_dev : nullptr, ep ? static_cast<const __nv_bfloat16*>(ep->residual_dev) : nullptr,
-          ep ? ep->relu : 0);
+          static_cast<__nv_bfloat16*>(y), first, fold_tail, cin, cout, channel_affine_of(ep),
+          ep ? static_cast<const __nv_bfloat16*>(ep->residual_dev) : nullptr,
+          epilogue_relu(ep));
     OCNN_LAUNCH_OK("fold_tail_kernel");
     note_launches(1);
     if (h_out < s.fold_nodes) return OCNN_OK;
@@ -1658,10 +1661,9 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
             (!(ep && ep->residual_dev) || (uintptr_t)ep->residual_dev % 32 == 0)) ? 1 : 0;
   if (s.group)
     OCNN_REQUIRE(h_out % 8 == 0, "%s: an octree level holds whole sibling groups (got %d nodes)", who, h_out);
-  a.scale = ep ? ep->scale_dev : nullptr;
-  a.bias = ep ? ep->bias_dev : nullptr;
+  a.aff = channel_affine_of(ep);
   a.residual = ep ? static_cast<const __nv_bfloat16*>(ep->residual_dev) : nullptr;
-  a.relu = ep ? ep->relu : 0;
+  a.relu = epilogue_relu(ep);
   a.status = status;
   for (int i = 0; i < 27; ++i) {
     int tap = i < tl.count ? tl.tap[i] : 0;

@@ -12,7 +12,7 @@ import torch
 from torch import nn as _nn
 
 from . import nn
-from .octree_conv import OctreeConv, OctreeDeconv, tc_status, _tensor_core_ready
+from .octree_conv import OctreeConv, OctreeDeconv, bn_vectors, tc_status
 from .octree_pool import OctreeMaxPool
 from .octree_pad import OctreeTile  # noqa: F401  (re-exported: the reference defines it here)
 
@@ -49,8 +49,7 @@ class _OctreeBlock(_nn.Module):
       assert data_in.size(1) == op.channel_in
       if not op.is_conv_layer() and op.stride == 2 and not op.nempty:
         data_in = nn.octree_depad(data_in, octree, op.depth)
-      scale, bias = _folded(self.bn)
-      return op._run(data_in, octree, (scale, bias, residual, relu))
+      return op._run(data_in, octree, self.bn, residual, relu)
     out = self.bn(op(data_in, octree))
     if residual is not None:
       out = out + residual
@@ -84,41 +83,39 @@ class FcBnRelu(_nn.Module):
 class OctreeConv1x1(_nn.Module):
   """A per-node linear map.  The parameters live in a torch Conv1d (as in the reference, so the
   state_dict keys match); the product runs on this library's pointwise kernels."""
+  _layer = None
 
   def __init__(self, channel_in, channel_out, use_bias=False):
     super().__init__()
     self.conv1x1 = _nn.Conv1d(channel_in, channel_out, kernel_size=1, bias=use_bias)
-    self._packed = {}
 
-  def run(self, data_in, scale=None, bias=None, residual=None, relu=False):
+  def run(self, data_in, bn=None, residual=None, relu=False):
+    """The product, and the BatchNorm on its running statistics, residual and ReLU that follow it."""
+    conv = self.conv1x1
     if torch.is_grad_enabled() and (data_in.requires_grad or
-                                    (self.training and self.conv1x1.weight.requires_grad)):
+                                    (self.training and conv.weight.requires_grad)):
       # training: torch's own 1x1 convolution (as the reference), which autograd differentiates
-      out = self.conv1x1(data_in.squeeze(-1)).unsqueeze(-1)
-      if scale is not None:
-        out = out * scale.view(1, -1, 1, 1)
-      if bias is not None and self.conv1x1.bias is None:
-        out = out + bias.view(1, -1, 1, 1)
+      out = conv(data_in.squeeze(-1)).unsqueeze(-1)
+      if bn is not None:
+        scale, bias = _folded(bn)
+        out = out * scale.view(1, -1, 1, 1) + bias.view(1, -1, 1, 1)
       if residual is not None:
         out = out + residual
       return torch.relu(out) if relu else out
-    w = self.conv1x1.weight.detach()
-    cout, cin = w.shape[0], w.shape[1]
-    w2 = w.reshape(cout, cin).float()
-    if self.conv1x1.bias is not None:
-      b = self.conv1x1.bias.detach().float()
-      bias = b if bias is None else bias + (b * scale if scale is not None else b)
-    with torch.no_grad():
-      if _tensor_core_ready(data_in) and cout % 8 == 0 and (cout <= 256 or cout % 256 == 0):
-        half = data_in.dtype == torch.float16
-        key = (w.data_ptr(), w._version, half)
-        if key not in self._packed:
-          self._packed.clear()
-          self._packed[key] = nn.conv_pack_weights_general(w2.contiguous(), cin, cout, [1, 1, 1], 1,
-                                                           False, False, half)
-        return nn.pointwise_conv_tc(data_in, self._packed[key], cout, scale, bias, residual, relu,
-                                    tc_status(data_in.device))
-      return nn.pointwise_conv(data_in, w2.contiguous(), scale, bias, residual, relu)
+    if self._layer is None:
+      cout, cin = conv.weight.shape[:2]
+      self._layer = nn.ConvLayer(cin, cout, [1, 1, 1], 1, False, False, True)
+    affine = bn_vectors(bn)
+    if conv.bias is not None:
+      with torch.no_grad():
+        b = conv.bias.detach().float()
+        if bn is None:
+          affine = (None, b, None, None, 0.0)
+        else:
+          scale, bias = _folded(bn)
+          affine = (scale, bias + b * scale, None, None, 0.0)
+    return self._layer.run(data_in, conv.weight, None, 0, *affine, residual, relu,
+                           tc_status(data_in.device))
 
   def forward(self, data_in):
     return self.run(data_in)
@@ -137,8 +134,7 @@ class _Conv1x1Block(_nn.Module):
   def forward(self, data_in, residual=None, relu=None):
     relu = self.with_relu if relu is None else relu
     if FUSE_EVAL_BN and not self.training:
-      scale, bias = _folded(self.bn)
-      return self.conv1x1.run(data_in, scale, bias, residual, relu)
+      return self.conv1x1.run(data_in, self.bn, residual, relu)
     out = self.bn(self.conv1x1(data_in))
     if residual is not None:
       out = out + residual

@@ -6,7 +6,7 @@ index c * K + tap — so a reference state_dict loads unchanged.  Every variant 
 nodes or non-empty nodes only) is one implicit-GEMM CUDA kernel; no column buffer is built.
 
 Data in bfloat16 / float16 with torch's channels_last memory format runs on the tensor-core
-kernel (weights are packed once per module and dtype and cached); float32 data, or the
+kernel (weights are packed when they change, `nn.ConvLayer`); float32 data, or the
 reference's contiguous [1,C,H,1] layout, runs on the CUDA-core kernel.  float32 data that takes
 part in autograd (training) goes through `OctreeConvFunction` / `OctreeDeconvFunction`, whose
 backward is the transposed operator for the data and a node-reduction kernel for the weights.
@@ -38,9 +38,13 @@ def resize_with_last_val(list_in, num=3):
   return out
 
 
-def _tensor_core_ready(data):
-  return (data.is_cuda and data.dtype in (torch.bfloat16, torch.float16) and data.dim() == 4 and
-          data.shape[1] % 8 == 0 and data.is_contiguous(memory_format=torch.channels_last))
+def bn_vectors(bn):
+  """(weight, bias, running mean, running variance, eps) of a BatchNorm for the native layer call."""
+  if bn is None:
+    return None, None, None, None, 0.0
+  if bn.running_var is None:
+    raise RuntimeError('a BatchNorm without running statistics cannot be applied in eval mode')
+  return bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.eps
 
 
 class _ConvFunctionBase(torch.autograd.Function):
@@ -107,6 +111,8 @@ def octree_deconv(data_in, weights, octree, depth, channel_out, kernel_size, str
 
 
 class OctreeConvBase(_nn.Module):
+  _layer = None                # the native side of the layer: packed weights, kernel choice
+
   def __init__(self, depth, channel_in, channel_out, kernel_size=[3], stride=1, nempty=False):
     super().__init__()
     self.depth = depth
@@ -121,40 +127,25 @@ class OctreeConvBase(_nn.Module):
     self.cdim = self.conv_in * self.kdim
     self.weights = _nn.Parameter(torch.Tensor(self.conv_out, self.cdim))
     _nn.init.xavier_uniform_(self.weights)
-    self._packed = {}
 
   def is_conv_layer(self):
     raise NotImplementedError
 
-  def _run(self, data, octree, fused=None):
-    """One kernel for the layer; `fused` = (scale, bias, residual, relu) applied in its epilogue."""
-    scale, bias, residual, relu = fused if fused is not None else (None, None, None, False)
-    transposed = not self.is_conv_layer()
-    if (fused is None and data.dtype == torch.float32 and torch.is_grad_enabled() and
+  def _run(self, data, octree, bn=None, residual=None, relu=False):
+    """One kernel for the layer, with a BatchNorm on its running statistics, the residual and the
+    ReLU that follow it applied in its epilogue."""
+    plain = bn is None and residual is None and not relu
+    if (plain and data.dtype == torch.float32 and torch.is_grad_enabled() and
         (data.requires_grad or (self.training and self.weights.requires_grad))):
-      fn = OctreeDeconvFunction if transposed else OctreeConvFunction
+      fn = OctreeConvFunction if self.is_conv_layer() else OctreeDeconvFunction
       return fn.apply(data, self.weights, octree, self.depth, self.channel_out, self.kernel_size,
                       self.stride, self.nempty)
-    w = self.weights.detach()
-    with torch.no_grad():
-      if _tensor_core_ready(data) and self.channel_out % 8 == 0:
-        half = data.dtype == torch.float16
-        key = (w.data_ptr(), w._version, half)
-        if key not in self._packed:
-          self._packed.clear()
-          try:
-            self._packed[key] = nn.conv_pack_weights_general(
-                w, self.channel_in, self.channel_out, self.kernel_size, self.stride, transposed,
-                self.nempty, half)
-          except RuntimeError:
-            self._packed[key] = None          # a shape the tensor-core kernel does not take
-        packed = self._packed[key]
-        if packed is not None:
-          return nn.octree_conv_tc_general(
-              data, packed, octree, self.depth, self.channel_out, self.kernel_size, self.stride,
-              self.nempty, transposed, scale, bias, residual, relu, tc_status(data.device))
-      return nn.octree_conv_general(data, w, octree, self.depth, self.channel_out, self.kernel_size,
-                                    self.stride, self.nempty, transposed, scale, bias, residual, relu)
+    layer = self._layer
+    if layer is None:
+      layer = self._layer = nn.ConvLayer(self.channel_in, self.channel_out, self.kernel_size,
+                                         self.stride, self.nempty, not self.is_conv_layer())
+    return layer.run(data, self.weights, octree, self.depth, *bn_vectors(bn), residual, relu,
+                     tc_status(data.device))
 
   def extra_repr(self) -> str:
     return ('depth={}, channel_in={}, channel_out={}, kernel_size={}, stride={}, '

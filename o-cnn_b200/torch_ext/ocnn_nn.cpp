@@ -12,6 +12,7 @@
 //    channels_last (node-major).  Outputs keep the dtype and layout of the input.
 //  * Errors raise Python exceptions; nothing aborts (pytorch/cpp uses CHECK -> abort()).
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime.h>
 #include <torch/extension.h>
@@ -19,6 +20,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -45,11 +48,22 @@ void* current_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 // ---- octree header cache ------------------------------------------------------------------------
 // Keyed by the tensor's StorageImpl; the weak reference keeps that address from being reused for
 // another storage while the entry lives, so a hit is always the same buffer.
+//
+// An entry also owns the index tables that operators on the non-empty nodes derive from the
+// octree: the inverse of a level's child array is the same for every layer that works on the level (a
+// U-Net's forward asked for it 55 times).  They are kept per (depth, stream), so a table is only
+// ever read on the stream that wrote it, and leave with the entry: at the latest when the next
+// octree is registered after this one's storage is gone.
+struct OctreeTables {
+  std::mutex mutex;
+  std::map<std::pair<int, void*>, Tensor> ichild;
+};
 struct CachedHeader {
   c10::weak_intrusive_ptr<c10::StorageImpl> storage;
   int64_t offset;
   uint32_t version;
   ocnn_octree_meta meta;
+  std::shared_ptr<OctreeTables> tables;
   uint8_t raw[OCNN_HEADER_BYTES];
 };
 std::mutex g_cache_mutex;
@@ -60,7 +74,22 @@ struct OctreeRef {
   uint8_t raw[OCNN_HEADER_BYTES];
   uint8_t* base;   // device (or host) pointer of byte 0
   bool cuda;
+  std::shared_ptr<OctreeTables> tables;   // CUDA octrees only
 };
+
+// Entries of octrees that no longer exist are dropped (the map holds an entry per live octree, so
+// the walk is short).  Call with the mutex held; the tables are released by the caller afterwards,
+// outside of it.
+void drop_expired(std::vector<std::shared_ptr<OctreeTables>>* released) {
+  for (auto it = g_cache.begin(); it != g_cache.end();) {
+    if (it->second.storage.expired()) {
+      released->push_back(std::move(it->second.tables));
+      it = g_cache.erase(it);
+    } else {
+      ++it;
+    }
+  }
+}
 
 OctreeRef get_octree(const Tensor& octree) {
   TORCH_CHECK(octree.scalar_type() == torch::kUInt8 && octree.dim() == 1 && octree.is_contiguous(),
@@ -84,6 +113,7 @@ OctreeRef get_octree(const Tensor& octree) {
       CachedHeader& c = it->second;
       if (!c.storage.expired() && c.offset == octree.storage_offset() && c.version == version) {
         ref.meta = c.meta;
+        ref.tables = c.tables;
         memcpy(ref.raw, c.raw, sizeof(ref.raw));
         return ref;
       }
@@ -98,15 +128,14 @@ OctreeRef get_octree(const Tensor& octree) {
   OCNN_CALL(ocnn_parse_header(ref.raw, (size_t)octree.numel(), &ref.meta));
   TORCH_CHECK(ref.meta.ptr_dis[OCNN_PROP_COUNT] <= octree.numel(),
               "the octree tensor is shorter than its header says");
-  std::lock_guard<std::mutex> lock(g_cache_mutex);
-  if (g_cache.size() > 256) {
-    for (auto it = g_cache.begin(); it != g_cache.end();)
-      it = it->second.storage.expired() ? g_cache.erase(it) : std::next(it);
-  }
+  ref.tables = std::make_shared<OctreeTables>();
   CachedHeader c{c10::weak_intrusive_ptr<c10::StorageImpl>(
                      c10::intrusive_ptr<c10::StorageImpl>::reclaim_copy(impl)),
-                 octree.storage_offset(), version, ref.meta, {}};
+                 octree.storage_offset(), version, ref.meta, ref.tables, {}};
   memcpy(c.raw, ref.raw, sizeof(c.raw));
+  std::vector<std::shared_ptr<OctreeTables>> released;
+  std::lock_guard<std::mutex> lock(g_cache_mutex);
+  drop_expired(&released);
   g_cache.emplace(impl, std::move(c));
   return ref;
 }
@@ -115,9 +144,12 @@ void remember_header(const Tensor& octree, const ocnn_octree_meta& meta, const u
   c10::StorageImpl* impl = octree.storage().unsafeGetStorageImpl();
   CachedHeader c{c10::weak_intrusive_ptr<c10::StorageImpl>(
                      c10::intrusive_ptr<c10::StorageImpl>::reclaim_copy(impl)),
-                 octree.storage_offset(), (uint32_t)octree._version(), meta, {}};
+                 octree.storage_offset(), (uint32_t)octree._version(), meta,
+                 std::make_shared<OctreeTables>(), {}};
   memcpy(c.raw, raw, sizeof(c.raw));
+  std::vector<std::shared_ptr<OctreeTables>> released;
   std::lock_guard<std::mutex> lock(g_cache_mutex);
+  drop_expired(&released);
   g_cache.erase(impl);
   g_cache.emplace(impl, std::move(c));
 }
@@ -349,9 +381,20 @@ std::tuple<Tensor, Tensor> conv1x1_chain(Tensor data_in, Tensor w1, c10::optiona
 // ichild of a level (node of the i-th non-empty node), as pytorch/cpp/octree2col.cpp:8-18 builds it.
 Tensor make_ichild(const OctreeRef& o, int depth, const torch::TensorOptions& like, const char* what) {
   const int nne = o.meta.nnum_nempty[depth], nnum = o.meta.nnum[depth];
+  const std::pair<int, void*> key(depth, current_stream());
+  if (o.tables) {
+    std::lock_guard<std::mutex> lock(o.tables->mutex);
+    auto it = o.tables->ichild.find(key);
+    if (it != o.tables->ichild.end()) return it->second;
+  }
   Tensor ichild = torch::zeros({std::max(nne, 1)}, like.dtype(torch::kInt32));
   OCNN_CALL(ocnn_octree_ichild(level_ptr(o, OCNN_PROP_CHILD, depth, what), nnum,
                                ichild.data_ptr<int32_t>(), current_stream()));
+  // (a table written inside a graph capture holds nothing until the graph runs)
+  if (o.tables && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
+    std::lock_guard<std::mutex> lock(o.tables->mutex);
+    o.tables->ichild.emplace(key, ichild);
+  }
   return ichild;
 }
 
@@ -453,7 +496,8 @@ ocnn_conv_epilogue make_epilogue(const c10::optional<Tensor>& scale, const c10::
                                  const c10::optional<Tensor>& residual, bool relu, int cout,
                                  const Tensor& y) {
   ocnn_conv_epilogue ep;
-  ep.scale_dev = nullptr; ep.bias_dev = nullptr; ep.residual_dev = nullptr; ep.relu = relu ? 1 : 0;
+  memset(&ep, 0, sizeof(ep));
+  ep.relu = relu ? 1 : 0;
   if (scale.has_value() && scale->defined()) {
     TORCH_CHECK(scale->is_cuda() && scale->scalar_type() == torch::kFloat32 && scale->is_contiguous() &&
                     scale->numel() == cout, "scale must be a contiguous float32 CUDA tensor of Cout values");
@@ -509,7 +553,7 @@ Tensor octree_conv_nempty(Tensor data_in, Tensor weights, Tensor octree, int dep
   need_cuda(data_in, "octree_conv");
   c10::cuda::CUDAGuard guard(data_in.device());
   DataRef x = get_data(data_in, "octree_conv");
-  const int nne = o.meta.nnum_nempty[depth], nnum = o.meta.nnum[depth];
+  const int nne = o.meta.nnum_nempty[depth];
   TORCH_CHECK(x.H == nne, "octree_conv (nempty): data height ", x.H, " != non-empty node number ", nne);
   const int kdim = ks[0] * ks[1] * ks[2];
   TORCH_CHECK(weights.is_cuda() && weights.scalar_type() == torch::kFloat32 &&
@@ -518,8 +562,7 @@ Tensor octree_conv_nempty(Tensor data_in, Tensor weights, Tensor octree, int dep
   Tensor w = weights.contiguous();
   Tensor y = new_data(num_output, nne, x);
   const int32_t* child = level_ptr(o, OCNN_PROP_CHILD, depth, "octree_conv");
-  Tensor ichild = torch::empty({std::max(nne, 1)}, x.t.options().dtype(torch::kInt32));
-  OCNN_CALL(ocnn_octree_ichild(child, nnum, ichild.data_ptr<int32_t>(), current_stream()));
+  Tensor ichild = make_ichild(o, depth, x.t.options(), "octree_conv");
   const int32_t* neigh = kdim > 1 ? level_ptr(o, OCNN_PROP_NEIGH, depth, "octree_conv") : nullptr;
   OCNN_CALL(ocnn_octree_conv_nempty(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), neigh, child,
                                     ichild.data_ptr<int32_t>(), nne, x.C, num_output, ks.data(),
@@ -628,7 +671,7 @@ Tensor octree_conv_tc_nempty(Tensor data_in, Tensor packed, Tensor octree, int d
   TORCH_CHECK(x.dtype == OCNN_BF16 && (x.layout == OCNN_NODE_MAJOR || x.C == 1 || x.H == 1),
               "octree_conv_tc_nempty takes bfloat16 channels_last data");
   x.layout = OCNN_NODE_MAJOR;
-  const int nne = o.meta.nnum_nempty[depth], nnum = o.meta.nnum[depth];
+  const int nne = o.meta.nnum_nempty[depth];
   TORCH_CHECK(x.H == nne, "octree_conv_tc_nempty: data height ", x.H, " != non-empty node number ", nne);
   TORCH_CHECK(packed.is_cuda() && packed.scalar_type() == torch::kUInt8 &&
                   (size_t)packed.numel() == ocnn_conv_packed_weight_bytes_nempty(x.C, num_output, ks.data()),
@@ -638,8 +681,7 @@ Tensor octree_conv_tc_nempty(Tensor data_in, Tensor packed, Tensor octree, int d
   Tensor y = new_data(num_output, nne, x);
   ocnn_conv_epilogue ep = make_epilogue(scale, bias, residual, relu, num_output, y);
   const int32_t* child = level_ptr(o, OCNN_PROP_CHILD, depth, "octree_conv_tc_nempty");
-  Tensor ichild = torch::empty({std::max(nne, 1)}, x.t.options().dtype(torch::kInt32));
-  OCNN_CALL(ocnn_octree_ichild(child, nnum, ichild.data_ptr<int32_t>(), current_stream()));
+  Tensor ichild = make_ichild(o, depth, x.t.options(), "octree_conv_tc_nempty");
   const int kdim = ks[0] * ks[1] * ks[2];
   const int32_t* neigh = kdim > 1 ? level_ptr(o, OCNN_PROP_NEIGH, depth, "octree_conv_tc_nempty") : nullptr;
   OCNN_CALL(ocnn_octree_conv_tc_nempty(x.t.data_ptr(), packed.data_ptr(), y.data_ptr(), neigh, child,
@@ -912,6 +954,119 @@ Tensor pointwise_conv_tc(Tensor data_in, Tensor packed, int num_output, c10::opt
                                         current_stream()));
   return y;
 }
+
+// ---- a module's layer -------------------------------------------------------------------------------
+// What OctreeConv / OctreeDeconv (point = false) and OctreeConv1x1 (point = true) do for one call in
+// eval mode, with the BatchNorm, residual and ReLU that follow: choose the kernel, pack the weights when
+// they have changed, launch.  The module hands over its parameters as they are; the BatchNorm is
+// folded inside the kernel (ChannelAffine), so a layer is one call from Python and one launch.
+// (In Python, with the folded vectors computed by tensor operations, it was about 60 us of host time
+// and six launches per layer.)
+class ConvLayer {
+ public:
+  ConvLayer(int cin, int cout, vector<int> ks, int stride, bool nempty, bool transposed, bool point)
+      : cin_(cin), cout_(cout), ks_(kernel3(ks)), stride_(stride), nempty_(nempty),
+        transposed_(transposed), point_(point) {}
+  ConvLayer(const ConvLayer& o)
+      : cin_(o.cin_), cout_(o.cout_), ks_(o.ks_), stride_(o.stride_), nempty_(o.nempty_),
+        transposed_(o.transposed_), point_(o.point_) {}
+
+  Tensor run(Tensor data, Tensor weights, c10::optional<Tensor> octree, int depth,
+             c10::optional<Tensor> scale, c10::optional<Tensor> bias, c10::optional<Tensor> bn_mean,
+             c10::optional<Tensor> bn_var, double bn_eps, c10::optional<Tensor> residual, bool relu,
+             Tensor status) {
+    torch::NoGradGuard no_grad;
+    const char* what = transposed_ ? "octree_deconv" : "octree_conv";
+    need_cuda(data, what);
+    c10::cuda::CUDAGuard guard(data.device());
+    DataRef x = get_data(data, what);
+    const int K = ks_[0] * ks_[1] * ks_[2];
+    TORCH_CHECK(x.C == cin_, what, ": the data has ", x.C, " channels, the layer takes ", cin_);
+    Geometry geo;
+    if (point_) {
+      memset(&geo.g, 0, sizeof(geo.g));
+      geo.g.stride = 1; geo.g.h_in = x.H; geo.g.h_out = x.H;
+    } else {
+      TORCH_CHECK(octree.has_value(), what, ": octree required");
+      OctreeRef o = get_octree(*octree);
+      TORCH_CHECK(o.cuda, what, ": the octree must be a CUDA tensor");
+      geo = make_geometry(o, x, depth, ks_, stride_, nempty_, transposed_, what);
+    }
+    Tensor keep[5];     // float32 copies of parameters that are held in another type
+    auto f32 = [&](const c10::optional<Tensor>& t, int slot) -> const float* {
+      if (!t.has_value() || !t->defined()) return nullptr;
+      TORCH_CHECK(t->is_cuda() && t->numel() == cout_, what, ": per-channel vectors must be CUDA tensors of ",
+                  cout_, " values");
+      keep[slot] = t->to(torch::kFloat32).contiguous();
+      return keep[slot].data_ptr<float>();
+    };
+    const bool has_bn = bn_var.has_value() && bn_var->defined();
+    Tensor y = new_data(cout_, geo.g.h_out, x);
+    ocnn_conv_epilogue ep = make_epilogue(c10::nullopt, c10::nullopt, residual, relu, cout_, y);
+    ep.scale_dev = f32(scale, 0);
+    ep.bias_dev = f32(bias, 1);
+    if (has_bn) {
+      ep.relu = OCNN_EPILOGUE_BATCHNORM | (relu ? 1 : 0);
+      ep.bn_mean_dev = f32(bn_mean, 2);
+      ep.bn_var_dev = f32(bn_var, 3);
+      ep.bn_eps = (float)bn_eps;
+    }
+    Tensor w = point_ ? weights.to(torch::kFloat32).contiguous() : weights;
+    check_weights(w, cin_, cout_, K);
+    const bool tc_layout = x.dtype != OCNN_F32 && cin_ % 8 == 0 && cout_ % 8 == 0 &&
+                           data.is_contiguous(at::MemoryFormat::ChannelsLast);
+    if (tc_layout) {
+      Tensor packed = packed_for(weights, w, x.dtype == OCNN_F16);
+      if (packed.defined()) {
+        TORCH_CHECK(status.is_cuda() && status.scalar_type() == torch::kInt32 && status.numel() >= 1,
+                    "status must be an int32 CUDA tensor");
+        OCNN_CALL(ocnn_octree_conv_tc_general(x.t.data_ptr(), packed.data_ptr(), y.data_ptr(), &geo.g, cin_,
+                                              cout_, ks_.data(), x.dtype, &ep,
+                                              status.data_ptr<int32_t>(), current_stream()));
+        return y;
+      }
+    }
+    w = w.contiguous();
+    if (point_) {
+      OCNN_CALL(ocnn_octree_conv(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), nullptr, x.H, x.H, cin_,
+                                 cout_, ks_.data(), 1, x.dtype, x.layout, &ep, current_stream()));
+    } else {
+      OCNN_CALL(ocnn_octree_conv_general(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), &geo.g, cin_,
+                                         cout_, ks_.data(), x.dtype, x.layout, &ep, current_stream()));
+    }
+    return y;
+  }
+
+  pybind11::tuple state() const {
+    return pybind11::make_tuple(cin_, cout_, ks_, stride_, nempty_, transposed_, point_);
+  }
+
+ private:
+  // The packed image of the module's parameter `weights` (`w`: its float32 values), made when it was
+  // not seen before (another tensor, or written to since); undefined for a shape the tensor-core
+  // kernel does not take.
+  Tensor packed_for(const Tensor& weights, const Tensor& w, bool half) {
+    const bool versioned = !weights.is_inference();
+    const void* ptr = weights.data_ptr();
+    const int64_t version = versioned ? (int64_t)weights._version() : -1;
+    std::lock_guard<std::mutex> lock(mutex_);
+    if (versioned && ptr == ptr_ && version == version_ && half == half_) return packed_;
+    packed_ = Tensor();
+    if (ocnn_conv_packed_weight_bytes_general(cin_, cout_, ks_.data(), stride_, transposed_, nempty_) > 0)
+      packed_ = conv_pack_weights_general(w, cin_, cout_, ks_, stride_, transposed_, nempty_, half);
+    ptr_ = ptr; version_ = version; half_ = half;
+    return packed_;
+  }
+  int cin_, cout_;
+  vector<int> ks_;
+  int stride_;
+  bool nempty_, transposed_, point_;
+  std::mutex mutex_;
+  Tensor packed_;
+  const void* ptr_ = nullptr;
+  int64_t version_ = -1;
+  bool half_ = false;
+};
 
 // 1x1x1 convolution over the concatenated channels of two tensors of the same rows: the sum of a
 // residual block's conv1x1b and its shortcut conv1x1c (pytorch/ocnn/modules.py OctreeResBlock) in
@@ -2187,6 +2342,17 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("bf16") = true, py::arg("half") = false);
   m.def("set_key_bits", &set_key_bits);
   m.def("get_key_bits", &get_key_bits);
+  py::class_<ConvLayer>(m, "ConvLayer")
+      .def(py::init<int, int, vector<int>, int, bool, bool, bool>(), py::arg("cin"), py::arg("cout"),
+           py::arg("kernel_size"), py::arg("stride") = 1, py::arg("nempty") = false,
+           py::arg("transposed") = false, py::arg("point") = false)
+      .def("run", &ConvLayer::run)
+      .def(py::pickle([](const ConvLayer& l) { return l.state(); },
+                      [](py::tuple t) {
+                        return std::make_unique<ConvLayer>(
+                            t[0].cast<int>(), t[1].cast<int>(), t[2].cast<vector<int>>(), t[3].cast<int>(),
+                            t[4].cast<bool>(), t[5].cast<bool>(), t[6].cast<bool>());
+                      }));
   py::class_<NetExecutor>(m, "NetExecutor")
       .def(py::init<>())
       .def("add_feature", &NetExecutor::add_feature)

@@ -1,0 +1,98 @@
+"""The native layer call behind the modules (`ocnn.nn.ConvLayer`): BatchNorm folded inside the kernels,
+weights packed again when they change, copies and pickles of a module, the per-octree tables."""
+import copy
+import pickle
+
+import pytest
+import torch
+
+import gpu_util as gu
+from oracle import oracle as oc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope='module')
+def ocnn():
+  import ocnn as mod
+  mod.set_key_bits(64)
+  return mod
+
+
+@pytest.fixture(scope='module')
+def batch():
+  _, merged, _ = gu.oracle_batch(gu.small_clouds(3, 3000, 500), 5, 2, 64)
+  return gu.to_cuda_u8(merged), oc.OctreeView(merged)
+
+
+def randomised(bn, seed):
+  g = torch.Generator().manual_seed(seed)
+  with torch.no_grad():
+    for t, lo in ((bn.weight, 0.5), (bn.bias, -0.3), (bn.running_mean, -0.3), (bn.running_var, 0.5)):
+      t.copy_(torch.rand(t.shape, generator=g) + lo)
+  return bn
+
+
+# (cin, cout, kernel, dtype): group mode, node mode, folded 1x1 (with a node count that leaves a tail on
+# non-empty nodes), CUDA-core kernel
+@pytest.mark.parametrize('cin,cout,ks,nempty', [
+    (8, 16, [3], False), (64, 64, [3], False), (24, 40, [3], True), (32, 8, [1], False),
+    (16, 32, [1], True), (64, 256, [1], False), (5, 7, [3], False)])
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16, torch.float16])
+def test_batchnorm_in_the_epilogue(ocnn, batch, cin, cout, ks, nempty, dtype):
+  octree, v = batch
+  if dtype != torch.float32 and cin % 8:
+    pytest.skip('16-bit layers take multiples of eight channels')
+  d = 5
+  h = int(v.nnum_nempty[d] if nempty else v.nnum[d])
+  torch.manual_seed(cin + cout)
+  x = torch.randn(1, cin, h, 1, device='cuda').to(dtype)
+  res = torch.randn(1, cout, h, 1, device='cuda').to(dtype)
+  if dtype != torch.float32:
+    x = x.contiguous(memory_format=torch.channels_last)
+    res = res.contiguous(memory_format=torch.channels_last)
+  bn = randomised(torch.nn.BatchNorm2d(cout, 1e-3), 3).cuda().eval()
+  if ks == [1]:
+    layer = ocnn.OctreeConv1x1(cin, cout).cuda().eval()
+    call = lambda *a: layer.run(x, *a)
+  else:
+    layer = ocnn.OctreeConv(d, cin, cout, ks, nempty=nempty).cuda().eval()
+    call = lambda *a: layer._run(x, octree, *a)
+  with torch.no_grad():
+    for _ in range(2):                     # the second pass after the parameters have changed in place
+      got = call(bn, res, True).float()
+      want = torch.relu(bn(call().float()) + res.float())
+      scale = float(want.abs().max())
+      assert float((got - want).abs().max()) < (1e-5 if dtype == torch.float32 else 2e-2) * scale
+      for p in list(layer.parameters()) + [bn.running_mean, bn.running_var]:
+        p.mul_(1.25)
+
+
+def test_copies_of_a_used_layer(ocnn, batch):
+  octree, v = batch
+  x = torch.randn(1, 8, int(v.nnum[5]), 1, device='cuda').to(torch.bfloat16)
+  x = x.contiguous(memory_format=torch.channels_last)
+  net = ocnn.OctreeConvBnRelu(5, 8, 16).cuda().eval()
+  with torch.no_grad():
+    want = net(x, octree)
+    for other in (copy.deepcopy(net), pickle.loads(pickle.dumps(net))):
+      assert torch.equal(other(x, octree), want)
+
+
+def test_tables_follow_the_octree(ocnn, batch):
+  """The inverse child table kept with an octree: per stream, and gone with the octree's content."""
+  octree, v = batch
+  other = torch.cuda.Stream()
+  conv = ocnn.OctreeConv(5, 8, 8, nempty=True).cuda().eval()
+  x = torch.randn(1, 8, int(v.nnum_nempty[5]), 1, device='cuda')
+  with torch.no_grad():
+    mine = octree.clone()
+    want = conv(x, octree)
+    assert torch.equal(conv(x, mine), want) and torch.equal(conv(x, mine), want)
+    other.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(other):
+      got = conv(x, mine)
+    torch.cuda.current_stream().wait_stream(other)
+    assert torch.equal(got, want)
+    mine.copy_(octree)                     # the same storage, written to: the tables are made again
+    assert torch.equal(conv(x, mine), want)
