@@ -247,6 +247,18 @@ int ocnn_octree_conv_general(const void* x_dev, const float* weights_dev, void* 
                              const int kernel_size[3], int dtype, int layout,
                              const ocnn_conv_epilogue* epilogue, void* stream);
 
+/* The fp32 layers of ocnn_octree_conv_general on the tensor cores: every value as three bf16 parts,
+ * six bf16 products accumulated in fp32 (conv_f32.cu).  workspace: 256-byte aligned device memory
+ * of ocnn_octree_conv_f32_workspace_bytes (0: this layer is left to ocnn_octree_conv_general);
+ * status_dev as for ocnn_octree_conv_tc. */
+size_t ocnn_octree_conv_f32_workspace_bytes(const ocnn_conv_geometry* geometry, int cin, int cout,
+                                            const int kernel_size[3]);
+int ocnn_octree_conv_f32(const float* x_dev, const float* weights_dev, float* y_dev,
+                         const ocnn_conv_geometry* geometry, int cin, int cout, const int kernel_size[3],
+                         int layout, const ocnn_conv_epilogue* epilogue, void* workspace,
+                         size_t workspace_bytes, int32_t* status_dev, void* stream);
+
+
 /* Training support.  The gradient with respect to the data of a convolution is the deconvolution
  * with the same weights and vice versa (ocnn_octree_conv_general with `transposed` flipped).  The
  * gradient with respect to the weights, replacing OctreeBaseConv::weight_gpu_gemm
@@ -261,6 +273,17 @@ int ocnn_octree_conv_general(const void* x_dev, const float* weights_dev, void* 
 int ocnn_octree_conv_weight_grad(const float* a_dev, const float* x_dev, float* dw_dev,
                                  const ocnn_conv_geometry* geometry, int m_channels, int x_channels,
                                  const int kernel_size[3], int layout, void* stream);
+
+/* The same on the tensor cores (three bf16 parts per value, fp32 accumulation; conv_f32_wgrad.cu), with a
+ * fixed summation order.  workspace: 256-byte aligned device memory of the first call's size (0: not
+ * served); h_out and h_in must be positive. */
+size_t ocnn_octree_conv_weight_grad_f32_workspace_bytes(const ocnn_conv_geometry* geometry, int m_channels,
+                                                        int x_channels, const int kernel_size[3]);
+int ocnn_octree_conv_weight_grad_f32(const float* a_dev, const float* x_dev, float* dw_dev,
+                                     const ocnn_conv_geometry* geometry, int m_channels, int x_channels,
+                                     const int kernel_size[3], int layout, void* workspace,
+                                     size_t workspace_bytes, int32_t* status_dev, void* stream);
+
 /* The transposes of the max-pool through its argmax mask.  Replace octree_max_unpool_gpu /
  * octree_mask_pool_gpu, octree/octree/octree_nn.cu:293-329 (bindings pytorch/cpp/octree_pool.cpp:
  * 36-95).  top, mask: [C, top_h]; btm: [C, 8*top_h]; fp32.  unpool: btm = 0, btm[., mask] = top;

@@ -16,6 +16,8 @@ namespace ocnn {
 
 int conv_pointwise_bf16(const void* x, const float* w, void* y, int h, int cin, int cout,
                         const ocnn_conv_epilogue* ep, cudaStream_t st, bool f16);   // conv_pw.cu
+int conv_group_f32(const float* x, const float* w, float* y, const ocnn_conv_geometry* g, int cin, int cout,
+                   const TapList& tl, int layout, const ocnn_conv_epilogue* ep, cudaStream_t st);   // conv_group.cu
 int conv_pointwise_pool_bf16(const void* x, const float* w, void* top, const int* child_parent, int h,
                              int top_h, int cin, int cout, const ocnn_conv_epilogue* ep, int* inv,
                              cudaStream_t st, bool f16);                            // conv_pw.cu
@@ -315,6 +317,13 @@ extern "C" int ocnn_octree_conv(const void* x, const float* w, void* y, const in
                                       dtype == OCNN_F16);
     if (s >= 0) return s;
   }
+  if (dtype == OCNN_F32) {
+    ocnn_conv_geometry g = {};
+    g.stride = stride; g.h_in = h_in; g.h_out = h_out; g.neigh_dev = neigh;
+    const int s = conv_group_f32(static_cast<const float*>(x), w, static_cast<float*>(y), &g, cin, cout, tl, layout,
+                                 ep, static_cast<cudaStream_t>(stream));
+    if (s >= 0) return s;
+  }
   return conv_simt_launch(x, w, y, neigh, nullptr, nullptr, h_in, h_out, cin, cout, tl, stride, dtype,
                           layout, ep, stream);
 }
@@ -445,6 +454,11 @@ extern "C" int ocnn_octree_conv_general(const void* x, const float* w, void* y,
   const bool identity = tl.count == 1 && g->stride == 1;
   const int32_t* child = (g->nempty && !identity && !(g->transposed && g->stride == 2)) ? g->child_dev : nullptr;
   const int32_t* ichild = (g->nempty && !identity && !(g->stride == 2 && !g->transposed)) ? g->ichild_dev : nullptr;
+  if (dtype == OCNN_F32) {
+    const int s = conv_group_f32(static_cast<const float*>(x), w, static_cast<float*>(y), g, cin, cout, tl, layout,
+                                 ep, static_cast<cudaStream_t>(stream));
+    if (s >= 0) return s;
+  }
   return conv_simt_launch(x, w, y, identity ? nullptr : g->neigh_dev, child, ichild, g->h_in, g->h_out,
                           cin, cout, tl, g->stride, dtype, layout, ep, stream, g->transposed != 0);
 }

@@ -80,6 +80,31 @@ class FcBnRelu(_nn.Module):
     return self.relu(self.bn(self.fc(self.flatten(data_in))))
 
 
+class _Conv1x1Function(torch.autograd.Function):
+  """torch's own 1x1 convolution with this library's kernel for the weight gradient."""
+
+  @staticmethod
+  def forward(ctx, data, weight, bias):
+    ctx.save_for_backward(data, weight)
+    ctx.bias = None if bias is None else list(bias.shape)
+    return torch.conv1d(data.squeeze(-1), weight, bias).unsqueeze(-1)
+
+  @staticmethod
+  def backward(ctx, grad):
+    data, weight = ctx.saved_tensors
+    need_x, need_w, need_b = ctx.needs_input_grad
+    grad = grad.contiguous()
+    gx = gw = gb = None
+    if need_x or need_b:
+      gx, _, gb = torch.ops.aten.convolution_backward(
+          grad.squeeze(-1), data.squeeze(-1), weight, ctx.bias, [1], [0], [1], False, [0], 1,
+          [need_x, False, need_b])
+      gx = gx if gx is None else gx.unsqueeze(-1)
+    if need_w:
+      gw = nn.pointwise_conv_weight_grad(data, grad).view_as(weight)
+    return gx, gw, gb
+
+
 class OctreeConv1x1(_nn.Module):
   """A per-node linear map.  The parameters live in a torch Conv1d (as in the reference, so the
   state_dict keys match); the product runs on this library's pointwise kernels."""
@@ -94,8 +119,14 @@ class OctreeConv1x1(_nn.Module):
     conv = self.conv1x1
     if torch.is_grad_enabled() and (data_in.requires_grad or
                                     (self.training and conv.weight.requires_grad)):
-      # training: torch's own 1x1 convolution (as the reference), which autograd differentiates
-      out = conv(data_in.squeeze(-1)).unsqueeze(-1)
+      # Training: torch's own 1x1 convolution (as the reference), which autograd differentiates. At
+      # 64 to 128 output channels cuDNN forms the weight gradient with a direct fp32 kernel (16 -> 64
+      # at 107 k nodes: 395 us); ours is used there. Elsewhere cuDNN takes a GEMM (about 55 us).
+      if (64 <= conv.weight.shape[0] <= 128 and data_in.dtype == conv.weight.dtype == torch.float32 and
+          data_in.is_cuda and data_in.is_contiguous() and not torch.is_autocast_enabled()):
+        out = _Conv1x1Function.apply(data_in, conv.weight, conv.bias)
+      else:
+        out = conv(data_in.squeeze(-1)).unsqueeze(-1)
       if bn is not None:
         scale, bias = _folded(bn)
         out = out * scale.view(1, -1, 1, 1) + bias.view(1, -1, 1, 1)

@@ -26,7 +26,7 @@ def tc_status(device):
   device; 0 = no kernel ever gave up)."""
   key = torch.device(device)
   if key not in _STATUS:
-    _STATUS[key] = torch.zeros(1, dtype=torch.int32, device=key)
+    _STATUS[key] = nn.tc_status(key)
   return _STATUS[key]
 
 
@@ -55,13 +55,14 @@ class _ConvFunctionBase(torch.autograd.Function):
     ctx.save_for_backward(data_in, weights, octree)     # (either memory layout is taken as it is)
     ctx.args = (depth, channel_out, resize_with_last_val(list(kernel_size)), stride, nempty)
     op = nn.octree_deconv if cls.deconv else nn.octree_conv
-    return op(data_in, weights, octree, *ctx.args)
+    return op(data_in, weights, octree, *ctx.args, fma_chain=True)
 
   @classmethod
   def _backward(cls, ctx, grad_in):
     data_in, weights, octree = ctx.saved_tensors
     op = nn.octree_deconv_grad if cls.deconv else nn.octree_conv_grad
-    grad_out, grad_w = op(data_in, weights, octree, grad_in.contiguous(), *ctx.args)
+    grad_out, grad_w = op(data_in, weights, octree, grad_in.contiguous(), *ctx.args,
+                          *ctx.needs_input_grad[:2])
     return (grad_out, grad_w) + (None,) * 6
 
 

@@ -517,9 +517,71 @@ ocnn_conv_epilogue make_epilogue(const c10::optional<Tensor>& scale, const c10::
   return ep;
 }
 
+// The int32 status word the tensor-core kernels write when a bounded wait runs out: one per device.
+Tensor tc_status(c10::Device device) {
+  static std::mutex mutex;
+  static auto& words = *new std::map<int, Tensor>();   // (never destroyed: outlives the CUDA context)
+  TORCH_CHECK(device.is_cuda(), "tc_status: a CUDA device");
+  const int index = device.has_index() ? device.index() : c10::cuda::current_device();
+  std::lock_guard<std::mutex> lock(mutex);
+  auto it = words.find(index);
+  if (it == words.end())
+    it = words.emplace(index, torch::zeros({1}, torch::dtype(torch::kInt32)
+                                                    .device(torch::kCUDA, (c10::DeviceIndex)index))).first;
+  return it->second;
+}
+
+bool use_conv_f32() {
+  static const bool use = [] {
+    const char* e = getenv("OCNN_CONV_F32");
+    return e == nullptr || atoi(e) != 0;
+  }();
+  return use;
+}
+
+// A layer through the kernels that take the caller's own weights and layout: fp32 data on the
+// tensor cores (three bf16 parts per value) where that kernel serves the layer, everything else on
+// the CUDA cores.  OCNN_CONV_F32=0 keeps fp32 on the CUDA cores.
+//
+// fma_chain: every output as one chain of rounded multiply-adds in the weights' order.  Training asks
+// for it, in both directions: its networks take maxima and ReLUs of these values and feed them to TF32
+// products, so a sum that differs in its last bit sends single nodes' gradients elsewhere (1e-7 in a
+// forward pass is 1e-2 in a weight gradient), and a run should not depend on the kernel.  It is kept
+// up to 4 GFLOP a layer, where it costs a tenth of a millisecond at most; beyond that the tensor
+// cores are four times faster (24 GFLOP, 32 -> 64 at 217 k nodes: 598 us against 176).
+// Few channels stay on the CUDA cores in any case: the tensor-core kernel's gather moves 16-byte
+// pieces whatever the channel count (3 -> 32 at 222 k nodes: 40 us against 77; 16 -> 16 at 217 k, where
+// the two meet: 88 against 91); for every kind of layer, so that few channels give the same bits in and
+// outside of training, on all nodes and on the non-empty ones.
+void run_conv(const DataRef& x, const Tensor& w, Tensor& y, const ocnn_conv_geometry& g, int cin, int cout,
+              const vector<int>& ks, const ocnn_conv_epilogue* ep, bool fma_chain = false) {
+  const int taps = ks[0] * ks[1] * ks[2];
+  const bool few = cin * cout <= 256;
+  const bool chain = fma_chain && 2.0 * taps * cin * cout * g.h_out < 4e9;
+  if (x.dtype == OCNN_F32 && use_conv_f32() && !chain && !few) {
+    const size_t bytes = ocnn_octree_conv_f32_workspace_bytes(&g, cin, cout, ks.data());
+    if (bytes > 0) {
+      Tensor ws = torch::empty({(int64_t)bytes}, torch::dtype(torch::kUInt8).device(x.t.device()));
+      OCNN_CALL(ocnn_octree_conv_f32(x.t.data_ptr<float>(), w.data_ptr<float>(), y.data_ptr<float>(), &g, cin,
+                                     cout, ks.data(), x.layout, ep, ws.data_ptr(), bytes,
+                                     tc_status(x.t.device()).data_ptr<int32_t>(), current_stream()));
+      return;
+    }
+  }
+  const bool point = ks[0] * ks[1] * ks[2] == 1 && g.stride == 1 && !g.transposed;
+  if (point) {      // (16-bit node-major data: its own streaming kernels)
+    OCNN_CALL(ocnn_octree_conv(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), nullptr, x.H, x.H, cin, cout,
+                               ks.data(), 1, x.dtype, x.layout, ep, current_stream()));
+  } else {
+    OCNN_CALL(ocnn_octree_conv_general(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), &g, cin, cout,
+                                       ks.data(), x.dtype, x.layout, ep, current_stream()));
+  }
+}
+
 Tensor octree_conv_fused(Tensor data_in, Tensor weights, Tensor octree, int depth, int num_output,
                          vector<int> kernel_size, int stride, c10::optional<Tensor> scale,
-                         c10::optional<Tensor> bias, c10::optional<Tensor> residual, bool relu) {
+                         c10::optional<Tensor> bias, c10::optional<Tensor> residual, bool relu,
+                         bool fma_chain = false) {
   vector<int> ks = kernel3(kernel_size);
   TORCH_CHECK(num_output > 0, "The num_output should be larger than 0");
   OctreeRef o = get_octree(octree);
@@ -535,16 +597,17 @@ Tensor octree_conv_fused(Tensor data_in, Tensor weights, Tensor octree, int dept
   Tensor w = weights.contiguous();
   Tensor y = new_data(num_output, s.h_out, x);
   ocnn_conv_epilogue ep = make_epilogue(scale, bias, residual, relu, num_output, y);
-  OCNN_CALL(ocnn_octree_conv(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), s.neigh, s.h_in,
-                             s.h_out, x.C, num_output, ks.data(), stride, x.dtype, x.layout, &ep,
-                             current_stream()));
+  ocnn_conv_geometry g;
+  memset(&g, 0, sizeof(g));
+  g.stride = stride; g.h_in = s.h_in; g.h_out = s.h_out; g.neigh_dev = s.neigh;
+  run_conv(x, w, y, g, x.C, num_output, ks, &ep, fma_chain);
   return y;
 }
 
 // OctreeConv(nempty=True), stride 1: data and result live on the non-empty nodes of `depth` only
 // (pytorch/cpp/octree_conv.cpp:61-120 with non_empty_).
 Tensor octree_conv_nempty(Tensor data_in, Tensor weights, Tensor octree, int depth, int num_output,
-                          vector<int> kernel_size) {
+                          vector<int> kernel_size, bool fma_chain) {
   vector<int> ks = kernel3(kernel_size);
   TORCH_CHECK(num_output > 0, "The num_output should be larger than 0");
   OctreeRef o = get_octree(octree);
@@ -561,29 +624,34 @@ Tensor octree_conv_nempty(Tensor data_in, Tensor weights, Tensor octree, int dep
               "weights must be a float32 CUDA tensor of shape [Cout, Cin*K]");
   Tensor w = weights.contiguous();
   Tensor y = new_data(num_output, nne, x);
-  const int32_t* child = level_ptr(o, OCNN_PROP_CHILD, depth, "octree_conv");
-  Tensor ichild = make_ichild(o, depth, x.t.options(), "octree_conv");
-  const int32_t* neigh = kdim > 1 ? level_ptr(o, OCNN_PROP_NEIGH, depth, "octree_conv") : nullptr;
-  OCNN_CALL(ocnn_octree_conv_nempty(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), neigh, child,
-                                    ichild.data_ptr<int32_t>(), nne, x.C, num_output, ks.data(),
-                                    x.dtype, x.layout, nullptr, current_stream()));
+  ocnn_conv_geometry g;
+  memset(&g, 0, sizeof(g));
+  g.stride = 1; g.nempty = 1; g.h_in = nne; g.h_out = nne;
+  Tensor ichild;
+  if (kdim > 1) {
+    ichild = make_ichild(o, depth, x.t.options(), "octree_conv");
+    g.child_dev = level_ptr(o, OCNN_PROP_CHILD, depth, "octree_conv");
+    g.ichild_dev = ichild.data_ptr<int32_t>();
+    g.neigh_dev = level_ptr(o, OCNN_PROP_NEIGH, depth, "octree_conv");
+  }
+  run_conv(x, w, y, g, x.C, num_output, ks, nullptr, fma_chain);
   return y;
 }
 
 Tensor octree_conv_general(Tensor data_in, Tensor weights, Tensor octree, int depth, int num_output,
                            vector<int> kernel_size, int stride, bool nempty, bool transposed,
                            c10::optional<Tensor> scale, c10::optional<Tensor> bias,
-                           c10::optional<Tensor> residual, bool relu);
+                           c10::optional<Tensor> residual, bool relu, bool fma_chain = false);
 
 Tensor octree_conv(Tensor data_in, Tensor weights, Tensor octree, int depth, int num_output,
-                   vector<int> kernel_size, int stride, bool nempty) {
+                   vector<int> kernel_size, int stride, bool nempty, bool fma_chain) {
   if (nempty && stride == 1)
-    return octree_conv_nempty(data_in, weights, octree, depth, num_output, kernel_size);
+    return octree_conv_nempty(data_in, weights, octree, depth, num_output, kernel_size, fma_chain);
   if (nempty)
     return octree_conv_general(data_in, weights, octree, depth, num_output, kernel_size, stride, true,
-                               false, c10::nullopt, c10::nullopt, c10::nullopt, false);
+                               false, c10::nullopt, c10::nullopt, c10::nullopt, false, fma_chain);
   return octree_conv_fused(data_in, weights, octree, depth, num_output, kernel_size, stride,
-                           c10::nullopt, c10::nullopt, c10::nullopt, false);
+                           c10::nullopt, c10::nullopt, c10::nullopt, false, fma_chain);
 }
 
 Tensor conv_pack_weights(Tensor weights, int cin, int cout, vector<int> kernel_size, int stride) {
@@ -744,7 +812,7 @@ void check_weights(const Tensor& weights, int cin, int cout, int kdim) {
 Tensor octree_conv_general(Tensor data_in, Tensor weights, Tensor octree, int depth, int num_output,
                            vector<int> kernel_size, int stride, bool nempty, bool transposed,
                            c10::optional<Tensor> scale, c10::optional<Tensor> bias,
-                           c10::optional<Tensor> residual, bool relu) {
+                           c10::optional<Tensor> residual, bool relu, bool fma_chain) {
   const char* what = transposed ? "octree_deconv" : "octree_conv";
   vector<int> ks = kernel3(kernel_size);
   TORCH_CHECK(num_output > 0, "The num_output should be larger than 0");
@@ -758,15 +826,14 @@ Tensor octree_conv_general(Tensor data_in, Tensor weights, Tensor octree, int de
   Tensor w = weights.contiguous();
   Tensor y = new_data(num_output, geo.g.h_out, x);
   ocnn_conv_epilogue ep = make_epilogue(scale, bias, residual, relu, num_output, y);
-  OCNN_CALL(ocnn_octree_conv_general(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), &geo.g, x.C,
-                                     num_output, ks.data(), x.dtype, x.layout, &ep, current_stream()));
+  run_conv(x, w, y, geo.g, x.C, num_output, ks, &ep, fma_chain);
   return y;
 }
 
 Tensor octree_deconv(Tensor data_in, Tensor weights, Tensor octree, int depth, int num_output,
-                     vector<int> kernel_size, int stride, bool nempty) {
+                     vector<int> kernel_size, int stride, bool nempty, bool fma_chain) {
   return octree_conv_general(data_in, weights, octree, depth, num_output, kernel_size, stride, nempty,
-                             true, c10::nullopt, c10::nullopt, c10::nullopt, false);
+                             true, c10::nullopt, c10::nullopt, c10::nullopt, false, fma_chain);
 }
 
 Tensor conv_pack_weights_general(Tensor weights, int cin, int cout, vector<int> kernel_size,
@@ -815,12 +882,27 @@ Tensor octree_conv_tc_general(Tensor data_in, Tensor packed, Tensor octree, int 
   return y;
 }
 
+// dW of a layer from the rows of `a` and the gathered rows of `src` (ocnn_octree_conv_weight_grad).
+void run_weight_grad(const DataRef& a, const DataRef& src, Tensor& gw, const ocnn_conv_geometry& g,
+                     const vector<int>& ks) {
+  const size_t bytes = use_conv_f32() ? ocnn_octree_conv_weight_grad_f32_workspace_bytes(&g, a.C, src.C, ks.data()) : 0;
+  if (bytes > 0) {
+    Tensor ws = torch::empty({(int64_t)bytes}, torch::dtype(torch::kUInt8).device(a.t.device()));
+    OCNN_CALL(ocnn_octree_conv_weight_grad_f32(a.t.data_ptr<float>(), src.t.data_ptr<float>(), gw.data_ptr<float>(),
+                                               &g, a.C, src.C, ks.data(), a.layout, ws.data_ptr(), bytes,
+                                               tc_status(a.t.device()).data_ptr<int32_t>(), current_stream()));
+  } else {
+    OCNN_CALL(ocnn_octree_conv_weight_grad(a.t.data_ptr<float>(), src.t.data_ptr<float>(), gw.data_ptr<float>(), &g,
+                                           a.C, src.C, ks.data(), a.layout, current_stream()));
+  }
+}
+
 // ---- gradients (pytorch/cpp/octree_conv.cpp:159-189, 219-253, 262-298; octree_pool.cpp:36-95) ---------
 // Returns {gradient of the data, gradient of the weights} of OctreeConv (deconv = false) or
 // OctreeDeconv (deconv = true) given the gradient of its output.  fp32.
 vector<Tensor> conv_grad_impl(Tensor data_in, Tensor weights, Tensor octree, Tensor grad_in, int depth,
                               int num_output, vector<int> kernel_size, int stride, bool nempty,
-                              bool deconv) {
+                              bool deconv, bool need_data, bool need_weights) {
   const char* what = deconv ? "octree_deconv_grad" : "octree_conv_grad";
   vector<int> ks = kernel3(kernel_size);
   OctreeRef o = get_octree(octree);
@@ -844,31 +926,33 @@ vector<Tensor> conv_grad_impl(Tensor data_in, Tensor weights, Tensor octree, Ten
   const int back_depth = stride == 1 ? depth : (deconv ? depth + 1 : depth - 1);
   Geometry back = make_geometry(o, gy, back_depth, ks, stride, nempty, !deconv, what);
   TORCH_CHECK(back.g.h_out == x.H, what, ": inconsistent octree");
-  Tensor gx = new_data(x.C, x.H, x);
-  OCNN_CALL(ocnn_octree_conv_general(gy.t.data_ptr(), w.data_ptr<float>(), gx.data_ptr(), &back.g, gy.C,
-                                     x.C, ks.data(), OCNN_F32, x.layout, nullptr, current_stream()));
+  Tensor gx, gw;
+  if (need_data) {
+    gx = new_data(x.C, x.H, x);
+    run_conv(gy, w, gx, back.g, gy.C, x.C, ks, nullptr, true);
+  }
+  if (!need_weights) return {gx, gw};
   // weight gradient: reduction over the rows of the convolution-type column matrix
-  Tensor gw = torch::empty_like(w);
+  gw = torch::empty_like(w);
   const Geometry& conv_geo = deconv ? back : fwd;
   const DataRef& a = deconv ? x : gy;      // the operand with one row per column-matrix row
   const DataRef& src = deconv ? gy : x;    // the operand that is gathered
-  OCNN_CALL(ocnn_octree_conv_weight_grad(a.t.data_ptr<float>(), src.t.data_ptr<float>(),
-                                         gw.data_ptr<float>(), &conv_geo.g, a.C, src.C, ks.data(),
-                                         x.layout, current_stream()));
+  run_weight_grad(a, src, gw, conv_geo.g, ks);
   return {gx, gw};
 }
 
 vector<Tensor> octree_conv_grad(Tensor data_in, Tensor weights, Tensor octree, Tensor grad_in, int depth,
-                                int num_output, vector<int> kernel_size, int stride, bool nempty) {
+                                int num_output, vector<int> kernel_size, int stride, bool nempty,
+                                bool need_data, bool need_weights) {
   return conv_grad_impl(data_in, weights, octree, grad_in, depth, num_output, kernel_size, stride,
-                        nempty, false);
+                        nempty, false, need_data, need_weights);
 }
 
 vector<Tensor> octree_deconv_grad(Tensor data_in, Tensor weights, Tensor octree, Tensor grad_in,
                                   int depth, int num_output, vector<int> kernel_size, int stride,
-                                  bool nempty) {
+                                  bool nempty, bool need_data, bool need_weights) {
   return conv_grad_impl(data_in, weights, octree, grad_in, depth, num_output, kernel_size, stride,
-                        nempty, true);
+                        nempty, true, need_data, need_weights);
 }
 
 Tensor octree_max_unpool(Tensor top_data, Tensor mask, Tensor octree, int depth) {
@@ -923,10 +1007,31 @@ Tensor pointwise_conv(Tensor data_in, Tensor weights, c10::optional<Tensor> scal
   Tensor w = weights.contiguous();
   Tensor y = new_data(cout, x.H, x);
   ocnn_conv_epilogue ep = make_epilogue(scale, bias, residual, relu, cout, y);
-  const int ks[3] = {1, 1, 1};
-  OCNN_CALL(ocnn_octree_conv(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), nullptr, x.H, x.H, x.C,
-                             cout, ks, 1, x.dtype, x.layout, &ep, current_stream()));
+  ocnn_conv_geometry g;
+  memset(&g, 0, sizeof(g));
+  g.stride = 1; g.h_in = x.H; g.h_out = x.H;
+  run_conv(x, w, y, g, x.C, cout, {1, 1, 1}, &ep);
   return y;
+}
+
+// Gradient of a 1x1x1 layer's weights [Cout, Cin] from its input and its output's gradient, fp32.
+Tensor pointwise_conv_weight_grad(Tensor data_in, Tensor grad) {
+  const char* what = "pointwise_conv_weight_grad";
+  need_cuda(data_in, what);
+  need_cuda(grad, what);
+  c10::cuda::CUDAGuard guard(data_in.device());
+  TORCH_CHECK(data_in.scalar_type() == torch::kFloat32 && grad.scalar_type() == torch::kFloat32, what,
+              ": float32 data only");
+  DataRef x = get_data(data_in, what);
+  DataRef gy = get_data(x.layout == OCNN_NODE_MAJOR ? grad.contiguous(at::MemoryFormat::ChannelsLast)
+                                                    : grad.contiguous(), what);
+  TORCH_CHECK(x.H == gy.H, what, ": the gradient has ", gy.H, " rows, the data ", x.H);
+  Tensor gw = torch::empty({gy.C, x.C}, torch::dtype(torch::kFloat32).device(data_in.device()));
+  ocnn_conv_geometry g;
+  memset(&g, 0, sizeof(g));
+  g.stride = 1; g.h_in = x.H; g.h_out = x.H;
+  run_weight_grad(gy, x, gw, g, {1, 1, 1});
+  return gw;
 }
 
 Tensor pointwise_conv_tc(Tensor data_in, Tensor packed, int num_output, c10::optional<Tensor> scale,
@@ -1026,14 +1131,7 @@ class ConvLayer {
         return y;
       }
     }
-    w = w.contiguous();
-    if (point_) {
-      OCNN_CALL(ocnn_octree_conv(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), nullptr, x.H, x.H, cin_,
-                                 cout_, ks_.data(), 1, x.dtype, x.layout, &ep, current_stream()));
-    } else {
-      OCNN_CALL(ocnn_octree_conv_general(x.t.data_ptr(), w.data_ptr<float>(), y.data_ptr(), &geo.g, cin_,
-                                         cout_, ks_.data(), x.dtype, x.layout, &ep, current_stream()));
-    }
+    run_conv(x, w.contiguous(), y, geo.g, cin_, cout_, ks_, &ep);
     return y;
   }
 
@@ -2243,10 +2341,19 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("points2octree", &points2octree, "convert points to octree");
   m.def("octree2col", &octree2col, "octree2col");
   m.def("col2octree", &col2octree, "col2octree");
-  m.def("octree_conv", &octree_conv, "octree based convolution");
-  m.def("octree_deconv", &octree_deconv, "octree based deconvolution");
-  m.def("octree_conv_grad", &octree_conv_grad, "octree based convolution");
-  m.def("octree_deconv_grad", &octree_deconv_grad, "octree based deconvolution");
+  m.def("octree_conv", &octree_conv, "octree based convolution", py::arg("data_in"), py::arg("weights"),
+        py::arg("octree"), py::arg("depth"), py::arg("num_output"), py::arg("kernel_size"), py::arg("stride"),
+        py::arg("nempty"), py::arg("fma_chain") = false);
+  m.def("octree_deconv", &octree_deconv, "octree based deconvolution", py::arg("data_in"), py::arg("weights"),
+        py::arg("octree"), py::arg("depth"), py::arg("num_output"), py::arg("kernel_size"), py::arg("stride"),
+        py::arg("nempty"), py::arg("fma_chain") = false);
+  m.def("octree_conv_grad", &octree_conv_grad, "octree based convolution", py::arg("data_in"), py::arg("weights"),
+        py::arg("octree"), py::arg("grad_in"), py::arg("depth"), py::arg("num_output"), py::arg("kernel_size"),
+        py::arg("stride"), py::arg("nempty"), py::arg("need_data") = true, py::arg("need_weights") = true);
+  m.def("octree_deconv_grad", &octree_deconv_grad, "octree based deconvolution", py::arg("data_in"),
+        py::arg("weights"), py::arg("octree"), py::arg("grad_in"), py::arg("depth"), py::arg("num_output"),
+        py::arg("kernel_size"), py::arg("stride"), py::arg("nempty"), py::arg("need_data") = true,
+        py::arg("need_weights") = true);
   m.def("octree_max_unpool", &octree_max_unpool, "octree max unpooling");
   m.def("octree_mask_pool", &octree_mask_pool, "octree mask pooling");
   m.def("octree_pad", &octree_pad, "octree pad", py::arg("data_in"), py::arg("octree"),
@@ -2273,7 +2380,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("octree_conv_fused", &octree_conv_fused, py::arg("data_in"), py::arg("weights"),
         py::arg("octree"), py::arg("depth"), py::arg("num_output"), py::arg("kernel_size"),
         py::arg("stride"), py::arg("scale") = py::none(), py::arg("bias") = py::none(),
-        py::arg("residual") = py::none(), py::arg("relu") = false);
+        py::arg("residual") = py::none(), py::arg("relu") = false, py::arg("fma_chain") = false);
   m.def("conv_pack_weights", &conv_pack_weights, py::arg("weights"), py::arg("cin"), py::arg("cout"),
         py::arg("kernel_size"), py::arg("stride") = 1);
   m.def("conv_tc_wait_selftest", &conv_tc_wait_selftest);
@@ -2291,7 +2398,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("octree"), py::arg("depth"), py::arg("num_output"), py::arg("kernel_size"),
         py::arg("stride") = 1, py::arg("nempty") = false, py::arg("transposed") = false,
         py::arg("scale") = py::none(), py::arg("bias") = py::none(),
-        py::arg("residual") = py::none(), py::arg("relu") = false);
+        py::arg("residual") = py::none(), py::arg("relu") = false, py::arg("fma_chain") = false);
   m.def("conv_pack_weights_general", &conv_pack_weights_general, py::arg("weights"), py::arg("cin"),
         py::arg("cout"), py::arg("kernel_size"), py::arg("stride") = 1,
         py::arg("transposed") = false, py::arg("nempty") = false, py::arg("half") = false);
@@ -2303,6 +2410,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("pointwise_conv", &pointwise_conv, py::arg("data_in"), py::arg("weights"),
         py::arg("scale") = py::none(), py::arg("bias") = py::none(),
         py::arg("residual") = py::none(), py::arg("relu") = false);
+  m.def("pointwise_conv_weight_grad", &pointwise_conv_weight_grad);
   m.def("pointwise_conv_tc", &pointwise_conv_tc, py::arg("data_in"), py::arg("packed"),
         py::arg("num_output"), py::arg("scale") = py::none(), py::arg("bias") = py::none(),
         py::arg("residual") = py::none(), py::arg("relu") = false, py::arg("status"));
@@ -2330,6 +2438,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("octree_align", &octree_align, "align octree data", py::arg("src_data"),
         py::arg("src_octree"), py::arg("des_octree"), py::arg("depth"));
   m.def("octree_align_grad", &octree_align_grad, "backward of align-octree-data");
+  m.def("tc_status", [](py::object device) {
+    return tc_status(torch::python::detail::py_object_to_device(device));
+  });
   m.def("octree_info", &octree_info);
   // (pytorch/cpp/pybind.cpp:35-41)
   m.def("octree_grow", &octree_grow, "octree growing", py::arg("octree"), py::arg("target_depth"),

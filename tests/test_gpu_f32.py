@@ -1,0 +1,122 @@
+"""fp32 layers on the tensor cores (three bf16 parts per value) and on whole sibling groups: every width of
+the accumulator tile, more than one slice of output channels, K splits, chunk remainders, node counts
+that do not fill a tile, against the column formulation in float64."""
+import numpy as np
+import pytest
+import torch
+
+import gpu_util as gu
+from oracle import oracle as oc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope='module')
+def ocnn():
+  import ocnn as mod
+  mod.set_key_bits(64)
+  return mod
+
+
+@pytest.fixture(scope='module')
+def octree(ocnn):
+  _, merged, _ = gu.oracle_batch(gu.small_clouds(3, 3000, 500), 5, 2, 64)
+  return gu.to_cuda_u8(merged), oc.OctreeView(merged)
+
+
+@pytest.fixture(scope='module')
+def big_octree(ocnn):
+  """A level large enough for two groups per warp and several tiles per CTA."""
+  _, merged, _ = gu.oracle_batch(gu.small_clouds(12, 6000, 500), 6, 2, 64)
+  return gu.to_cuda_u8(merged), oc.OctreeView(merged)
+
+
+def columns(ocnn, x, octree, d, nempty):
+  return ocnn.nn.octree2col(x, octree, d, [3, 3, 3], 1, nempty).flatten(0, 1).double()
+
+
+def off(got, want):
+  return float((got.double() - want).norm() / want.norm())
+
+
+# (cin, cout): each NG = cout / 16 of conv_f32_kernel, a slice boundary, channel counts that leave a
+# K-block or an 8-channel chunk unfilled; few channels stay on the group kernel
+CHANNELS = [(3, 5), (3, 64), (16, 16), (33, 16), (40, 32), (24, 48), (64, 64), (72, 80), (9, 96), (32, 112),
+            (64, 128), (40, 130), (17, 257)]
+
+
+@pytest.mark.parametrize('cin,cout', CHANNELS)
+@pytest.mark.parametrize('depth,nempty,node_major', [(5, False, False), (5, True, False), (5, True, True), (2, False, True)])
+def test_forward(ocnn, octree, cin, cout, depth, nempty, node_major):
+  tree, v = octree
+  h = int(v.nnum_nempty[depth] if nempty else v.nnum[depth])
+  torch.manual_seed(cin * cout)
+  x, w = torch.randn(1, cin, h, 1, device='cuda'), torch.randn(cout, cin * 27, device='cuda') * 0.1
+  want = (w.double() @ columns(ocnn, x, tree, depth, nempty)).view(1, cout, h, 1)
+  xin = x.contiguous(memory_format=torch.channels_last) if node_major else x
+  got = ocnn.octree_conv(xin, w, tree, depth, cout, [3, 3, 3], 1, nempty)
+  assert off(got, want) < 6e-7 and gu.rel_err(gu.to_np(got), want.view(cout, h).cpu().numpy()) < 1e-5
+  chain = ocnn.nn.octree_conv(xin, w, tree, depth, cout, [3, 3, 3], 1, nempty, True)
+  assert off(chain, want) < 2e-6
+
+
+@pytest.mark.parametrize('cin,cout', [(3, 16), (4, 64), (20, 12), (32, 40), (64, 96)])
+def test_forward_and_gradients_of_a_big_level(ocnn, big_octree, cin, cout):
+  tree, v = big_octree
+  d, h = 6, int(v.nnum[6])
+  assert h > 2 * 148 * 16 * 8
+  torch.manual_seed(cin)
+  x, w = torch.randn(1, cin, h, 1, device='cuda'), torch.randn(cout, cin * 27, device='cuda') * 0.1
+  g = torch.randn(1, cout, h, 1, device='cuda')
+  col = columns(ocnn, x, tree, d, False)
+  want = (w.double() @ col).view(1, cout, h, 1)
+  for chain in (False, True):
+    assert off(ocnn.nn.octree_conv(x, w, tree, d, cout, [3, 3, 3], 1, False, chain), want) < 2e-6
+  gx, gw = ocnn.nn.octree_conv_grad(x, w, tree, g, d, cout, [3, 3, 3], 1, False)
+  assert off(gw, g.view(cout, h).double() @ col.t()) < 2e-6
+  gcol = (w.double().t() @ g.view(cout, h).double()).view(cin, 27, h).float()
+  want = ocnn.nn.col2octree(gcol, tree, d, [3, 3, 3], 1, False).double()
+  assert off(gx, want) < 2e-6
+  only = ocnn.nn.octree_conv_grad(x, w, tree, g, d, cout, [3, 3, 3], 1, False, False, True)
+  assert only[0] is None and torch.equal(only[1], gw)
+
+
+@pytest.mark.parametrize('cin,cout', [(3, 5), (8, 32), (40, 33), (16, 64), (64, 96), (24, 128), (130, 257)])
+@pytest.mark.parametrize('rows', [1, 31, 33, 250, 4111])
+def test_pointwise_weight_gradient(ocnn, cin, cout, rows):
+  torch.manual_seed(rows)
+  x, g = torch.randn(1, cin, rows, 1, device='cuda'), torch.randn(1, cout, rows, 1, device='cuda')
+  want = g.view(cout, rows).double() @ x.view(cin, rows).double().t()
+  for nm in (False, True):
+    xin = x.contiguous(memory_format=torch.channels_last) if nm else x
+    assert off(ocnn.nn.pointwise_conv_weight_grad(xin, g), want) < 1e-6
+
+
+def test_pointwise_training_layer(ocnn):
+  """OctreeConv1x1 in training: every gradient, with and without a bias."""
+  torch.manual_seed(5)
+  for bias in (False, True):
+    layer = ocnn.OctreeConv1x1(24, 64, bias).cuda().train()
+    x = torch.randn(1, 24, 1000, 1, device='cuda', requires_grad=True)
+    g = torch.randn(1, 64, 1000, 1, device='cuda')
+    params = [x] + list(layer.parameters())
+    got = torch.autograd.grad(layer(x), params, g)
+    want = torch.autograd.grad(layer.conv1x1(x.squeeze(-1)).unsqueeze(-1), params, g)
+    for a, b in zip(got, want):
+      assert a.shape == b.shape and off(a, b.double()) < 2e-3     # (torch's own may run in TF32)
+
+
+def test_extreme_values(ocnn, octree):
+  """Values whose high part would round to infinity, and tiny ones, keep their fp32 result."""
+  tree, v = octree
+  h = int(v.nnum[5])
+  rng = np.random.default_rng(3)
+  scale = torch.tensor(10.0 ** rng.uniform(-30, 30, size=h), dtype=torch.float32, device='cuda')
+  x = torch.randn(1, 40, h, 1, device='cuda') * scale.view(1, 1, h, 1)
+  x[0, 0, :4, 0] = torch.tensor([3.4e38, -3.4e38, 1e-40, 0.0], device='cuda')
+  w = torch.zeros(32, 40 * 27, device='cuda')
+  w[:, 13::27] = torch.randn(32, 40, device='cuda') * 1e-4      # the centre tap: a 1x1 layer
+  got = ocnn.octree_conv(x, w, tree, 5, 32, [3, 3, 3], 1)
+  want = (w[:, 13::27].double() @ x.view(40, h).double()).view(1, 32, h, 1)
+  mag = (w[:, 13::27].double().abs() @ x.view(40, h).double().abs()).view(1, 32, h, 1)
+  assert float(((got.double() - want).abs() / (mag + 1e-36)).max()) < 1e-6
