@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
       if (a.rowsplit == 3) {
         const int slot = (tid & ~31) + ((tid & 3) << 3) + ((tid >> 2) & 7);
         const int* blk = a.neigh + ((long long)(live ? h : 0) << 6);
-#pragma unroll
+#pragma unroll 1
         for (int t0 = 0; t0 < 64; t0 += 16) {
           int pv[16];
 #pragma unroll
@@ -254,38 +254,44 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
       if (a.identity) {
         nbr[a.rowsplit >= 2 ? (tid & ~31) + ((tid & 3) << 3) + ((tid >> 2) & 7) : tid] = live ? h : -1;
       } else {
-      // all (up to 27) table reads are issued before the first result is used: a load-then-store
-      // loop would expose the L2 latency once per tap
       // with the four-rows-per-instruction mapping a thread serves rows sub + 4*i of its warp: their
       // entries are stored next to each other so that it reads them as two 16-byte words
       const int slot = a.rowsplit >= 2 ? (tid & ~31) + ((tid & 3) << 3) + ((tid >> 2) & 7) : tid;
       const int tstride = a.rowsplit == 4 ? kGroupTableStride : kTileM;
-      int pv[27];
-#pragma unroll
-      for (int t = 0; t < 27; ++t) {
-        int p = -1;
-        if (t < a.T && live) {
-          // a.tap[t] holds (tx<<4)|(ty<<2)|tz; adding the octant's (ox<<4)|(oy<<2)|oz gives the
-          // position in the sibling group's 4x4x4 block (no field can carry: each sum is <= 3)
-          if (GENERAL && a.up) {
-            const int code = a.tap[t];
-            p = up_source_group(a.neigh, hn, (code >> 4) * 9 + ((code >> 2) & 3) * 3 + (code & 3));
-          } else {
-            const long long at = a.stride == 2 ? ((long long)hn << 6) + a.tap[t]
-                                               : ((long long)(hn >> 3) << 6) + a.tap[t] + oct_code;
-            p = a.neigh[at];
-          }
+      // a.tap[t] holds (tx<<4)|(ty<<2)|tz; adding the octant's (ox<<4)|(oy<<2)|oz gives the position in
+      // the sibling group's 4x4x4 block (no field can carry: each sum is <= 3)
+      if (GENERAL && a.up) {
+#pragma unroll 1
+        for (int t = 0; t < a.T; ++t) {
+          const int code = a.tap[t];
+          nbr[t * tstride + slot] =
+              live ? up_source_group(a.neigh, hn, (code >> 4) * 9 + ((code >> 2) & 3) * 3 + (code & 3)) : -1;
         }
-        pv[t] = p;
-      }
-      if (a.child != nullptr) {
+      } else {
+        // Nine table reads are in flight before the first result is used. (All 27 unrolled are several
+        // KB of code that a CTA runs once: fetching it took longer than the reads.)
+#pragma unroll 1
+        for (int t0 = 0; t0 < a.T; t0 += 9) {
+          int pv[9];
 #pragma unroll
-        for (int t = 0; t < 27; ++t)
-          if (t < a.T && pv[t] >= 0) pv[t] = a.child[pv[t]];
-      }
+          for (int j = 0; j < 9; ++j) {
+            pv[j] = -1;
+            if (t0 + j < a.T && live) {
+              const long long at = a.stride == 2 ? ((long long)hn << 6) + a.tap[t0 + j]
+                                                 : ((long long)(hn >> 3) << 6) + a.tap[t0 + j] + oct_code;
+              pv[j] = a.neigh[at];
+            }
+          }
+          if (a.child != nullptr) {
 #pragma unroll
-      for (int t = 0; t < 27; ++t)
-        if (t < a.T) nbr[t * tstride + slot] = pv[t];
+            for (int j = 0; j < 9; ++j)
+              if (pv[j] >= 0) pv[j] = a.child[pv[j]];
+          }
+#pragma unroll
+          for (int j = 0; j < 9; ++j)
+            if (t0 + j < a.T) nbr[(t0 + j) * tstride + slot] = pv[j];
+        }
+      }
       }
     }
   }
@@ -839,25 +845,27 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
         const int hn = (a.ichild != nullptr && live) ? a.ichild[h] : h;
         const int oct_code = ((hn & 4) << 2) | ((hn & 2) << 1) | (hn & 1);
         {
-          int pv[27];
+#pragma unroll 1
+          for (int t0 = 0; t0 < a.T; t0 += 9) {          // (as in conv_tc_kernel)
+            int pv[9];
 #pragma unroll
-          for (int t = 0; t < 27; ++t) {
-            int p = -1;
-            if (t < a.T && live) {
-              const long long at = a.stride == 2 ? ((long long)hn << 6) + a.tap[t]
-                                                 : ((long long)(hn >> 3) << 6) + a.tap[t] + oct_code;
-              p = a.neigh[at];
+            for (int j = 0; j < 9; ++j) {
+              pv[j] = -1;
+              if (t0 + j < a.T && live) {
+                const long long at = a.stride == 2 ? ((long long)hn << 6) + a.tap[t0 + j]
+                                                   : ((long long)(hn >> 3) << 6) + a.tap[t0 + j] + oct_code;
+                pv[j] = a.neigh[at];
+              }
             }
-            pv[t] = p;
-          }
-          if (a.child != nullptr) {
+            if (a.child != nullptr) {
 #pragma unroll
-            for (int t = 0; t < 27; ++t)
-              if (t < a.T && pv[t] >= 0) pv[t] = a.child[pv[t]];
-          }
+              for (int j = 0; j < 9; ++j)
+                if (pv[j] >= 0) pv[j] = a.child[pv[j]];
+            }
 #pragma unroll
-          for (int t = 0; t < 27; ++t)
-            if (t < a.T) nbr[t * kRows + slot] = pv[t];
+            for (int j = 0; j < 9; ++j)
+              if (t0 + j < a.T) nbr[(t0 + j) * kRows + slot] = pv[j];
+          }
         }
       }
       gather_bar<R>();
