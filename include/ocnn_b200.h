@@ -110,6 +110,11 @@ int ocnn_octree_max_pool(const void* btm_dev, void* top_dev, int32_t* mask_dev, 
 int ocnn_octree_tile(const void* y_dev, void* out_dev, const int32_t* child_dev, int channels,
                      int hy, int hout, int dtype, int layout, void* stream);
 
+/* Rows of two node-major tensors side by side: out[h] = [a[h] | b[h]], row sizes in bytes, multiples of 16. */
+int ocnn_cat_rows(const void* a_dev, const void* b_dev, void* out_dev, int64_t rows, int a_bytes, int b_bytes,
+                  void* stream);
+
+
 /* OctreeMaxPool in one pass: octree_max_pool followed by octree_pad with 0, the pair the
  * reference's module runs (pytorch/ocnn/octree_pool.py, OctreeMaxPool.forward: octree_max_pool
  * then octree_pad at depth - 1).  btm: [btm_h, C] rows of level `depth`; top: [top_h, C] rows of
@@ -352,6 +357,17 @@ int ocnn_octree_conv_tc_general(const void* x_dev, const void* packed_dev, void*
                                 const ocnn_conv_geometry* geometry, int cin, int cout,
                                 const int kernel_size[3], int dtype,
                                 const ocnn_conv_epilogue* epilogue, int32_t* status_dev, void* stream);
+
+/* The same with device memory for layers that gain from splitting K over CTAs (few tiles, a long K):
+ * workspace of ocnn_octree_conv_tc_workspace_bytes (0: none needed; NULL: never split), 32-byte
+ * aligned. */
+size_t ocnn_octree_conv_tc_workspace_bytes(const ocnn_conv_geometry* geometry, int cin, int cout,
+                                           const int kernel_size[3]);
+int ocnn_octree_conv_tc_general_ws(const void* x_dev, const void* packed_dev, void* y_dev,
+                                   const ocnn_conv_geometry* geometry, int cin, int cout,
+                                   const int kernel_size[3], int dtype, const ocnn_conv_epilogue* epilogue,
+                                   int32_t* status_dev, void* workspace, size_t workspace_bytes, void* stream);
+
 
 /* ------------------------------------------------------------------------------------------
  * Octree editing for the generative networks.  Replace octree_new / octree_grow / octree_update

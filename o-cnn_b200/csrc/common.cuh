@@ -196,6 +196,7 @@ __device__ __forceinline__ int up_source_group(const int* __restrict__ neigh, in
     if (bit == 0 ? off[a] != 0 : off[a] == 0) return -1;
     pos = (pos << 2) | ((bit == 1 && off[a] == -1) ? 3 : 1);
   }
+  if (pos == 21) return node >> 3;      // the node's own group (all there is for kernel 2): no look-up
   const int q = neigh[((long long)(node >> 3) << 6) + pos];
   return q >= 0 ? (q >> 3) : -1;
 }

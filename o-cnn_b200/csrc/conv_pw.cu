@@ -774,6 +774,76 @@ int try_pw_mma(const PwArgs& a, int cout, cudaStream_t st) {
   return -1;
 }
 
+// Any even Cout up to 64 (a segmentation head's class count): one node row per thread, COP = Cout
+// rounded up to 8 accumulators, fp32 weights broadcast from shared memory, one chain of
+// multiply-adds per output in channel order. 64 -> 20 at 200 k nodes took 103 us on the general kernel,
+// whose 64-column tiles were two thirds empty.
+template <int COP, bool HALF>
+__global__ void __launch_bounds__(128) conv_pw_any_kernel(const PwArgs a, const int cout) {
+  extern __shared__ __align__(16) float wsm[];       // [cin][COP]
+  __shared__ float2 saff[COP];
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  for (int i = threadIdx.x; i < a.cin * COP; i += blockDim.x) {
+    const int ci = i / COP, co = i - ci * COP;
+    wsm[i] = co < cout ? a.w[co * a.cin + ci] : 0.f;
+  }
+  for (int i = threadIdx.x; i < COP; i += blockDim.x)
+    saff[i] = i < cout ? channel_affine(a.aff, i) : make_float2(1.f, 0.f);
+  __syncthreads();
+  for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < a.h; h += (long long)gridDim.x * blockDim.x) {
+    float acc[COP];
+#pragma unroll
+    for (int j = 0; j < COP; ++j) acc[j] = 0.f;
+    const uint4* row = reinterpret_cast<const uint4*>(a.x + h * a.cin);
+    uint4 nxt = row[0];
+    for (int c8 = 0; c8 < (a.cin >> 3); ++c8) {
+      const uint4 cur = nxt;
+      if (c8 + 1 < (a.cin >> 3)) nxt = row[c8 + 1];
+      const uint32_t p[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float2 f = unpack2(p[k >> 1], HALF);
+        const float xv = k & 1 ? f.y : f.x;
+        const float4* wr = reinterpret_cast<const float4*>(wsm + (c8 * 8 + k) * COP);
+#pragma unroll
+        for (int q = 0; q < COP / 4; ++q) {
+          const float4 wv = wr[q];
+          acc[4 * q] = fmaf(xv, wv.x, acc[4 * q]);
+          acc[4 * q + 1] = fmaf(xv, wv.y, acc[4 * q + 1]);
+          acc[4 * q + 2] = fmaf(xv, wv.z, acc[4 * q + 2]);
+          acc[4 * q + 3] = fmaf(xv, wv.w, acc[4 * q + 3]);
+        }
+      }
+    }
+    uint32_t* out = reinterpret_cast<uint32_t*>(a.y + h * cout);
+    const uint32_t* res = a.residual ? reinterpret_cast<const uint32_t*>(a.residual + h * cout) : nullptr;
+#pragma unroll
+    for (int j = 0; j < COP; j += 2) {
+      if (j >= cout) break;
+      float lo = fmaf(acc[j], saff[j].x, saff[j].y), hi = fmaf(acc[j + 1], saff[j + 1].x, saff[j + 1].y);
+      if (res) {
+        const float2 rf = unpack2(res[j >> 1], HALF);
+        lo += rf.x;
+        hi += rf.y;
+      }
+      if (a.relu) {
+        lo = fmaxf(lo, 0.f);
+        hi = fmaxf(hi, 0.f);
+      }
+      out[j >> 1] = pack2(lo, hi, HALF);
+    }
+  }
+}
+
+template <int COP>
+int launch_pw_any(const PwArgs& a, int cout, cudaStream_t st) {
+  OCNN_CUDA_OK(launch_chained(a.f16 ? conv_pw_any_kernel<COP, true> : conv_pw_any_kernel<COP, false>,
+                              dim3(grid_for(a.h, 128)), dim3(128), (size_t)a.cin * COP * sizeof(float), st, a, cout));
+  OCNN_LAUNCH_OK("conv_pw_any_kernel");
+  return OCNN_OK;
+}
+
 }  // namespace
 
 // Used by ocnn_octree_conv for 1x1x1 stride-1 bf16 node-major convolutions.  Returns -1 when the
@@ -781,7 +851,9 @@ int try_pw_mma(const PwArgs& a, int cout, cudaStream_t st) {
 int conv_pointwise_bf16(const void* x, const float* w, void* y, int h, int cin, int cout,
                         const ocnn_conv_epilogue* ep, cudaStream_t st, bool f16) {
   if (cin % 8 != 0 || cin > 256 || (long long)cin * cout > 16384) return -1;
-  if (cout != 8 && cout != 16 && cout != 32 && cout != 64) return -1;
+  const bool any = cout != 8 && cout != 16 && cout != 32 && cout != 64;
+  // (shared memory: cin x Cout weights)
+  if (any && (cout % 2 != 0 || cout > 64 || (long long)cin * ((cout + 7) / 8 * 8) > 11 * 1024)) return -1;
   if (((uintptr_t)x % 16) != 0 || ((uintptr_t)y % 16) != 0) return -1;
   if (ep && ep->residual_dev && ((uintptr_t)ep->residual_dev % 16) != 0) return -1;
   PwArgs a;
@@ -798,6 +870,18 @@ int conv_pointwise_bf16(const void* x, const float* w, void* y, int h, int cin, 
   a.w2 = nullptr; a.aff2 = channel_affine_of(nullptr); a.y2 = nullptr; a.relu2 = 0;
   a.wide = (((uintptr_t)x % 32) == 0 && ((uintptr_t)y % 32) == 0 &&
             (!(ep && ep->residual_dev) || ((uintptr_t)ep->residual_dev % 32) == 0)) ? 1 : 0;
+  if (any) {
+    switch ((cout + 7) / 8) {
+      case 1: return launch_pw_any<8>(a, cout, st);
+      case 2: return launch_pw_any<16>(a, cout, st);
+      case 3: return launch_pw_any<24>(a, cout, st);
+      case 4: return launch_pw_any<32>(a, cout, st);
+      case 5: return launch_pw_any<40>(a, cout, st);
+      case 6: return launch_pw_any<48>(a, cout, st);
+      case 7: return launch_pw_any<56>(a, cout, st);
+      default: return launch_pw_any<64>(a, cout, st);
+    }
+  }
   {
     static const int use_mma = [] { const char* e = getenv("OCNN_PW_MMA"); return e ? atoi(e) : 1; }();
     if (use_mma) {

@@ -80,11 +80,12 @@ struct TcArgs {
   int fold_cout;    // > 0: a 1x1x1 layer with Cin < 64 run on rows of 64/Cin nodes (one 128-byte
                     // line) against block-diagonal weights: column n is channel n % fold_cout of
                     // node n / fold_cout of the row
-  const int* scatter_child;   // with expand_cout: Child block of the finer level; octant o of tile
-                              // row h is written to row scatter_child[8h + o] (skipped when < 0)
   ChannelAffine aff;
   const __nv_bfloat16* residual;
   int relu;
+  int late_affine;  // scale and bias are staged over the neighbour table, after the gather
+  float* partial;   // K split: fp32 sums [split][rows][row_elems] instead of y, finished by a reduction
+  int kb_per_split;
   int* status;
   signed char tap[27];
 };
@@ -167,8 +168,8 @@ __device__ __forceinline__ void chunk_src(int cpt, int kb, int chunk, int& t, ui
 }
 
 // GENERAL compiles in the rarely used layer kinds (stride-2 deconvolution in gather form, the
-// expanded kernel-2 deconvolution with its scattered epilogue); the convolutions of the
-// classification networks run the variant without them.
+// expanded kernel-2 deconvolution); the convolutions of the classification networks run the variant
+// without them.
 template <int CPT, bool HALF, bool GENERAL>
 __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
   extern __shared__ uint8_t smem_raw[];
@@ -181,11 +182,13 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
   // per-column scale and bias of the epilogue, staged once per CTA: read from global memory in
   // the epilogue they were a chain of cold misses (one per 128-byte line of each array) that every
   // thread of a one-wave launch sat through
-  float* s_scale = reinterpret_cast<float*>(
-      nbr + (a.group ? (a.rowsplit == 3 ? 64 * kGroupTableStride : 0)
-                     : a.T * (a.rowsplit == 4 ? kGroupTableStride : kTileM)));
+  // (they take the neighbour table's place after the gather where that is what lets two CTAs share
+  // the SM: 256 columns)
+  int* table_end = nbr + (a.group ? (a.rowsplit == 3 ? 64 * kGroupTableStride : 0)
+                                  : a.T * (a.rowsplit == 4 ? kGroupTableStride : kTileM));
+  float* s_scale = reinterpret_cast<float*>(a.late_affine ? nbr : table_end);
   float* s_bias = s_scale + a.npad;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_bias + a.npad);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(a.late_affine ? reinterpret_cast<float*>(table_end) : s_bias + a.npad);
   uint64_t* full = bars;
   uint64_t* empty = bars + a.stages;
   uint64_t* accum = bars + 2 * a.stages;
@@ -196,6 +199,8 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
   const int h0 = blockIdx.x * a.tile_rows;
   // blockIdx.y = 256-channel slice of the output (layers with more than 256 output channels)
   const int co_base = blockIdx.y * a.cout;
+  const int kb_first = blockIdx.z * a.kb_per_split;
+  const int kb_end = min(a.nkb, kb_first + a.kb_per_split);
   const uint8_t* wpacked = a.wpacked + (size_t)blockIdx.y * a.nkb * (a.npad * 128);
   grid_dependency_trigger();     // the next layer's CTAs may queue up behind this grid's last wave
 
@@ -217,16 +222,19 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
   // everything above is private to the CTA; from here on global memory is read, so the previous
   // kernel of the stream must have completed
   grid_dependency_wait();
-  for (int n = tid; n < a.npad; n += kThreads) {
-    // output channel of column n: columns are (octant, channel) pairs in group mode
-    int co = a.group ? (n & (a.cout - 1)) : co_base + n;
-    if (a.fold_cout) co = n % a.fold_cout;
-    if (GENERAL && a.expand_cout) co = (co_base + n) % a.expand_cout;
-    const bool live = n < a.row_elems;
-    const float2 sb = live ? channel_affine(a.aff, co) : make_float2(1.f, 0.f);
-    s_scale[n] = sb.x;
-    s_bias[n] = sb.y;
-  }
+  auto stage_affine = [&](int threads) {
+    for (int n = tid; n < a.npad; n += threads) {
+      // output channel of column n: columns are (octant, channel) pairs in group mode
+      int co = a.group ? (n & (a.cout - 1)) : co_base + n;
+      if (a.fold_cout) co = n % a.fold_cout;
+      if (GENERAL && a.expand_cout) co = (co_base + n) % a.expand_cout;
+      const bool live = n < a.row_elems;
+      const float2 sb = live ? channel_affine(a.aff, co) : make_float2(1.f, 0.f);
+      s_scale[n] = sb.x;
+      s_bias[n] = sb.y;
+    }
+  };
+  if (!a.late_affine) stage_affine(kThreads);
   if (tid < kTileM) {
     const int h = h0 + tid;          // node, or sibling group in group mode
     const bool live = tid < a.tile_rows && h < a.rows;
@@ -324,15 +332,15 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
         int p[8];
         int s = 0;
         uint32_t pe = 1;
-        int t = 0, part = 0;
-        for (int kb = 0; kb < a.nkb; ++kb) {
-          if (part == 0) {
+        int t = kb_first / kBlocksPerTap, part = kb_first - t * kBlocksPerTap;
+        for (int kb = kb_first; kb < kb_end; ++kb) {
+          if (part == 0 || kb == kb_first) {
             const int4 lo = *reinterpret_cast<const int4*>(my_idx + t * kTileM);
             const int4 hi = *reinterpret_cast<const int4*>(my_idx + t * kTileM + 4);
             p[0] = lo.x; p[1] = lo.y; p[2] = lo.z; p[3] = lo.w;
             p[4] = hi.x; p[5] = hi.y; p[6] = hi.z; p[7] = hi.w;
           }
-          if (alive && kb >= a.stages)
+          if (alive && kb - kb_first >= a.stages)
             alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrEmptyWait);
           if (alive) {
             const uint32_t stage_base = smem_u32(sA + s * kStageA);
@@ -396,13 +404,13 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
       uint32_t pe = 1;
       int p_cur[8];
       uint32_t off_cur;
-      fetch(0, p_cur, off_cur);
-      for (int kb = 0; kb < a.nkb; ++kb) {
+      fetch(kb_first, p_cur, off_cur);
+      for (int kb = kb_first; kb < kb_end; ++kb) {
         // the indices of the next block are requested before this block's copies are issued
         int p_nxt[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
         uint32_t off_nxt = 0;
-        if (kb + 1 < a.nkb) fetch(kb + 1, p_nxt, off_nxt);
-        if (alive && kb >= a.stages)
+        if (kb + 1 < kb_end) fetch(kb + 1, p_nxt, off_nxt);
+        if (alive && kb - kb_first >= a.stages)
           alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrEmptyWait);
         if (alive) {
           const uint32_t stage_base = smem_u32(sA + s * kStageA);
@@ -435,9 +443,14 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
       const int nbr_stride = a.group ? 1 : kTileM;
       const int T = a.T;
       int s = 0, t_run = 0, cc_run = 0;
+      if constexpr (CPT == 0) {
+        const int g = kb_first * 8, cpt = a.cin >> 3;
+        t_run = g / cpt;
+        cc_run = g - t_run * cpt;
+      }
       uint32_t pe = 1;                       // parity of the next empty[] wait, flips per ring turn
-      for (int kb = 0; kb < a.nkb; ++kb) {
-        if (alive && kb >= a.stages)
+      for (int kb = kb_first; kb < kb_end; ++kb) {
+        if (alive && kb - kb_first >= a.stages)
           alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrEmptyWait);
         bool paired = false;
         if constexpr (CPT == 0) paired = a.x2 != nullptr;
@@ -467,6 +480,11 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");   // nothing of ours in flight past this point
+    if (a.late_affine) {
+      asm volatile("bar.sync 1, 128;" ::: "memory");   // every gather thread has read its last table entry
+      stage_affine(kTileM);
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+    }
 
     // ---------------- epilogue: TMEM -> registers -> global ----------------
     // The residual is read 64 bytes (32 channels) of the row at a time, the four 16-byte pieces at
@@ -501,7 +519,6 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
     if (alive) {
       __nv_bfloat16* y_row = a.y + (long long)h * a.y_stride + co_base;
       const bool has_sb = a.aff.any();
-      const bool scatter = GENERAL && a.scatter_child != nullptr;
       for (int c0 = 0; c0 < a.npad; c0 += 32) {
         uint4 res_cur[4];
 #pragma unroll
@@ -517,6 +534,18 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
           const int n0 = c0 + 16 * step;
           if (n0 >= a.npad) break;
           const uint32_t (&v)[16] = v2[step];
+          if (a.partial != nullptr) {
+            if (row_ok && n0 < a.row_elems) {
+              uint32_t* out = reinterpret_cast<uint32_t*>(a.partial) +
+                              ((long long)blockIdx.z * a.rows + h) * a.y_stride + co_base + n0;
+#pragma unroll
+              for (int j = 0; j < 16; j += 8)
+                if (n0 + j < a.row_elems)
+                  st_global_32B(out + j, make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]),
+                                make_uint4(v[j + 4], v[j + 5], v[j + 6], v[j + 7]));
+            }
+            continue;
+          }
           uint4 ov[2];
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
@@ -551,20 +580,11 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
             uint32_t* op = reinterpret_cast<uint32_t*>(&ov[half]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) op[j] = pack2(f[2 * j], f[2 * j + 1], f16);
-            if (scatter) {
-              // column (co_base + n) = octant * Cout + channel of this parent's children; the child
-              // of octant o lives in row scatter_child[8h + o] of the output (if it is non-empty)
-              const int ng = co_base + n;
-              const int o = ng / a.expand_cout;
-              const int dst = a.scatter_child[((long long)h << 3) + o];
-              if (dst >= 0)
-                *reinterpret_cast<uint4*>(a.y + (long long)dst * a.expand_cout + (ng - o * a.expand_cout)) =
-                    ov[half];
-            } else if (!a.wide) {
+            if (!a.wide) {
               *reinterpret_cast<uint4*>(y_row + n) = ov[half];
             }
           }
-          if (a.wide && !scatter && row_ok && n0 < a.row_elems) st_global_32B(y_row + n0, ov[0], ov[1]);
+          if (a.wide && row_ok && n0 < a.row_elems) st_global_32B(y_row + n0, ov[0], ov[1]);
         }
       }
     }
@@ -580,7 +600,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
       bool alive = true;
       int s = 0;
       uint32_t pf = 0;
-      for (int kb = 0; kb < a.nkb && alive; ++kb) {
+      for (int kb = kb_first; kb < kb_end && alive; ++kb) {
         alive = mbar_wait(smem_u32(&full[s]), pf, abort_flag, a.status, kErrFullWait);
         if (!alive) break;
         // the gathered bytes were written through the generic proxy (cp.async) and have been
@@ -593,7 +613,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
 #pragma unroll
         for (int k4 = 0; k4 < kBlockK / 16; ++k4) {
           umma_bf16(tmem_base, smem_desc_sw128(a_addr + k4 * 32), smem_desc_sw128(b_addr + k4 * 32),
-                    idesc, (kb > 0 || k4 > 0) ? 1u : 0u);
+                    idesc, (kb > kb_first || k4 > 0) ? 1u : 0u);
         }
         umma_commit(smem_u32(&empty[s]));     // stage reusable once these MMAs retire
         if (++s == a.stages) { s = 0; pf ^= 1u; }
@@ -625,8 +645,8 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
       bool alive = true;
       int s = 0;
       uint32_t pe = 1;
-      for (int kb = 0; kb < a.nkb && alive; ++kb) {
-        if (kb >= a.stages)
+      for (int kb = kb_first; kb < kb_end && alive; ++kb) {
+        if (kb - kb_first >= a.stages)
           alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrWeightWait);
         if (!alive) break;
         const uint32_t bar = smem_u32(&full[s]);
@@ -1125,6 +1145,47 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
   }
 }
 
+// Sum of the K splits and the epilogue: one thread per eight columns.
+template <bool HALF>
+__global__ void __launch_bounds__(256) conv_tc_reduce_kernel(const float* __restrict__ partial, uint4* __restrict__ y,
+                                                             long long chunks, int splits, int cout,
+                                                             const ChannelAffine aff,
+                                                             const uint4* __restrict__ residual, int relu) {
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < chunks; i += gridDim.x * 256LL) {
+    float f[8] = {};
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) {
+      uint4 lo, hi;
+      ld_global_32B(partial + (s * chunks + i) * 8, lo, hi);
+      const uint32_t v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] += __uint_as_float(v[j]);
+    }
+    const int c0 = (int)(i % (cout >> 3)) * 8;
+    const uint4 r = residual ? residual[i] : make_uint4(0, 0, 0, 0);
+    const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+    uint32_t out[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 a0 = channel_affine(aff, c0 + 2 * j), a1 = channel_affine(aff, c0 + 2 * j + 1);
+      float lo = fmaf(f[2 * j], a0.x, a0.y), hi = fmaf(f[2 * j + 1], a1.x, a1.y);
+      if (residual) {
+        const float2 rf = unpack2(rw[j], HALF);
+        lo += rf.x;
+        hi += rf.y;
+      }
+      if (relu) {
+        lo = fmaxf(lo, 0.f);
+        hi = fmaxf(hi, 0.f);
+      }
+      out[j] = pack2(lo, hi, HALF);
+    }
+    y[i] = make_uint4(out[0], out[1], out[2], out[3]);
+  }
+}
+
 // ---- self-test of the bounded waits -------------------------------------------------------------
 // One CTA, two waiting threads, a barrier that nobody ever arrives on: the first waiter must run
 // out of polls, write its code to status[0] and raise the abort flag; the second must come back
@@ -1289,6 +1350,15 @@ int fold_mode() {
   return mode;
 }
 
+// 0: K is never split over CTAs.
+int split_mode() {
+  static const int mode = [] {
+    const char* e = getenv("OCNN_CONV_SPLIT");
+    return e ? atoi(e) : 1;
+  }();
+  return mode;
+}
+
 struct TcShape {
   int T, npad, nkb, tmem_cols, stages, group, slices, tile_rows, gtable, ntable_stride;
   int fold_in, expand_out;   // kernel 2, stride 2 as a dense product (see WeightView)
@@ -1297,10 +1367,11 @@ struct TcShape {
   size_t smem;
   size_t fixed_bytes, stage_bytes;   // shared memory outside the ring / per ring stage
   bool small_grid;                   // the tiles do not fill the SMs once
+  int late_affine, splits, kb_per_split;
 };
 
 int tc_shape(int cin, int cout, const int ks[3], const LayerKind& kind, TcShape* s,
-             long long rows_hint = -1) {
+             long long rows_hint = -1, bool can_split = false) {
   const TapList tl = taps_for_kernel(ks);
   const int stride = kind.stride;
   if (tl.count < 0)
@@ -1313,10 +1384,12 @@ int tc_shape(int cin, int cout, const int ks[3], const LayerKind& kind, TcShape*
   const bool k222s2 = ks[0] == 2 && ks[1] == 2 && ks[2] == 2 && stride == 2;
   // kernel 2, stride 2: a sibling group's eight children are the whole neighbourhood.  On all nodes
   // the convolution reads them as one contiguous row of 8*Cin channels; the deconvolution writes a
-  // parent's eight children as one row of 8*Cout channels (scattered through child on non-empty
-  // nodes).  Both are then plain dense products with no gather.
+  // parent's eight children as one row of 8*Cout channels.  Both are then plain dense products with no
+  // gather.  (On non-empty nodes a parent has one or two of its eight children: the deconvolution
+  // runs there as a gather from the child, eight taps of which one is live.  Expanded and scattered it
+  // formed six times the rows: 96 -> 96 at 186 k nodes 243 us.)
   s->fold_in = (k222s2 && !kind.transposed && !kind.nempty) ? 1 : 0;
-  s->expand_out = (k222s2 && kind.transposed && (cout * 8 <= 256 || cout % 32 == 0) && cout * 8 <= 4096) ? 1 : 0;
+  s->expand_out = (k222s2 && kind.transposed && !kind.nempty && (cout * 8 <= 256 || cout % 32 == 0) && cout * 8 <= 4096) ? 1 : 0;
   // 1x1x1, stride 1, fewer than 64 channels in: a K-block of one node would be mostly padding and
   // a tile of 128 nodes only 128*Cin*2 bytes.  64/Cin consecutive nodes are one 128-byte line, so
   // the layer runs on rows of 64/Cin nodes with block-diagonal weights (K = 64 exactly, N =
@@ -1354,8 +1427,11 @@ int tc_shape(int cin, int cout, const int ks[3], const LayerKind& kind, TcShape*
   // node mode keeps a [taps][128] index table; Cin not a multiple of 64 reads it per K-block with
   // lanes on different taps, which wants the padded stride
   s->ntable_stride = (!s->group && s->cin_eff % 64 != 0 && s->T > 1) ? kGroupTableStride : kTileM;
-  const size_t fixed = 1024 + (s->group ? (s->gtable ? 64 * kGroupTableStride * 4 : 0) : (size_t)s->T * s->ntable_stride * 4) +
-                       (size_t)s->npad * 8 + 256;
+  const size_t table = s->group ? (s->gtable ? 64 * kGroupTableStride * 4 : 0) : (size_t)s->T * s->ntable_stride * 4;
+  // 256 columns: with scale and bias in the table's place two stages fit twice into an SM (149 tiles of
+  // 256 -> 256 ran as two waves of one CTA per SM, 109 us; as one wave of two)
+  s->late_affine = (!s->group && s->npad > 128 && table >= (size_t)s->npad * 8) ? 1 : 0;
+  const size_t fixed = 1024 + table + (s->late_affine ? 0 : (size_t)s->npad * 8) + 256;
   const size_t two_cta = 112 * 1024, one_cta = 200 * 1024;
   // every stage of the ring can be in flight at once, so prefer two CTAs per SM (set-up and
   // epilogue of one overlap the main loop of the other) whenever each still gets 2 stages
@@ -1372,7 +1448,20 @@ int tc_shape(int cin, int cout, const int ks[3], const LayerKind& kind, TcShape*
   while (rows >= 0 && s->tile_rows > 32 && 2 * ((rows + s->tile_rows - 1) / s->tile_rows) <= sms &&
          8.0 * s->tile_rows > 3.2 * s->npad)
     s->tile_rows >>= 1;
-  const bool small_grid = rows >= 0 && (rows + s->tile_rows - 1) / s->tile_rows <= sms;
+  // A level of few tiles and a long K (32 K-blocks or more): K is split over several CTAs per tile, eight
+  // blocks or more each, and a reduction adds their fp32 sums.  The tiles are whole then: with 64-row
+  // tiles half of every MMA was padding, and each CTA still walked all of K (256 -> 256, 27 taps, 4.2 k
+  // nodes: 66 CTAs of 108 K-blocks, 58 us).
+  s->splits = 1;
+  const long long whole = rows < 0 ? 0 : (rows + kTileM - 1) / kTileM * s->slices;
+  if (can_split && rows >= 0 && !s->group && !s->expand_out && s->nkb >= 32 && 2 * whole <= sms && split_mode() != 0) {
+    s->tile_rows = kTileM;
+    const long long want = sms / whole, most = s->nkb / 8;
+    s->splits = (int)(want < most ? want : most);
+  }
+  s->kb_per_split = (s->nkb + s->splits - 1) / s->splits;
+  s->splits = (s->nkb + s->kb_per_split - 1) / s->kb_per_split;
+  const bool small_grid = rows >= 0 && (rows + s->tile_rows - 1) / s->tile_rows * s->splits <= sms;
   if (st < 2 || 2 * s->tmem_cols > 512 || small_grid) {
     st = (int)((one_cta - fixed) / stage_bytes);
     if (st > 7) st = 7;
@@ -1481,7 +1570,7 @@ int pack_weights_impl(const float* w, void* packed, int cin, int cout, const int
 int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geometry* g, int cin,
                  int cout, const int kernel_size[3], int dtype, const ocnn_conv_epilogue* ep,
                  int32_t* status, void* stream, const char* who, const void* x2 = nullptr,
-                 int cin_a = 0) {
+                 int cin_a = 0, void* workspace = nullptr, size_t workspace_bytes = 0) {
   OCNN_REQUIRE(kernel_size != nullptr, "%s: null kernel size", who);
   OCNN_REQUIRE(dtype == OCNN_BF16 || dtype == OCNN_F16, "%s: bf16 or fp16 data only (dtype %d)", who, dtype);
   const TapList tl = taps_for_kernel(kernel_size);
@@ -1497,7 +1586,11 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
   {
     TcShape probe;
     if (int st = tc_shape(cin, cout, kernel_size, kind, &probe, -1)) return st;
-    if (int st = tc_shape(cin, cout, kernel_size, kind, &s, probe.expand_out ? h_in : h_out)) return st;
+    const long long rows = probe.expand_out ? h_in : h_out;
+    if (int st = tc_shape(cin, cout, kernel_size, kind, &s, rows, workspace != nullptr)) return st;
+    const size_t need = s.splits > 1 ? (size_t)s.splits * rows * s.cout_eff * 4 : 0;
+    if (need > workspace_bytes)       // (the caller's workspace was for another layer: run unsplit)
+      if (int st = tc_shape(cin, cout, kernel_size, kind, &s, rows, false)) return st;
   }
   if (h_out == 0 || (s.expand_out && h_in == 0)) return OCNN_OK;
   const bool identity = s.T == 1 && (stride == 1 || s.fold_in || s.expand_out);
@@ -1506,11 +1599,6 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
                "%s: data and weight pointers must be 16-byte aligned", who);
   if (ep && ep->residual_dev)
     OCNN_REQUIRE((uintptr_t)ep->residual_dev % 16 == 0, "%s: residual must be 16-byte aligned", who);
-  const bool scatter = s.expand_out && g->nempty;
-  if (scatter) {
-    OCNN_REQUIRE(g->child_dev != nullptr, "%s: child array of the finer level required", who);
-    OCNN_REQUIRE(!(ep && ep->residual_dev), "%s: no residual on a scattered deconvolution", who);
-  }
   if (x2 != nullptr && identity && !g->nempty && !g->transposed && s.fold_nodes == 1 && s.slices == 1 &&
       cin_a > 0 && cin_a < cin) {
     // few channels on a big level: the streaming kernel, on the same packed weights
@@ -1560,7 +1648,6 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
     note_launches(1);
     if (h_out < s.fold_nodes) return OCNN_OK;
   }
-  a.scatter_child = scatter ? g->child_dev : nullptr;
   a.h_in = h_in; a.h_out = h_out; a.cin = s.cin_eff; a.npad = s.npad; a.T = s.T;
   a.stride = (s.fold_in || s.expand_out) ? 1 : stride;
   a.identity = identity ? 1 : 0; a.nkb = s.nkb; a.stages = s.stages;
@@ -1585,6 +1672,13 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
   a.aff = channel_affine_of(ep);
   a.residual = ep ? static_cast<const __nv_bfloat16*>(ep->residual_dev) : nullptr;
   a.relu = epilogue_relu(ep);
+  a.late_affine = s.late_affine;
+  a.kb_per_split = s.kb_per_split;
+  a.partial = s.splits > 1 ? static_cast<float*>(workspace) : nullptr;
+  if (s.splits > 1) {
+    OCNN_REQUIRE((uintptr_t)workspace % 32 == 0, "%s: the workspace must be 32-byte aligned", who);
+    a.residual = nullptr;
+  }
   a.status = status;
   for (int i = 0; i < 27; ++i) {
     int tap = i < tl.count ? tl.tap[i] : 0;
@@ -1699,9 +1793,18 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
       return OCNN_OK;
     }
   }
-  OCNN_CUDA_OK(launch_chained(kernel, dim3(ntiles, s.slices), dim3(kThreads), s.smem,
+  OCNN_CUDA_OK(launch_chained(kernel, dim3(ntiles, s.slices, s.splits), dim3(kThreads), s.smem,
                               static_cast<cudaStream_t>(stream), a));
   OCNN_LAUNCH_OK("conv_tc_kernel");
+  if (s.splits > 1) {
+    const long long chunks = (long long)a.rows * a.y_stride / 8;
+    const uint4* res = ep ? static_cast<const uint4*>(ep->residual_dev) : nullptr;
+    OCNN_CUDA_OK(launch_chained(a.f16 ? conv_tc_reduce_kernel<true> : conv_tc_reduce_kernel<false>,
+                                dim3(grid_for(chunks, 256)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                (const float*)a.partial, static_cast<uint4*>(y), chunks, s.splits, s.cout_eff, a.aff,
+                                res, a.relu));
+    OCNN_LAUNCH_OK("conv_tc_reduce_kernel");
+  }
   return OCNN_OK;
 }
 
@@ -1793,6 +1896,26 @@ int ocnn_octree_conv_tc_general(const void* x, const void* packed, void* y,
                                 int32_t* status, void* stream) {
   return ocnn::conv_tc_impl(x, packed, y, geometry, cin, cout, kernel_size, dtype, ep, status, stream,
                             "ocnn_octree_conv_tc_general");
+}
+
+size_t ocnn_octree_conv_tc_workspace_bytes(const ocnn_conv_geometry* g, int cin, int cout,
+                                           const int kernel_size[3]) {
+  using namespace ocnn;
+  if (g == nullptr || kernel_size == nullptr) return 0;
+  const LayerKind kind{g->stride, g->transposed != 0, g->nempty != 0};
+  TcShape s;
+  if (tc_shape(cin, cout, kernel_size, kind, &s, -1) != OCNN_OK) return 0;
+  const long long rows = s.expand_out ? g->h_in : g->h_out;
+  if (tc_shape(cin, cout, kernel_size, kind, &s, rows, true) != OCNN_OK || s.splits <= 1) return 0;
+  return (size_t)s.splits * rows * s.cout_eff * 4;
+}
+
+int ocnn_octree_conv_tc_general_ws(const void* x, const void* packed, void* y,
+                                   const ocnn_conv_geometry* geometry, int cin, int cout,
+                                   const int kernel_size[3], int dtype, const ocnn_conv_epilogue* ep,
+                                   int32_t* status, void* workspace, size_t workspace_bytes, void* stream) {
+  return ocnn::conv_tc_impl(x, packed, y, geometry, cin, cout, kernel_size, dtype, ep, status, stream,
+                            "ocnn_octree_conv_tc_general_ws", nullptr, 0, workspace, workspace_bytes);
 }
 
 }  // extern "C"

@@ -425,6 +425,30 @@ int check_common(const char* op, const void* a, const void* b, const void* c, in
   return OCNN_OK;
 }
 
+// Rows of two node-major tensors side by side (a U-Net's skip connection): 16-byte pieces, four in
+// flight per thread.
+__global__ void __launch_bounds__(256) cat_rows_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b,
+                                                       uint4* __restrict__ out, long long rows, int ca, int cb) {
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  const int c = ca + cb;
+  const long long total = rows * c, stride = (long long)gridDim.x * blockDim.x;
+  for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < total; i0 += 4 * stride) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * stride;
+      if (i >= total) break;
+      const long long h = i / c;
+      const int k = (int)(i - h * c);
+      v[u] = k < ca ? a[h * ca + k] : b[h * cb + (k - ca)];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * stride < total) out[i0 + u * stride] = v[u];
+  }
+}
+
 }  // namespace
 }  // namespace ocnn
 
@@ -500,6 +524,21 @@ int ocnn_octree_tile(const void* y, void* out, const int32_t* child, int C, int 
         (const __nv_bfloat16*)y, (__nv_bfloat16*)out, child, C, hy, hout, layout == OCNN_NODE_MAJOR);
   }
   OCNN_LAUNCH_OK("octree_tile");
+  return OCNN_OK;
+}
+
+int ocnn_cat_rows(const void* a, const void* b, void* out, int64_t rows, int a_bytes, int b_bytes, void* stream) {
+  using namespace ocnn;
+  OCNN_REQUIRE(rows >= 0 && a_bytes > 0 && b_bytes > 0 && a_bytes % 16 == 0 && b_bytes % 16 == 0,
+               "ocnn_cat_rows: rows of %d and %d bytes", a_bytes, b_bytes);
+  if (rows == 0) return OCNN_OK;
+  OCNN_REQUIRE(a && b && out && (uintptr_t)a % 16 == 0 && (uintptr_t)b % 16 == 0 && (uintptr_t)out % 16 == 0,
+               "ocnn_cat_rows: null or misaligned pointer");
+  const int ca = a_bytes / 16, cb = b_bytes / 16;
+  OCNN_CUDA_OK(launch_chained(cat_rows_kernel, dim3(grid_for(rows * (ca + cb), 4 * 256)), dim3(256), 0,
+                              static_cast<cudaStream_t>(stream), (const uint4*)a, (const uint4*)b, (uint4*)out,
+                              (long long)rows, ca, cb));
+  OCNN_LAUNCH_OK("cat_rows_kernel");
   return OCNN_OK;
 }
 

@@ -5,8 +5,21 @@ optional interpolation at query points and a two-layer 1x1 head.  Forward only."
 import torch
 from torch import nn as _nn
 
+from . import nn
 from .modules import (OctreeConvBnRelu, OctreeDeConvBnRelu, OctreeResBlocks, OctreeResBlock2,
                       OctreeConv1x1BnRelu, OctreeConv1x1, OctreeInterp, octree_feature)
+
+
+def _cat(skip, up):
+  """The skip connection: both tensors' channels side by side, in `up`'s memory layout."""
+  rows = all(t.is_contiguous(memory_format=torch.channels_last) and not t.is_contiguous() and
+             t.shape[1] * t.element_size() % 16 == 0 and t.data_ptr() % 16 == 0 for t in (skip, up))
+  if rows and up.is_cuda and up.dtype == skip.dtype and not (
+      torch.is_grad_enabled() and (skip.requires_grad or up.requires_grad)):
+    return nn.cat_channels(skip, up)
+  fmt = torch.channels_last if up.is_contiguous(memory_format=torch.channels_last) and \
+      not up.is_contiguous() else torch.contiguous_format
+  return torch.cat([skip, up], dim=1).contiguous(memory_format=fmt)
 
 
 class UNet(_nn.Module):
@@ -63,9 +76,7 @@ class UNet(_nn.Module):
     for i in range(self.stages):
       d += 1
       up = self.upsample[i](x, octree)
-      fmt = torch.channels_last if up.is_contiguous(memory_format=torch.channels_last) and \
-          not up.is_contiguous() else torch.contiguous_format
-      x = torch.cat([level[d], up], dim=1).contiguous(memory_format=fmt)
+      x = _cat(level[d], up)
       x = self.decoder[i](x, octree)
     if pts is not None:
       x = self.octree_interp(x, octree, pts)

@@ -270,6 +270,22 @@ Tensor octree_tile(Tensor data_in, Tensor octree, int depth) {
   return out;
 }
 
+// torch.cat([a, b], dim=1) of two node-major tensors of the same rows.
+Tensor cat_channels(Tensor a, Tensor b) {
+  need_cuda(a, "cat_channels");
+  need_cuda(b, "cat_channels");
+  c10::cuda::CUDAGuard guard(a.device());
+  TORCH_CHECK(a.scalar_type() == b.scalar_type() && a.dim() == 4 && b.dim() == 4 && a.size(0) == 1 &&
+                  b.size(0) == 1 && a.size(2) == b.size(2) && a.size(3) == 1 && b.size(3) == 1 &&
+                  a.is_contiguous(at::MemoryFormat::ChannelsLast) && b.is_contiguous(at::MemoryFormat::ChannelsLast),
+              "cat_channels: two channels_last tensors [1, C, H, 1] of one dtype and height");
+  Tensor out = torch::empty({1, a.size(1) + b.size(1), a.size(2), 1},
+                            a.options().memory_format(at::MemoryFormat::ChannelsLast));
+  OCNN_CALL(ocnn_cat_rows(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.size(2),
+                          (int)(a.size(1) * a.element_size()), (int)(b.size(1) * b.element_size()), current_stream()));
+  return out;
+}
+
 vector<Tensor> octree_max_pool(Tensor data_in, Tensor octree, int depth) {
   OctreeRef o = get_octree(octree);
   TORCH_CHECK(depth > 1, "Depth should be larger than 1");
@@ -578,6 +594,16 @@ void run_conv(const DataRef& x, const Tensor& w, Tensor& y, const ocnn_conv_geom
   }
 }
 
+// A layer on the 16-bit tensor-core kernel, with the workspace it asks for.
+void run_conv_tc(const void* x, const Tensor& packed, Tensor& y, const ocnn_conv_geometry& g, int cin, int cout,
+                 const vector<int>& ks, int dtype, const ocnn_conv_epilogue* ep, int32_t* status) {
+  const size_t bytes = ocnn_octree_conv_tc_workspace_bytes(&g, cin, cout, ks.data());
+  Tensor ws;
+  if (bytes > 0) ws = torch::empty({(int64_t)bytes}, torch::dtype(torch::kUInt8).device(y.device()));
+  OCNN_CALL(ocnn_octree_conv_tc_general_ws(x, packed.data_ptr(), y.data_ptr(), &g, cin, cout, ks.data(), dtype, ep,
+                                           status, bytes > 0 ? ws.data_ptr() : nullptr, bytes, current_stream()));
+}
+
 Tensor octree_conv_fused(Tensor data_in, Tensor weights, Tensor octree, int depth, int num_output,
                          vector<int> kernel_size, int stride, c10::optional<Tensor> scale,
                          c10::optional<Tensor> bias, c10::optional<Tensor> residual, bool relu,
@@ -693,9 +719,10 @@ Tensor octree_conv_tc(Tensor data_in, Tensor packed, Tensor octree, int depth, i
               "status must be an int32 CUDA tensor");
   Tensor y = new_data(num_output, s.h_out, x);
   ocnn_conv_epilogue ep = make_epilogue(scale, bias, residual, relu, num_output, y);
-  OCNN_CALL(ocnn_octree_conv_tc(x.t.data_ptr(), packed.data_ptr(), y.data_ptr(), s.neigh, s.h_in,
-                                s.h_out, x.C, num_output, ks.data(), stride, &ep,
-                                status.data_ptr<int32_t>(), current_stream()));
+  ocnn_conv_geometry g;
+  memset(&g, 0, sizeof(g));
+  g.stride = stride; g.h_in = s.h_in; g.h_out = s.h_out; g.neigh_dev = s.neigh;
+  run_conv_tc(x.t.data_ptr(), packed, y, g, x.C, num_output, ks, OCNN_BF16, &ep, status.data_ptr<int32_t>());
   return y;
 }
 
@@ -876,9 +903,7 @@ Tensor octree_conv_tc_general(Tensor data_in, Tensor packed, Tensor octree, int 
               "status must be an int32 CUDA tensor");
   Tensor y = new_data(num_output, geo.g.h_out, x);
   ocnn_conv_epilogue ep = make_epilogue(scale, bias, residual, relu, num_output, y);
-  OCNN_CALL(ocnn_octree_conv_tc_general(x.t.data_ptr(), packed.data_ptr(), y.data_ptr(), &geo.g, x.C,
-                                        num_output, ks.data(), x.dtype, &ep,
-                                        status.data_ptr<int32_t>(), current_stream()));
+  run_conv_tc(x.t.data_ptr(), packed, y, geo.g, x.C, num_output, ks, x.dtype, &ep, status.data_ptr<int32_t>());
   return y;
 }
 
@@ -1125,9 +1150,7 @@ class ConvLayer {
       if (packed.defined()) {
         TORCH_CHECK(status.is_cuda() && status.scalar_type() == torch::kInt32 && status.numel() >= 1,
                     "status must be an int32 CUDA tensor");
-        OCNN_CALL(ocnn_octree_conv_tc_general(x.t.data_ptr(), packed.data_ptr(), y.data_ptr(), &geo.g, cin_,
-                                              cout_, ks_.data(), x.dtype, &ep,
-                                              status.data_ptr<int32_t>(), current_stream()));
+        run_conv_tc(x.t.data_ptr(), packed, y, geo.g, cin_, cout_, ks_, x.dtype, &ep, status.data_ptr<int32_t>());
         return y;
       }
     }
@@ -2055,6 +2078,15 @@ class NetExecutor {
         pool_tmp = std::max<int64_t>(pool_tmp, (int64_t)o.meta.nnum[op.depth] / 8 * 4);
     const int64_t tmp_off = total;
     total += (pool_tmp + 255) / 256 * 256;
+    // workspace of the layers whose K is split over CTAs
+    int64_t split_ws = 0;
+    for (auto& op : ops_)
+      if (op.kind == ExecOp::kConvTc && op.in2 < 0) {
+        const ocnn_conv_geometry g = op_geometry(o, op);
+        split_ws = std::max<int64_t>(split_ws, ocnn_octree_conv_tc_workspace_bytes(&g, op.cin, op.cout, op.ks.data()));
+      }
+    const int64_t split_off = total;
+    total += (split_ws + 255) / 256 * 256;
     if (!arena_.defined() || arena_.numel() < total || arena_.device() != octree.device())
       arena_ = torch::empty({total + total / 4}, octree.options());
     uint8_t* base = arena_.data_ptr<uint8_t>();
@@ -2124,9 +2156,10 @@ class NetExecutor {
                                                op.packed.data_ptr(), slot(op.out), h, op.cout,
                                                OCNN_BF16, &ep, status_.data_ptr<int32_t>(), st));
           } else if (op.kind == ExecOp::kConvTc && !stream_pw) {
-            OCNN_CALL(ocnn_octree_conv_tc(slot(op.in), op.packed.data_ptr(), slot(op.out), neigh, h, h,
-                                          op.cin, op.cout, op.ks.data(), 1, &ep,
-                                          status_.data_ptr<int32_t>(), st));
+            const ocnn_conv_geometry g = op_geometry(o, op);
+            OCNN_CALL(ocnn_octree_conv_tc_general_ws(
+                slot(op.in), op.packed.data_ptr(), slot(op.out), &g, op.cin, op.cout, op.ks.data(), OCNN_BF16, &ep,
+                status_.data_ptr<int32_t>(), split_ws > 0 ? base + split_off : nullptr, (size_t)split_ws, st));
           } else {
             OCNN_CALL(ocnn_octree_conv(slot(op.in), op.weights.data_ptr<float>(), slot(op.out), neigh,
                                        h, h, op.cin, op.cout, op.ks.data(), 1, OCNN_BF16,
@@ -2260,6 +2293,13 @@ class NetExecutor {
   int status() { return status_.defined() ? status_.item<int>() : 0; }
 
  private:
+  static ocnn_conv_geometry op_geometry(const OctreeRef& o, const ExecOp& op) {
+    ocnn_conv_geometry g;
+    memset(&g, 0, sizeof(g));
+    g.stride = 1; g.h_in = g.h_out = o.meta.nnum[op.depth];
+    if (op.ks[0] * op.ks[1] * op.ks[2] > 1) g.neigh_dev = level_ptr(o, OCNN_PROP_NEIGH, op.depth, "conv");
+    return g;
+  }
   int push(const ExecOp& op) { ops_.push_back(op); return (int)ops_.size() - 1; }
   struct Ev { int index; cudaEvent_t e0, e1; };
   vector<ExecOp> ops_;
@@ -2360,6 +2400,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("depth"), py::arg("val") = 0.0f);
   m.def("octree_depad", &octree_depad, "octree depad");
   m.def("octree_tile", &octree_tile, "nearest upsampling: depad + repeat each row for its 8 children");
+  m.def("cat_channels", &cat_channels, "torch.cat over the channels of two channels_last tensors");
   m.def("octree_max_pool", &octree_max_pool, "octree max pooling");
   m.def("octree_max_pool_pad", &octree_max_pool_pad, "octree max pooling + pad to depth - 1 (bf16 node-major)");
   m.def("points_new", &points_new, "create a point cloud");
