@@ -2,21 +2,27 @@
 //
 // What the reference does per cloud on one CPU core (Octree::build, octree/octree/octree.cpp:74-121)
 // and then per batch (merge_octrees, octree/octree/merge_octrees.cpp:7-198) is done here in one
-// pass over all clouds: every point gets the composite key  (cloud << 3*depth) | morton(cell),
-// one stable LSD radix sort orders all clouds at once (equal to the reference's std::sort of
-// (key, index) pairs per cloud), and each level is then a segmented "unique" of the level below.
+// pass over all clouds: every point gets the composite key  (cloud << 3*depth) | morton(cell), the
+// clouds' own key bits are radix-sorted (the clouds already lie one behind the other, so the sort is
+// segmented by cloud and never looks at the cloud bits; equal to the reference's std::sort of (key,
+// index) pairs per cloud), and every level is a segmented "unique" of the sorted keys.
 // The composite key of a level-d node is also its rank basis: ranks in the batch-wide unique list
 // are exactly the rebased child indices that merge_octrees produces.
 //
 // Phase 1 (plan) leaves in the workspace, for d = full..depth, the sorted unique composite keys
 // Kd of the non-empty nodes and, for each such node, where its children (or its points, at the
-// finest level) start in the list below.  One device->host copy of the per-level counts follows;
-// the caller allocates the exact output.  Phase 2 (emit) writes header, keys, children, split
+// finest level) start in the list below.  The per-level counts reach the host through a mapped
+// word; the caller allocates the exact output.  Phase 2 (emit) writes header, keys, children, split
 // labels, finest-level signal and — for a merged batch — the neighbour table.
 //
 // All scans are reduce-then-scan over a fixed grid (no inter-block waiting anywhere).
 // This file is compiled with --fmad=false: the signal must round exactly like the reference's
 // separate multiplies and adds (octree.cpp:330-348).
+//
+// A depth-6 batch is 16 launches: encode + first histogram, two sort passes of 9 bits, count and
+// compact for all levels at once, averages, emit, neighbour tables.  (A count and a compact launch
+// per level, a sort over the cloud bits too and separate header / table copies made it 33, most of
+// them shorter than their launch.)
 #include <cstring>
 #include <vector>
 
@@ -26,30 +32,35 @@ namespace ocnn {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / 32;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kThreads * kScanItems;
 constexpr int kMaxScanGrid = kSMs * 4;   // 592 blocks: 4 CTAs of 256 threads per SM
 constexpr int kSortItems = 8;            // keys per thread per sort tile
 constexpr int kSortTile = kThreads * kSortItems;   // 2048 keys
 
-// One entry per cloud (plus a sentinel holding the total point count), uploaded by the plan call.
+// One entry per cloud (plus a sentinel holding the totals).
 struct CloudRef {
   const float* xyz;
   const float* normal;
   const float* feat;
   const float* label;
   long long offset;     // index of the cloud's first point in the batch-wide numbering
+  int chunk0;           // first sort chunk (= sort CTA) of the cloud: a chunk never crosses clouds
+  int pad;
 };
+constexpr int kInlineClouds = 63;        // a table of this many clouds rides in the launch parameters
 
 // ---- workspace layout --------------------------------------------------------------------------
 struct Layout {
   int64_t n;            // total points
   int batch, depth, full;
-  int key_bytes_sort;   // 4 or 8: width of the sort key
-  int nvb;              // sort: number of CTAs, each owning one contiguous chunk of the keys
-  int vchunk;           // sort: keys per CTA chunk (multiple of the 2048-key tile)
+  int key_bytes;        // 4 or 8: width of the composite keys
+  int radix_bits, passes;
+  int max_chunks;       // sort: bound on the number of chunks, whatever the clouds' sizes
   int64_t cap[OCNN_MAX_DEPTH + 1];   // capacity of Kd
-  size_t off_offsets, off_counts, off_blockcnt, off_hist, off_bintot;
+  size_t off_clouds, off_counts, off_bintot, off_blockcnt, off_hist, off_avg;
+  size_t zero_bytes;    // counts + digit totals, cleared together
   size_t off_keys[2], off_idx[2];
   size_t off_K[OCNN_MAX_DEPTH + 1], off_start[OCNN_MAX_DEPTH + 2];
   size_t total;
@@ -63,36 +74,44 @@ int bits_for(int64_t v) {  // number of bits needed to represent values 0..v-1
   return b;
 }
 
+// Points per sort chunk: one tile until the batch has four tiles per SM, several tiles then.
+int chunk_points(int64_t n) {
+  const int64_t tiles = (n + kSortTile - 1) / kSortTile;
+  const int64_t per = (tiles + kSMs * 4 - 1) / (kSMs * 4);
+  return (int)((per < 1 ? 1 : per) * kSortTile);
+}
+
 Layout make_layout(int64_t n, int batch, int depth, int full) {
   Layout L;
   memset(&L, 0, sizeof(L));
   L.n = n; L.batch = batch; L.depth = depth; L.full = full;
-  L.key_bytes_sort = (3 * depth + bits_for(batch) <= 32) ? 4 : 8;
-  int64_t nvb = (n + kSortTile - 1) / kSortTile;       // one tile per CTA until the grid is 4 waves
-  if (nvb < 1) nvb = 1;
-  if (nvb > kSMs * 4) nvb = kSMs * 4;
-  int64_t vchunk = (n + nvb - 1) / nvb;
-  vchunk = (vchunk + kSortTile - 1) / kSortTile * kSortTile;
-  nvb = (n + vchunk - 1) / vchunk;                   // drop chunks the rounding left empty
-  L.nvb = (int)nvb;
-  L.vchunk = (int)vchunk;
+  L.key_bytes = (3 * depth + bits_for(batch) <= 32) ? 4 : 8;
+  // 9-bit digits where they save a pass over 8-bit ones (depth 6: two passes instead of three,
+  // depth 9: three instead of four)
+  const int p8 = (3 * depth + 7) / 8, p9 = (3 * depth + 8) / 9;
+  L.radix_bits = p9 < p8 ? 9 : 8;
+  L.passes = p9 < p8 ? p9 : p8;
+  const int bins = 1 << L.radix_bits;
+  L.max_chunks = (int)(n / chunk_points(n)) + batch;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes); return at; };
-  L.off_offsets = take(sizeof(CloudRef) * (size_t)(batch + 1));
+  L.off_clouds = take(sizeof(CloudRef) * (size_t)(batch + 1));
   L.off_counts = take(sizeof(int) * 32);
-  L.off_blockcnt = take(sizeof(int) * kMaxScanGrid);
-  L.off_hist = take(sizeof(int) * 256 * (size_t)L.nvb);
-  L.off_bintot = take(sizeof(int) * 256 * 8);      // one row of digit totals per sort pass (<= 8)
-  for (int i = 0; i < 2; ++i) L.off_keys[i] = take((size_t)L.key_bytes_sort * (size_t)n);
+  L.off_bintot = take(sizeof(int) * (size_t)bins * batch * L.passes);   // digit totals per pass and cloud
+  L.zero_bytes = o - L.off_counts;
+  L.off_blockcnt = take(sizeof(int) * kMaxScanGrid * (OCNN_MAX_DEPTH + 1));
+  L.off_hist = take(sizeof(int) * (size_t)bins * L.max_chunks);
+  for (int i = 0; i < 2; ++i) L.off_keys[i] = take((size_t)L.key_bytes * (size_t)n);
   for (int i = 0; i < 2; ++i) L.off_idx[i] = take(sizeof(uint32_t) * (size_t)n);
   for (int d = full; d <= depth; ++d) {
     int64_t full_nodes = d >= 20 ? INT64_MAX : (int64_t)batch << (3 * d);
     L.cap[d] = n < full_nodes ? n : full_nodes;
-    L.off_K[d] = take(sizeof(uint64_t) * (size_t)L.cap[d]);
+    L.off_K[d] = take((size_t)L.key_bytes * (size_t)L.cap[d]);
     // start[d][a]: first entry, in the list below Kd (K(d+1), or the sorted points for d = depth),
     // that belongs to node a of Kd
     L.off_start[d] = take(sizeof(int) * (size_t)(L.cap[d] + 1));
   }
+  L.off_avg = take(3 * sizeof(float) * (size_t)L.cap[depth]);   // averaged normals of the finest nodes
   L.total = o;
   return L;
 }
@@ -109,114 +128,161 @@ __device__ __forceinline__ uint64_t spread3(uint32_t v) {
   return x;
 }
 
-struct EncodeArgs {
-  const CloudRef* clouds;   // device table, batch + 1 entries
-  int batch, depth;
-  long long n;
-  float bbmin[3];
-  float mul;
-};
-
-__device__ __forceinline__ int cloud_of(const CloudRef* clouds, int batch, long long i) {
-  int lo = 0, hi = batch;          // clouds[lo].offset <= i < clouds[hi].offset
+// The cloud that sort chunk `chunk` belongs to.
+__device__ __forceinline__ int cloud_of_chunk(const CloudRef* clouds, int batch, int chunk) {
+  int lo = 0, hi = batch;          // clouds[lo].chunk0 <= chunk < clouds[hi].chunk0
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (clouds[mid].offset <= i) lo = mid; else hi = mid;
+    if (clouds[mid].chunk0 <= chunk) lo = mid; else hi = mid;
   }
   return lo;
 }
 
-// normalize_pts + sort_keys' key computation (octree.cpp:155-170, 180-186): cell = trunc((p -
-// bbmin) * mul), only `depth` bits per axis enter the key.
-template <typename KeyT>
-__global__ void encode_kernel(EncodeArgs a, KeyT* __restrict__ keys, int* __restrict__ bintot,
-                              int bintot_n) {
-  grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
-  // the sort's per-pass digit totals start at zero (the histogram kernels add into them)
-  if (blockIdx.x == 0)
-    for (int i = threadIdx.x; i < bintot_n; i += blockDim.x) bintot[i] = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int b = cloud_of(a.clouds, a.batch, i);
-    const float* xyz = a.clouds[b].xyz + 3 * (i - a.clouds[b].offset);
-    const uint32_t mask = (1u << a.depth) - 1u;
-    uint32_t c[3];
+// One chunk of one cloud: its points, and where its digit counts go (hist holds, cloud by cloud, a
+// [digit][chunk of the cloud] table).
+struct Chunk {
+  int cloud, first, chunks;        // cloud, index inside it, the cloud's number of chunks
+  long long beg, end;
+};
+__device__ __forceinline__ Chunk chunk_of(const CloudRef* clouds, int batch, int chunk_pts) {
+  Chunk c;
+  c.cloud = cloud_of_chunk(clouds, batch, blockIdx.x);
+  const CloudRef a = clouds[c.cloud];
+  const long long next = clouds[c.cloud + 1].offset;
+  c.first = (int)blockIdx.x - a.chunk0;
+  c.chunks = clouds[c.cloud + 1].chunk0 - a.chunk0;
+  c.beg = a.offset + (long long)c.first * chunk_pts;
+  c.end = c.beg + chunk_pts < next ? c.beg + chunk_pts : next;
+  return c;
+}
+
+// Per-warp digit counters of a CTA, summed and published: hist gets the chunk's counts, bintot the
+// cloud's totals (integer additions: their order does not matter).
+template <int RB>
+__device__ __forceinline__ void publish_counts(int (&sh)[kWarps][1 << RB], const Chunk& c, int chunk0,
+                                               int* __restrict__ hist, int* __restrict__ bintot) {
+  constexpr int kBins = 1 << RB;
+  __syncthreads();
+  int* to = hist + (long long)chunk0 * kBins + c.first;
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const float s = (xyz[j] - a.bbmin[j]) * a.mul;
-      c[j] = (uint32_t)s & mask;
-    }
-    const uint64_t key = (spread3(c[0]) << 2) | (spread3(c[1]) << 1) | spread3(c[2]);
-    keys[i] = (KeyT)(((uint64_t)b << (3 * a.depth)) | key);
+  for (int d = threadIdx.x; d < kBins; d += kThreads) {
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) total += sh[w][d];
+    to[(long long)d * c.chunks] = total;
+    if (total) atomicAdd(&bintot[c.cloud * kBins + d], total);
   }
+}
+
+// Adds one digit per lane to the warp's counters. Keys that are close in memory often share the
+// digit: a run of equal digits in consecutive lanes is added once, by its first lane.  Lanes without
+// a key pass `none`, which no counter has.
+__device__ __forceinline__ void count_digit(int* counters, int digit, int none) {
+  const int lane = threadIdx.x & 31;
+  const int prev = __shfl_up_sync(0xffffffffu, digit, 1);
+  const bool head = lane == 0 || prev != digit;
+  const unsigned heads = __ballot_sync(0xffffffffu, head);
+  if (head && digit != none) {
+    const unsigned later = lane == 31 ? 0u : (heads >> (lane + 1));
+    atomicAdd(&counters[digit], later ? __ffs(later) : 32 - lane);
+  }
+}
+
+struct EncodeArgs {
+  const CloudRef* table;    // device table (written by this kernel when the clouds ride along)
+  int inline_clouds;        // 1: `clouds` holds them
+  int batch, depth, chunk_pts;
+  float bbmin[3];
+  float mul;
+  CloudRef clouds[kInlineClouds + 1];
+};
+
+// normalize_pts + sort_keys' key computation (octree.cpp:155-170, 180-186): cell = trunc((p -
+// bbmin) * mul), only `depth` bits per axis enter the key.  One CTA per sort chunk, so the cloud is the
+// CTA's and the first sort pass's digits are counted on the way.
+template <typename KeyT, int RB>
+__global__ void __launch_bounds__(kThreads) encode_kernel(const __grid_constant__ EncodeArgs a,
+                                                          KeyT* __restrict__ keys, int* __restrict__ hist,
+                                                          int* __restrict__ bintot) {
+  __shared__ int sh[kWarps][1 << RB];
+  for (int d = threadIdx.x; d < (1 << RB); d += kThreads)
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) sh[w][d] = 0;
+  grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
+  const CloudRef* clouds = a.inline_clouds ? a.clouds : a.table;
+  if (a.inline_clouds && blockIdx.x == 0)
+    for (int i = threadIdx.x; i <= a.batch; i += kThreads) const_cast<CloudRef*>(a.table)[i] = a.clouds[i];
+  const Chunk c = chunk_of(clouds, a.batch, a.chunk_pts);
+  const float* xyz = clouds[c.cloud].xyz - 3 * clouds[c.cloud].offset;
+  const uint64_t top = (uint64_t)c.cloud << (3 * a.depth);
+  const uint32_t mask = (1u << a.depth) - 1u;
+  __syncthreads();
+  for (long long i0 = c.beg; i0 < c.end; i0 += 4 * kThreads) {
+    float p[4][3];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * kThreads + threadIdx.x;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) p[u][j] = i < c.end ? xyz[3 * i + j] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * kThreads + threadIdx.x;
+      uint32_t cell[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const float s = (p[u][j] - a.bbmin[j]) * a.mul;
+        cell[j] = (uint32_t)s & mask;
+      }
+      const uint64_t key = (spread3(cell[0]) << 2) | (spread3(cell[1]) << 1) | spread3(cell[2]);
+      if (i < c.end) keys[i] = (KeyT)(top | key);
+      count_digit(sh[threadIdx.x >> 5], i < c.end ? (int)(key & ((1 << RB) - 1)) : (1 << RB), 1 << RB);
+    }
+  }
+  publish_counts<RB>(sh, c, clouds[c.cloud].chunk0, hist, bintot);
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
-// ---- stable LSD radix sort, 8 bits per pass -------------------------------------------------------
-// Each CTA owns one contiguous chunk of the keys.  A pass is: per-CTA digit histogram -> exclusive
-// scan over (digit, CTA) -> stable scatter.  The scatter works in tiles of 2048 keys: every warp
-// ranks its 256 keys 32 at a time with match_any (stable inside the warp), the per-warp digit counts
+// ---- stable LSD radix sort, RB bits per pass, segmented by cloud -----------------------------------
+// Each CTA owns one chunk of one cloud.  A pass is: per-CTA digit histogram -> exclusive scan over
+// (digit, chunk) inside the cloud -> stable scatter.  The scatter works in tiles of 2048 keys: every
+// warp ranks its 256 keys 32 at a time with ballots (stable inside the warp), the per-warp digit counts
 // are prefixed across warps and digits, the tile is written to shared memory in digit order, and
 // only then copied out — consecutive threads then write consecutive global addresses of one digit
 // run, so the 4-byte scatter of the naive formulation becomes coalesced runs.
-template <typename KeyT>
+template <typename KeyT, int RB>
 __global__ void __launch_bounds__(kThreads) sort_hist_kernel(const KeyT* __restrict__ keys,
-                                                             long long n, int shift, int vchunk,
-                                                             int nvb, int* __restrict__ hist,
+                                                             const CloudRef* __restrict__ clouds, int batch,
+                                                             int chunk_pts, int shift, int* __restrict__ hist,
                                                              int* __restrict__ bintot) {
-  grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
   // one private histogram per warp (shared-memory atomics never cross warps), summed at the end
-  __shared__ int sh[kThreads / 32][256];
-  const int warp = threadIdx.x >> 5;
+  __shared__ int sh[kWarps][1 << RB];
+  for (int d = threadIdx.x; d < (1 << RB); d += kThreads)
 #pragma unroll
-  for (int w = 0; w < kThreads / 32; ++w) sh[w][threadIdx.x] = 0;
+    for (int w = 0; w < kWarps; ++w) sh[w][d] = 0;
+  grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
+  const Chunk c = chunk_of(clouds, batch, chunk_pts);
   __syncthreads();
-  const long long beg = (long long)blockIdx.x * vchunk;
-  long long end = beg + vchunk;
-  if (end > n) end = n;
-  // Eight keys per thread are requested before the first is counted.  Keys that are close in
-  // memory often share the digit (the input is sorted by the lower digits, and the top digit is
-  // the cloud index): a run of equal digits in consecutive lanes is added once, by its first lane.
-  const int lane = threadIdx.x & 31;
-  for (long long i0 = beg; i0 < end; i0 += 8 * kThreads) {
-    KeyT k[8];
+  for (long long i0 = c.beg; i0 < c.end; i0 += 8 * kThreads) {
+    KeyT k[8];                  // all requested before the first is counted
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const long long i = i0 + u * kThreads + threadIdx.x;
-      k[u] = i < end ? keys[i] : 0;
+      k[u] = i < c.end ? keys[i] : 0;
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const long long i = i0 + u * kThreads + threadIdx.x;
-      // lanes past the end carry digit 256, which no counted lane has
-      const int digit = i < end ? (int)((k[u] >> shift) & 255) : 256;
-      const int prev = __shfl_up_sync(0xffffffffu, digit, 1);
-      const bool head = lane == 0 || prev != digit;
-      const unsigned heads = __ballot_sync(0xffffffffu, head);
-      if (head && digit < 256) {
-        // the run ends before the next head (or at the end of the warp)
-        const unsigned later = lane == 31 ? 0u : (heads >> (lane + 1));
-        const int run = later ? __ffs(later) : 32 - lane;
-        atomicAdd(&sh[warp][digit], run);
-      }
+      count_digit(sh[threadIdx.x >> 5], i < c.end ? (int)((k[u] >> shift) & ((1 << RB) - 1)) : (1 << RB), 1 << RB);
     }
   }
-  __syncthreads();
-  int total = 0;
-#pragma unroll
-  for (int w = 0; w < kThreads / 32; ++w) total += sh[w][threadIdx.x];
-  hist[(long long)threadIdx.x * nvb + blockIdx.x] = total;
-  // digit totals over all CTAs (integer additions: the order does not matter); bintot was cleared
-  // by the encode kernel
-  if (total) atomicAdd(&bintot[threadIdx.x], total);
+  publish_counts<RB>(sh, c, clouds[c.cloud].chunk0, hist, bintot);
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
-// Exclusive scan of hist[256][nvb] in (digit, CTA) order: one CTA per digit row (sort_rowscan_kernel
-// below); the digit totals it starts from were accumulated by the histogram kernel.
 __device__ __forceinline__ int block_exclusive_scan(int v, int* total) {
   // exclusive prefix of v over the CTA's kThreads threads
-  __shared__ int wsum[kThreads / 32];
+  __shared__ int wsum[kWarps];
   __shared__ int wtot;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int inc = v;
@@ -228,45 +294,62 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* total) {
   if (lane == 31) wsum[warp] = inc;
   __syncthreads();
   if (warp == 0) {
-    int w = lane < kThreads / 32 ? wsum[lane] : 0;
+    int w = lane < kWarps ? wsum[lane] : 0;
     int winc = w;
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(0xffffffffu, winc, o);
       if (lane >= o) winc += t;
     }
-    if (lane < kThreads / 32) wsum[lane] = winc - w;
-    if (lane == kThreads / 32 - 1) wtot = winc;
+    if (lane < kWarps) wsum[lane] = winc - w;
+    if (lane == kWarps - 1) wtot = winc;
   }
   __syncthreads();
   *total = wtot;
   return inc - v + wsum[warp];
 }
 
-__global__ void __launch_bounds__(kThreads) sort_rowscan_kernel(int* __restrict__ hist, int nvb,
+// Exclusive scan of every cloud's hist[digit][chunk] in that order, starting at the cloud's first
+// point: one warp per (cloud, digit) row.
+template <int RB>
+__global__ void __launch_bounds__(kThreads) sort_rowscan_kernel(int* __restrict__ hist,
+                                                                const CloudRef* __restrict__ clouds, int batch,
                                                                 const int* __restrict__ bintot) {
+  constexpr int kBins = 1 << RB;
   grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
-  // first slot of this digit = number of keys with a smaller digit (kThreads == 256 digits)
-  int below_total;
-  block_exclusive_scan(threadIdx.x < blockIdx.x ? bintot[threadIdx.x] : 0, &below_total);
-  int base = below_total;
-  int* row = hist + (long long)blockIdx.x * nvb;
-  for (int i0 = 0; i0 < nvb; i0 += kThreads) {
-    const int i = i0 + threadIdx.x;
-    const int v = i < nvb ? row[i] : 0;
-    int total;
-    const int ex = block_exclusive_scan(v, &total);
-    if (i < nvb) row[i] = base + ex;
-    base += total;
+  const int lane = threadIdx.x & 31;
+  const long long row = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+  if (row < (long long)batch * kBins) {
+    const int b = (int)(row >> RB), digit = (int)(row & (kBins - 1));
+    const CloudRef c = clouds[b];
+    const int chunks = clouds[b + 1].chunk0 - c.chunk0;
+    // first slot of this digit = number of the cloud's keys with a smaller digit
+    int below = 0;
+    for (int d = lane; d < digit; d += 32) below += bintot[b * kBins + d];
+    for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
+    int base = (int)c.offset + below;
+    int* at = hist + (long long)c.chunk0 * kBins + (long long)digit * chunks;
+    for (int i0 = 0; i0 < chunks; i0 += 32) {
+      const int i = i0 + lane;
+      const int v = i < chunks ? at[i] : 0;
+      int inc = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+      }
+      if (i < chunks) at[i] = base + inc - v;
+      base += __shfl_sync(0xffffffffu, inc, 31);
+    }
   }
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
-// The lanes of `mask` whose 8-bit digit equals this lane's: eight ballots, one per bit.  (Measured
-// several times faster here than match.any, which the histogram used to spend most of its time in.)
+// The lanes of `mask` whose RB-bit digit equals this lane's: one ballot per bit.  (Measured several
+// times faster here than match.any.)
+template <int RB>
 __device__ __forceinline__ unsigned match_digit(unsigned mask, int digit) {
   unsigned peers = mask;
 #pragma unroll
-  for (int b = 0; b < 8; ++b) {
+  for (int b = 0; b < RB; ++b) {
     const bool bit = (digit >> b) & 1;
     const unsigned with = __ballot_sync(mask, bit);
     peers &= bit ? with : ~with;
@@ -274,27 +357,33 @@ __device__ __forceinline__ unsigned match_digit(unsigned mask, int digit) {
   return peers;
 }
 
-template <typename KeyT, bool FIRST>
+template <typename KeyT, bool FIRST, int RB>
 __global__ void __launch_bounds__(kThreads) sort_scatter_kernel(
     const KeyT* __restrict__ keys_in, const uint32_t* __restrict__ idx_in,
-    KeyT* __restrict__ keys_out, uint32_t* __restrict__ idx_out, long long n, int shift,
-    int vchunk, int nvb, const int* __restrict__ hist) {
-  grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
-  constexpr int kWarps = kThreads / 32;
-  __shared__ int cnt[kWarps][256];        // per-warp digit counts, then per-warp digit bases
-  __shared__ int tile_start[256];         // first slot of each digit inside the sorted tile
-  __shared__ int gofs[256];               // next global slot of each digit for this CTA
+    KeyT* __restrict__ keys_out, uint32_t* __restrict__ idx_out, const CloudRef* __restrict__ clouds, int batch,
+    int chunk_pts, int shift, const int* __restrict__ hist) {
+  constexpr int kBins = 1 << RB, kPer = kBins / kThreads;     // digits per thread: 1 or 2, neighbours
+  __shared__ int cnt[kWarps][kBins];      // per-warp digit counts, then per-warp digit bases
+  __shared__ int tile_start[kBins];       // first slot of each digit inside the sorted tile
+  __shared__ int gofs[kBins];             // next global slot of each digit for this CTA
   __shared__ KeyT skey[kSortTile];
   __shared__ uint32_t sidx[kSortTile];
+  grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  gofs[threadIdx.x] = hist[(long long)threadIdx.x * nvb + blockIdx.x];
-  const long long beg = (long long)blockIdx.x * vchunk;
-  long long end = beg + vchunk;
-  if (end > n) end = n;
-  for (long long t0 = beg; t0 < end; t0 += kSortTile) {
-    const int tile_n = (int)((end - t0) < kSortTile ? (end - t0) : kSortTile);
+  const Chunk c = chunk_of(clouds, batch, chunk_pts);
+  {
+    const int* from = hist + (long long)clouds[c.cloud].chunk0 * kBins + c.first;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) cnt[w][threadIdx.x] = 0;
+    for (int q = 0; q < kPer; ++q) {
+      const int d = threadIdx.x * kPer + q;
+      gofs[d] = from[(long long)d * c.chunks];
+    }
+  }
+  for (long long t0 = c.beg; t0 < c.end; t0 += kSortTile) {
+    const int tile_n = (int)((c.end - t0) < kSortTile ? (c.end - t0) : kSortTile);
+    for (int d = threadIdx.x; d < kBins; d += kThreads)
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) cnt[w][d] = 0;
     __syncthreads();
     // 1. rank inside the warp's 256 keys (index order = rank order: stable)
     KeyT key[kSortItems];
@@ -317,8 +406,8 @@ __global__ void __launch_bounds__(kThreads) sort_scatter_kernel(
       const unsigned mask = __ballot_sync(0xffffffffu, valid);
       rank[r] = -1;
       if (valid) {
-        const int digit = (int)((key[r] >> shift) & 255);
-        const unsigned peers = match_digit(mask, digit);
+        const int digit = (int)((key[r] >> shift) & (kBins - 1));
+        const unsigned peers = match_digit<RB>(mask, digit);
         const int before = __popc(peers & ((1u << lane) - 1));
         rank[r] = cnt[warp][digit] + before;
         __syncwarp(mask);
@@ -327,23 +416,34 @@ __global__ void __launch_bounds__(kThreads) sort_scatter_kernel(
       __syncwarp();
     }
     __syncthreads();
-    // 2. thread d: prefix digit d over the warps, then over the digits
-    int total_d = 0;
+    // 2. every thread: prefix its digits over the warps, then over the digits
+    int total_d[kPer], sum = 0;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const int c = cnt[w][threadIdx.x];
-      cnt[w][threadIdx.x] = total_d;
-      total_d += c;
+    for (int q = 0; q < kPer; ++q) {
+      const int d = threadIdx.x * kPer + q;
+      int t = 0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const int v = cnt[w][d];
+        cnt[w][d] = t;
+        t += v;
+      }
+      total_d[q] = t;
+      sum += t;
     }
     int tile_total;
-    const int start_d = block_exclusive_scan(total_d, &tile_total);
-    tile_start[threadIdx.x] = start_d;
+    int start_d = block_exclusive_scan(sum, &tile_total);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      tile_start[threadIdx.x * kPer + q] = start_d;
+      start_d += total_d[q];
+    }
     __syncthreads();
     // 3. tile into shared memory in digit order
 #pragma unroll
     for (int r = 0; r < kSortItems; ++r) {
       if (rank[r] >= 0) {
-        const int digit = (int)((key[r] >> shift) & 255);
+        const int digit = (int)((key[r] >> shift) & (kBins - 1));
         const int pos = tile_start[digit] + cnt[warp][digit] + rank[r];
         skey[pos] = key[r];
         sidx[pos] = idx[r];
@@ -353,116 +453,206 @@ __global__ void __launch_bounds__(kThreads) sort_scatter_kernel(
     // 4. copy out: slot i of the sorted tile goes to gofs[digit] + (i - tile_start[digit])
     for (int i = threadIdx.x; i < tile_n; i += kThreads) {
       const KeyT k = skey[i];
-      const int digit = (int)((k >> shift) & 255);
+      const int digit = (int)((k >> shift) & (kBins - 1));
       const long long pos = (long long)gofs[digit] + (i - tile_start[digit]);
       keys_out[pos] = k;
       idx_out[pos] = sidx[i];
     }
     __syncthreads();
-    gofs[threadIdx.x] += total_d;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) gofs[threadIdx.x * kPer + q] += total_d[q];
     __syncthreads();
   }
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
-// ---- segmented unique (reduce, then scan) ---------------------------------------------------------
-// out = unique(in >> shift) for sorted `in`; start[a] = first i with (in[i] >> shift) == out[a];
-// start[count] = n; *count_out = count.  n is read from n_ptr when given (a count produced on the
-// device by the previous stage).
-template <typename InT>
-__device__ __forceinline__ bool is_head(const InT* __restrict__ in, long long i, int shift) {
-  return i == 0 || (in[i] >> shift) != (in[i - 1] >> shift);
+// ---- unique for every level at once (reduce, then scan) -------------------------------------------
+// In the sorted composite keys, point i opens a new node at level d iff its key differs from the one
+// before it above bit 3 (depth - d); a node opened at one level opens one at every finer level too,
+// so a point is described by the coarsest level it opens (`levels` = none).  Level l = 0 is the full
+// level, l = levels - 1 the finest.  K_l[rank] = key >> 3 (levels - 1 - l), start_l[rank] = the rank the
+// same point has one level finer (the point itself at the finest), so that a node's children are
+// start_l[a] .. start_l[a + 1].
+template <typename KeyT>
+struct UniqueArgs {
+  const KeyT* keys;
+  long long n;
+  int depth, full, levels;
+  int* blockcnt;            // [levels][blocks]
+  int* counts;              // by depth
+  int* host_counts;         // the same in mapped host memory
+  KeyT* K[OCNN_MAX_DEPTH + 1];
+  int* start[OCNN_MAX_DEPTH + 1];
+};
+
+__device__ __forceinline__ int top_bit(uint32_t v) { return 31 - __clz(v); }
+__device__ __forceinline__ int top_bit(uint64_t v) { return 63 - __clzll((long long)v); }
+
+template <typename KeyT>
+__device__ __forceinline__ int opened_level(const UniqueArgs<KeyT>& a, KeyT key, KeyT prev, bool first) {
+  if (first) return 0;
+  const KeyT x = key ^ prev;
+  if (x == 0) return a.levels;
+  const int l = a.depth - top_bit(x) / 3 - a.full;
+  return l < 0 ? 0 : l;
 }
 
 __device__ __forceinline__ void scan_range(long long n, long long* beg, long long* end) {
   long long chunk = (n + gridDim.x - 1) / gridDim.x;
   chunk = (chunk + kScanTile - 1) / kScanTile * kScanTile;
   *beg = (long long)blockIdx.x * chunk;
-  long long e = *beg + chunk;
+  if (*beg > n) *beg = n;
+  const long long e = *beg + chunk;
   *end = e < n ? e : n;
 }
 
-template <typename InT>
-__global__ void __launch_bounds__(kThreads) unique_count_kernel(const InT* __restrict__ in,
-                                                                const int* __restrict__ n_ptr,
-                                                                long long n_host, int shift,
-                                                                int* __restrict__ blockcnt) {
+// Four consecutive keys per thread (16-byte reads of 32-bit keys) and the key before them.
+template <typename KeyT>
+__device__ __forceinline__ void load_items(const UniqueArgs<KeyT>& a, long long i0, long long end,
+                                           KeyT (&key)[kScanItems], int (&lvl)[kScanItems]) {
+  KeyT prev = (i0 > 0 && i0 < end) ? a.keys[i0 - 1] : 0;
+  if (sizeof(KeyT) == 4 && i0 + kScanItems <= end) {
+    const uint4 q = *reinterpret_cast<const uint4*>(a.keys + i0);
+    key[0] = (KeyT)q.x; key[1] = (KeyT)q.y; key[2] = (KeyT)q.z; key[3] = (KeyT)q.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) key[k] = i0 + k < end ? a.keys[i0 + k] : 0;
+  }
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    lvl[k] = i0 + k < end ? opened_level(a, key[k], prev, i0 + k == 0) : a.levels;
+    prev = key[k];
+  }
+}
+
+template <typename KeyT, int LV>       // LV: bound on the levels
+__global__ void __launch_bounds__(kThreads) unique_count_kernel(const __grid_constant__ UniqueArgs<KeyT> a) {
+  __shared__ int red[kWarps][LV];
   grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
-  __shared__ int red[kThreads / 32];
-  const long long n = n_ptr ? (long long)*n_ptr : n_host;
   long long beg, end;
-  scan_range(n, &beg, &end);
-  int c = 0;
-  for (long long i = beg + threadIdx.x; i < end; i += kThreads) c += is_head(in, i, shift) ? 1 : 0;
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
+  scan_range(a.n, &beg, &end);
+  int cnt[LV];
+#pragma unroll
+  for (int l = 0; l < LV; ++l) cnt[l] = 0;
+  for (long long t0 = beg; t0 < end; t0 += kScanTile) {
+    KeyT key[kScanItems];
+    int lvl[kScanItems];
+    load_items(a, t0 + (long long)threadIdx.x * kScanItems, end, key, lvl);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k)
+#pragma unroll
+      for (int l = 0; l < LV; ++l) cnt[l] += (lvl[k] <= l && lvl[k] < a.levels) ? 1 : 0;
+  }
+#pragma unroll
+  for (int l = 0; l < LV; ++l) {
+    for (int o = 16; o > 0; o >>= 1) cnt[l] += __shfl_down_sync(0xffffffffu, cnt[l], o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][l] = cnt[l];
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < a.levels) {
     int t = 0;
-    for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-    blockcnt[blockIdx.x] = t;
+    for (int w = 0; w < kWarps; ++w) t += red[w][threadIdx.x];
+    a.blockcnt[threadIdx.x * gridDim.x + blockIdx.x] = t;
   }
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
-template <typename InT>
-__global__ void __launch_bounds__(kThreads) unique_compact_kernel(
-    const InT* __restrict__ in, const int* __restrict__ n_ptr, long long n_host, int shift,
-    const int* __restrict__ blockcnt, uint64_t* __restrict__ out, int* __restrict__ start,
-    int* __restrict__ count_out) {
+template <typename KeyT, int LV>
+__global__ void __launch_bounds__(kThreads) unique_compact_kernel(const __grid_constant__ UniqueArgs<KeyT> a) {
+  constexpr int W = (LV + 1) / 2;         // two levels' counts per word, 16 bits each (a tile has 1024 keys)
+  __shared__ int s_base[LV];              // nodes of the level in all tiles before this one
+  __shared__ unsigned s_warp[kWarps][W];
   grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
-  __shared__ int red[kThreads / 32];
-  __shared__ int base_s;
-  const long long n = n_ptr ? (long long)*n_ptr : n_host;
-  // base = heads in all lower blocks
-  int c = 0;
-  for (int g = threadIdx.x; g < (int)blockIdx.x; g += kThreads) c += blockcnt[g];
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-    base_s = t;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int l = warp; l < a.levels; l += kWarps) {
+    int c = 0;
+    for (int g = lane; g < (int)blockIdx.x; g += 32) c += a.blockcnt[l * gridDim.x + g];
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if (lane == 0) s_base[l] = c;
   }
   __syncthreads();
-  int base = base_s;
   long long beg, end;
-  scan_range(n, &beg, &end);
+  scan_range(a.n, &beg, &end);
   for (long long t0 = beg; t0 < end; t0 += kScanTile) {
     const long long i0 = t0 + (long long)threadIdx.x * kScanItems;
-    bool head[kScanItems];
-    int local = 0;
+    KeyT key[kScanItems];
+    int lvl[kScanItems];
+    load_items(a, i0, end, key, lvl);
+    unsigned own[W], inc[W];
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      head[k] = (i0 + k < end) && is_head(in, i0 + k, shift);
-      local += head[k] ? 1 : 0;
-    }
-    int total;
-    int at = base + block_exclusive_scan(local, &total);
+    for (int w = 0; w < W; ++w) {
+      own[w] = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      if (head[k]) {
-        out[at] = (uint64_t)(in[i0 + k] >> shift);
-        start[at] = (int)(i0 + k);
-        ++at;
+      for (int k = 0; k < kScanItems; ++k)
+        if (lvl[k] < a.levels)
+          own[w] += (lvl[k] <= 2 * w ? 1u : 0u) + (lvl[k] <= 2 * w + 1 ? 0x10000u : 0u);
+      inc[w] = own[w];
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, inc[w], o);
+        if (lane >= o) inc[w] += t;
       }
+      if (lane == 31) s_warp[warp][w] = inc[w];
     }
-    base += total;
+    __syncthreads();
+    int rank[LV];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      unsigned before = inc[w] - own[w];
+      for (int v = 0; v < warp; ++v) before += s_warp[v][w];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (2 * w + h < LV) rank[2 * w + h] = (2 * w + h < a.levels ? s_base[2 * w + h] : 0) +
+                                              (int)((before >> (16 * h)) & 0xffffu);
+    }
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      if (lvl[k] >= a.levels) continue;
+#pragma unroll
+      for (int l = 0; l < LV; ++l) {
+        if (l < lvl[k] || l >= a.levels) continue;
+        a.K[l][rank[l]] = key[k] >> (3 * (a.levels - 1 - l));
+        a.start[l][rank[l]] = l == a.levels - 1 ? (int)(i0 + k) : rank[l + 1 < LV ? l + 1 : l];
+      }
+#pragma unroll
+      for (int l = 0; l < LV; ++l)
+        if (l >= lvl[k]) ++rank[l];
+    }
+    __syncthreads();
+    if (threadIdx.x < a.levels) {
+      unsigned t = 0;
+      for (int v = 0; v < kWarps; ++v) t += (s_warp[v][threadIdx.x >> 1] >> (16 * (threadIdx.x & 1))) & 0xffffu;
+      s_base[threadIdx.x] += (int)t;
+    }
+    __syncthreads();
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
-    *count_out = base;
-    start[base] = (int)n;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x < a.levels) {
+    const int l = threadIdx.x, c = s_base[l];
+    a.counts[a.full + l] = c;
+    a.host_counts[a.full + l] = c;
+    a.start[l][c] = l == a.levels - 1 ? (int)a.n : s_base[l + 1];
   }
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
 // ---- emit ------------------------------------------------------------------------------------
-struct EmitLevelArgs {
-  uint8_t* out;               // octree buffer
+struct EmitLevel {
   long long off_key, off_child, off_split;   // byte offsets of this level (split < 0: absent)
-  int key_bytes;
-  int d;
+  long long nnum;
+  const void* Kp;            // K(d-1), levels above the full ones only
+  const void* Kc;            // Kd
+  const int* start;          // first entry of Kc under each parent
+  int d, block0;             // first block of the level
+};
+struct EmitAll {
+  uint8_t* out;              // octree buffer
+  int nlev, batch, full, depth, key_bytes;
+  const void* K_full;        // the full level's non-empty nodes, for its children
+  const int* count_full;
+  float* feat;               // finest level's feature block, [channels, nnum]; NULL: written elsewhere
+  int channels;
+  const float* avg[6];       // a channel's values on the non-empty finest nodes
+  EmitLevel lev[OCNN_MAX_DEPTH + 1];
+  uint8_t header[OCNN_HEADER_BYTES];
 };
 
 __device__ __forceinline__ void store_key(uint8_t* base, long long off, long long i, uint64_t local,
@@ -476,89 +666,101 @@ __device__ __forceinline__ void store_key(uint8_t* base, long long off, long lon
   }
 }
 
-// levels 0..full: every node exists; key = index inside its octree; child = itself below the
-// full level, -1 at the full level (filled from K_full afterwards) — octree.cpp:210-224.
-// All levels in one launch: a block serves one level (EmitAll::block0 is the first block of each).
-struct EmitAll {
-  int nlev, batch, full;
-  int block0[OCNN_MAX_DEPTH + 2];
-  long long nnum[OCNN_MAX_DEPTH + 1];
-  EmitLevelArgs a[OCNN_MAX_DEPTH + 1];
-  const uint64_t* Kp[OCNN_MAX_DEPTH + 1];     // K(d-1), levels above the full ones only
-  const uint64_t* Kc[OCNN_MAX_DEPTH + 1];     // Kd
-  const int* start[OCNN_MAX_DEPTH + 1];       // first entry of Kc under each parent
-};
+constexpr int kEmitNodes = kThreads * 8;      // nodes per block: 32 parents per warp
 
-__device__ __forceinline__ void emit_full_node(const EmitLevelArgs& a, long long i, int batch, int full) {
-  const long long per = 1LL << (3 * a.d);
-  const int b = (int)(i / per);
-  store_key(a.out, a.off_key, i, (uint64_t)(i - b * per), b, a.key_bytes);
-  const int ch = a.d < full ? (int)i : -1;
-  reinterpret_cast<int*>(a.out + a.off_child)[i] = ch;
-  if (a.off_split >= 0) reinterpret_cast<float*>(a.out + a.off_split)[i] = ch < 0 ? 0.f : 1.f;
-}
-
-// children of the full level: the composite key of a level-`full` node IS its batch-wide node
-// index, so child[K_full[r]] = r (octree.cpp:277-282 + the rebasing of merge_octrees.cpp:136-144).
-__global__ void emit_full_children_kernel(EmitLevelArgs a, const uint64_t* __restrict__ K,
-                                          const int* __restrict__ count) {
+// All levels in one launch, a block serves one level.
+// Levels 0..full hold every node: key = index inside its octree, child = itself below the full level
+// (octree.cpp:210-224); at the full level the rank of the node in K_full, whose composite key IS the
+// batch-wide node index (octree.cpp:277-282 + the rebasing of merge_octrees.cpp:136-144).
+// Level d > full: node 8a+j is the j-th child slot of the a-th non-empty node of level d-1
+// (octree.cpp:226-273).  A lane fetches one parent and the octants of its children as a bit mask; its
+// 8 nodes are then written by the warp 32 at a time, in order.  Everything a warp's 256 nodes need is
+// requested before the first of them is written (one node per thread was a chain of three reads per
+// 12 bytes written: 258 us for 23 M nodes).
+template <typename KeyT>
+__global__ void __launch_bounds__(kThreads) emit_levels_kernel(const __grid_constant__ EmitAll A) {
   grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
-  const int n = *count;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    const long long node = (long long)K[r];
-    reinterpret_cast<int*>(a.out + a.off_child)[node] = r;
-    if (a.off_split >= 0) reinterpret_cast<float*>(a.out + a.off_split)[node] = 1.f;
-  }
-  grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
-}
-
-// level d > full: node 8a+j is the j-th child slot of the a-th non-empty node of level d-1
-// (octree.cpp:226-273).  Kp = K(d-1), Kc = Kd, start = first entry of Kc under each parent.
-__global__ void __launch_bounds__(kThreads) emit_levels_kernel(const EmitAll A) {
-  grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
-  int l = 0;
-  while (l + 1 < A.nlev && (int)blockIdx.x >= A.block0[l + 1]) ++l;
-  const EmitLevelArgs& a = A.a[l];
-  const long long i = (long long)((int)blockIdx.x - A.block0[l]) * kThreads + threadIdx.x;
-  if (i >= A.nnum[l]) return;          // (whole sibling groups leave together: nnum is a multiple of 8)
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < OCNN_HEADER_BYTES / 4; i += kThreads)
+      reinterpret_cast<int*>(A.out)[i] = reinterpret_cast<const int*>(A.header)[i];
+  int li = 0;
+  while (li + 1 < A.nlev && (int)blockIdx.x >= A.lev[li + 1].block0) ++li;
+  const EmitLevel& a = A.lev[li];
+  const int lane = threadIdx.x & 31;
+  const long long i0 = (long long)((int)blockIdx.x - a.block0) * kEmitNodes;
+  int* child = reinterpret_cast<int*>(A.out + a.off_child);
+  float* split = a.off_split >= 0 ? reinterpret_cast<float*>(A.out + a.off_split) : nullptr;
+  const bool with_feat = A.feat != nullptr && a.d == A.depth;
   if (a.d <= A.full) {
-    emit_full_node(a, i, A.batch, A.full);
-    return;
-  }
-  const uint64_t* __restrict__ Kp = A.Kp[l];
-  const uint64_t* __restrict__ Kc = A.Kc[l];
-  const int* __restrict__ start = A.start[l];
-  const uint64_t local_mask = (1ULL << (3 * (a.d - 1))) - 1ULL;
-  const long long p = i >> 3;
-  const int j = (int)(i & 7);
-  const uint64_t pk = Kp[p];
-  const int b = (int)(pk >> (3 * (a.d - 1)));
-  store_key(a.out, a.off_key, i, ((pk & local_mask) << 3) | (uint64_t)j, b, a.key_bytes);
-  // The group's children are the s1 - s0 <= 8 keys Kc[s0..s1): lane j of the group's 8 lanes
-  // fetches Kc[s0 + j], and each lane then picks, among the group's lanes, the one whose key
-  // ends in its own octant.  (A level above the full ones holds whole sibling groups and a block
-  // starts on a multiple of 8, so the 8 lanes of a group always run together.)
-  const int s0 = start[p], s1 = start[p + 1];
-  const int mine = s0 + j < s1 ? (int)(Kc[s0 + j] & 7) : -1;
-  const unsigned group_mask = 0xffu << (threadIdx.x & 24);
-  int ch = -1;
+    const long long per = 1LL << (3 * a.d);
+    const KeyT* K = static_cast<const KeyT*>(A.K_full);
+    const int nk = a.d == A.full && K != nullptr ? *A.count_full : 0;
+    for (long long i = i0 + threadIdx.x; i < i0 + kEmitNodes && i < a.nnum; i += kThreads) {
+      const int b = (int)(i / per);
+      store_key(A.out, a.off_key, i, (uint64_t)(i - b * per), b, A.key_bytes);
+      int ch = a.d < A.full ? (int)i : -1;
+      if (nk > 0) {
+        int lo = 0, hi = nk;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if ((long long)K[mid] < i) lo = mid + 1; else hi = mid;
+        }
+        if (lo < nk && (long long)K[lo] == i) ch = lo;
+      }
+      child[i] = ch;
+      if (split) split[i] = ch < 0 ? 0.f : 1.f;
+      if (with_feat)            // (the full level is the finest: no node has a signal)
+        for (int c = 0; c < A.channels; ++c) A.feat[c * a.nnum + i] = 0.f;
+    }
+  } else {
+    const KeyT* __restrict__ Kp = static_cast<const KeyT*>(a.Kp);
+    const KeyT* __restrict__ Kc = static_cast<const KeyT*>(a.Kc);
+    const long long w0 = i0 + (threadIdx.x & ~31) * 8;          // the warp's first node
+    const long long p = (w0 >> 3) + lane, np = a.nnum >> 3;
+    KeyT pk = 0;
+    int s0 = 0, s1 = 0;
+    if (p < np) {
+      pk = Kp[p];
+      s0 = a.start[p];
+      s1 = a.start[p + 1];
+    }
+    unsigned octants = 0;
 #pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const int oct = __shfl_sync(group_mask, mine, u, 8);
-    if (oct == j) ch = s0 + u;
+    for (int u = 0; u < 8; ++u)
+      if (s0 + u < s1) octants |= 1u << (int)(Kc[s0 + u] & 7);
+    const uint64_t local_mask = (1ULL << (3 * (a.d - 1))) - 1ULL;
+    const int o = lane & 7;
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const long long i = w0 + it * 32 + lane;
+      const int src = it * 4 + (lane >> 3);
+      const KeyT key = __shfl_sync(0xffffffffu, pk, src);
+      const int first = __shfl_sync(0xffffffffu, s0, src);
+      const unsigned have = __shfl_sync(0xffffffffu, octants, src);
+      if (i >= a.nnum) continue;       // (whole sibling groups leave together; shuffles precede)
+      const int ch = (have >> o) & 1 ? first + __popc(have & ((1u << o) - 1)) : -1;
+      store_key(A.out, a.off_key, i, (((uint64_t)key & local_mask) << 3) | (uint64_t)o,
+                (int)((uint64_t)key >> (3 * (a.d - 1))), A.key_bytes);
+      child[i] = ch;
+      if (split) split[i] = ch < 0 ? 0.f : 1.f;
+      if (with_feat) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c)
+          if (c < A.channels) A.feat[c * a.nnum + i] = ch < 0 ? 0.f : A.avg[c][ch];
+      }
+    }
   }
-  reinterpret_cast<int*>(a.out + a.off_child)[i] = ch;
-  if (a.off_split >= 0) reinterpret_cast<float*>(a.out + a.off_split)[i] = ch < 0 ? 0.f : 1.f;
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
 // finest-level signal, octree.cpp:312-452 restated per node.  Rows of the feature block, in
 // order: normals, displacement, point features, average points (octree.cpp:916-926).
+template <typename KeyT>
 struct SignalArgs {
   const int* child;          // level `depth` children = index into seg
   const int* seg;            // point segment starts per non-empty finest node
   const uint32_t* sorted_idx;
-  const uint64_t* K;         // composite keys of the non-empty finest nodes (cloud in the top bits)
+  const KeyT* K;             // composite keys of the non-empty finest nodes (cloud in the top bits)
   const CloudRef* clouds;
   int depth;
   int has_normal, has_feat;
@@ -568,86 +770,85 @@ struct SignalArgs {
   int cf, node_dis, save_pts;
   float bbmin[3];
   float mul;
+  float* avg[6];             // signal_average_kernel: where each channel goes
+  int nodes;                 // ... and the number of non-empty nodes
 };
 
-// The common case — normals only, no displacement, point features, labels or average points —
-// with four nodes per thread in lock step: child, then segment + key, then the first point's
-// index, then its normal are each requested for all four nodes before any is used, so a thread has
-// four dependent-load chains in flight instead of one (with one chain the grid-stride loop of the
-// general kernel below is a latency loop: ~5 dependent reads per node).  The arithmetic and its
-// order are those of the general kernel, so the results are bit-identical.
-__global__ void __launch_bounds__(256) signal_normals_kernel(SignalArgs a) {
+// Normals and / or point features (no displacement, labels or average points), averaged per
+// non-empty node into compact arrays that the emit kernel spreads over the level's nodes.  Two nodes
+// per thread in lock step, every stage of the chain segment -> point index -> values requested for
+// both before any is used.  The arithmetic and its order are signal_kernel's: bit-identical.
+template <typename KeyT>
+__global__ void __launch_bounds__(256) signal_average_kernel(const __grid_constant__ SignalArgs<KeyT> a) {
   grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
-  constexpr int U = 4;
-  const long long nn = a.nnum;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  float* f_normal = a.f_out;
-  for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < nn; i0 += stride * U) {
-    int t[U], s0[U], s1[U];
-    uint64_t key[U];
+  constexpr int U = 2;
+  const int stride = gridDim.x * blockDim.x;
+  for (int r0 = blockIdx.x * blockDim.x + threadIdx.x; r0 < a.nodes; r0 += stride * U) {
+    int s0[U], s1[U];
+    KeyT key[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + u * stride;
+      s0[u] = s1[u] = 0;
+      key[u] = 0;
+      if (r < a.nodes) { s0[u] = a.seg[r]; s1[u] = a.seg[r + 1]; key[u] = a.K[r]; }
+    }
     long long h0[U];
     const float* normals[U];
+    const float* feats[U];
     long long base[U];
-    float first[U][3];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const long long i = i0 + u * stride;
-      t[u] = i < nn ? a.child[i] : -2;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      s0[u] = 0; s1[u] = 0; key[u] = 0;
-      if (t[u] >= 0) { s0[u] = a.seg[t[u]]; s1[u] = a.seg[t[u] + 1]; key[u] = a.K[t[u]]; }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      h0[u] = 0; normals[u] = nullptr; base[u] = 0;
-      if (t[u] >= 0) {
-        const CloudRef cl = a.clouds[(int)(key[u] >> (3 * a.depth))];
+      h0[u] = 0; normals[u] = feats[u] = nullptr; base[u] = 0;
+      if (s1[u] > s0[u]) {
+        const CloudRef& cl = a.clouds[(int)((uint64_t)key[u] >> (3 * a.depth))];
         normals[u] = cl.normal;
+        feats[u] = cl.feat;
         base[u] = cl.offset;
         h0[u] = a.sorted_idx[s0[u]] - base[u];
       }
     }
+    float first[U][3];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) first[u][c] = (a.has_normal && s1[u] > s0[u]) ? normals[u][3 * h0[u] + c] : 0.f;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      first[u][0] = first[u][1] = first[u][2] = 0.f;
-      if (t[u] >= 0) {
-        first[u][0] = normals[u][3 * h0[u]];
-        first[u][1] = normals[u][3 * h0[u] + 1];
-        first[u][2] = normals[u][3 * h0[u] + 2];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long i = i0 + u * stride;
-      if (t[u] == -2) continue;
-      if (t[u] < 0) {
-        for (int c = 0; c < 3; ++c) f_normal[c * nn + i] = 0.f;
-        continue;
-      }
-      float nrm[3] = {0.f, 0.f, 0.f};
-      nrm[0] += first[u][0]; nrm[1] += first[u][1]; nrm[2] += first[u][2];
-      for (int j = s0[u] + 1; j < s1[u]; ++j) {
-        const long long h = a.sorted_idx[j] - base[u];
-        nrm[0] += normals[u][3 * h]; nrm[1] += normals[u][3 * h + 1]; nrm[2] += normals[u][3 * h + 2];
-      }
-      float len = 0.f;
-      len += nrm[0] * nrm[0]; len += nrm[1] * nrm[1]; len += nrm[2] * nrm[2];
-      float factor = sqrtf(len);
-      if (factor < 1.0e-6f) {
-        nrm[0] = first[u][0]; nrm[1] = first[u][1]; nrm[2] = first[u][2];
-        len = 0.f;
+      const int r = r0 + u * stride;
+      if (s1[u] <= s0[u]) continue;
+      if (a.has_normal) {
+        float nrm[3] = {0.f, 0.f, 0.f};
+        nrm[0] += first[u][0]; nrm[1] += first[u][1]; nrm[2] += first[u][2];
+        for (int j = s0[u] + 1; j < s1[u]; ++j) {
+          const long long h = a.sorted_idx[j] - base[u];
+          nrm[0] += normals[u][3 * h]; nrm[1] += normals[u][3 * h + 1]; nrm[2] += normals[u][3 * h + 2];
+        }
+        float len = 0.f;
         len += nrm[0] * nrm[0]; len += nrm[1] * nrm[1]; len += nrm[2] * nrm[2];
-        factor = sqrtf(len) + 1.0e-30f;
+        float factor = sqrtf(len);
+        if (factor < 1.0e-6f) {
+          nrm[0] = first[u][0]; nrm[1] = first[u][1]; nrm[2] = first[u][2];
+          len = 0.f;
+          len += nrm[0] * nrm[0]; len += nrm[1] * nrm[1]; len += nrm[2] * nrm[2];
+          factor = sqrtf(len) + 1.0e-30f;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a.avg[c][r] = nrm[c] / factor;
       }
-      for (int c = 0; c < 3; ++c) { nrm[c] = nrm[c] / factor; f_normal[c * nn + i] = nrm[c]; }
+      const float cnt = (float)(unsigned)(s1[u] - s0[u]) + 1.0e-30f;
+      for (int c = 0; c < a.cf; ++c) {
+        float acc = 0.f;
+        for (int j = s0[u]; j < s1[u]; ++j) acc += feats[u][(long long)a.cf * (a.sorted_idx[j] - base[u]) + c];
+        a.avg[(a.has_normal ? 3 : 0) + c][r] = acc / cnt;
+      }
     }
   }
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
-__global__ void signal_kernel(SignalArgs a) {
+template <typename KeyT>
+__global__ void signal_kernel(const __grid_constant__ SignalArgs<KeyT> a) {
   grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
   const long long nn = a.nnum;
   const int cn = a.has_normal ? 3 : 0;
@@ -667,7 +868,7 @@ __global__ void signal_kernel(SignalArgs a) {
     }
     const int s0 = a.seg[t], s1 = a.seg[t + 1];
     // every point of a node comes from the node's own cloud; sorted_idx is batch-wide
-    const CloudRef cl = a.clouds[(int)(a.K[t] >> (3 * a.depth))];
+    const CloudRef cl = a.clouds[(int)((uint64_t)a.K[t] >> (3 * a.depth))];
     const float* normals = cl.normal;
     const float* feats = cl.feat;
     const float* labels = cl.label;
@@ -736,59 +937,172 @@ __global__ void signal_kernel(SignalArgs a) {
 }
 
 // ---- host drivers -----------------------------------------------------------------------------
-template <typename KeyT>
-int sort_and_unique(const ocnn_points_batch* pts, const ocnn_build_params* prm, const Layout& L,
-                    uint8_t* ws, cudaStream_t st, int* final_buf) {
-  const int64_t n = L.n;
-  KeyT* keys[2] = {reinterpret_cast<KeyT*>(ws + L.off_keys[0]), reinterpret_cast<KeyT*>(ws + L.off_keys[1])};
-  uint32_t* idx[2] = {reinterpret_cast<uint32_t*>(ws + L.off_idx[0]), reinterpret_cast<uint32_t*>(ws + L.off_idx[1])};
-  int* hist = reinterpret_cast<int*>(ws + L.off_hist);
-  int* bintot = reinterpret_cast<int*>(ws + L.off_bintot);
+// The counts' way back: a mapped, pinned word per host thread, written by the last kernel of the plan.
+struct HostCounts {
+  int* host = nullptr;
+  ~HostCounts() {
+    if (host) cudaFreeHost(host);
+  }
+  int* get() {
+    if (host == nullptr) {
+      void* p = nullptr;
+      if (cudaHostAlloc(&p, 32 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+      host = static_cast<int*>(p);
+    }
+    return host;
+  }
+};
 
-  EncodeArgs ea;
-  ea.clouds = reinterpret_cast<const CloudRef*>(ws + L.off_offsets);
-  ea.batch = pts->batch; ea.depth = prm->depth; ea.n = n;
+float cell_scale(const ocnn_build_params* prm) {
   float width = prm->bbmax[0] - prm->bbmin[0];
   for (int j = 1; j < 3; ++j) {
     const float w = prm->bbmax[j] - prm->bbmin[j];
     if (w > width) width = w;
   }
   if (width == 0.0f) width = 1.0e-10f;
-  ea.mul = (float)(1 << prm->depth) / width;
-  for (int j = 0; j < 3; ++j) ea.bbmin[j] = prm->bbmin[j];
-  OCNN_CUDA_OK(launch_chained(encode_kernel<KeyT>, dim3(grid_for(n, kThreads)), dim3(kThreads), 0, st, ea, keys[0], bintot, 256 * 8));
-  OCNN_LAUNCH_OK("encode_kernel");
+  return (float)(1 << prm->depth) / width;
+}
 
-  const int nbits = 3 * prm->depth + bits_for(pts->batch);
-  const int passes = (nbits + 7) / 8 < 1 ? 1 : (nbits + 7) / 8;
-  const int sort_grid = L.nvb;
+template <typename KeyT, int RB>
+int sort_keys(const EncodeArgs& ea, const Layout& L, int chunks, uint8_t* ws, cudaStream_t st) {
+  constexpr int kBins = 1 << RB;
+  KeyT* keys[2] = {reinterpret_cast<KeyT*>(ws + L.off_keys[0]), reinterpret_cast<KeyT*>(ws + L.off_keys[1])};
+  uint32_t* idx[2] = {reinterpret_cast<uint32_t*>(ws + L.off_idx[0]), reinterpret_cast<uint32_t*>(ws + L.off_idx[1])};
+  const CloudRef* clouds = reinterpret_cast<const CloudRef*>(ws + L.off_clouds);
+  int* hist = reinterpret_cast<int*>(ws + L.off_hist);
+  OCNN_CUDA_OK(launch_chained(encode_kernel<KeyT, RB>, dim3(chunks), dim3(kThreads), 0, st, ea, keys[0], hist,
+                              reinterpret_cast<int*>(ws + L.off_bintot)));
+  OCNN_LAUNCH_OK("encode_kernel");
+  const int rows = ceil_div((long long)L.batch * kBins, kWarps);
   int cur = 0;
-  for (int p = 0; p < passes; ++p) {
-    const int shift = 8 * p;
-    OCNN_CUDA_OK(launch_chained(sort_hist_kernel<KeyT>, dim3(sort_grid), dim3(kThreads), 0, st, keys[cur], n, shift, L.vchunk, L.nvb, hist, bintot + 256 * p));
-    OCNN_CUDA_OK(launch_chained(sort_rowscan_kernel, dim3(256), dim3(kThreads), 0, st, hist, L.nvb, bintot + 256 * p));
+  for (int p = 0; p < L.passes; ++p) {
+    const int shift = RB * p;
+    int* bintot = reinterpret_cast<int*>(ws + L.off_bintot) + (size_t)p * L.batch * kBins;
+    if (p > 0)
+      OCNN_CUDA_OK(launch_chained(sort_hist_kernel<KeyT, RB>, dim3(chunks), dim3(kThreads), 0, st,
+                                  (const KeyT*)keys[cur], clouds, L.batch, ea.chunk_pts, shift, hist, bintot));
+    OCNN_CUDA_OK(launch_chained(sort_rowscan_kernel<RB>, dim3(rows), dim3(kThreads), 0, st, hist, clouds, L.batch,
+                                (const int*)bintot));
     if (p == 0)
-      OCNN_CUDA_OK(launch_chained(sort_scatter_kernel<KeyT, true>, dim3(sort_grid), dim3(kThreads), 0, st, keys[cur], nullptr, keys[cur ^ 1], idx[cur ^ 1], n, shift, L.vchunk, L.nvb, hist));
+      OCNN_CUDA_OK(launch_chained(sort_scatter_kernel<KeyT, true, RB>, dim3(chunks), dim3(kThreads), 0, st,
+                                  (const KeyT*)keys[cur], (const uint32_t*)nullptr, keys[cur ^ 1], idx[cur ^ 1],
+                                  clouds, L.batch, ea.chunk_pts, shift, (const int*)hist));
     else
-      OCNN_CUDA_OK(launch_chained(sort_scatter_kernel<KeyT, false>, dim3(sort_grid), dim3(kThreads), 0, st, keys[cur], idx[cur], keys[cur ^ 1], idx[cur ^ 1], n, shift, L.vchunk, L.nvb, hist));
-    OCNN_LAUNCHES_OK("radix sort pass", 3);
+      OCNN_CUDA_OK(launch_chained(sort_scatter_kernel<KeyT, false, RB>, dim3(chunks), dim3(kThreads), 0, st,
+                                  (const KeyT*)keys[cur], (const uint32_t*)idx[cur], keys[cur ^ 1], idx[cur ^ 1],
+                                  clouds, L.batch, ea.chunk_pts, shift, (const int*)hist));
+    OCNN_LAUNCHES_OK("radix sort pass", p == 0 ? 2 : 3);
     cur ^= 1;
   }
-  *final_buf = cur;
+  return OCNN_OK;
+}
 
-  int* counts = reinterpret_cast<int*>(ws + L.off_counts);
-  int* blockcnt = reinterpret_cast<int*>(ws + L.off_blockcnt);
+template <typename KeyT>
+int sort_and_unique(const EncodeArgs& ea, const Layout& L, int chunks, uint8_t* ws, int* host_counts,
+                    cudaStream_t st) {
+  const int rc = L.radix_bits == 9 ? sort_keys<KeyT, 9>(ea, L, chunks, ws, st) : sort_keys<KeyT, 8>(ea, L, chunks, ws, st);
+  if (rc != OCNN_OK) return rc;
+  UniqueArgs<KeyT> u;
+  memset(&u, 0, sizeof(u));
+  u.keys = reinterpret_cast<const KeyT*>(ws + L.off_keys[L.passes & 1]);
+  u.n = L.n; u.depth = L.depth; u.full = L.full; u.levels = L.depth - L.full + 1;
+  u.blockcnt = reinterpret_cast<int*>(ws + L.off_blockcnt);
+  u.counts = reinterpret_cast<int*>(ws + L.off_counts);
+  u.host_counts = host_counts;
+  for (int l = 0; l < u.levels; ++l) {
+    u.K[l] = reinterpret_cast<KeyT*>(ws + L.off_K[L.full + l]);
+    u.start[l] = reinterpret_cast<int*>(ws + L.off_start[L.full + l]);
+  }
+  const int grid = grid_for(L.n, kScanTile, 4) < kMaxScanGrid ? grid_for(L.n, kScanTile, 4) : kMaxScanGrid;
+  if (u.levels <= 8) {
+    OCNN_CUDA_OK(launch_chained(unique_count_kernel<KeyT, 8>, dim3(grid), dim3(kThreads), 0, st, u));
+    OCNN_CUDA_OK(launch_chained(unique_compact_kernel<KeyT, 8>, dim3(grid), dim3(kThreads), 0, st, u));
+  } else {
+    OCNN_CUDA_OK(launch_chained(unique_count_kernel<KeyT, 14>, dim3(grid), dim3(kThreads), 0, st, u));
+    OCNN_CUDA_OK(launch_chained(unique_compact_kernel<KeyT, 14>, dim3(grid), dim3(kThreads), 0, st, u));
+  }
+  OCNN_LAUNCHES_OK("unique", 2);
+  return OCNN_OK;
+}
+
+template <typename KeyT>
+int emit_impl(const ocnn_points_batch* pts, const ocnn_build_params* prm, const ocnn_octree_meta* meta,
+              const Layout& L, uint8_t* ws, uint8_t* o, const uint8_t (&hdr)[OCNN_HEADER_BYTES], cudaStream_t st) {
   const int D = prm->depth, F = prm->full_depth;
-  const int g0 = grid_for(n, kScanTile, 4);
-  OCNN_CUDA_OK(launch_chained(unique_count_kernel<KeyT>, dim3(g0), dim3(kThreads), 0, st, keys[cur], nullptr, n, 0, blockcnt));
-  OCNN_CUDA_OK(launch_chained(unique_compact_kernel<KeyT>, dim3(g0), dim3(kThreads), 0, st, keys[cur], nullptr, n, 0, blockcnt, reinterpret_cast<uint64_t*>(ws + L.off_K[D]), reinterpret_cast<int*>(ws + L.off_start[D]), counts + D));
-  OCNN_LAUNCHES_OK("unique (finest level)", 2);
-  for (int d = D; d > F; --d) {
-    const uint64_t* Kd = reinterpret_cast<const uint64_t*>(ws + L.off_K[d]);
-    const int g = grid_for(L.cap[d], kScanTile, 4);
-    OCNN_CUDA_OK(launch_chained(unique_count_kernel<uint64_t>, dim3(g), dim3(kThreads), 0, st, Kd, counts + d, 0, 3, blockcnt));
-    OCNN_CUDA_OK(launch_chained(unique_compact_kernel<uint64_t>, dim3(g), dim3(kThreads), 0, st, Kd, counts + d, 0, 3, blockcnt, reinterpret_cast<uint64_t*>(ws + L.off_K[d - 1]), reinterpret_cast<int*>(ws + L.off_start[d - 1]), counts + d - 1));
-    OCNN_LAUNCHES_OK("unique (parent level)", 2);
+  SignalArgs<KeyT> sa;
+  memset(&sa, 0, sizeof(sa));
+  sa.seg = reinterpret_cast<const int*>(ws + L.off_start[D]);
+  sa.sorted_idx = reinterpret_cast<const uint32_t*>(ws + L.off_idx[L.passes & 1]);
+  sa.K = reinterpret_cast<const KeyT*>(ws + L.off_K[D]);
+  sa.clouds = reinterpret_cast<const CloudRef*>(ws + L.off_clouds);
+  sa.depth = D;
+  sa.has_normal = pts->normal_dev != nullptr;
+  sa.has_feat = pts->feature_dev != nullptr;
+  sa.nnum = meta->nnum[D];
+  sa.cf = pts->feature_dev ? pts->feature_channels : 0;
+  sa.node_dis = prm->node_dis; sa.save_pts = prm->save_pts;
+  sa.mul = cell_scale(prm);
+  for (int j = 0; j < 3; ++j) sa.bbmin[j] = prm->bbmin[j];
+  sa.f_out = reinterpret_cast<float*>(o + ocnn_prop_offset(meta, OCNN_PROP_FEATURE, D));
+  sa.l_out = pts->label_dev ? reinterpret_cast<float*>(o + ocnn_prop_offset(meta, OCNN_PROP_LABEL, D)) : nullptr;
+  sa.nodes = D > F ? meta->nnum_nempty[D] : 0;
+  // Normals and features alone (up to six channels): averaged per non-empty node, spread by the emit
+  // kernel. The sort's buffers are free by now and hold the channels beyond the first three.
+  const int channels = (sa.has_normal ? 3 : 0) + sa.cf;
+  const bool compact = channels >= 1 && channels <= 6 && sa.l_out == nullptr && !sa.node_dis && !sa.save_pts;
+  if (compact) {
+    float* avg = reinterpret_cast<float*>(ws + L.off_avg);
+    for (int c = 0; c < 3; ++c) sa.avg[c] = avg + (size_t)c * L.cap[D];
+    sa.avg[3] = reinterpret_cast<float*>(ws + L.off_keys[0]);
+    sa.avg[4] = reinterpret_cast<float*>(ws + L.off_keys[1]);
+    sa.avg[5] = reinterpret_cast<float*>(ws + L.off_idx[(L.passes & 1) ^ 1]);
+    if (sa.nodes > 0) {
+      OCNN_CUDA_OK(launch_chained(signal_average_kernel<KeyT>, dim3(grid_for((sa.nodes + 1) / 2, 256, 8)), dim3(256), 0,
+                                  st, sa));
+      OCNN_LAUNCH_OK("signal_average_kernel");
+    }
+  }
+
+  EmitAll all;
+  memset(&all, 0, sizeof(all));
+  all.out = o; all.batch = L.batch; all.full = F; all.depth = D; all.key_bytes = prm->key_bits / 8;
+  if (D > F && meta->nnum_nempty[F] > 0) {
+    all.K_full = ws + L.off_K[F];
+    all.count_full = reinterpret_cast<const int*>(ws + L.off_counts) + F;
+  }
+  if (compact) {
+    all.feat = sa.f_out;
+    all.channels = channels;
+    for (int c = 0; c < 6; ++c) all.avg[c] = sa.avg[c];
+  }
+  memcpy(all.header, hdr, OCNN_HEADER_BYTES);
+  int blocks = 0;
+  for (int d = 0; d <= D; ++d) {
+    if (meta->nnum[d] == 0) continue;
+    EmitLevel& a = all.lev[all.nlev++];
+    a.off_key = ocnn_prop_offset(meta, OCNN_PROP_KEY, d);
+    a.off_child = ocnn_prop_offset(meta, OCNN_PROP_CHILD, d);
+    a.off_split = meta->channels[OCNN_PROP_SPLIT] ? ocnn_prop_offset(meta, OCNN_PROP_SPLIT, d) : -1;
+    a.d = d;
+    a.nnum = meta->nnum[d];
+    a.block0 = blocks;
+    blocks += ceil_div(a.nnum, kEmitNodes);
+    if (d > F) {
+      a.Kp = ws + L.off_K[d - 1];
+      a.Kc = ws + L.off_K[d];
+      a.start = reinterpret_cast<const int*>(ws + L.off_start[d - 1]);
+    }
+  }
+  OCNN_CUDA_OK(launch_chained(emit_levels_kernel<KeyT>, dim3(blocks), dim3(kThreads), 0, st, all));
+  OCNN_LAUNCH_OK("emit_levels_kernel");
+
+  if (meta->nnum[D] > 0 && !compact) {
+    sa.child = reinterpret_cast<const int*>(o + ocnn_prop_offset(meta, OCNN_PROP_CHILD, D));
+    OCNN_CUDA_OK(launch_chained(signal_kernel<KeyT>, dim3(grid_for(sa.nnum, 256, 8)), dim3(256), 0, st, sa));
+    OCNN_LAUNCH_OK("signal_kernel");
   }
   return OCNN_OK;
 }
@@ -872,30 +1186,42 @@ int ocnn_octree_build_plan(const ocnn_points_batch* pts, const ocnn_build_params
   if (workspace_bytes < L.total)
     return fail(OCNN_ERR_CAPACITY, "ocnn_octree_build_plan: workspace of %zu bytes, need %zu",
                 workspace_bytes, L.total);
+  static thread_local HostCounts host_counts;
+  int* counts = host_counts.get();
+  if (counts == nullptr)
+    return fail(OCNN_ERR_CUDA, "ocnn_octree_build_plan: no pinned memory for the node counts");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  {
-    std::vector<CloudRef> table((size_t)pts->batch + 1);
-    for (int b = 0; b <= pts->batch; ++b) {
-      CloudRef& c = table[b];
-      const bool real = b < pts->batch;
-      c.xyz = real ? pts->xyz_dev[b] : nullptr;
-      c.normal = real && pts->normal_dev ? pts->normal_dev[b] : nullptr;
-      c.feat = real && pts->feature_dev ? pts->feature_dev[b] : nullptr;
-      c.label = real && pts->label_dev ? pts->label_dev[b] : nullptr;
-      c.offset = pts->offsets_host[b];
-    }
-    // pageable source: the runtime stages it before returning, so `table` may go out of scope
-    OCNN_CUDA_OK(cudaMemcpyAsync(ws + L.off_offsets, table.data(), sizeof(CloudRef) * table.size(),
-                                 cudaMemcpyHostToDevice, st));
+
+  EncodeArgs ea;
+  ea.table = reinterpret_cast<const CloudRef*>(ws + L.off_clouds);
+  ea.inline_clouds = pts->batch <= kInlineClouds ? 1 : 0;
+  ea.batch = pts->batch; ea.depth = prm->depth; ea.chunk_pts = chunk_points(n);
+  ea.mul = cell_scale(prm);
+  for (int j = 0; j < 3; ++j) ea.bbmin[j] = prm->bbmin[j];
+  std::vector<CloudRef> big(ea.inline_clouds ? 0 : (size_t)pts->batch + 1);
+  CloudRef* table = ea.inline_clouds ? ea.clouds : big.data();
+  int chunks = 0;
+  for (int b = 0; b <= pts->batch; ++b) {
+    CloudRef& c = table[b];
+    const bool real = b < pts->batch;
+    c.xyz = real ? pts->xyz_dev[b] : nullptr;
+    c.normal = real && pts->normal_dev ? pts->normal_dev[b] : nullptr;
+    c.feat = real && pts->feature_dev ? pts->feature_dev[b] : nullptr;
+    c.label = real && pts->label_dev ? pts->label_dev[b] : nullptr;
+    c.offset = pts->offsets_host[b];
+    c.chunk0 = chunks;
+    c.pad = 0;
+    if (real) chunks += ceil_div(pts->offsets_host[b + 1] - pts->offsets_host[b], ea.chunk_pts);
   }
-  OCNN_CUDA_OK(cudaMemsetAsync(ws + L.off_counts, 0, sizeof(int) * 32, st));
-  int final_buf = 0;
-  int s = L.key_bytes_sort == 4 ? sort_and_unique<uint32_t>(pts, prm, L, ws, st, &final_buf)
-                                : sort_and_unique<uint64_t>(pts, prm, L, ws, st, &final_buf);
+  // (pageable source: the runtime stages it before returning, so `big` may go out of scope)
+  if (!ea.inline_clouds)
+    OCNN_CUDA_OK(cudaMemcpyAsync(ws + L.off_clouds, big.data(), sizeof(CloudRef) * big.size(),
+                                 cudaMemcpyHostToDevice, st));
+  OCNN_CUDA_OK(cudaMemsetAsync(ws + L.off_counts, 0, L.zero_bytes, st));
+  const int s = L.key_bytes == 4 ? sort_and_unique<uint32_t>(ea, L, chunks, ws, counts, st)
+                                 : sort_and_unique<uint64_t>(ea, L, chunks, ws, counts, st);
   if (s != OCNN_OK) return s;
-  int counts[32];
-  OCNN_CUDA_OK(cudaMemcpyAsync(counts, ws + L.off_counts, sizeof(counts), cudaMemcpyDeviceToHost, st));
   OCNN_CUDA_OK(cudaStreamSynchronize(st));
 
   fill_static_meta(pts, prm, meta);
@@ -932,11 +1258,6 @@ int ocnn_octree_build_emit(const ocnn_points_batch* pts, const ocnn_build_params
   if ((int64_t)out_bytes < meta->ptr_dis[OCNN_PROP_COUNT])
     return fail(OCNN_ERR_CAPACITY, "ocnn_octree_build_emit: output of %zu bytes, need %lld",
                 out_bytes, (long long)meta->ptr_dis[OCNN_PROP_COUNT]);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  uint8_t* ws = static_cast<uint8_t*>(workspace);
-  uint8_t* o = static_cast<uint8_t*>(out);
-  const int D = prm->depth, F = prm->full_depth, B = pts->batch;
-
   uint8_t hdr[OCNN_HEADER_BYTES];
   HeaderExtras ex;
   ex.adp_depth = prm->adp_depth;
@@ -945,83 +1266,12 @@ int ocnn_octree_build_emit(const ocnn_points_batch* pts, const ocnn_build_params
   for (int j = 0; j < 3; ++j) { ex.bbmin[j] = prm->bbmin[j]; ex.bbmax[j] = prm->bbmax[j]; }
   write_header(meta, ex, hdr);
   if (header_host_out) memcpy(header_host_out, hdr, OCNN_HEADER_BYTES);
-  OCNN_CUDA_OK(cudaMemcpyAsync(o, hdr, OCNN_HEADER_BYTES, cudaMemcpyHostToDevice, st));
-
-  const int* counts = reinterpret_cast<const int*>(ws + L.off_counts);
-  EmitAll all;
-  memset(&all, 0, sizeof(all));
-  all.batch = B; all.full = F;
-  int blocks = 0;
-  EmitLevelArgs full_args;
-  memset(&full_args, 0, sizeof(full_args));
-  for (int d = 0; d <= D; ++d) {
-    EmitLevelArgs a;
-    a.out = o;
-    a.off_key = ocnn_prop_offset(meta, OCNN_PROP_KEY, d);
-    a.off_child = ocnn_prop_offset(meta, OCNN_PROP_CHILD, d);
-    a.off_split = meta->channels[OCNN_PROP_SPLIT] ? ocnn_prop_offset(meta, OCNN_PROP_SPLIT, d) : -1;
-    a.key_bytes = prm->key_bits / 8;
-    a.d = d;
-    if (d == F) full_args = a;
-    const long long nnum = meta->nnum[d];
-    if (nnum == 0) continue;
-    const int l = all.nlev++;
-    all.a[l] = a;
-    all.nnum[l] = nnum;
-    all.block0[l] = blocks;
-    blocks += (int)((nnum + kThreads - 1) / kThreads);
-    if (d > F) {
-      all.Kp[l] = reinterpret_cast<const uint64_t*>(ws + L.off_K[d - 1]);
-      all.Kc[l] = reinterpret_cast<const uint64_t*>(ws + L.off_K[d]);
-      all.start[l] = reinterpret_cast<const int*>(ws + L.off_start[d - 1]);
-    }
-  }
-  all.block0[all.nlev] = blocks;
-  if (blocks > 0) {
-    OCNN_CUDA_OK(launch_chained(emit_levels_kernel, dim3(blocks), dim3(kThreads), 0, st, all));
-    OCNN_LAUNCH_OK("emit_levels_kernel");
-  }
-  if (D > F && meta->nnum_nempty[F] > 0) {
-    // (after the level itself: it overwrites the -1 the full level wrote for every node)
-    OCNN_CUDA_OK(launch_chained(emit_full_children_kernel, dim3(grid_for(meta->nnum_nempty[F], kThreads)),
-                                dim3(kThreads), 0, st, full_args,
-                                reinterpret_cast<const uint64_t*>(ws + L.off_K[F]), counts + F));
-    OCNN_LAUNCH_OK("emit_full_children_kernel");
-  }
-
-  if (meta->nnum[D] > 0) {
-    // which of the two sort buffers holds the final order: passes are a function of (depth, batch)
-    const int nbits = 3 * D + bits_for(B);
-    const int passes = (nbits + 7) / 8 < 1 ? 1 : (nbits + 7) / 8;
-    SignalArgs sa;
-    sa.child = reinterpret_cast<const int*>(o + ocnn_prop_offset(meta, OCNN_PROP_CHILD, D));
-    sa.seg = reinterpret_cast<const int*>(ws + L.off_start[D]);
-    sa.sorted_idx = reinterpret_cast<const uint32_t*>(ws + L.off_idx[passes & 1]);
-    sa.K = reinterpret_cast<const uint64_t*>(ws + L.off_K[D]);
-    sa.clouds = reinterpret_cast<const CloudRef*>(ws + L.off_offsets);
-    sa.depth = D;
-    sa.has_normal = pts->normal_dev != nullptr;
-    sa.has_feat = pts->feature_dev != nullptr;
-    sa.f_out = reinterpret_cast<float*>(o + ocnn_prop_offset(meta, OCNN_PROP_FEATURE, D));
-    sa.l_out = pts->label_dev ? reinterpret_cast<float*>(o + ocnn_prop_offset(meta, OCNN_PROP_LABEL, D)) : nullptr;
-    sa.nnum = meta->nnum[D];
-    sa.cf = pts->feature_dev ? pts->feature_channels : 0;
-    sa.node_dis = prm->node_dis; sa.save_pts = prm->save_pts;
-    float width = prm->bbmax[0] - prm->bbmin[0];
-    for (int j = 1; j < 3; ++j) {
-      const float w = prm->bbmax[j] - prm->bbmin[j];
-      if (w > width) width = w;
-    }
-    if (width == 0.0f) width = 1.0e-10f;
-    sa.mul = (float)(1 << D) / width;
-    for (int j = 0; j < 3; ++j) sa.bbmin[j] = prm->bbmin[j];
-    if (sa.has_normal && sa.cf == 0 && sa.l_out == nullptr && !sa.node_dis && !sa.save_pts)
-      OCNN_CUDA_OK(launch_chained(signal_normals_kernel, dim3(grid_for((sa.nnum + 3) / 4, 256, 8)), dim3(256), 0, st, sa));
-    else
-      OCNN_CUDA_OK(launch_chained(signal_kernel, dim3(grid_for(sa.nnum, 256, 8)), dim3(256), 0, st, sa));
-    OCNN_LAUNCH_OK("signal_kernel");
-  }
-
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  uint8_t* o = static_cast<uint8_t*>(out);
+  const int s = L.key_bytes == 4 ? emit_impl<uint32_t>(pts, prm, meta, L, ws, o, hdr, st)
+                                 : emit_impl<uint64_t>(pts, prm, meta, L, ws, o, hdr, st);
+  if (s != OCNN_OK) return s;
   if (prm->merged) return ocnn_calc_neigh(out, meta, stream);
   return OCNN_OK;
 }

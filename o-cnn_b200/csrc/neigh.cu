@@ -46,6 +46,33 @@ __global__ void neigh_full_kernel(int* __restrict__ out, int depth, long long pe
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
+// Levels 0 .. full of a batch octree in one launch: level d's table is out + 8 * 8^d-node prefix, i.e.
+// the levels lie one behind the other. Level 0 has no neighbour table; the reference leaves its slot
+// zero-filled (merge_octrees.cpp:108-112 resizes a fresh vector, the loop at :184 starts at d = 1).
+__global__ void neigh_full_levels_kernel(int* __restrict__ out, int batch, int full, long long total) {
+  grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+       i += (long long)gridDim.x * blockDim.x) {
+    long long at = i;
+    int depth = 0;
+    while (depth < full && at >= 8LL * batch << (3 * depth)) { at -= 8LL * batch << (3 * depth); ++depth; }
+    if (depth == 0) { out[i] = 0; continue; }
+    const int per = 1 << (3 * depth), side = 1 << depth;
+    const int j = (int)(at & 63);
+    const long long node = at >> 6 << 3;           // first node of the sibling group, over the batch
+    const int n = (int)(node / per);
+    const unsigned g = (unsigned)(node - (long long)n * per);
+    const int x = (int)gather3(g >> 2) + (j >> 4) - 1;
+    const int y = (int)gather3(g >> 1) + ((j >> 2) & 3) - 1;
+    const int z = (int)gather3(g) + (j & 3) - 1;
+    int v = -1;
+    if (x >= 0 && y >= 0 && z >= 0 && x < side && y < side && z < side)
+      v = (int)((spread3(x) << 2) | (spread3(y) << 1) | spread3(z)) + n * per;
+    out[i] = v;
+  }
+  grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
+}
+
 // Split level, one warp per sibling group of PARENT nodes.  The eight parents of a group share one
 // 4x4x4 neighbour block at their own level, and every entry any of their children's blocks needs
 // is "the child group of one of those 64 cells".  So the warp reads the group's 64 neighbour
@@ -73,17 +100,34 @@ __global__ void __launch_bounds__(kNeighWarps * 32) neigh_split_kernel(
     tapcode[k] = ((x >> 1) << 4) | ((y >> 1) << 2) | (z >> 1);
     oct[k] = ((x & 1) << 2) | ((y & 1) << 1) | (z & 1);
   }
-  for (long long g = blockIdx.x * (long long)kNeighWarps + warp; g < ngroups;
-       g += (long long)gridDim.x * kNeighWarps) {
+  // Three stages in flight per warp: the block of the group after next is requested, then the child
+  // pointers behind the next group's block, then this group's tables are written.  (One group at a
+  // time was a chain of two reads per 700 bytes written: 3.7 TB/s where the writes alone go at 7.4.)
+  const long long stride = (long long)gridDim.x * kNeighWarps;
+  const long long first = blockIdx.x * (long long)kNeighWarps + warp;
+  auto cells = [&](long long g, int (&cell)[2], int& mine) {
+    cell[0] = cell[1] = mine = -1;
+    if (g >= ngroups) return;
     const int* blk = neigh + (g << 6);
+    cell[0] = blk[lane];
+    cell[1] = blk[lane + 32];
+    if (lane < 8) mine = child[(g << 3) + lane];     // the eight parents themselves
+  };
+  auto kids = [&](const int (&cell)[2], int (&kid)[2]) {
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int cell = blk[lane + 32 * k];
-      cblk[warp][lane + 32 * k] = cell >= 0 ? child[cell] : -1;
-    }
-    // the eight parents themselves: lanes 0..7 read their child pointers
-    const int mine = lane < 8 ? child[(g << 3) + lane] : -1;
+    for (int k = 0; k < 2; ++k) kid[k] = cell[k] >= 0 ? child[cell[k]] : -1;
+  };
+  int cell[2], kid[2], mine, mine_next;
+  cells(first, cell, mine);
+  kids(cell, kid);
+  cells(first + stride, cell, mine_next);
+  for (long long g = first; g < ngroups; g += stride) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) cblk[warp][lane + 32 * k] = kid[k];
     __syncwarp();
+    kids(cell, kid);
+    int mine_after;
+    cells(g + 2 * stride, cell, mine_after);
 #pragma unroll
     for (int o = 0; o < 8; ++o) {
       const int l0 = __shfl_sync(0xffffffffu, mine, o);
@@ -96,6 +140,8 @@ __global__ void __launch_bounds__(kNeighWarps * 32) neigh_split_kernel(
         dst[lane + 32 * k] = c >= 0 ? (c << 3) + oct[k] : -1;
       }
     }
+    mine = mine_next;
+    mine_next = mine_after;
     __syncwarp();
   }
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
@@ -141,23 +187,23 @@ int ocnn_calc_neigh(void* octree_dev, const ocnn_octree_meta* m, void* stream) {
   OCNN_REQUIRE(m->channels[OCNN_PROP_CHILD] == 1 && m->locations[OCNN_PROP_CHILD] == -1,
                "ocnn_calc_neigh: the octree has no child block");
   uint8_t* base = static_cast<uint8_t*>(octree_dev);
-  // level 0 has no neighbour table; the reference leaves its slot zero-filled
-  // (merge_octrees.cpp:108-112 resizes a fresh vector, the loop at :184 starts at d = 1)
-  if (m->nnum[0] > 0)
-    OCNN_CUDA_OK(cudaMemsetAsync(base + ocnn_prop_offset(m, OCNN_PROP_NEIGH, 0), 0,
-                                 (size_t)m->nnum[0] * 8 * sizeof(int32_t),
-                                 static_cast<cudaStream_t>(stream)));
-  for (int d = 1; d <= m->depth; ++d) {
-    int32_t* nd = reinterpret_cast<int32_t*>(base + ocnn_prop_offset(m, OCNN_PROP_NEIGH, d));
-    int s;
-    if (d <= m->full_depth) {
-      s = ocnn_calc_neigh_full(nd, d, m->batch_size, stream);
-    } else {
-      s = ocnn_calc_neigh_split(
-          nd, reinterpret_cast<const int32_t*>(base + ocnn_prop_offset(m, OCNN_PROP_NEIGH, d - 1)),
-          reinterpret_cast<const int32_t*>(base + ocnn_prop_offset(m, OCNN_PROP_CHILD, d - 1)),
-          m->nnum[d - 1], stream);
-    }
+  const int full = m->full_depth < m->depth ? m->full_depth : m->depth;
+  OCNN_REQUIRE(full >= 0 && full <= 10, "ocnn_calc_neigh: full depth %d out of range", full);
+  long long total = 0;
+  for (int d = 0; d <= full; ++d) {
+    OCNN_REQUIRE(m->nnum[d] == (long long)m->batch_size << (3 * d), "ocnn_calc_neigh: level %d is not full", d);
+    total += 8LL * m->nnum[d];
+  }
+  int* all = reinterpret_cast<int*>(base + ocnn_prop_offset(m, OCNN_PROP_NEIGH, 0));
+  OCNN_CUDA_OK(launch_chained(neigh_full_levels_kernel, dim3(grid_for(total, 256)), dim3(256), 0,
+                              static_cast<cudaStream_t>(stream), all, m->batch_size, full, total));
+  OCNN_LAUNCH_OK("neigh_full_levels_kernel");
+  for (int d = full + 1; d <= m->depth; ++d) {
+    const int s = ocnn_calc_neigh_split(
+        reinterpret_cast<int32_t*>(base + ocnn_prop_offset(m, OCNN_PROP_NEIGH, d)),
+        reinterpret_cast<const int32_t*>(base + ocnn_prop_offset(m, OCNN_PROP_NEIGH, d - 1)),
+        reinterpret_cast<const int32_t*>(base + ocnn_prop_offset(m, OCNN_PROP_CHILD, d - 1)), m->nnum[d - 1],
+        stream);
     if (s != OCNN_OK) return s;
   }
   return OCNN_OK;
