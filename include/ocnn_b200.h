@@ -526,6 +526,27 @@ int ocnn_octree_align_backward(const void* dst_grad_dev, void* src_grad_dev, con
  * orient_normal / clip, octree/octree/points_parser.cpp:42-259, and bounding_box,
  * octree/octree/math_functions.cpp:113-128 (bindings pytorch/cpp/transform_points.cpp:7-125).
  * ------------------------------------------------------------------------------------------ */
+/* normalise + transform + clip of one points buffer in two launches (PointsParser::uniform scale and shift,
+ * then displace / rotate / translate / scale / orient, then clip to the open box): every step as in
+ * ocnn_points_transform and ocnn_points_clip, bit for bit. in, work, out: whole points buffers of `bytes`
+ * bytes (work may be in; out must not); offsets / channels of the four properties, coordinates and
+ * normals one behind the other; mask [n]; workspace of ocnn_points_clip_workspace_bytes; total_out: a
+ * device-visible word (mapped host memory will do) that receives the kept count. */
+typedef struct ocnn_point_transform {
+  float offset;
+  int32_t rotate;      /* rot is used */
+  float rot[9];
+  int32_t translate;   /* shift is used */
+  float shift[3];
+  float scale[3];      /* 1,1,1: none */
+  int32_t orient;
+} ocnn_point_transform;
+int ocnn_points_prepare(const void* in_dev, void* work_dev, void* out_dev, int64_t bytes, int64_t n,
+                        const int64_t offsets[4], const int channels[4], const ocnn_point_transform* first,
+                        const ocnn_point_transform* second, const float bbmin[3], const float bbmax[3],
+                        int32_t* mask_dev, void* workspace, size_t workspace_bytes, int32_t* total_out,
+                        void* stream);
+
 /* In place, in the reference's order: p += normal * offset (when offset > 1e-10 and normals
  * exist); p, normal = R p, R normal (rot9: out[m] = sum_k rot9[k*3 + m] * in[k], or NULL);
  * p += shift3 (or NULL); p *= scale3 (or NULL; with unequal factors the normals are divided by

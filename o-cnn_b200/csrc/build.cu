@@ -234,8 +234,9 @@ __global__ void __launch_bounds__(kThreads) encode_kernel(const __grid_constant_
         const float s = (p[u][j] - a.bbmin[j]) * a.mul;
         cell[j] = (uint32_t)s & mask;
       }
-      const uint64_t key = (spread3(cell[0]) << 2) | (spread3(cell[1]) << 1) | spread3(cell[2]);
-      if (i < c.end) keys[i] = (KeyT)(top | key);
+      // (with the cloud's bits: the top digit of a shallow tree reaches into them, here as in the scatter)
+      const uint64_t key = top | (spread3(cell[0]) << 2) | (spread3(cell[1]) << 1) | spread3(cell[2]);
+      if (i < c.end) keys[i] = (KeyT)key;
       count_digit(sh[threadIdx.x >> 5], i < c.end ? (int)(key & ((1 << RB) - 1)) : (1 << RB), 1 << RB);
     }
   }

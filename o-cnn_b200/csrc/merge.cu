@@ -19,6 +19,7 @@ struct MergeEntry {
   int node0;              // first destination node
   int ne0;                // non-empty nodes of earlier octrees at this level
   int b, d;
+  int block0;             // first block of merge_kernel that works on this entry
 };
 
 struct MergeDst {
@@ -27,40 +28,92 @@ struct MergeDst {
       label[OCNN_MAX_DEPTH], split[OCNN_MAX_DEPTH];
   int nnum[OCNN_MAX_DEPTH];
   int key_bytes, cfeat;
+  uint8_t header[OCNN_HEADER_BYTES];
 };
 
-__global__ void merge_kernel(const MergeEntry* __restrict__ entries, int nentries, MergeDst dst) {
-  for (int e = blockIdx.y; e < nentries; e += gridDim.y) {
-    const MergeEntry en = entries[e];
-    const int d = en.d;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < en.n; j += gridDim.x * blockDim.x) {
-      const long long o = en.node0 + j;
-      if (en.key >= 0) {
-        if (dst.key_bytes == 8) {
-          const uint64_t k = reinterpret_cast<const uint64_t*>(en.src + en.key)[j];
-          reinterpret_cast<uint64_t*>(dst.out + dst.key[d])[o] =
-              (k & 0x0000ffffffffffffULL) | ((uint64_t)(en.b & 0xffff) << 48);
-        } else {
-          const uint32_t k = reinterpret_cast<const uint32_t*>(en.src + en.key)[j];
-          reinterpret_cast<uint32_t*>(dst.out + dst.key[d])[o] =
-              (k & 0x00ffffffu) | ((uint32_t)(en.b & 0xff) << 24);
-        }
-      }
-      if (en.child >= 0) {
-        const int c = reinterpret_cast<const int*>(en.src + en.child)[j];
-        reinterpret_cast<int*>(dst.out + dst.child[d])[o] = c == -1 ? -1 : c + en.ne0;
-      }
-      if (en.feat >= 0) {
-        const float* fs = reinterpret_cast<const float*>(en.src + en.feat);
-        float* fd = reinterpret_cast<float*>(dst.out + dst.feat[d]);
-        for (int c = 0; c < dst.cfeat; ++c) fd[(long long)c * dst.nnum[d] + o] = fs[(long long)c * en.n + j];
-      }
-      if (en.label >= 0)
-        reinterpret_cast<float*>(dst.out + dst.label[d])[o] = reinterpret_cast<const float*>(en.src + en.label)[j];
-      if (en.split >= 0)
-        reinterpret_cast<float*>(dst.out + dst.split[d])[o] = reinterpret_cast<const float*>(en.src + en.split)[j];
-    }
+constexpr int kMergeNodes = 1024;        // nodes per block: four per thread, all requested together
+constexpr int kParamEntries = 352;       // a table of this many entries rides in the launch parameters
+
+template <int N>
+struct MergeTable {
+  MergeEntry e[N];
+};
+
+// A block copies kMergeNodes nodes of one entry (block0 is the entry's first block).  The header goes
+// along with block 0.
+__device__ __forceinline__ void merge_block(const MergeEntry* __restrict__ entries, int nentries, const MergeDst& dst) {
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < OCNN_HEADER_BYTES / 4; i += 256)
+      reinterpret_cast<int*>(dst.out)[i] = reinterpret_cast<const int*>(dst.header)[i];
+  int lo = 0, hi = nentries;               // entries[lo].block0 <= blockIdx.x < entries[hi].block0
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (entries[mid].block0 <= (int)blockIdx.x) lo = mid; else hi = mid;
   }
+  const MergeEntry en = entries[lo];
+  const int d = en.d;
+  const int j0 = ((int)blockIdx.x - en.block0) * kMergeNodes + threadIdx.x;
+  constexpr int U = kMergeNodes / 256;
+  const bool wide = dst.key_bytes == 8;
+  uint64_t key[U];
+  int child[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int j = j0 + 256 * u;
+    if (j >= en.n) continue;
+    if (en.key >= 0)
+      key[u] = wide ? reinterpret_cast<const uint64_t*>(en.src + en.key)[j]
+                    : (uint64_t)reinterpret_cast<const uint32_t*>(en.src + en.key)[j];
+    if (en.child >= 0) child[u] = reinterpret_cast<const int*>(en.src + en.child)[j];
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int j = j0 + 256 * u;
+    if (j >= en.n) continue;
+    const long long o = en.node0 + j;
+    if (en.key >= 0) {
+      if (wide)
+        reinterpret_cast<uint64_t*>(dst.out + dst.key[d])[o] =
+            (key[u] & 0x0000ffffffffffffULL) | ((uint64_t)(en.b & 0xffff) << 48);
+      else
+        reinterpret_cast<uint32_t*>(dst.out + dst.key[d])[o] =
+            ((uint32_t)key[u] & 0x00ffffffu) | ((uint32_t)(en.b & 0xff) << 24);
+    }
+    if (en.child >= 0)
+      reinterpret_cast<int*>(dst.out + dst.child[d])[o] = child[u] == -1 ? -1 : child[u] + en.ne0;
+  }
+  auto copy_row = [&](const float* from, float* to) {
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = j0 + 256 * u < en.n ? from[j0 + 256 * u] : 0.f;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (j0 + 256 * u < en.n) to[j0 + 256 * u] = v[u];
+  };
+  if (en.feat >= 0)
+    for (int c = 0; c < dst.cfeat; ++c)
+      copy_row(reinterpret_cast<const float*>(en.src + en.feat) + (long long)c * en.n,
+               reinterpret_cast<float*>(dst.out + dst.feat[d]) + (long long)c * dst.nnum[d] + en.node0);
+  if (en.label >= 0)
+    copy_row(reinterpret_cast<const float*>(en.src + en.label),
+             reinterpret_cast<float*>(dst.out + dst.label[d]) + en.node0);
+  if (en.split >= 0)
+    copy_row(reinterpret_cast<const float*>(en.src + en.split),
+             reinterpret_cast<float*>(dst.out + dst.split[d]) + en.node0);
+}
+
+__global__ void __launch_bounds__(256) merge_kernel(const MergeEntry* __restrict__ entries, int nentries,
+                                                    const __grid_constant__ MergeDst dst) {
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  merge_block(entries, nentries, dst);
+}
+
+__global__ void __launch_bounds__(256) merge_param_kernel(const __grid_constant__ MergeTable<kParamEntries> table,
+                                                          int nentries, const __grid_constant__ MergeDst dst) {
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  merge_block(table.e, nentries, dst);
 }
 
 bool at_level(const ocnn_octree_meta* m, int prop, int d) {
@@ -90,11 +143,11 @@ void merged_header(const void* first_header_host, const ocnn_octree_meta* merged
 }
 
 // The (octree, level) table merge_kernel walks, written to `entries` (room for batch*(depth+1));
-// returns the number of entries; *max_n = the largest node count of any entry.
+// returns the number of entries; *blocks = the number of blocks they take.
 int merge_table(const void* const* octrees_dev, const ocnn_octree_meta* in, int batch, int depth,
-                MergeEntry* entries, int* max_n) {
+                MergeEntry* entries, int* blocks) {
   int ne = 0;
-  *max_n = 1;
+  *blocks = 0;
   for (int d = 0; d <= depth; ++d) {
     int node0 = 0, ne0 = 0;
     for (int b = 0; b < batch; ++b) {
@@ -107,8 +160,11 @@ int merge_table(const void* const* octrees_dev, const ocnn_octree_meta* in, int 
       e.label = at_level(m, OCNN_PROP_LABEL, d) ? ocnn_prop_offset(m, OCNN_PROP_LABEL, d) : -1;
       e.split = at_level(m, OCNN_PROP_SPLIT, d) ? ocnn_prop_offset(m, OCNN_PROP_SPLIT, d) : -1;
       e.n = m->nnum[d]; e.node0 = node0; e.ne0 = ne0; e.b = b; e.d = d;
-      if (e.n > 0) entries[ne++] = e;
-      if (e.n > *max_n) *max_n = e.n;
+      e.block0 = *blocks;
+      if (e.n > 0) {
+        entries[ne++] = e;
+        *blocks += ceil_div(e.n, kMergeNodes);
+      }
       node0 += m->nnum[d];
       ne0 += m->nnum_nempty[d];
     }
@@ -116,11 +172,12 @@ int merge_table(const void* const* octrees_dev, const ocnn_octree_meta* in, int 
   return ne;
 }
 
-MergeDst merge_destination(const ocnn_octree_meta* merged, uint8_t* out) {
+MergeDst merge_destination(const ocnn_octree_meta* merged, uint8_t* out, const uint8_t (&hdr)[OCNN_HEADER_BYTES]) {
   MergeDst dst;
   memset(&dst, 0, sizeof(dst));
   dst.out = out;
   dst.key_bytes = merged->key_bits / 8;
+  memcpy(dst.header, hdr, OCNN_HEADER_BYTES);
   dst.cfeat = merged->channels[OCNN_PROP_FEATURE];
   for (int d = 0; d <= merged->depth; ++d) {
     dst.key[d] = ocnn_prop_offset(merged, OCNN_PROP_KEY, d);
@@ -131,15 +188,6 @@ MergeDst merge_destination(const ocnn_octree_meta* merged, uint8_t* out) {
     dst.nnum[d] = merged->nnum[d];
   }
   return dst;
-}
-
-// Enqueue the merge of `ne` table entries already resident at table_dev.
-int launch_merge(const MergeEntry* table_dev, int ne, int max_n, const MergeDst& dst,
-                 cudaStream_t st, const char* what) {
-  dim3 grid(ceil_div(max_n, 256) < 64 ? ceil_div(max_n, 256) : 64, ne < 4096 ? ne : 4096);
-  merge_kernel<<<grid, 256, 0, st>>>(table_dev, ne, dst);
-  OCNN_LAUNCH_OK(what);
-  return OCNN_OK;
 }
 
 }  // namespace
@@ -205,19 +253,25 @@ int ocnn_octree_batch(const void* const* octrees_dev, const ocnn_octree_meta* in
   uint8_t hdr[OCNN_HEADER_BYTES];
   merged_header(first_header_host, merged, hdr);
   if (header_host_out) memcpy(header_host_out, hdr, OCNN_HEADER_BYTES);
-  OCNN_CUDA_OK(cudaMemcpyAsync(o, hdr, OCNN_HEADER_BYTES, cudaMemcpyHostToDevice, st));
 
-  std::vector<MergeEntry> entries((size_t)batch * (depth + 1));
-  int max_n = 1;
-  const int ne = merge_table(octrees_dev, in, batch, depth, entries.data(), &max_n);
-  if (ne > 0) {
+  std::vector<MergeEntry> big;
+  MergeTable<kParamEntries> table;
+  const bool inline_table = (long long)batch * (depth + 1) <= kParamEntries;
+  if (!inline_table) big.resize((size_t)batch * (depth + 1));
+  int blocks = 0;
+  const int ne = merge_table(octrees_dev, in, batch, depth, inline_table ? table.e : big.data(), &blocks);
+  const MergeDst dst = merge_destination(merged, o, hdr);
+  OCNN_REQUIRE(ne > 0, "ocnn_octree_batch: the octrees have no nodes");
+  if (inline_table) {
+    OCNN_CUDA_OK(launch_chained(merge_param_kernel, dim3(blocks), dim3(256), 0, st, table, ne, dst));
+  } else {
     // the staging vector is pageable memory: the runtime has copied it out before returning
-    OCNN_CUDA_OK(cudaMemcpyAsync(workspace, entries.data(), sizeof(MergeEntry) * (size_t)ne,
+    OCNN_CUDA_OK(cudaMemcpyAsync(workspace, big.data(), sizeof(MergeEntry) * (size_t)ne,
                                  cudaMemcpyHostToDevice, st));
-    if (int rc = launch_merge(static_cast<const MergeEntry*>(workspace), ne, max_n,
-                              merge_destination(merged, o), st, "merge_kernel"))
-      return rc;
+    OCNN_CUDA_OK(launch_chained(merge_kernel, dim3(blocks), dim3(256), 0, st,
+                                static_cast<const MergeEntry*>(workspace), ne, dst));
   }
+  OCNN_LAUNCH_OK("merge_kernel");
   return ocnn_calc_neigh(out, merged, stream);
 }
 
@@ -277,20 +331,18 @@ extern "C" int ocnn_octree_batch_noalloc(const void* const* octrees_dev, const o
   uint8_t hdr[OCNN_HEADER_BYTES];
   merged_header(first_header_host, merged, hdr);
   if (header_host_out) memcpy(header_host_out, hdr, OCNN_HEADER_BYTES);
-  OCNN_CUDA_OK(cudaMemcpyAsync(o, hdr, OCNN_HEADER_BYTES, cudaMemcpyHostToDevice, st));
 
-  int max_n = 1;
-  const int ne = merge_table(octrees_dev, in, batch, depth, g_static_stage, &max_n);
-  if (ne > 0) {
-    // Only the first `ne` entries are read by the kernel and all of them are rewritten here, so
-    // nothing left over from an earlier call needs clearing.  The staging array is pageable
-    // memory: the runtime has copied it out when cudaMemcpyAsync returns, which is what lets the
-    // mutex be released at the end of this function.
-    OCNN_CUDA_OK(cudaMemcpyAsync(table_dev, g_static_stage, sizeof(MergeEntry) * (size_t)ne,
-                                 cudaMemcpyHostToDevice, st));
-    if (int rc = launch_merge(table_dev, ne, max_n, merge_destination(merged, o), st,
-                              "merge_kernel (built-in scratch)"))
-      return rc;
-  }
+  int blocks = 0;
+  const int ne = merge_table(octrees_dev, in, batch, depth, g_static_stage, &blocks);
+  OCNN_REQUIRE(ne > 0, "ocnn_octree_batch_noalloc: the octrees have no nodes");
+  // Only the first `ne` entries are read by the kernel and all of them are rewritten here, so
+  // nothing left over from an earlier call needs clearing.  The staging array is pageable
+  // memory: the runtime has copied it out when cudaMemcpyAsync returns, which is what lets the
+  // mutex be released at the end of this function.
+  OCNN_CUDA_OK(cudaMemcpyAsync(table_dev, g_static_stage, sizeof(MergeEntry) * (size_t)ne,
+                               cudaMemcpyHostToDevice, st));
+  OCNN_CUDA_OK(launch_chained(merge_kernel, dim3(blocks), dim3(256), 0, st,
+                              static_cast<const MergeEntry*>(table_dev), ne, merge_destination(merged, o, hdr)));
+  OCNN_LAUNCH_OK("merge_kernel (built-in scratch)");
   return ocnn_calc_neigh(out, merged, stream);
 }

@@ -115,6 +115,15 @@ class TransformCompose:
     self.points2octree = Points2Octree(**flags)
 
   def __call__(self, points, idx=None):
+    norm, transform, build = self.normalize_points, self.transform_points, self.points2octree
+    if (type(norm) is NormalizePoints and type(transform) is TransformPoints and type(build) is Points2Octree and
+        (norm.radius >= 0 or norm.bsphere == 'box')):
+      # the stock steps: one native call
+      angle, scale, jitter = transform.draw()
+      octree, points, inbox_mask = nn.prepare_cloud(
+          points, norm.radius if norm.radius >= 0 else -1.0, list(norm.center), angle, scale, jitter,
+          transform.offset, transform.normal_axis, *build._args())
+      return {'octree': octree, 'points': points, 'inbox_mask': inbox_mask}
     points = self.normalize_points(points)
     points, inbox_mask = self.transform_points(points)
     return {'octree': self.points2octree(points), 'points': points, 'inbox_mask': inbox_mask}

@@ -1484,42 +1484,57 @@ void euler_rotation(const float* angle, float* rot) {
   prod(rot, tmp, rz);
 }
 
-Tensor transform_points(Tensor data_in, vector<float> angle, vector<float> scale, vector<float> jitter,
-                        float offset, string normal_axis) {
-  PointsHeader h = read_points_header(data_in);
-  Tensor out = data_in.to(torch::kCUDA).contiguous().clone();
-  c10::cuda::CUDAGuard guard(out.device());
+// The two steps' parameters as the kernels take them.
+ocnn_point_transform transform_steps(vector<float> angle, vector<float> scale, vector<float> jitter, float offset,
+                                     const string& normal_axis) {
   angle = three(angle, "angle"); scale = three(scale, "scale"); jitter = three(jitter, "jitter");
   const float eps = 1.0e-10f;
-  float rot[9];
-  const bool do_rot = fabsf(angle[0]) > eps || fabsf(angle[1]) > eps || fabsf(angle[2]) > eps;
-  if (do_rot) euler_rotation(angle.data(), rot);
-  const bool do_jit = fabsf(jitter[0]) > eps || fabsf(jitter[1]) > eps || fabsf(jitter[2]) > eps;
-  const bool do_scale = scale[0] != 1.0f || scale[1] != 1.0f || scale[2] != 1.0f;
-  int orient = 0;
-  if (normal_axis == "x") orient = 1;
-  else if (normal_axis == "y") orient = 2;
-  else if (normal_axis == "z") orient = 3;
-  else if (normal_axis == "xyz") orient = 4;
-  OCNN_CALL(ocnn_points_transform(points_block(out, h, 0), points_block(out, h, 1), h.pt_num, offset,
-                                  do_rot ? rot : nullptr, do_jit ? jitter.data() : nullptr,
-                                  do_scale ? scale.data() : nullptr, orient, current_stream()));
+  ocnn_point_transform t;
+  memset(&t, 0, sizeof(t));
+  t.offset = offset;
+  t.rotate = fabsf(angle[0]) > eps || fabsf(angle[1]) > eps || fabsf(angle[2]) > eps;
+  if (t.rotate) euler_rotation(angle.data(), t.rot);
+  t.translate = fabsf(jitter[0]) > eps || fabsf(jitter[1]) > eps || fabsf(jitter[2]) > eps;
+  for (int j = 0; j < 3; ++j) { t.shift[j] = jitter[j]; t.scale[j] = scale[j]; }
+  if (normal_axis == "x") t.orient = 1;
+  else if (normal_axis == "y") t.orient = 2;
+  else if (normal_axis == "z") t.orient = 3;
+  else if (normal_axis == "xyz") t.orient = 4;
+  return t;
+}
+
+ocnn_point_transform normalize_steps(float radius, const vector<float>& center) {
+  TORCH_CHECK(radius >= 0.0f, "normalize_points: the radius must not be negative");
+  TORCH_CHECK(center.size() == 3, "normalize_points: center must hold 3 values");
+  ocnn_point_transform t;
+  memset(&t, 0, sizeof(t));
+  const float inv = 1.0f / radius;
+  for (int j = 0; j < 3; ++j) {
+    t.shift[j] = -center[j];
+    if (t.shift[j] != 0.0f) t.translate = 1;
+    t.scale[j] = inv;
+  }
+  return t;
+}
+
+Tensor apply_steps(Tensor data_in, const ocnn_point_transform& t) {
+  PointsHeader h = read_points_header(data_in);
+  Tensor out = data_in.is_cuda() ? data_in.contiguous().clone() : data_in.contiguous().to(torch::kCUDA);
+  c10::cuda::CUDAGuard guard(out.device());
+  OCNN_CALL(ocnn_points_transform(points_block(out, h, 0), points_block(out, h, 1), h.pt_num, t.offset,
+                                  t.rotate ? t.rot : nullptr, t.translate ? t.shift : nullptr,
+                                  t.scale[0] != 1.0f || t.scale[1] != 1.0f || t.scale[2] != 1.0f ? t.scale : nullptr,
+                                  t.orient, current_stream()));
   return out;
 }
 
+Tensor transform_points(Tensor data_in, vector<float> angle, vector<float> scale, vector<float> jitter,
+                        float offset, string normal_axis) {
+  return apply_steps(data_in, transform_steps(angle, scale, jitter, offset, normal_axis));
+}
+
 Tensor normalize_points(Tensor data_in, float radius, vector<float> center) {
-  TORCH_CHECK(radius >= 0.0f, "normalize_points: the radius must not be negative");
-  TORCH_CHECK(center.size() == 3, "normalize_points: center must hold 3 values");
-  PointsHeader h = read_points_header(data_in);
-  Tensor out = data_in.to(torch::kCUDA).contiguous().clone();
-  c10::cuda::CUDAGuard guard(out.device());
-  const float dis[3] = {-center[0], -center[1], -center[2]};
-  const bool do_shift = dis[0] != 0.0f || dis[1] != 0.0f || dis[2] != 0.0f;
-  const float inv = 1.0f / radius;
-  const float sc[3] = {inv, inv, inv};
-  OCNN_CALL(ocnn_points_transform(points_block(out, h, 0), points_block(out, h, 1), h.pt_num, 0.f, nullptr,
-                                  do_shift ? dis : nullptr, inv != 1.0f ? sc : nullptr, 0, current_stream()));
-  return out;
+  return apply_steps(data_in, normalize_steps(radius, center));
 }
 
 vector<Tensor> clip_points(Tensor data_in, vector<float> bbmin, vector<float> bbmax) {
@@ -1543,19 +1558,36 @@ vector<Tensor> clip_points(Tensor data_in, vector<float> bbmin, vector<float> bb
   return {out, mask};
 }
 
-vector<float> bounding_sphere(Tensor data_in, string method) {
-  TORCH_CHECK(method != "sphere", "bounding_sphere(method='sphere') needs the reference's external "
-              "Miniball code and is not implemented; use method='box'");
-  PointsHeader h = read_points_header(data_in);
-  Tensor src = data_in.to(torch::kCUDA).contiguous();
-  c10::cuda::CUDAGuard guard(src.device());
-  const size_t ws_bytes = ocnn_points_bbox_workspace_bytes();
-  Tensor ws = torch::empty({(int64_t)ws_bytes}, src.options());
-  Tensor box = torch::empty({6}, src.options().dtype(torch::kFloat32));
-  OCNN_CALL(ocnn_points_bbox(points_block(src, h, 0), h.pt_num, box.data_ptr<float>(), ws.data_ptr(),
-                             ws_bytes, current_stream()));
-  Tensor b = box.cpu();
-  const float* p = b.data_ptr<float>();
+// The bounding box of a cloud that is still in host memory: looking at it here costs less than the
+// upload, two kernels and read-back it would take on the device before the cloud is needed there.
+void host_box(const float* xyz, int64_t n, float (&box)[6]) {
+  float lo[12], hi[12];
+  for (int k = 0; k < 12; ++k) { lo[k] = INFINITY; hi[k] = -INFINITY; }
+  int64_t i = 0;
+  for (; i + 4 <= n; i += 4)            // four points = twelve independent chains
+    for (int k = 0; k < 12; ++k) {
+      const float v = xyz[3 * i + k];
+      lo[k] = v < lo[k] ? v : lo[k];
+      hi[k] = v > hi[k] ? v : hi[k];
+    }
+  for (; i < n; ++i)
+    for (int k = 0; k < 3; ++k) {
+      const float v = xyz[3 * i + k];
+      lo[k] = v < lo[k] ? v : lo[k];
+      hi[k] = v > hi[k] ? v : hi[k];
+    }
+  for (int k = 0; k < 3; ++k) {
+    box[k] = lo[k];
+    box[3 + k] = hi[k];
+    for (int q = 1; q < 4; ++q) {
+      box[k] = lo[3 * q + k] < box[k] ? lo[3 * q + k] : box[k];
+      box[3 + k] = hi[3 * q + k] > box[3 + k] ? hi[3 * q + k] : box[3 + k];
+    }
+  }
+}
+
+// (radius, centre) of the sphere around a box
+vector<float> box_sphere(const float (&p)[6]) {
   float radius = 0.f, center[3];
   for (int j = 0; j < 3; ++j) {
     center[j] = (p[3 + j] + p[j]) / 2.0f;
@@ -1564,6 +1596,28 @@ vector<float> bounding_sphere(Tensor data_in, string method) {
   }
   radius = sqrtf(radius + 1.0e-20f);
   return {radius, center[0], center[1], center[2]};
+}
+
+vector<float> bounding_sphere(Tensor data_in, string method) {
+  TORCH_CHECK(method != "sphere", "bounding_sphere(method='sphere') needs the reference's external "
+              "Miniball code and is not implemented; use method='box'");
+  PointsHeader h = read_points_header(data_in);
+  float box[6];
+  if (data_in.is_cuda()) {
+    Tensor src = data_in.contiguous();
+    c10::cuda::CUDAGuard guard(src.device());
+    const size_t ws_bytes = ocnn_points_bbox_workspace_bytes();
+    Tensor ws = torch::empty({(int64_t)ws_bytes}, src.options());
+    Tensor dev = torch::empty({6}, src.options().dtype(torch::kFloat32));
+    OCNN_CALL(ocnn_points_bbox(points_block(src, h, 0), h.pt_num, dev.data_ptr<float>(), ws.data_ptr(),
+                               ws_bytes, current_stream()));
+    Tensor b = dev.cpu();
+    memcpy(box, b.data_ptr<float>(), sizeof(box));
+  } else {
+    Tensor src = data_in.contiguous();
+    host_box(points_block(src, h, 0), h.pt_num, box);
+  }
+  return box_sphere(box);
 }
 
 int points_prop_index(const string& property) {
@@ -1628,8 +1682,10 @@ struct BuildFlags {
 };
 
 // Build the (merged or single) octree of clouds stored back to back in one CUDA uint8 buffer.
+// kept (one cloud): a mapped word that holds, once the stream has come to it, how many of the cloud's
+// points there really are; the plan is made again when they are fewer.
 Tensor build_from_device(const Tensor& packed_dev, const vector<CloudInfo>& clouds,
-                         const BuildFlags& f, bool merged) {
+                         const BuildFlags& f, bool merged, const int32_t* kept = nullptr) {
   TORCH_CHECK(!f.adaptive, "points2octree: adaptive octrees are not implemented");
   TORCH_CHECK(!f.node_feature, "points2octree: node_feature=True is not implemented");
   TORCH_CHECK(!f.extrapolate, "points2octree: extrapolate=True is not implemented");
@@ -1676,6 +1732,10 @@ Tensor build_from_device(const Tensor& packed_dev, const vector<CloudInfo>& clou
   Tensor ws = torch::empty({(int64_t)ws_bytes}, opts);
   ocnn_octree_meta meta;
   OCNN_CALL(ocnn_octree_build_plan(&pb, &prm, ws.data_ptr(), ws_bytes, &meta, current_stream()));
+  if (kept != nullptr && *static_cast<const volatile int32_t*>(kept) != offsets[1]) {
+    offsets[1] = *static_cast<const volatile int32_t*>(kept);
+    OCNN_CALL(ocnn_octree_build_plan(&pb, &prm, ws.data_ptr(), ws_bytes, &meta, current_stream()));
+  }
   Tensor out = torch::empty({(int64_t)meta.ptr_dis[OCNN_PROP_COUNT]}, opts);
   uint8_t raw[OCNN_HEADER_BYTES];
   OCNN_CALL(ocnn_octree_build_emit(&pb, &prm, &meta, ws.data_ptr(), ws_bytes, out.data_ptr(),
@@ -1805,6 +1865,92 @@ Tensor points2octree_batch(vector<Tensor> points, int depth, int full_depth, boo
                             make_flags(depth, full_depth, node_dis, node_feature, split_label, adaptive,
                                        adp_depth, th_normal, th_distance, extrapolate, save_pts, key2xyz),
                             true);
+}
+
+// ---- a data loader's sample: normalise + transform + clip + octree in one call -----------------------
+// Pinned memory of a host thread: a staging area for uploads (a cloud larger than it is uploaded as it
+// lies) and a word that kernels answer in.  Whoever uses it waits for its stream before returning.
+struct HostStage {
+  static constexpr size_t kBytes = 4 << 20;
+  uint8_t* bytes = nullptr;
+  int32_t* word = nullptr;
+  ~HostStage() {
+    if (bytes) cudaFreeHost(bytes);
+    if (word) cudaFreeHost(word);
+  }
+  bool ready() {
+    void* p = nullptr;
+    if (word == nullptr && cudaHostAlloc(&p, 64, cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess)
+      word = static_cast<int32_t*>(p);
+    if (bytes == nullptr && cudaHostAlloc(&p, kBytes, cudaHostAllocPortable) == cudaSuccess)
+      bytes = static_cast<uint8_t*>(p);
+    cudaGetLastError();
+    return word != nullptr;
+  }
+};
+
+// (octree, points, mask) of TransformCompose: NormalizePoints (bounding box when radius < 0),
+// TransformPoints with the drawn parameters, the clip to (-1, 1)^3 and points2octree — the values of
+// the four calls bit for bit, with one upload, two launches for the points, and one wait: the octree
+// is planned for all points, which the clip nearly always keeps, and planned again if it did not.
+// (Call by call a 5 k-point cloud took five round trips, 24 launches and 12 copies.)
+std::tuple<Tensor, Tensor, Tensor> prepare_cloud(
+    Tensor points, float radius, vector<float> center, vector<float> angle, vector<float> scale,
+    vector<float> jitter, float offset, string normal_axis, int depth, int full_depth, bool node_dis,
+    bool node_feature, bool split_label, bool adaptive, int adp_depth, float th_normal, float th_distance,
+    bool extrapolate, bool save_pts, bool key2xyz) {
+  PointsHeader h = read_points_header(points);
+  const BuildFlags flags = make_flags(depth, full_depth, node_dis, node_feature, split_label, adaptive, adp_depth,
+                                      th_normal, th_distance, extrapolate, save_pts, key2xyz);
+  Tensor host_pts = points.contiguous();
+  if (radius < 0) {
+    vector<float> sphere = bounding_sphere(host_pts, "box");
+    radius = sphere[0];
+    center = {sphere[1], sphere[2], sphere[3]};
+  }
+  const ocnn_point_transform first = normalize_steps(radius, center);
+  const ocnn_point_transform second = transform_steps(angle, scale, jitter, offset, normal_axis);
+  static thread_local HostStage stage;
+  TORCH_CHECK(stage.ready(), "prepare_cloud: no pinned host memory");
+  const c10::Device device = points.is_cuda() ? points.device()
+                                              : c10::Device(c10::kCUDA, c10::cuda::current_device());
+  c10::cuda::CUDAGuard guard(device);
+  cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
+  struct Wait {                     // the staging area is free again when this call is over
+    cudaStream_t st;
+    ~Wait() { cudaStreamSynchronize(st); }
+  };
+  auto opts = torch::dtype(torch::kUInt8).device(device);
+  const int64_t bytes = host_pts.numel();
+  Tensor work = torch::empty({bytes}, opts), out = torch::empty({bytes}, opts);
+  Tensor mask = torch::empty({(int64_t)h.pt_num}, opts.dtype(torch::kInt32));
+  const size_t ws_bytes = ocnn_points_clip_workspace_bytes(h.pt_num);
+  Tensor ws = torch::empty({(int64_t)ws_bytes}, opts);
+  Tensor octree;
+  {
+    Wait wait{st};
+    const void* in = host_pts.data_ptr();
+    if (!points.is_cuda()) {
+      const void* from = in;
+      if (stage.bytes != nullptr && (size_t)bytes <= HostStage::kBytes && !host_pts.is_pinned()) {
+        memcpy(stage.bytes, in, bytes);
+        from = stage.bytes;
+      }
+      TORCH_CHECK(cudaMemcpyAsync(work.data_ptr(), from, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess,
+                  "prepare_cloud: the upload failed");
+      in = work.data_ptr();
+    }
+    int64_t offsets[4];
+    int channels[4];
+    for (int t = 0; t < 4; ++t) { offsets[t] = h.ptr_dis[t]; channels[t] = h.channels[t]; }
+    const float lo[3] = {-1.f, -1.f, -1.f}, hi[3] = {1.f, 1.f, 1.f};
+    OCNN_CALL(ocnn_points_prepare(in, work.data_ptr(), out.data_ptr(), bytes, h.pt_num, offsets, channels, &first,
+                                  &second, lo, hi, mask.data_ptr<int32_t>(), ws.data_ptr(), ws_bytes, stage.word,
+                                  st));
+    CloudInfo cloud{0, h};
+    octree = build_from_device(out, {cloud}, flags, false, stage.word);
+  }
+  return std::make_tuple(octree, out, mask);
 }
 
 // ---- octree_batch -------------------------------------------------------------------------------------
@@ -2415,6 +2561,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("points2octree_batch", &points2octree_batch,
         "build the merged batch octree of a list of point clouds in one pass");
   m.def("points_pack", &points_pack, py::arg("points"), py::arg("pin") = false);
+  m.def("prepare_cloud", &prepare_cloud, py::call_guard<py::gil_scoped_release>());
   // (the GIL is released: the build blocks once on its stream, and a second Python thread may be
   // enqueueing a forward pass meanwhile)
   m.def("points2octree_packed", &points2octree_packed, py::call_guard<py::gil_scoped_release>());

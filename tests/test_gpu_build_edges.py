@@ -37,7 +37,7 @@ def check(ocnn, pts, depth, full, key_bits):
   assert got.shape == want.shape and np.array_equal(got, want)
 
 
-@pytest.mark.parametrize('depth,full,key_bits', [(2, 2, 64), (3, 1, 32), (5, 2, 64), (6, 2, 32), (6, 4, 64), (7, 2, 64),
+@pytest.mark.parametrize('depth,full,key_bits', [(1, 1, 64), (2, 1, 32), (2, 2, 64), (3, 1, 32), (5, 2, 64), (6, 2, 32), (6, 4, 64), (7, 2, 64),
                                                  (8, 2, 32), (9, 2, 64), (10, 3, 64), (11, 2, 64)])
 def test_chunk_sizes(ocnn, depth, full, key_bits):
   check(ocnn, clouds_of([1, 2047, 2048, 2049, 4097, 700], 40 + depth), depth, full, key_bits)
