@@ -530,7 +530,7 @@ int ocnn_octree_align_backward(const void* dst_grad_dev, void* src_grad_dev, con
  * then displace / rotate / translate / scale / orient, then clip to the open box): every step as in
  * ocnn_points_transform and ocnn_points_clip, bit for bit. in, work, out: whole points buffers of `bytes`
  * bytes (work may be in; out must not); offsets / channels of the four properties, coordinates and
- * normals one behind the other; mask [n]; workspace of ocnn_points_clip_workspace_bytes; total_out: a
+ * normals one behind the other; mask [n]; workspace: one int per 256 points; total_out: a
  * device-visible word (mapped host memory will do) that receives the kept count. */
 typedef struct ocnn_point_transform {
   float offset;

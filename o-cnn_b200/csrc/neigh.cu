@@ -88,7 +88,9 @@ __global__ void __launch_bounds__(kNeighWarps * 32) neigh_split_kernel(
     int* __restrict__ out, const int* __restrict__ neigh, const int* __restrict__ child,
     long long ngroups) {
   grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
-  __shared__ int cblk[kNeighWarps][64];     // child group of each cell of the parents' block
+  // 8 * child group of each cell of the parents' block, -1 where there is none: an output is that
+  // value | octant either way
+  __shared__ int cblk[kNeighWarps][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // child-level block position j = (x,y,z) in 0..3 -> which parent-level cell (tap, as a
   // (tx<<4)|(ty<<2)|tz code relative to the parent) and which octant inside it; two per lane
@@ -123,7 +125,7 @@ __global__ void __launch_bounds__(kNeighWarps * 32) neigh_split_kernel(
   cells(first + stride, cell, mine_next);
   for (long long g = first; g < ngroups; g += stride) {
 #pragma unroll
-    for (int k = 0; k < 2; ++k) cblk[warp][lane + 32 * k] = kid[k];
+    for (int k = 0; k < 2; ++k) cblk[warp][lane + 32 * k] = kid[k] >= 0 ? kid[k] << 3 : -1;
     __syncwarp();
     kids(cell, kid);
     int mine_after;
@@ -135,10 +137,7 @@ __global__ void __launch_bounds__(kNeighWarps * 32) neigh_split_kernel(
       const int octcode = ((o & 4) << 2) | ((o & 2) << 1) | (o & 1);
       int* dst = out + ((long long)l0 << 6);
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int c = cblk[warp][tapcode[k] + octcode];
-        dst[lane + 32 * k] = c >= 0 ? (c << 3) + oct[k] : -1;
-      }
+      for (int k = 0; k < 2; ++k) dst[lane + 32 * k] = cblk[warp][tapcode[k] + octcode] | oct[k];
     }
     mine = mine_next;
     mine_next = mine_after;

@@ -219,15 +219,12 @@ struct PrepareCloudArgs {
 __global__ void __launch_bounds__(kClipThreads) prepare_cloud_kernel(const __grid_constant__ PrepareCloudArgs a) {
   grid_dependency_wait();
   __shared__ int warp_sum[kClipThreads / 32];
-  const long long base = (long long)blockIdx.x * kClipTile;
+  const long long i = (long long)blockIdx.x * kClipThreads + threadIdx.x;
   const bool has_n = a.normal_off >= 0;
   const float* xyz = reinterpret_cast<const float*>(a.in + a.xyz_off);
   const float* nrm = reinterpret_cast<const float*>(a.in + a.normal_off);
   int mine = 0;
-#pragma unroll
-  for (int j = 0; j < kClipItems; ++j) {
-    const long long i = base + (long long)j * kClipThreads + threadIdx.x;
-    if (i >= a.n) continue;
+  if (i < a.n) {
     float p[3] = {xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]};
     float q[3] = {0.f, 0.f, 0.f};
     if (has_n) { q[0] = nrm[3 * i]; q[1] = nrm[3 * i + 1]; q[2] = nrm[3 * i + 2]; }
@@ -245,7 +242,7 @@ __global__ void __launch_bounds__(kClipThreads) prepare_cloud_kernel(const __gri
     const int in = (a.box.lo[0] < p[0] && p[0] < a.box.hi[0] && a.box.lo[1] < p[1] && p[1] < a.box.hi[1] &&
                     a.box.lo[2] < p[2] && p[2] < a.box.hi[2]) ? 1 : 0;
     a.mask[i] = in;
-    mine += in;
+    mine = in;
   }
   // everything else of the buffer: the header before the coordinates, features and labels after them
   const long long tail = a.xyz_off + 12 * a.n * (has_n ? 2 : 1);
@@ -282,7 +279,6 @@ __global__ void __launch_bounds__(kClipThreads) prepare_move_kernel(long long n,
   grid_dependency_wait();
   __shared__ int red[2][kClipThreads / 32];
   __shared__ int warp_base[kClipThreads / 32];
-  __shared__ int carry;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int below = 0, all = 0;
   for (int t = threadIdx.x; t < tiles; t += kClipThreads) {
@@ -313,29 +309,18 @@ __global__ void __launch_bounds__(kClipThreads) prepare_move_kernel(long long n,
     return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *pt_num_out = total;
-  if (threadIdx.x == 0) carry = first;
-  const long long base = (long long)blockIdx.x * kClipTile;
-  for (int j = 0; j < kClipItems; ++j) {   // (as clip_move_kernel)
-    const long long i = base + (long long)j * kClipThreads + threadIdx.x;
-    const int in = (i < n) ? mask[i] : 0;
-    const unsigned ballot = __ballot_sync(0xffffffffu, in);
-    if (lane == 0) warp_base[warp] = __popc(ballot);
-    __syncthreads();
-    int before = 0, round_total = 0;
-    for (int w = 0; w < kClipThreads / 32; ++w) {
-      if (w < warp) before += warp_base[w];
-      round_total += warp_base[w];
+  const long long i = (long long)blockIdx.x * kClipThreads + threadIdx.x;
+  const int in = (i < n) ? mask[i] : 0;
+  const unsigned ballot = __ballot_sync(0xffffffffu, in);
+  if (lane == 0) warp_base[warp] = __popc(ballot);
+  __syncthreads();
+  int rank = first + __popc(ballot & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) rank += warp_base[w];
+  if (in) {
+    for (int t = 0; t < 4; ++t) {
+      const int ch = pr.channels[t];
+      for (int c = 0; c < ch; ++c) pr.dst[t][(long long)rank * ch + c] = pr.src[t][i * ch + c];
     }
-    const int rank = carry + before + __popc(ballot & ((1u << lane) - 1u));
-    if (in) {
-      for (int t = 0; t < 4; ++t) {
-        const int ch = pr.channels[t];
-        for (int c = 0; c < ch; ++c) pr.dst[t][(long long)rank * ch + c] = pr.src[t][i * ch + c];
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) carry += round_total;
-    __syncthreads();
   }
   grid_dependency_trigger();
 }
@@ -429,10 +414,10 @@ int ocnn_points_prepare(const void* in, void* work, void* out, int64_t bytes, in
                "%s: coordinates and normals must lie one behind the other", who);
   OCNN_REQUIRE(first->orient >= 0 && first->orient <= 4 && second->orient >= 0 && second->orient <= 4,
                "%s: orient must be 0..4", who);
-  if (workspace == nullptr || workspace_bytes < ocnn_points_clip_workspace_bytes(n))
+  const int tiles = ceil_div(n, kClipThreads);       // one point per thread: a cloud is a few thousand points
+  if (workspace == nullptr || workspace_bytes < (size_t)tiles * sizeof(int))
     return fail(OCNN_ERR_CAPACITY, "%s: workspace of %zu bytes, need %zu", who, workspace_bytes,
-                ocnn_points_clip_workspace_bytes(n));
-  const int tiles = ceil_div(n, kClipTile);
+                (size_t)tiles * sizeof(int));
   PrepareCloudArgs a;
   a.in = static_cast<const uint8_t*>(in);
   a.work = static_cast<uint8_t*>(work);

@@ -1916,19 +1916,20 @@ std::tuple<Tensor, Tensor, Tensor> prepare_cloud(
                                               : c10::Device(c10::kCUDA, c10::cuda::current_device());
   c10::cuda::CUDAGuard guard(device);
   cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
-  struct Wait {                     // the staging area is free again when this call is over
-    cudaStream_t st;
-    ~Wait() { cudaStreamSynchronize(st); }
+  struct Wait {                     // the staging area is free again when this call is over: the plan
+    cudaStream_t st;                // has waited for the stream, an exception on the way there does so here
+    bool done;
+    ~Wait() { if (!done) cudaStreamSynchronize(st); }
   };
   auto opts = torch::dtype(torch::kUInt8).device(device);
   const int64_t bytes = host_pts.numel();
   Tensor work = torch::empty({bytes}, opts), out = torch::empty({bytes}, opts);
   Tensor mask = torch::empty({(int64_t)h.pt_num}, opts.dtype(torch::kInt32));
-  const size_t ws_bytes = ocnn_points_clip_workspace_bytes(h.pt_num);
+  const size_t ws_bytes = ((size_t)h.pt_num + 255) / 256 * 4;
   Tensor ws = torch::empty({(int64_t)ws_bytes}, opts);
   Tensor octree;
   {
-    Wait wait{st};
+    Wait wait{st, false};
     const void* in = host_pts.data_ptr();
     if (!points.is_cuda()) {
       const void* from = in;
@@ -1949,6 +1950,7 @@ std::tuple<Tensor, Tensor, Tensor> prepare_cloud(
                                   st));
     CloudInfo cloud{0, h};
     octree = build_from_device(out, {cloud}, flags, false, stage.word);
+    wait.done = true;
   }
   return std::make_tuple(octree, out, mask);
 }
