@@ -1,12 +1,14 @@
-"""Building blocks of the reference's networks (pytorch/ocnn/modules.py:1-345), forward only:
+"""Building blocks of the reference's networks (pytorch/ocnn/modules.py:1-345):
 convolution + BatchNorm (+ ReLU) blocks, 1x1 blocks, the two residual blocks, nearest /
 trilinear interpolation at points, and `octree_feature`.  Class names, constructor arguments and
 parameter names follow the reference, so its state_dicts load.
 
 In eval mode a block folds its BatchNorm (running statistics) and ReLU into the convolution
 kernel's epilogue — one launch per block instead of three; set `FUSE_EVAL_BN = False` to run the
-torch BatchNorm / ReLU modules after the convolution instead.  In training mode the torch modules
-always run (the convolution itself has no backward here).
+torch BatchNorm / ReLU modules after the convolution instead.  In training mode an fp32 block is one
+native autograd node around the same convolution kernel and torch's own BatchNorm (`_train_block`);
+under autocast, with hooks on the inner modules, or with another normalisation the modules run one
+by one.
 """
 import torch
 from torch import nn as _nn
@@ -14,10 +16,33 @@ from torch import nn as _nn
 from . import nn
 from .octree_conv import OctreeConv, OctreeDeconv, bn_vectors, tc_status
 from .octree_pool import OctreeMaxPool
+from .octree_pad import octree_depad
 from .octree_pad import OctreeTile  # noqa: F401  (re-exported: the reference defines it here)
 
 bn_momentum, bn_eps = 0.01, 0.001       # pytorch/ocnn/modules.py:5
 FUSE_EVAL_BN = True
+
+
+def _trainable(data, weight, bn, residual):
+  """Whether a block in training mode can run as the one native autograd node: plain fp32 on the GPU,
+  a BatchNorm with parameters and running statistics, no hooks that would have to see the modules inside."""
+  return (torch.is_grad_enabled() and bn.training and data.is_cuda and data.dtype == torch.float32 and
+          data.is_contiguous() and weight.dtype == torch.float32 and weight.is_cuda and bn.affine and
+          bn.track_running_stats and bn.momentum is not None and bn.weight.dtype == torch.float32 and
+          (residual is None or residual.dtype == torch.float32) and not torch.is_autocast_enabled() and
+          not _hooked(bn))
+
+
+def _hooked(module):
+  return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or
+              module._backward_pre_hooks)
+
+
+def _train_block(data, weight, bias, bn, residual, octree, kind, depth, cout, kernel_size, stride, nempty, relu):
+  if bn.num_batches_tracked is not None:
+    bn.num_batches_tracked.add_(1)
+  return nn.train_block(data, weight, bias, bn.weight, bn.bias, residual, bn.running_mean, bn.running_var,
+                        bn.momentum, bn.eps, octree, kind, depth, cout, kernel_size, stride, nempty, relu)
 
 
 def _folded(bn):
@@ -50,6 +75,13 @@ class _OctreeBlock(_nn.Module):
       if not op.is_conv_layer() and op.stride == 2 and not op.nempty:
         data_in = nn.octree_depad(data_in, octree, op.depth)
       return op._run(data_in, octree, self.bn, residual, relu)
+    if foldable and type(self.bn) is _nn.BatchNorm2d and type(op) in (OctreeConv, OctreeDeconv) and \
+        _trainable(data_in, op.weights, self.bn, residual) and not _hooked(op):
+      assert data_in.size(1) == op.channel_in
+      if not op.is_conv_layer() and op.stride == 2 and not op.nempty:
+        data_in = octree_depad(data_in, octree, op.depth)
+      return _train_block(data_in, op.weights, None, self.bn, residual, octree, int(not op.is_conv_layer()),
+                          op.depth, op.channel_out, op.kernel_size, op.stride, op.nempty, relu)
     out = self.bn(op(data_in, octree))
     if residual is not None:
       out = out + residual
@@ -166,6 +198,11 @@ class _Conv1x1Block(_nn.Module):
     relu = self.with_relu if relu is None else relu
     if FUSE_EVAL_BN and not self.training:
       return self.conv1x1.run(data_in, self.bn, residual, relu)
+    conv = self.conv1x1.conv1x1
+    if type(self.bn) is _nn.BatchNorm2d and type(self.conv1x1) is OctreeConv1x1 and \
+        _trainable(data_in, conv.weight, self.bn, residual) and not (_hooked(conv) or _hooked(self.conv1x1)):
+      return _train_block(data_in, conv.weight, conv.bias, self.bn, residual, None, 2, 0, conv.weight.shape[0],
+                          [1], 1, False, relu)
     out = self.bn(self.conv1x1(data_in))
     if residual is not None:
       out = out + residual

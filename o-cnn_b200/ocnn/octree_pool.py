@@ -83,6 +83,8 @@ class OctreeMaxPool(OctreePoolBase):
         not (torch.is_grad_enabled() and data.requires_grad)):
       with torch.no_grad():      # both steps in one kernel
         return nn.octree_max_pool_pad(data, octree, self.depth)
+    if not self.return_indices and data.dtype == torch.float32 and torch.is_grad_enabled() and data.requires_grad:
+      return nn.train_max_pool(data, octree, self.depth)      # both steps as one autograd node
     pool, mask = octree_max_pool(data, octree, self.depth)
     output = octree_pad(pool, octree, self.depth - 1)
     return output if not self.return_indices else (output, mask)

@@ -1246,6 +1246,142 @@ Tensor global_pool_fc(Tensor data_in, Tensor weights, c10::optional<Tensor> bias
   return out;
 }
 
+// ---- training blocks ----------------------------------------------------------------------------------
+// The autograd forms of a block as one node each: (de)convolution or 1x1 layer + BatchNorm (batch
+// statistics) + residual + ReLU, and pool + pad.  The arithmetic is that of the separate modules, call
+// by call (torch's BatchNorm, the same convolution kernels), so results are bit-identical; what goes
+// away is host time: six autograd nodes, two of them in Python, and the modules around them were about
+// 150 us per block and direction, and a training step was bound by them.
+using torch::autograd::AutogradContext;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+
+struct TrainBlock : public torch::autograd::Function<TrainBlock> {
+  // kind: 0 convolution, 1 deconvolution, 2 1x1 layer
+  static Variable forward(AutogradContext* ctx, const Tensor& data, const Tensor& weight,
+                          const c10::optional<Tensor>& bias, const Tensor& bn_weight, const Tensor& bn_bias,
+                          const c10::optional<Tensor>& residual, const Tensor& running_mean,
+                          const Tensor& running_var, double momentum, double eps,
+                          const c10::optional<Tensor>& octree, int64_t kind, int64_t depth,
+                          int64_t num_output, const vector<int64_t>& kernel_size, int64_t stride, bool nempty,
+                          bool relu) {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    const vector<int> ks(kernel_size.begin(), kernel_size.end());
+    Tensor z;
+    if (kind == 2) {
+      z = at::conv1d(data.squeeze(-1), weight, bias).unsqueeze(-1);
+    } else if (kind == 1) {
+      z = octree_deconv(data, weight, *octree, (int)depth, (int)num_output, ks, (int)stride, nempty, true);
+    } else {
+      z = octree_conv(data, weight, *octree, (int)depth, (int)num_output, ks, (int)stride, nempty, true);
+    }
+    TORCH_CHECK_VALUE(z.numel() > z.size(1), "Expected more than 1 value per channel when training, got input size ",
+                      z.sizes());
+    Tensor out, save_mean, save_var, reserve;
+    int64_t impl = 0;
+    std::tie(out, save_mean, save_var, reserve, impl) =
+        at::_batch_norm_impl_index(z, bn_weight, bn_bias, running_mean, running_var, /*training=*/true, momentum,
+                                   eps, at::globalContext().userEnabledCuDNN());
+    if (residual.has_value() && residual->defined()) out = at::add(out, *residual);
+    if (relu) at::relu_(out);
+    ctx->save_for_backward({data, weight, z, bn_weight, save_mean, save_var, reserve, relu ? out : Tensor(),
+                            octree.has_value() ? *octree : Tensor(), running_mean, running_var});
+    ctx->saved_data["impl"] = impl;
+    ctx->saved_data["eps"] = eps;
+    ctx->saved_data["kind"] = kind;
+    ctx->saved_data["depth"] = depth;
+    ctx->saved_data["num_output"] = num_output;
+    ctx->saved_data["ks"] = kernel_size;
+    ctx->saved_data["stride"] = stride;
+    ctx->saved_data["nempty"] = nempty;
+    ctx->saved_data["bias"] = bias.has_value() && bias->defined();
+    ctx->saved_data["residual"] = residual.has_value() && residual->defined();
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &data = saved[0], &weight = saved[1], &z = saved[2], &bn_weight = saved[3], &out = saved[7],
+                 &octree = saved[8];
+    const int64_t kind = ctx->saved_data["kind"].toInt();
+    const bool has_bias = ctx->saved_data["bias"].toBool(), has_res = ctx->saved_data["residual"].toBool();
+    // (positions among the tensor inputs that were given)
+    int at_input = 0;
+    const bool need_data = ctx->needs_input_grad(at_input++), need_weight = ctx->needs_input_grad(at_input++);
+    const bool need_bias = has_bias && ctx->needs_input_grad(at_input);
+    at_input += has_bias ? 1 : 0;
+    Tensor g = grads[0];
+    if (out.defined()) g = at::threshold_backward(g, out, 0);
+    variable_list res(18);
+    if (has_res) res[5] = g;
+    Tensor gz, gbw, gbb;
+    std::tie(gz, gbw, gbb) = at::_batch_norm_impl_index_backward(
+        ctx->saved_data["impl"].toInt(), z, g, bn_weight, saved[9], saved[10], saved[4], saved[5], /*train=*/true,
+        ctx->saved_data["eps"].toDouble(), {true, true, true}, saved[6]);
+    res[3] = gbw;
+    res[4] = gbb;
+    gz = gz.contiguous();
+    if (kind == 2) {
+      const bool ours = own_weight_grad(weight, data);
+      if (need_data || need_bias || (need_weight && !ours)) {
+        c10::optional<at::IntArrayRef> bias_sizes;
+        vector<int64_t> bs = {weight.size(0)};
+        if (has_bias) bias_sizes = bs;
+        auto gr = at::convolution_backward(gz.squeeze(-1), data.squeeze(-1), weight, bias_sizes, {1}, {0}, {1}, false,
+                                           {0}, 1, {need_data, need_weight && !ours, need_bias});
+        if (need_data) res[0] = std::get<0>(gr).unsqueeze(-1);
+        if (need_weight && !ours) res[1] = std::get<1>(gr);
+        if (need_bias) res[2] = std::get<2>(gr);
+      }
+      if (need_weight && ours) res[1] = pointwise_conv_weight_grad(data, gz).view_as(weight);
+    } else {
+      const auto k64 = ctx->saved_data["ks"].toIntVector();
+      const vector<int> ks(k64.begin(), k64.end());
+      auto gr = conv_grad_impl(data, weight, octree, gz, (int)ctx->saved_data["depth"].toInt(),
+                               (int)ctx->saved_data["num_output"].toInt(), ks,
+                               (int)ctx->saved_data["stride"].toInt(), ctx->saved_data["nempty"].toBool(), kind == 1,
+                               need_data, need_weight);
+      res[0] = gr[0];
+      res[1] = gr[1];
+    }
+    return res;
+  }
+
+  // At 64 to 128 output channels cuDNN forms a 1x1 layer's weight gradient with a direct fp32 kernel (16 ->
+  // 64 at 107 k nodes: 395 us); ours is used there.  Elsewhere cuDNN takes a GEMM (about 55 us).
+  static bool own_weight_grad(const Tensor& weight, const Tensor& data) {
+    return weight.size(0) >= 64 && weight.size(0) <= 128 && weight.scalar_type() == torch::kFloat32 &&
+           data.scalar_type() == torch::kFloat32 && data.is_contiguous();
+  }
+};
+
+Tensor train_block(Tensor data, Tensor weight, c10::optional<Tensor> bias, Tensor bn_weight, Tensor bn_bias,
+                   c10::optional<Tensor> residual, Tensor running_mean, Tensor running_var, double momentum,
+                   double eps, c10::optional<Tensor> octree, int64_t kind, int64_t depth, int64_t num_output,
+                   vector<int64_t> kernel_size, int64_t stride, bool nempty, bool relu) {
+  return TrainBlock::apply(data, weight, bias, bn_weight, bn_bias, residual, running_mean, running_var, momentum, eps,
+                           octree, kind, depth, num_output, kernel_size, stride, nempty, relu);
+}
+
+// OctreeMaxPool: pool level `depth`, pad to every node of the level above.
+struct TrainPool : public torch::autograd::Function<TrainPool> {
+  static Variable forward(AutogradContext* ctx, const Tensor& data, const Tensor& octree, int64_t depth) {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    auto pooled = octree_max_pool(data.contiguous(), octree, (int)depth);
+    ctx->save_for_backward({pooled[1], octree});
+    ctx->saved_data["depth"] = depth;
+    return octree_pad(pooled[0], octree, (int)depth - 1, 0.f);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const int depth = (int)ctx->saved_data["depth"].toInt();
+    Tensor g = octree_depad(grads[0].contiguous(), saved[1], depth - 1);
+    return {octree_max_unpool(g.contiguous(), saved[0], saved[1], depth), Tensor(), Tensor()};
+  }
+};
+
+Tensor train_max_pool(Tensor data, Tensor octree, int64_t depth) { return TrainPool::apply(data, octree, depth); }
+
 // ---- keys, search, interpolation, alignment (pytorch/cpp/octree_key.cpp, octree_align.cpp) ------------
 // The reference's binding is compiled with 64-bit keys only (pytorch/cpp/octree_key.cpp:1-3), so
 // key tensors are int64; a 32-bit-key octree is rejected here with a message.
@@ -2631,6 +2767,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("tc_status", [](py::object device) {
     return tc_status(torch::python::detail::py_object_to_device(device));
   });
+  m.def("train_block", &train_block);
+  m.def("train_max_pool", &train_max_pool);
   m.def("octree_info", &octree_info);
   // (pytorch/cpp/pybind.cpp:35-41)
   m.def("octree_grow", &octree_grow, "octree growing", py::arg("octree"), py::arg("target_depth"),

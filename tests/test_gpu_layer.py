@@ -96,3 +96,42 @@ def test_tables_follow_the_octree(ocnn, batch):
     assert torch.equal(got, want)
     mine.copy_(octree)                     # the same storage, written to: the tables are made again
     assert torch.equal(conv(x, mine), want)
+
+
+# (1x1 with cuDNN's and with our own weight gradient, sibling-group and node mode, deconvolution)
+@pytest.mark.parametrize('kind,cin,cout,nempty', [
+    ('conv1x1', 16, 32, False), ('conv1x1', 16, 64, False), ('conv', 8, 16, False), ('conv', 16, 8, True),
+    ('deconv', 16, 8, False), ('deconv', 8, 8, True)])
+@pytest.mark.parametrize('with_res', [False, True])
+def test_training_block_is_the_modules_one_by_one(ocnn, batch, kind, cin, cout, nempty, with_res):
+  octree, v = batch
+  torch.manual_seed(cin + cout)
+  h_in = h_out = int(v.nnum_nempty[4] if nempty else v.nnum[4])
+  if kind == 'conv1x1':
+    block = ocnn.OctreeConv1x1BnRelu(cin, cout, use_bias=with_res).cuda().train()
+    args = ()
+  elif kind == 'conv':
+    block = ocnn.OctreeConvBnRelu(4, cin, cout, nempty=nempty).cuda().train()
+    args = (octree,)
+  else:
+    block = ocnn.OctreeDeConvBnRelu(4, cin, cout, [3], 2, nempty).cuda().train()
+    args = (octree,)
+    h_out = int(v.nnum_nempty[5] if nempty else v.nnum[5])
+  one = copy.deepcopy(block)
+  one.bn.register_forward_hook(lambda *a: None)            # a hook inside: no single node
+  data = torch.randn(1, cin, h_in, 1, device='cuda')
+  res = torch.randn(1, cout, h_out, 1, device='cuda') if with_res else None
+  g = torch.randn(1, cout, h_out, 1, device='cuda')
+  got = []
+  for b in (block, one):
+    x = data.clone().requires_grad_()
+    r = None if res is None else res.clone().requires_grad_()
+    y = b(x, *args, residual=r)
+    y.backward(g)
+    got.append([y.detach(), x.grad] + ([] if r is None else [r.grad]) + [p.grad for p in b.parameters()] +
+               [t.float() for t in b.bn.buffers()])
+  assert len(got[0]) == len(got[1]) > 5
+  for a, b in zip(*got):
+    torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
+  with pytest.raises(ValueError):
+    ocnn.OctreeConv1x1BnRelu(4, 4).cuda().train()(torch.ones(1, 4, 1, 1, device='cuda'))
