@@ -338,17 +338,31 @@ __global__ void __launch_bounds__(256) conv_f32_wgrad_reduce_kernel(const float*
                                                                     int T) {
   grid_dependency_trigger();
   grid_dependency_wait();
+  // 32 outputs per block, the splits of each dealt to eight warps: with few output tiles there are up to
+  // some 290 splits, and one thread adding them was a chain of that many loads
+  __shared__ float part[8][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long width = (long long)groups * 128;
   const long long stride = width * slices * npad;
-  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < width * M; i += gridDim.x * 256LL) {
+  for (long long base = blockIdx.x * 32LL; base < width * M; base += gridDim.x * 32LL) {
+    const long long i = base + lane;                       // (width is a multiple of 128: no tail)
     const int m = (int)(i / width), lin = (int)(i - m * width);
     const int t = lin / cp, c = lin - t * cp;
-    if (t >= T || c >= channels) continue;
     const int slice = m / npad, n = m - slice * npad, group = lin >> 7;
-    const float* p = partial + (((long long)group * slices + slice) * npad + n) * 128 + (lin & 127);
+    const bool on = t < T && c < channels;
     float v = 0.f;
-    for (int s = 0; s < splits; ++s) v += p[s * stride];
-    dw[((long long)m * channels + c) * T + t] = v;
+    if (on) {
+      const float* p = partial + (((long long)group * slices + slice) * npad + n) * 128 + (lin & 127);
+#pragma unroll 4
+      for (int s = warp; s < splits; s += 8) v += p[s * stride];
+    }
+    part[warp][lane] = v;
+    __syncthreads();
+    if (warp == 0 && on) {
+      for (int w = 1; w < 8; ++w) v += part[w][lane];
+      dw[((long long)m * channels + c) * T + t] = v;
+    }
+    __syncthreads();
   }
 }
 
@@ -472,7 +486,7 @@ extern "C" int ocnn_octree_conv_weight_grad_f32(const float* a, const float* x, 
   }
   OCNN_CUDA_OK(launch_chained(table[s.npad / 32 - 1], dim3(s.ctas), dim3(kF32Threads), s.smem, st, w));
   OCNN_LAUNCH_OK("conv_f32_wgrad_kernel");
-  OCNN_CUDA_OK(launch_chained(conv_f32_wgrad_reduce_kernel, dim3(grid_for((long long)s.groups * 128 * m_channels, 256)),
+  OCNN_CUDA_OK(launch_chained(conv_f32_wgrad_reduce_kernel, dim3(grid_for((long long)s.groups * 4 * m_channels, 1)),
                               dim3(256), 0, st, (const float*)w.partial, dw, s.splits, s.groups, s.slices, s.npad,
                               m_channels, x_channels, s.cp, tl.count));
   OCNN_LAUNCH_OK("conv_f32_wgrad_reduce_kernel");
