@@ -77,20 +77,26 @@ __global__ void neigh_full_levels_kernel(int* __restrict__ out, int batch, int f
 // 4x4x4 neighbour block at their own level, and every entry any of their children's blocks needs
 // is "the child group of one of those 64 cells".  So the warp reads the group's 64 neighbour
 // entries (256 contiguous bytes) and the 64 child pointers behind them ONCE (two gathers per
-// lane), keeps them in shared memory, and then writes the 64-int block of each non-empty parent
-// with two coalesced 128-byte stores: 8 child gathers per parent instead of the 64 of the
-// one-thread-per-output formulation.  Restates calc_neigh_cpu(neigh_split, neigh, children,
+// lane), keeps them in shared memory, and then writes the 64-int block of each non-empty parent:
+// 8 child gathers per parent instead of the 64 of the one-thread-per-output formulation.
+// WIDE (the output on a 16-byte boundary: a level's table starts 12 * batch bytes past one with
+// 64-bit keys, so batches of a multiple of four): two parents, z-neighbours, at a time, 16 lanes each,
+// a lane writes the four z positions of one (x, y) from one 16-byte read of the parents' block.  A
+// quarter of the stores and reads of the other form, one int per lane and store, which was bound
+// by instruction issue.  Depth 8 of 64 clouds of 100k points: 190 -> 178 us, 916 MB of DRAM traffic
+// at 5.1 TB/s (79 % of a copy).  Restates calc_neigh_cpu(neigh_split, neigh, children,
 // node_num), octree/octree/octree_nn.cpp:357-380, with the parent/displacement tables
 // (octree_nn.cpp:53-81) in arithmetic form.
 constexpr int kNeighWarps = 8;
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kNeighWarps * 32) neigh_split_kernel(
     int* __restrict__ out, const int* __restrict__ neigh, const int* __restrict__ child,
     long long ngroups) {
   grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
   // 8 * child group of each cell of the parents' block, -1 where there is none: an output is that
   // value | octant either way
-  __shared__ int cblk[kNeighWarps][64];
+  __shared__ __align__(16) int cblk[kNeighWarps][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // child-level block position j = (x,y,z) in 0..3 -> which parent-level cell (tap, as a
   // (tx<<4)|(ty<<2)|tz code relative to the parent) and which octant inside it; two per lane
@@ -102,6 +108,9 @@ __global__ void __launch_bounds__(kNeighWarps * 32) neigh_split_kernel(
     tapcode[k] = ((x >> 1) << 4) | ((y >> 1) << 2) | (z >> 1);
     oct[k] = ((x & 1) << 2) | ((y & 1) << 1) | (z & 1);
   }
+  // WIDE: the lane's (x, y) and half = the z bit of its parent
+  const int half = lane >> 4, wx = ((lane >> 2) & 3) + 1, wy = (lane & 3) + 1;
+  const int rowcode = ((wx >> 1) << 4) | ((wy >> 1) << 2), rowoct = ((wx & 1) << 2) | ((wy & 1) << 1);
   // Three stages in flight per warp: the block of the group after next is requested, then the child
   // pointers behind the next group's block, then this group's tables are written.  (One group at a
   // time was a chain of two reads per 700 bytes written: 3.7 TB/s where the writes alone go at 7.4.)
@@ -130,14 +139,26 @@ __global__ void __launch_bounds__(kNeighWarps * 32) neigh_split_kernel(
     kids(cell, kid);
     int mine_after;
     cells(g + 2 * stride, cell, mine_after);
+    if constexpr (WIDE) {
 #pragma unroll
-    for (int o = 0; o < 8; ++o) {
-      const int l0 = __shfl_sync(0xffffffffu, mine, o);
-      if (l0 < 0) continue;                                     // empty parent: no block
-      const int octcode = ((o & 4) << 2) | ((o & 2) << 1) | (o & 1);
-      int* dst = out + ((long long)l0 << 6);
+      for (int pair = 0; pair < 4; ++pair) {
+        const int l0 = __shfl_sync(0xffffffffu, mine, 2 * pair + half);
+        if (l0 < 0) continue;                                   // empty parent: no block
+        const int4 c = *reinterpret_cast<const int4*>(&cblk[warp][rowcode + ((pair & 2) << 3) + ((pair & 1) << 2)]);
+        const int lo = half ? c.y : c.x, mid = half ? c.z : c.y, hi = half ? c.w : c.z;
+        *reinterpret_cast<int4*>(out + ((long long)l0 << 6) + ((lane & 15) << 2)) =
+            make_int4(lo | rowoct | 1, mid | rowoct, mid | rowoct | 1, hi | rowoct);
+      }
+    } else {
 #pragma unroll
-      for (int k = 0; k < 2; ++k) dst[lane + 32 * k] = cblk[warp][tapcode[k] + octcode] | oct[k];
+      for (int o = 0; o < 8; ++o) {
+        const int l0 = __shfl_sync(0xffffffffu, mine, o);
+        if (l0 < 0) continue;                                     // empty parent: no block
+        const int octcode = ((o & 4) << 2) | ((o & 2) << 1) | (o & 1);
+        int* dst = out + ((long long)l0 << 6);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) dst[lane + 32 * k] = cblk[warp][tapcode[k] + octcode] | oct[k];
+      }
     }
     mine = mine_next;
     mine_next = mine_after;
@@ -173,7 +194,10 @@ int ocnn_calc_neigh_split(int32_t* neigh_child, const int32_t* neigh, const int3
                "ocnn_calc_neigh_split: parent level must hold whole sibling groups (got %d nodes)",
                nnum_parent);
   const long long ngroups = nnum_parent / 8;
-  OCNN_CUDA_OK(launch_chained(neigh_split_kernel, dim3(grid_for(ngroups, kNeighWarps, 16)), dim3(kNeighWarps * 32), 0, static_cast<cudaStream_t>(stream), neigh_child, neigh, child, ngroups));
+  const bool wide = (uintptr_t)neigh_child % 16 == 0;
+  OCNN_CUDA_OK(launch_chained(wide ? neigh_split_kernel<true> : neigh_split_kernel<false>,
+                              dim3(grid_for(ngroups, kNeighWarps, 16)), dim3(kNeighWarps * 32), 0,
+                              static_cast<cudaStream_t>(stream), neigh_child, neigh, child, ngroups));
   OCNN_LAUNCH_OK("neigh_split_kernel");
   return OCNN_OK;
 }
