@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(kF32Threads, NG <= 4 ? 2 : 1) conv_f32_kernel(
     bool alive = true;
     int s = 0, filled = -1;
     uint32_t pe = 1;
+    ZeroRows<4> zeros;
     long long gk = 0;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
       const int tile = item / per_tile;
@@ -233,6 +234,7 @@ __global__ void __launch_bounds__(kF32Threads, NG <= 4 ? 2 : 1) conv_f32_kernel(
           uint32_t off, width;
           chunk_place(cc, cpt, off, width);
           const int p[4] = {p4.x, p4.y, p4.z, p4.w};
+          const uint32_t copies = zeros.copies(s, live_rows<4>(p));
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int row = warp * 32 + 8 * i + rr;
@@ -240,8 +242,10 @@ __global__ void __launch_bounds__(kF32Threads, NG <= 4 ? 2 : 1) conv_f32_kernel(
             const bool have = p[i] >= 0;
             const uint8_t* src = have ? a.xs + (size_t)p[i] * row_bytes + off : a.xs;
             const uint32_t step = have ? width : 0u, n = have ? 16u : 0u;
+            if ((copies >> i) & 1u) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q) cp_async16(dst + q * kF32PartA, src + q * step, n);
+              for (int q = 0; q < 3; ++q) cp_async16(dst + q * kF32PartA, src + q * step, n);
+            }
           }
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s]))

@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(kF32Threads, NB <= 2 ? 2 : 1) conv_f32_wgrad_k
     int s = 0;
     uint32_t pe = 1;
     long long gk = 0;
+    ZeroRows<4> zeros;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
       const int group = item % per_split / a.slices;
       const int g = (group * 4 + warp) * 4 + c;              // chunk of eight (t, c) pairs
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(kF32Threads, NB <= 2 ? 2 : 1) conv_f32_wgrad_k
           alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrEmptyWait);
         if (alive) {
           const uint32_t block = smem_u32(sA + s * (3 * kF32PartA)) + (uint32_t)warp * kWgBlock;
+          const uint32_t copies = zeros.copies(s, live_rows<4>(p));
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int row = 8 * i + rr;
@@ -185,8 +187,10 @@ __global__ void __launch_bounds__(kF32Threads, NB <= 2 ? 2 : 1) conv_f32_wgrad_k
             const bool have = p[i] >= 0;
             const uint8_t* src = have ? a.xs + (size_t)p[i] * row_bytes + off : a.xs;
             const uint32_t stride = have ? width : 0u, n = have ? 16u : 0u;
+            if ((copies >> i) & 1u) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q) cp_async16(dst + q * kF32PartA, src + q * stride, n);
+              for (int q = 0; q < 3; ++q) cp_async16(dst + q * kF32PartA, src + q * stride, n);
+            }
           }
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s]))

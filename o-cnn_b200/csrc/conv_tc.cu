@@ -331,7 +331,8 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
           if (rbase + 4 * i < a.tile_rows && h0 + rbase + 4 * i < a.rows) row_mask |= 1u << i;
         int p[8];
         int s = 0;
-        uint32_t pe = 1;
+        uint32_t pe = 1, live = 0;
+        ZeroRows<8> zeros;
         int t = kb_first / kBlocksPerTap, part = kb_first - t * kBlocksPerTap;
         for (int kb = kb_first; kb < kb_end; ++kb) {
           if (part == 0 || kb == kb_first) {
@@ -339,12 +340,14 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
             const int4 hi = *reinterpret_cast<const int4*>(my_idx + t * kTileM + 4);
             p[0] = lo.x; p[1] = lo.y; p[2] = lo.z; p[3] = lo.w;
             p[4] = hi.x; p[5] = hi.y; p[6] = hi.z; p[7] = hi.w;
+            live = live_rows<8>(p);
           }
           if (alive && kb - kb_first >= a.stages)
             alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrEmptyWait);
           if (alive) {
             const uint32_t stage_base = smem_u32(sA + s * kStageA);
             const uint32_t off = (uint32_t)part * 128u + (uint32_t)chunk * 16u;
+            const uint32_t copies = zeros.copies(s, live) & row_mask;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int row = rbase + 4 * i;
@@ -352,7 +355,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
                                    (((uint32_t)chunk ^ (uint32_t)(row & 7)) << 4);
               const int pi = p[i];
               const char* src = pi >= 0 ? xb + (size_t)((uint32_t)pi * row_bytes) + off : xb;
-              if ((row_mask >> i) & 1u) cp_async16(dst, src, pi >= 0 ? 16u : 0u);
+              if ((copies >> i) & 1u) cp_async16(dst, src, pi >= 0 ? 16u : 0u);
             }
           }
           asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s]))
@@ -402,6 +405,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
       };
       int s = 0;
       uint32_t pe = 1;
+      ZeroRows<8> zeros;
       int p_cur[8];
       uint32_t off_cur;
       fetch(kb_first, p_cur, off_cur);
@@ -414,6 +418,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
           alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrEmptyWait);
         if (alive) {
           const uint32_t stage_base = smem_u32(sA + s * kStageA);
+          const uint32_t copies = zeros.copies(s, live_rows<8>(p_cur)) & row_mask;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int row = rbase + 4 * i;
@@ -423,7 +428,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
             const char* src = p >= 0 ? xb + (size_t)((uint32_t)p * row_bytes) + off_cur : xb;
             // rows the tile does not have are left as they are: their accumulator lanes are
             // never read
-            if ((row_mask >> i) & 1u) cp_async16(dst, src, p >= 0 ? 16u : 0u);
+            if ((copies >> i) & 1u) cp_async16(dst, src, p >= 0 ? 16u : 0u);
           }
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s]))
@@ -805,6 +810,7 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
           }
         }
       };
+      ZeroRows<8> zeros;
       int tile = blockIdx.x, kb0 = 0;
       int p_cur[kAhead][8];
       uint32_t off_cur[kAhead];
@@ -827,6 +833,7 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
             alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrEmptyWait);
           if (alive) {
             const uint32_t stage_base = smem_u32(sA + s * (R * kStageA));
+            const uint32_t copies = zeros.copies(s, live_rows<8>(p_cur[j]));
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int row = rbase + 4 * i;
@@ -834,9 +841,8 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
                                    (((uint32_t)chunk ^ (uint32_t)(row & 7)) << 4);
               const int pi = p_cur[j][i];
               const char* src = pi >= 0 ? xb + (size_t)((uint32_t)pi * row_bytes) + off_cur[j] : xb;
-              // rows past the level's last group are left as they are: their accumulator lanes
-              // are never read
-              if (tile * kRows + row < a.rows) cp_async16(dst, src, pi >= 0 ? 16u : 0u);
+              // (rows past the level's last group count as missing: their accumulator lanes are never read)
+              if ((copies >> i) & 1u) cp_async16(dst, src, pi >= 0 ? 16u : 0u);
             }
           }
           asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s]))
@@ -853,7 +859,8 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
         tile = tile_nxt;
         kb0 = kb_nxt;
       }
-    } else
+    } else {
+    ZeroRows<8> zeros;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
       const int h0 = tile * kRows;
       // 1x1x1: a tile row reads its own row, no table and no barriers
@@ -898,6 +905,7 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
       int p[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) p[i] = h0 + rbase + 4 * i;      // (identity; masked rows are not copied)
+      uint32_t live = 0xffu;           // (identity)
       int t = 0, part = 0;
       for (int kb = 0; kb < a.nkb; ++kb, ++gk) {
         if (part == 0 && !a.identity) {
@@ -905,6 +913,7 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
           const int4 hi = *reinterpret_cast<const int4*>(my_idx + t * kRows + 4);
           p[0] = lo.x; p[1] = lo.y; p[2] = lo.z; p[3] = lo.w;
           p[4] = hi.x; p[5] = hi.y; p[6] = hi.z; p[7] = hi.w;
+          live = live_rows<8>(p);
         }
         if (alive && gk >= a.stages)
           alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrEmptyWait);
@@ -916,7 +925,7 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
           const uint32_t stage_base = smem_u32(sA + s * (R * kStageA));
           const uint32_t g = (uint32_t)kb * 8u + (uint32_t)chunk;
           const uint32_t cpt_all = (uint32_t)a.cin >> 3, cpt_a = (uint32_t)a.cpt_a;
-          const bool from_a = g < cpt_a, live = g < cpt_all;
+          const bool from_a = g < cpt_a, inside = g < cpt_all;
           const char* base = from_a ? xb : reinterpret_cast<const char*>(a.x2);
           const uint32_t rb = (from_a ? cpt_a : cpt_all - cpt_a) * 16u;
           const uint32_t off = (from_a ? g : g - cpt_a) * 16u;
@@ -925,12 +934,13 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
             const int row = rbase + 4 * i;
             const uint32_t dst = stage_base + (uint32_t)row * 128u +
                                  (((uint32_t)chunk ^ (uint32_t)(row & 7)) << 4);
-            const char* src = live ? base + (size_t)p[i] * rb + off : xb;
-            if ((row_mask >> i) & 1u) cp_async16(dst, src, live ? 16u : 0u);
+            const char* src = inside ? base + (size_t)p[i] * rb + off : xb;
+            if ((row_mask >> i) & 1u) cp_async16(dst, src, inside ? 16u : 0u);
           }
         } else if (alive) {
           const uint32_t stage_base = smem_u32(sA + s * (R * kStageA));
           const uint32_t off = (uint32_t)part * 128u + (uint32_t)chunk * 16u;
+          const uint32_t copies = zeros.copies(s, live) & row_mask;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int row = rbase + 4 * i;
@@ -938,7 +948,7 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
                                  (((uint32_t)chunk ^ (uint32_t)(row & 7)) << 4);
             const int pi = p[i];
             const char* src = pi >= 0 ? xb + (size_t)((uint32_t)pi * row_bytes) + off : xb;
-            if ((row_mask >> i) & 1u) cp_async16(dst, src, pi >= 0 ? 16u : 0u);
+            if ((copies >> i) & 1u) cp_async16(dst, src, pi >= 0 ? 16u : 0u);
           }
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s]))
@@ -948,6 +958,7 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
       }
       // a thread that gave up keeps walking the tiles (without waiting or copying): the named
       // barrier above needs every gather thread every time
+    }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == kGatherWarps) {

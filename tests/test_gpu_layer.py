@@ -135,3 +135,32 @@ def test_training_block_is_the_modules_one_by_one(ocnn, batch, kind, cin, cout, 
     torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
   with pytest.raises(ValueError):
     ocnn.OctreeConv1x1BnRelu(4, 4).cuda().train()(torch.ones(1, 4, 1, 1, device='cuda'))
+
+
+@pytest.fixture(scope='module')
+def sparse_level(ocnn):
+  """About 97 k non-empty nodes at depth 7, a slab among scattered points: from 1 to 27 neighbours."""
+  gen = torch.Generator().manual_seed(7)
+  p = 0.99 * (2 * torch.rand(100000, 3, generator=gen) - 1)
+  p[50000:] = p[50000:] * torch.tensor([1.0, 1.0, 0.02])
+  n = torch.nn.functional.normalize(torch.randn(100000, 3, generator=gen), dim=1)
+  octree = ocnn.octree_batch([ocnn.Points2Octree(7, 2)(ocnn.points_new(p, n, torch.zeros(0), torch.zeros(0)))]).cuda()
+  return octree, int((ocnn.octree_property(octree, 'child', 7) >= 0).sum())
+
+
+# (one and several 64-channel parts per tap, one and several taps per K-block, padded columns, slices of
+# 256; 256 columns take the persistent kernel, fp32 the three-part one; the gradient its own gather)
+@pytest.mark.parametrize('cin,cout', [(64, 64), (96, 96), (128, 104), (32, 72), (8, 64), (192, 512), (64, 256)])
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
+def test_missing_neighbours_on_a_large_sparse_level(ocnn, sparse_level, cin, cout, dtype):
+  octree, h = sparse_level
+  torch.manual_seed(cin + cout)
+  op = ocnn.OctreeConv(7, cin, cout, [3], 1, True).cuda().eval()
+  x = torch.randn(1, cin, h, 1, device='cuda').to(dtype).contiguous(memory_format=torch.channels_last)
+  res = torch.randn(1, cout, h, 1, device='cuda').to(dtype).contiguous(memory_format=torch.channels_last)
+  bn = randomised(torch.nn.BatchNorm2d(cout, 1e-3), 3).cuda().eval()
+  with torch.no_grad():
+    op.weights.copy_(op.weights.to(dtype).float())
+    z = op._run(x.float().contiguous(), octree)
+    got, want = op._run(x, octree, bn, res, True).float(), torch.relu(bn(z) + res.float())
+    assert float((got - want).abs().max() / want.abs().max()) < (1e-2 if dtype == torch.bfloat16 else 2e-3)
