@@ -30,12 +30,13 @@ def _trainable(data, weight, bn, residual):
           data.is_contiguous() and weight.dtype == torch.float32 and weight.is_cuda and bn.affine and
           bn.track_running_stats and bn.momentum is not None and bn.weight.dtype == torch.float32 and
           (residual is None or residual.dtype == torch.float32) and not torch.is_autocast_enabled() and
-          not _hooked(bn))
+          not hooked(bn))
 
 
-def _hooked(module):
+def hooked(module):
+  """Whether someone asked to see this module's calls: a path that passes it by has to leave it alone."""
   return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or
-              module._backward_pre_hooks)
+              module._backward_pre_hooks or torch.nn.modules.module._has_any_global_hook())
 
 
 def _train_block(data, weight, bias, bn, residual, octree, kind, depth, cout, kernel_size, stride, nempty, relu):
@@ -76,7 +77,7 @@ class _OctreeBlock(_nn.Module):
         data_in = nn.octree_depad(data_in, octree, op.depth)
       return op._run(data_in, octree, self.bn, residual, relu)
     if foldable and type(self.bn) is _nn.BatchNorm2d and type(op) in (OctreeConv, OctreeDeconv) and \
-        _trainable(data_in, op.weights, self.bn, residual) and not _hooked(op):
+        _trainable(data_in, op.weights, self.bn, residual) and not hooked(op):
       assert data_in.size(1) == op.channel_in
       if not op.is_conv_layer() and op.stride == 2 and not op.nempty:
         data_in = octree_depad(data_in, octree, op.depth)
@@ -200,7 +201,7 @@ class _Conv1x1Block(_nn.Module):
       return self.conv1x1.run(data_in, self.bn, residual, relu)
     conv = self.conv1x1.conv1x1
     if type(self.bn) is _nn.BatchNorm2d and type(self.conv1x1) is OctreeConv1x1 and \
-        _trainable(data_in, conv.weight, self.bn, residual) and not (_hooked(conv) or _hooked(self.conv1x1)):
+        _trainable(data_in, conv.weight, self.bn, residual) and not (hooked(conv) or hooked(self.conv1x1)):
       return _train_block(data_in, conv.weight, conv.bias, self.bn, residual, None, 2, 0, conv.weight.shape[0],
                           [1], 1, False, relu)
     out = self.bn(self.conv1x1(data_in))

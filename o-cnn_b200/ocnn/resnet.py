@@ -5,7 +5,8 @@ import torch
 from torch import nn as _nn
 
 from . import nn
-from .modules import OctreeConvBnRelu, OctreeResBlocks
+from .modules import OctreeConvBnRelu, OctreeResBlocks, hooked
+from .octree2voxel import FullOctree2Voxel
 from .octree_pool import OctreeMaxPool, FullOctreeGlobalPool
 
 
@@ -29,9 +30,25 @@ class ResNet(_nn.Module):
     data = self.conv1(data, octree)
     for blocks, pool in zip(self.resblocks, self.pools):
       data = pool(blocks(data, octree), octree)
-    fc = self.header[1]
-    if (not self.training and data.dtype in (torch.bfloat16, torch.float16) and
-        not (torch.is_grad_enabled() and data.requires_grad) and
-        data.is_contiguous(memory_format=torch.channels_last) and fc.weight.dtype == torch.float32):
-      return nn.global_pool_fc(data, fc.weight, fc.bias, data.shape[2] // 64)   # one kernel
+    if self._head_is_one_kernel(data):
+      pool, fc = self.header
+      return nn.global_pool_fc(data, fc.weight, fc.bias, data.shape[2] // 8 ** pool.depth)
     return self.header(data.float() if data.dtype != torch.float32 else data)
+
+  def _head_is_one_kernel(self, data):
+    """Whether the header can run as pool + Linear in one launch: the two stock modules with nothing that
+    would have to see the tensors between them, on 16-bit node-major data, with no gradient to record
+    (a frozen network whose Linear is being trained records one)."""
+    if self.training or data.dtype not in (torch.bfloat16, torch.float16) or torch.is_autocast_enabled():
+      return False
+    head = self.header
+    if type(head) is not _nn.Sequential or len(head) != 2:
+      return False
+    pool, fc = head
+    if type(pool) is not FullOctreeGlobalPool or type(pool.octree2voxel) is not FullOctree2Voxel or \
+        type(fc) is not _nn.Linear or any(hooked(m) for m in (head, pool, pool.octree2voxel, fc)):
+      return False
+    params = [p for p in (fc.weight, fc.bias) if p is not None]
+    return (all(p.dtype == torch.float32 and p.device == data.device for p in params) and
+            data.is_contiguous(memory_format=torch.channels_last) and
+            not (torch.is_grad_enabled() and any(t.requires_grad for t in (data, *params))))
