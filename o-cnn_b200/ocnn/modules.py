@@ -39,6 +39,12 @@ def hooked(module):
               module._backward_pre_hooks or torch.nn.modules.module._has_any_global_hook())
 
 
+def _stock_conv1x1(conv):
+  """Whether a 1x1 layer's product may be formed from the weight and bias of `conv` without calling it."""
+  return (type(conv) is _nn.Conv1d and conv.kernel_size == (1,) and conv.stride == (1,) and
+          conv.padding == (0,) and conv.groups == 1 and not hooked(conv))
+
+
 def _train_block(data, weight, bias, bn, residual, octree, kind, depth, cout, kernel_size, stride, nempty, relu):
   if bn.num_batches_tracked is not None:
     bn.num_batches_tracked.add_(1)
@@ -141,7 +147,7 @@ class _Conv1x1Function(torch.autograd.Function):
 class OctreeConv1x1(_nn.Module):
   """A per-node linear map.  The parameters live in a torch Conv1d (as in the reference, so the
   state_dict keys match); the product runs on this library's pointwise kernels."""
-  _layer = None
+  _layer, _layer_shape = None, None
 
   def __init__(self, channel_in, channel_out, use_bias=False):
     super().__init__()
@@ -156,7 +162,8 @@ class OctreeConv1x1(_nn.Module):
       # 64 to 128 output channels cuDNN forms the weight gradient with a direct fp32 kernel (16 -> 64
       # at 107 k nodes: 395 us); ours is used there. Elsewhere cuDNN takes a GEMM (about 55 us).
       if (64 <= conv.weight.shape[0] <= 128 and data_in.dtype == conv.weight.dtype == torch.float32 and
-          data_in.is_cuda and data_in.is_contiguous() and not torch.is_autocast_enabled()):
+          data_in.is_cuda and data_in.is_contiguous() and not torch.is_autocast_enabled() and
+          _stock_conv1x1(conv)):
         out = _Conv1x1Function.apply(data_in, conv.weight, conv.bias)
       else:
         out = conv(data_in.squeeze(-1)).unsqueeze(-1)
@@ -166,9 +173,10 @@ class OctreeConv1x1(_nn.Module):
       if residual is not None:
         out = out + residual
       return torch.relu(out) if relu else out
-    if self._layer is None:
-      cout, cin = conv.weight.shape[:2]
+    cout, cin = conv.weight.shape[:2]
+    if self._layer is None or self._layer_shape != (cin, cout):      # (the Conv1d can be replaced)
       self._layer = nn.ConvLayer(cin, cout, [1, 1, 1], 1, False, False, True)
+      self._layer_shape = (cin, cout)
     affine = bn_vectors(bn)
     if conv.bias is not None:
       with torch.no_grad():
@@ -201,7 +209,7 @@ class _Conv1x1Block(_nn.Module):
       return self.conv1x1.run(data_in, self.bn, residual, relu)
     conv = self.conv1x1.conv1x1
     if type(self.bn) is _nn.BatchNorm2d and type(self.conv1x1) is OctreeConv1x1 and \
-        _trainable(data_in, conv.weight, self.bn, residual) and not (hooked(conv) or hooked(self.conv1x1)):
+        _stock_conv1x1(conv) and _trainable(data_in, conv.weight, self.bn, residual) and not hooked(self.conv1x1):
       return _train_block(data_in, conv.weight, conv.bias, self.bn, residual, None, 2, 0, conv.weight.shape[0],
                           [1], 1, False, relu)
     out = self.bn(self.conv1x1(data_in))

@@ -1,5 +1,7 @@
 """`ocnn.ResNet` with another classification header than its own: whatever stands there is what runs, and
 the one-launch form of pool + Linear keeps out of its way."""
+import copy
+
 import pytest
 import torch
 from torch import nn
@@ -71,11 +73,7 @@ def net_features(net, octree):
 def test_training_runs_a_replaced_header(setup):
   ocnn, net, octree, data, stock, feature = setup
   net.header = nn.Identity()
-  net.train()
-  try:
-    out = net(octree, octree_data(ocnn, octree))
-  finally:
-    net.eval()
+  out = copy.deepcopy(net).train()(octree, octree_data(ocnn, octree))     # (a copy: it updates its statistics)
   assert out.shape == feature.shape
 
 

@@ -164,3 +164,44 @@ def test_missing_neighbours_on_a_large_sparse_level(ocnn, sparse_level, cin, cou
     z = op._run(x.float().contiguous(), octree)
     got, want = op._run(x, octree, bn, res, True).float(), torch.relu(bn(z) + res.float())
     assert float((got - want).abs().max() / want.abs().max()) < (1e-2 if dtype == torch.bfloat16 else 2e-3)
+
+
+class _Tripled(torch.nn.Conv1d):
+  def forward(self, x):
+    return 3 * super().forward(x)
+
+
+@pytest.mark.parametrize('cout', [24, 64])                 # torch's weight gradient, and our own
+@pytest.mark.parametrize('block', [False, True])
+def test_replaced_or_hooked_conv1d_is_called(ocnn, cout, block):
+  """Training paths that pass the inner Conv1d by keep to the stock one."""
+  layer = (ocnn.OctreeConv1x1BnRelu if block else ocnn.OctreeConv1x1)(16, cout).cuda().train()
+  inner = layer.conv1x1 if block else layer
+  x = torch.randn(1, 16, 500, 1, device='cuda', requires_grad=True)
+  seen = []
+  handle = inner.conv1x1.register_forward_pre_hook(lambda m, i: seen.append(m))
+  layer(x)
+  handle.remove()
+  assert seen == [inner.conv1x1]
+  tripled = _Tripled(16, cout, 1, bias=False).cuda()
+  tripled.load_state_dict(inner.conv1x1.state_dict())
+  y = inner(x)
+  inner.conv1x1 = tripled
+  torch.testing.assert_close(inner(x), 3 * y, rtol=1e-3, atol=1e-3)
+  if block:
+    want = torch.relu(layer.bn(inner(x)))
+    torch.testing.assert_close(layer(x), want, rtol=1e-3, atol=1e-3)
+
+
+def test_conv1d_of_another_width(ocnn):
+  """The native side of a 1x1 layer follows a Conv1d of another shape."""
+  layer = ocnn.OctreeConv1x1(16, 24).cuda().eval()
+  with torch.no_grad():
+    for cin, cout in [(16, 24), (16, 8), (32, 8)]:
+      layer.conv1x1 = torch.nn.Conv1d(cin, cout, 1, bias=False).cuda()
+      for dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 1e-2)):
+        x = torch.randn(1, cin, 300, 1, device='cuda').to(dtype).contiguous(memory_format=torch.channels_last)
+        got = layer(x)
+        ref = torch.einsum('oc,ch->oh', layer.conv1x1.weight[:, :, 0].double(), x.squeeze(0).squeeze(-1).double())
+        assert got.shape == (1, cout, 300, 1)
+        assert float((got.double().squeeze(0).squeeze(-1) - ref).norm() / ref.norm()) < tol
