@@ -92,7 +92,8 @@ Layout make_layout(int64_t n, int batch, int depth, int full) {
   L.radix_bits = p9 < p8 ? 9 : 8;
   L.passes = p9 < p8 ? p9 : p8;
   const int bins = 1 << L.radix_bits;
-  L.max_chunks = (int)(n / chunk_points(n)) + batch;
+  // (a bound that grows with n although the chunks do too, so that the workspace of n points serves fewer)
+  L.max_chunks = (int)(n / kSortTile < kSMs * 4 ? n / kSortTile : kSMs * 4) + batch;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes); return at; };
   L.off_clouds = take(sizeof(CloudRef) * (size_t)(batch + 1));

@@ -184,3 +184,14 @@ def test_octree_new_and_grow_header_on_the_host(lib, kb):
   # a full level cannot follow a level with empty nodes
   assert lib.ocnn_octree_grow_header(cur[:720].tobytes(), 4, 1, hdr) != 0
   assert b'non-empty' in lib.ocnn_last_error()
+
+
+@pytest.mark.parametrize('depth', [5, 6, 8, 9])
+@pytest.mark.parametrize('batch', [1, 40])
+def test_build_workspace_grows_with_the_points(lib, depth, batch):
+  """A plan made again for fewer points (a loader's clip dropped some) runs in the workspace of all of them,
+  also where the sort goes over to longer chunks (every 592 * 2048 points)."""
+  size = lambda n: lib.ocnn_octree_build_workspace_bytes(n, batch, depth, 2)
+  for tiles in (592, 1184, 1776):
+    around = [size(tiles * 2048 + k) for k in (-5000, -1, 0, 1, 2, 100, 2047, 2048, 2049, 5000, 20000)]
+    assert around == sorted(around)
