@@ -4,8 +4,9 @@
 // and then per batch (merge_octrees, octree/octree/merge_octrees.cpp:7-198) is done here in one
 // pass over all clouds: every point gets the composite key  (cloud << 3*depth) | morton(cell), the
 // clouds' own key bits are radix-sorted (the clouds already lie one behind the other, so the sort is
-// segmented by cloud and never looks at the cloud bits; equal to the reference's std::sort of (key,
-// index) pairs per cloud), and every level is a segmented "unique" of the sorted keys.
+// segmented by cloud and never looks at the cloud bits, unless there are many small clouds: by_cloud; equal
+// to the reference's std::sort of (key, index) pairs per cloud), and every level is a segmented "unique" of the
+// sorted keys.
 // The composite key of a level-d node is also its rank basis: ranks in the batch-wide unique list
 // are exactly the rebased child indices that merge_octrees produces.
 //
@@ -49,6 +50,7 @@ struct CloudRef {
   int chunk0;           // first sort chunk (= sort CTA) of the cloud: a chunk never crosses clouds
   int pad;
 };
+constexpr int kCloudPoints = 7000;       // see by_cloud
 constexpr int kInlineClouds = 63;        // a table of this many clouds rides in the launch parameters
 
 // ---- workspace layout --------------------------------------------------------------------------
@@ -56,6 +58,7 @@ struct Layout {
   int64_t n;            // total points
   int batch, depth, full;
   int key_bytes;        // 4 or 8: width of the composite keys
+  int segments;         // of the sort: the clouds, or 1 (by_cloud)
   int radix_bits, passes;
   int max_chunks;       // sort: bound on the number of chunks, whatever the clouds' sizes
   int64_t cap[OCNN_MAX_DEPTH + 1];   // capacity of Kd
@@ -81,24 +84,35 @@ int chunk_points(int64_t n) {
   return (int)((per < 1 ? 1 : per) * kSortTile);
 }
 
+// Whether the sort runs cloud by cloud or over the whole batch, cloud bits and all.  By cloud saves the passes
+// over the cloud bits, but every cloud costs a chunk, a digit row per warp and its digit totals, whatever
+// it holds, so the cost of many small clouds has no bound: 60000 clouds of 8 points at depth 6 took 21 ms and
+// cleared 246 MB of totals; over the whole batch 3.5 ms.  Measured at depths 5 to 8 (us, by cloud /
+// over the batch): 65 clouds of 200 to 32000 points 102 / 116 to 631 / 659, by cloud at nearly every size; 128
+// of 500 140 / 127; 256 of 1000 224 / 188, of 6000 498 / 467, of 8000 302 / 311 and 566 / 564, of 12000 364 / 384; 512 of
+// 1000 385 / 296; 1024 of 2000 945 / 787.
+bool by_cloud(int64_t n, int batch) { return batch <= 64 || n >= (int64_t)batch * kCloudPoints; }
+
 Layout make_layout(int64_t n, int batch, int depth, int full) {
   Layout L;
   memset(&L, 0, sizeof(L));
   L.n = n; L.batch = batch; L.depth = depth; L.full = full;
   L.key_bytes = (3 * depth + bits_for(batch) <= 32) ? 4 : 8;
+  L.segments = by_cloud(n, batch) ? batch : 1;
+  const int bits = 3 * depth + (L.segments == batch ? 0 : bits_for(batch));
   // 9-bit digits where they save a pass over 8-bit ones (depth 6: two passes instead of three,
   // depth 9: three instead of four)
-  const int p8 = (3 * depth + 7) / 8, p9 = (3 * depth + 8) / 9;
+  const int p8 = (bits + 7) / 8, p9 = (bits + 8) / 9;
   L.radix_bits = p9 < p8 ? 9 : 8;
   L.passes = p9 < p8 ? p9 : p8;
   const int bins = 1 << L.radix_bits;
   // (a bound that grows with n although the chunks do too, so that the workspace of n points serves fewer)
-  L.max_chunks = (int)(n / kSortTile < kSMs * 4 ? n / kSortTile : kSMs * 4) + batch;
+  L.max_chunks = (int)(n / kSortTile < kSMs * 4 ? n / kSortTile : kSMs * 4) + L.segments;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes); return at; };
-  L.off_clouds = take(sizeof(CloudRef) * (size_t)(batch + 1));
+  L.off_clouds = take(sizeof(CloudRef) * (size_t)(batch + 3));    // the clouds, then the one segment of all of them
   L.off_counts = take(sizeof(int) * 32);
-  L.off_bintot = take(sizeof(int) * (size_t)bins * batch * L.passes);   // digit totals per pass and cloud
+  L.off_bintot = take(sizeof(int) * (size_t)bins * L.segments * L.passes);   // digit totals per pass and segment
   L.zero_bytes = o - L.off_counts;
   L.off_blockcnt = take(sizeof(int) * kMaxScanGrid * (OCNN_MAX_DEPTH + 1));
   L.off_hist = take(sizeof(int) * (size_t)bins * L.max_chunks);
@@ -129,8 +143,11 @@ __device__ __forceinline__ uint64_t spread3(uint32_t v) {
   return x;
 }
 
-// The cloud that sort chunk `chunk` belongs to.
-__device__ __forceinline__ int cloud_of_chunk(const CloudRef* clouds, int batch, int chunk) {
+// A table of the sort's segments has the form of the table of clouds: first point and first chunk of each, and a
+// sentinel.  It is that table where the sort runs cloud by cloud.
+
+// The segment that sort chunk `chunk` belongs to.
+__device__ __forceinline__ int segment_of_chunk(const CloudRef* clouds, int batch, int chunk) {
   int lo = 0, hi = batch;          // clouds[lo].chunk0 <= chunk < clouds[hi].chunk0
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -139,26 +156,35 @@ __device__ __forceinline__ int cloud_of_chunk(const CloudRef* clouds, int batch,
   return lo;
 }
 
-// One chunk of one cloud: its points, and where its digit counts go (hist holds, cloud by cloud, a
-// [digit][chunk of the cloud] table).
+// The cloud that point i belongs to, between clouds lo and hi.
+__device__ __forceinline__ int cloud_of_point(const CloudRef* clouds, int lo, int hi, long long i) {
+  while (hi > lo) {                // clouds[lo].offset <= i < clouds[hi + 1].offset
+    const int mid = (lo + hi + 1) >> 1;
+    if (clouds[mid].offset <= i) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// One chunk of one segment: its points, and where its digit counts go (hist holds, segment by segment, a
+// [digit][chunk of the segment] table).
 struct Chunk {
-  int cloud, first, chunks;        // cloud, index inside it, the cloud's number of chunks
+  int segment, first, chunks;      // segment, index inside it, the segment's number of chunks
   long long beg, end;
 };
 __device__ __forceinline__ Chunk chunk_of(const CloudRef* clouds, int batch, int chunk_pts) {
   Chunk c;
-  c.cloud = cloud_of_chunk(clouds, batch, blockIdx.x);
-  const CloudRef a = clouds[c.cloud];
-  const long long next = clouds[c.cloud + 1].offset;
+  c.segment = segment_of_chunk(clouds, batch, blockIdx.x);
+  const CloudRef a = clouds[c.segment];
+  const long long next = clouds[c.segment + 1].offset;
   c.first = (int)blockIdx.x - a.chunk0;
-  c.chunks = clouds[c.cloud + 1].chunk0 - a.chunk0;
+  c.chunks = clouds[c.segment + 1].chunk0 - a.chunk0;
   c.beg = a.offset + (long long)c.first * chunk_pts;
   c.end = c.beg + chunk_pts < next ? c.beg + chunk_pts : next;
   return c;
 }
 
 // Per-warp digit counters of a CTA, summed and published: hist gets the chunk's counts, bintot the
-// cloud's totals (integer additions: their order does not matter).
+// segment's totals (integer additions: their order does not matter).
 template <int RB>
 __device__ __forceinline__ void publish_counts(int (&sh)[kWarps][1 << RB], const Chunk& c, int chunk0,
                                                int* __restrict__ hist, int* __restrict__ bintot) {
@@ -171,7 +197,7 @@ __device__ __forceinline__ void publish_counts(int (&sh)[kWarps][1 << RB], const
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) total += sh[w][d];
     to[(long long)d * c.chunks] = total;
-    if (total) atomicAdd(&bintot[c.cloud * kBins + d], total);
+    if (total) atomicAdd(&bintot[c.segment * kBins + d], total);
   }
 }
 
@@ -191,6 +217,7 @@ __device__ __forceinline__ void count_digit(int* counters, int digit, int none) 
 
 struct EncodeArgs {
   const CloudRef* table;    // device table (written by this kernel when the clouds ride along)
+  const CloudRef* segments; // WHOLE: the one segment
   int inline_clouds;        // 1: `clouds` holds them
   int batch, depth, chunk_pts;
   float bbmin[3];
@@ -199,9 +226,10 @@ struct EncodeArgs {
 };
 
 // normalize_pts + sort_keys' key computation (octree.cpp:155-170, 180-186): cell = trunc((p -
-// bbmin) * mul), only `depth` bits per axis enter the key.  One CTA per sort chunk, so the cloud is the
-// CTA's and the first sort pass's digits are counted on the way.
-template <typename KeyT, int RB>
+// bbmin) * mul), only `depth` bits per axis enter the key.  One CTA per sort chunk, whose cloud is the
+// CTA's (WHOLE: each of its points is looked up among the chunk's clouds); the first sort pass's digits are
+// counted on the way.
+template <typename KeyT, int RB, bool WHOLE>
 __global__ void __launch_bounds__(kThreads) encode_kernel(const __grid_constant__ EncodeArgs a,
                                                           KeyT* __restrict__ keys, int* __restrict__ hist,
                                                           int* __restrict__ bintot) {
@@ -213,18 +241,27 @@ __global__ void __launch_bounds__(kThreads) encode_kernel(const __grid_constant_
   const CloudRef* clouds = a.inline_clouds ? a.clouds : a.table;
   if (a.inline_clouds && blockIdx.x == 0)
     for (int i = threadIdx.x; i <= a.batch; i += kThreads) const_cast<CloudRef*>(a.table)[i] = a.clouds[i];
-  const Chunk c = chunk_of(clouds, a.batch, a.chunk_pts);
-  const float* xyz = clouds[c.cloud].xyz - 3 * clouds[c.cloud].offset;
-  const uint64_t top = (uint64_t)c.cloud << (3 * a.depth);
+  const Chunk c = WHOLE ? chunk_of(a.segments, 1, a.chunk_pts) : chunk_of(clouds, a.batch, a.chunk_pts);
+  __shared__ int range[2];      // WHOLE: the chunk's first and last cloud
+  if (WHOLE && (threadIdx.x & 31) == 0 && threadIdx.x < 64)
+    range[threadIdx.x >> 5] = cloud_of_point(clouds, 0, a.batch - 1, threadIdx.x == 0 ? c.beg : c.end - 1);
+  const float* xyz = WHOLE ? nullptr : clouds[c.segment].xyz - 3 * clouds[c.segment].offset;
+  uint64_t top = (uint64_t)c.segment << (3 * a.depth);
   const uint32_t mask = (1u << a.depth) - 1u;
   __syncthreads();
   for (long long i0 = c.beg; i0 < c.end; i0 += 4 * kThreads) {
     float p[4][3];
+    int cloud[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const long long i = i0 + u * kThreads + threadIdx.x;
+      const float* from = xyz;
+      if (WHOLE && i < c.end) {
+        cloud[u] = cloud_of_point(clouds, range[0], range[1], i);
+        from = clouds[cloud[u]].xyz - 3 * clouds[cloud[u]].offset;
+      }
 #pragma unroll
-      for (int j = 0; j < 3; ++j) p[u][j] = i < c.end ? xyz[3 * i + j] : 0.f;
+      for (int j = 0; j < 3; ++j) p[u][j] = i < c.end ? from[3 * i + j] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -235,19 +272,20 @@ __global__ void __launch_bounds__(kThreads) encode_kernel(const __grid_constant_
         const float s = (p[u][j] - a.bbmin[j]) * a.mul;
         cell[j] = (uint32_t)s & mask;
       }
+      if (WHOLE) top = i < c.end ? (uint64_t)cloud[u] << (3 * a.depth) : 0;
       // (with the cloud's bits: the top digit of a shallow tree reaches into them, here as in the scatter)
       const uint64_t key = top | (spread3(cell[0]) << 2) | (spread3(cell[1]) << 1) | spread3(cell[2]);
       if (i < c.end) keys[i] = (KeyT)key;
       count_digit(sh[threadIdx.x >> 5], i < c.end ? (int)(key & ((1 << RB) - 1)) : (1 << RB), 1 << RB);
     }
   }
-  publish_counts<RB>(sh, c, clouds[c.cloud].chunk0, hist, bintot);
+  publish_counts<RB>(sh, c, WHOLE ? 0 : clouds[c.segment].chunk0, hist, bintot);
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
-// ---- stable LSD radix sort, RB bits per pass, segmented by cloud -----------------------------------
-// Each CTA owns one chunk of one cloud.  A pass is: per-CTA digit histogram -> exclusive scan over
-// (digit, chunk) inside the cloud -> stable scatter.  The scatter works in tiles of 2048 keys: every
+// ---- stable LSD radix sort, RB bits per pass, by segments (the clouds, or the batch: by_cloud) ---------
+// Each CTA owns one chunk of one segment.  A pass is: per-CTA digit histogram -> exclusive scan over
+// (digit, chunk) inside the segment -> stable scatter.  The scatter works in tiles of 2048 keys: every
 // warp ranks its 256 keys 32 at a time with ballots (stable inside the warp), the per-warp digit counts
 // are prefixed across warps and digits, the tile is written to shared memory in digit order, and
 // only then copied out — consecutive threads then write consecutive global addresses of one digit
@@ -278,7 +316,7 @@ __global__ void __launch_bounds__(kThreads) sort_hist_kernel(const KeyT* __restr
       count_digit(sh[threadIdx.x >> 5], i < c.end ? (int)((k[u] >> shift) & ((1 << RB) - 1)) : (1 << RB), 1 << RB);
     }
   }
-  publish_counts<RB>(sh, c, clouds[c.cloud].chunk0, hist, bintot);
+  publish_counts<RB>(sh, c, clouds[c.segment].chunk0, hist, bintot);
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
@@ -310,8 +348,8 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* total) {
   return inc - v + wsum[warp];
 }
 
-// Exclusive scan of every cloud's hist[digit][chunk] in that order, starting at the cloud's first
-// point: one warp per (cloud, digit) row.
+// Exclusive scan of every segment's hist[digit][chunk] in that order, starting at the segment's first
+// point: one warp per (segment, digit) row.
 template <int RB>
 __global__ void __launch_bounds__(kThreads) sort_rowscan_kernel(int* __restrict__ hist,
                                                                 const CloudRef* __restrict__ clouds, int batch,
@@ -324,7 +362,7 @@ __global__ void __launch_bounds__(kThreads) sort_rowscan_kernel(int* __restrict_
     const int b = (int)(row >> RB), digit = (int)(row & (kBins - 1));
     const CloudRef c = clouds[b];
     const int chunks = clouds[b + 1].chunk0 - c.chunk0;
-    // first slot of this digit = number of the cloud's keys with a smaller digit
+    // first slot of this digit = number of the segment's keys with a smaller digit
     int below = 0;
     for (int d = lane; d < digit; d += 32) below += bintot[b * kBins + d];
     for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
@@ -374,7 +412,7 @@ __global__ void __launch_bounds__(kThreads) sort_scatter_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const Chunk c = chunk_of(clouds, batch, chunk_pts);
   {
-    const int* from = hist + (long long)clouds[c.cloud].chunk0 * kBins + c.first;
+    const int* from = hist + (long long)clouds[c.segment].chunk0 * kBins + c.first;
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
       const int d = threadIdx.x * kPer + q;
@@ -991,29 +1029,30 @@ int sort_keys(const EncodeArgs& ea, const Layout& L, int chunks, uint8_t* ws, cu
   constexpr int kBins = 1 << RB;
   KeyT* keys[2] = {reinterpret_cast<KeyT*>(ws + L.off_keys[0]), reinterpret_cast<KeyT*>(ws + L.off_keys[1])};
   uint32_t* idx[2] = {reinterpret_cast<uint32_t*>(ws + L.off_idx[0]), reinterpret_cast<uint32_t*>(ws + L.off_idx[1])};
-  const CloudRef* clouds = reinterpret_cast<const CloudRef*>(ws + L.off_clouds);
+  const bool whole = L.segments != L.batch;
+  const CloudRef* segs = reinterpret_cast<const CloudRef*>(ws + L.off_clouds) + (whole ? L.batch + 1 : 0);
   int* hist = reinterpret_cast<int*>(ws + L.off_hist);
-  OCNN_CUDA_OK(launch_chained(encode_kernel<KeyT, RB>, dim3(chunks), dim3(kThreads), 0, st, ea, keys[0], hist,
-                              reinterpret_cast<int*>(ws + L.off_bintot)));
+  OCNN_CUDA_OK(launch_chained(whole ? encode_kernel<KeyT, RB, true> : encode_kernel<KeyT, RB, false>, dim3(chunks),
+                              dim3(kThreads), 0, st, ea, keys[0], hist, reinterpret_cast<int*>(ws + L.off_bintot)));
   OCNN_LAUNCH_OK("encode_kernel");
-  const int rows = ceil_div((long long)L.batch * kBins, kWarps);
+  const int rows = ceil_div((long long)L.segments * kBins, kWarps);
   int cur = 0;
   for (int p = 0; p < L.passes; ++p) {
     const int shift = RB * p;
-    int* bintot = reinterpret_cast<int*>(ws + L.off_bintot) + (size_t)p * L.batch * kBins;
+    int* bintot = reinterpret_cast<int*>(ws + L.off_bintot) + (size_t)p * L.segments * kBins;
     if (p > 0)
       OCNN_CUDA_OK(launch_chained(sort_hist_kernel<KeyT, RB>, dim3(chunks), dim3(kThreads), 0, st,
-                                  (const KeyT*)keys[cur], clouds, L.batch, ea.chunk_pts, shift, hist, bintot));
-    OCNN_CUDA_OK(launch_chained(sort_rowscan_kernel<RB>, dim3(rows), dim3(kThreads), 0, st, hist, clouds, L.batch,
+                                  (const KeyT*)keys[cur], segs, L.segments, ea.chunk_pts, shift, hist, bintot));
+    OCNN_CUDA_OK(launch_chained(sort_rowscan_kernel<RB>, dim3(rows), dim3(kThreads), 0, st, hist, segs, L.segments,
                                 (const int*)bintot));
     if (p == 0)
       OCNN_CUDA_OK(launch_chained(sort_scatter_kernel<KeyT, true, RB>, dim3(chunks), dim3(kThreads), 0, st,
                                   (const KeyT*)keys[cur], (const uint32_t*)nullptr, keys[cur ^ 1], idx[cur ^ 1],
-                                  clouds, L.batch, ea.chunk_pts, shift, (const int*)hist));
+                                  segs, L.segments, ea.chunk_pts, shift, (const int*)hist));
     else
       OCNN_CUDA_OK(launch_chained(sort_scatter_kernel<KeyT, false, RB>, dim3(chunks), dim3(kThreads), 0, st,
                                   (const KeyT*)keys[cur], (const uint32_t*)idx[cur], keys[cur ^ 1], idx[cur ^ 1],
-                                  clouds, L.batch, ea.chunk_pts, shift, (const int*)hist));
+                                  segs, L.segments, ea.chunk_pts, shift, (const int*)hist));
     OCNN_LAUNCHES_OK("radix sort pass", p == 0 ? 2 : 3);
     cur ^= 1;
   }
@@ -1215,11 +1254,12 @@ int ocnn_octree_build_plan(const ocnn_points_batch* pts, const ocnn_build_params
 
   EncodeArgs ea;
   ea.table = reinterpret_cast<const CloudRef*>(ws + L.off_clouds);
+  ea.segments = ea.table + pts->batch + 1;
   ea.inline_clouds = pts->batch <= kInlineClouds ? 1 : 0;
   ea.batch = pts->batch; ea.depth = prm->depth; ea.chunk_pts = chunk_points(n);
   ea.mul = cell_scale(prm);
   for (int j = 0; j < 3; ++j) ea.bbmin[j] = prm->bbmin[j];
-  std::vector<CloudRef> big(ea.inline_clouds ? 0 : (size_t)pts->batch + 1);
+  std::vector<CloudRef> big(ea.inline_clouds ? 0 : (size_t)pts->batch + 3);
   CloudRef* table = ea.inline_clouds ? ea.clouds : big.data();
   int chunks = 0;
   for (int b = 0; b <= pts->batch; ++b) {
@@ -1233,6 +1273,15 @@ int ocnn_octree_build_plan(const ocnn_points_batch* pts, const ocnn_build_params
     c.chunk0 = chunks;
     c.pad = 0;
     if (real) chunks += ceil_div(pts->offsets_host[b + 1] - pts->offsets_host[b], ea.chunk_pts);
+  }
+  if (L.segments != L.batch) {           // one segment of all clouds (by_cloud: more than ride along)
+    chunks = ceil_div(n, ea.chunk_pts);
+    for (int e = 0; e < 2; ++e) {
+      CloudRef& c = big[pts->batch + 1 + e];
+      memset(&c, 0, sizeof(c));
+      c.offset = e == 0 ? 0 : n;
+      c.chunk0 = e == 0 ? 0 : chunks;
+    }
   }
   // (pageable source: the runtime stages it before returning, so `big` may go out of scope)
   if (!ea.inline_clouds)

@@ -58,3 +58,18 @@ def test_signal_channels(ocnn, channels, normals, depth):
 def test_several_tiles_per_chunk(ocnn):
   """Enough points that a sort chunk is more than one tile, in clouds that do not divide it."""
   check(ocnn, clouds_of([700000, 3, 600001], 11), 7, 2, 64)
+
+
+@pytest.mark.parametrize('depth,key_bits,sizes', [
+    # as many clouds as are sorted one by one whatever their size, and one more; a chunk of 2048 points that
+    # holds a few clouds, hundreds, or the end of a large one; 32- and 64-bit composite keys, 8- and 9-bit digits
+    (5, 64, [5] * 64), (5, 64, [5] * 65), (1, 64, [1] * 300), (3, 64, [3] * 1000), (8, 64, [9] * 70),
+    (6, 32, [17, 1, 300] * 40), (9, 64, [40] * 500), (11, 64, [4000] + [2] * 200 + [2500, 1]),
+    (6, 64, [7] * 5000)])
+def test_batches_sorted_over_their_cloud_bits(ocnn, depth, key_bits, sizes):
+  check(ocnn, clouds_of(sizes, 300), depth, min(depth, 2), key_bits)
+
+
+@pytest.mark.parametrize('points', [6999, 7000])
+def test_average_size_at_which_clouds_are_sorted_one_by_one(ocnn, points):
+  check(ocnn, clouds_of([points - 500, points + 500] * 33, 77, channels=2), 6, 2, 64)
