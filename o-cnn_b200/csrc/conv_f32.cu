@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kF32Threads, NG <= 4 ? 2 : 1) conv_f32_kernel(
         tmem_ld8(lane_base + (uint32_t)(2 * N + 8 * g), v2);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[8 * g + j] += __uint_as_float(v2[j]) + __uint_as_float(v1[j]);
+        for (int j = 0; j < 8; ++j) acc[8 * g + j] = join_products(acc[8 * g + j], __uint_as_float(v1[j]), __uint_as_float(v2[j]));
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(smem_u32(dempty));

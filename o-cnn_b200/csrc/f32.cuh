@@ -89,6 +89,15 @@ __device__ __forceinline__ void split_rows(const float* __restrict__ x, uint8_t*
   for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(dst + q * width) = part[q];
 }
 
+// The sum of all products from that of the high ones and those of the small ones.  A sum that is infinite
+// or NaN is so because of its operands (or has overflowed) and the high products alone say which, as a chain of fp32
+// multiply-adds would: the small ones hold inf * 0 there (the lower parts of a value that bf16 holds are 0)
+// and infinities of either sign.  What is left: an infinity times a value below 2^-134, whose high part
+// is 0, gives NaN instead of an infinity.
+__device__ __forceinline__ float join_products(float high, float mid, float low) {
+  return fabsf(high) < __int_as_float(0x7f800000) ? high + (low + mid) : high;
+}
+
 // Offset of 16-byte chunk cc (of cpt per row) of part q in such a row: base + q * width.
 __device__ __forceinline__ void chunk_place(int cc, int cpt, uint32_t& base, uint32_t& width) {
   const uint32_t block = (uint32_t)cc >> 2;

@@ -120,3 +120,41 @@ def test_extreme_values(ocnn, octree):
   want = (w[:, 13::27].double() @ x.view(40, h).double()).view(1, 32, h, 1)
   mag = (w[:, 13::27].double().abs() @ x.view(40, h).double().abs()).view(1, 32, h, 1)
   assert float(((got.double() - want).abs() / (mag + 1e-36)).max()) < 1e-6
+
+
+def same_kinds(got, want):
+  """Infinities of the same sign and NaNs in the same places, the rest finite and close."""
+  finite = torch.isfinite(want)
+  assert torch.equal(torch.isnan(got), torch.isnan(want))
+  assert torch.equal(torch.isposinf(got), torch.isposinf(want)) and torch.equal(torch.isneginf(got), torch.isneginf(want))
+  assert 0 < int(finite.sum()) < finite.numel()
+  assert off(got[finite], want[finite].double()) < 2e-6
+
+
+# (one and four weight images a stage, K splits and none; weights that bf16 holds exactly, whose lower parts
+# are 0, and others, whose lower parts have either sign)
+@pytest.mark.parametrize('cin,cout', [(40, 32), (64, 96)])
+@pytest.mark.parametrize('depth', [5, 2])
+@pytest.mark.parametrize('exact', [True, False])
+def test_infinities(ocnn, octree, cin, cout, depth, exact):
+  """An infinite operand gives what the chain of fp32 multiply-adds gives: forward, data and weight gradient."""
+  tree, v = octree
+  h = int(v.nnum[depth])
+  torch.manual_seed(cin + depth)
+  x, w = torch.randn(1, cin, h, 1, device='cuda'), torch.randn(cout, cin * 27, device='cuda') * 0.1
+  g = torch.randn(1, cout, h, 1, device='cuda')
+  if exact:
+    x, w, g = (t.bfloat16().float() for t in (x, w, g))
+  x[0, 0, 3, 0], x[0, 5, 70, 0], x[0, 7, 71, 0] = float('inf'), -float('inf'), float('inf')
+  same_kinds(ocnn.nn.octree_conv(x, w, tree, depth, cout, [3, 3, 3], 1, False),
+             ocnn.nn.octree_conv(x, w, tree, depth, cout, [3, 3, 3], 1, False, True))
+  col = columns(ocnn, x, tree, depth, False)
+  same_kinds(ocnn.nn.octree_conv_grad(x, w, tree, g, depth, cout, [3, 3, 3], 1, False, False, True)[1], g.view(cout, h).double() @ col.t())
+  same_kinds(ocnn.nn.pointwise_conv(x, w[:, :cin].contiguous(), None, None, None, False),
+             (w[:, :cin].double() @ x.view(cin, h).double()).view(1, cout, h, 1))
+  g[0, 2, 9, 0] = -float('inf')
+  x = x.nan_to_num(posinf=1.0, neginf=1.0)
+  col = columns(ocnn, x, tree, depth, False)
+  same_kinds(ocnn.nn.octree_conv_grad(x, w, tree, g, depth, cout, [3, 3, 3], 1, False, False, True)[1], g.view(cout, h).double() @ col.t())
+  same_kinds(ocnn.nn.octree_deconv(g, w, tree, depth, cin, [3, 3, 3], 1, False),
+             ocnn.nn.octree_deconv(g, w, tree, depth, cin, [3, 3, 3], 1, False, True))
