@@ -1,6 +1,8 @@
 """fp32 layers on the tensor cores (three bf16 parts per value) and on whole sibling groups: every width of
 the accumulator tile, more than one slice of output channels, K splits, chunk remainders, node counts
 that do not fill a tile, against the column formulation in float64."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -104,6 +106,37 @@ def test_pointwise_training_layer(ocnn):
     want = torch.autograd.grad(layer.conv1x1(x.squeeze(-1)).unsqueeze(-1), params, g)
     for a, b in zip(got, want):
       assert a.shape == b.shape and off(a, b.double()) < 2e-3     # (torch's own may run in TF32)
+
+
+class _Geometry(ctypes.Structure):
+  _fields_ = [(n, ctypes.c_int32) for n in ('transposed', 'stride', 'nempty', 'h_in', 'h_out')] + \
+      [(n, ctypes.c_void_p) for n in ('neigh', 'child', 'ichild')]
+
+
+@pytest.mark.parametrize('ks', [[3, 3, 3], [2, 2, 2], [3, 1, 1], [1, 1, 1]])
+@pytest.mark.parametrize('stride,nempty', [(1, False), (1, True), (2, False), (2, True)])
+def test_weight_gradient_without_a_workspace(ocnn, octree, ks, stride, nempty):
+  """ocnn_octree_conv_weight_grad: the CUDA-core form that asks for no device memory, through the C interface."""
+  tree, v = octree
+  lib, d, m, c = ctypes.CDLL(ocnn.LIBRARY), 5, 20, 9
+  lib.ocnn_last_error.restype = ctypes.c_char_p
+  neigh, child = (ocnn.octree_property(tree, p, d).contiguous() for p in ('neigh', 'child'))
+  ichild = torch.nonzero(child >= 0).flatten().int()
+  h_in = int(v.nnum_nempty[d] if nempty else v.nnum[d])
+  h_out = int(v.nnum[d]) // 8 if stride == 2 else h_in
+  x, a = torch.randn(1, c, h_in, 1, device='cuda'), torch.randn(1, m, h_out, 1, device='cuda')
+  col = ocnn.nn.octree2col(x, tree, d, ks, stride, nempty).flatten(0, 1).double()
+  taps = ks[0] * ks[1] * ks[2]
+  want = a.view(m, h_out).double() @ col.view(c * taps, h_out).t()
+  geo = _Geometry(0, stride, nempty, h_in, h_out, neigh.data_ptr(), child.data_ptr(), ichild.data_ptr())
+  ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+  for node_major in (0, 1):
+    xa, aa = ((t.view(t.shape[1], -1).t() if node_major else t).contiguous() for t in (x, a))
+    got = torch.full((m, c * taps), 7.0, device='cuda')
+    status = lib.ocnn_octree_conv_weight_grad(ptr(aa), ptr(xa), ptr(got), ctypes.byref(geo), m, c, (ctypes.c_int * 3)(*ks),
+                                              node_major, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert status == 0, lib.ocnn_last_error()
+    assert off(got, want) < 1e-6
 
 
 def test_extreme_values(ocnn, octree):
