@@ -158,12 +158,10 @@ class OctreeConv1x1(_nn.Module):
     conv = self.conv1x1
     if torch.is_grad_enabled() and (data_in.requires_grad or
                                     (self.training and conv.weight.requires_grad)):
-      # Training: torch's own 1x1 convolution (as the reference), which autograd differentiates. At
-      # 64 to 128 output channels cuDNN forms the weight gradient with a direct fp32 kernel (16 -> 64
-      # at 107 k nodes: 395 us); ours is used there. Elsewhere cuDNN takes a GEMM (about 55 us).
-      if (64 <= conv.weight.shape[0] <= 128 and data_in.dtype == conv.weight.dtype == torch.float32 and
-          data_in.is_cuda and data_in.is_contiguous() and not torch.is_autocast_enabled() and
-          _stock_conv1x1(conv)):
+      # training: torch's own 1x1 convolution (as the reference), which autograd differentiates; for some
+      # widths with this library's weight gradient
+      if nn.own_pointwise_weight_grad(conv.weight, data_in) and not torch.is_autocast_enabled() and \
+          _stock_conv1x1(conv):
         out = _Conv1x1Function.apply(data_in, conv.weight, conv.bias)
       else:
         out = conv(data_in.squeeze(-1)).unsqueeze(-1)

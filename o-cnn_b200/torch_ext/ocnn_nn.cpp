@@ -1059,6 +1059,21 @@ Tensor pointwise_conv_weight_grad(Tensor data_in, Tensor grad) {
   return gw;
 }
 
+// Whether a 1x1 layer's weight gradient in training is pointwise_conv_weight_grad (fp32 throughout) or torch's:
+// 64 to 128 output channels.  There cuDNN mostly takes a direct fp32 kernel, elsewhere a GEMM that runs in
+// TF32 as torch's default allows.  Measured, us of cuDNN / ours:
+//   inside   16 -> 64: 1 k rows 6.6 / 9.2, 4 k 17 / 13, 16 k 60 / 22, 107 k 386 / 48, 440 k 2547 / 250
+//            64 -> 128: 1 k rows 18 / 12, 16 k 197 / 24, 107 k 1438 / 99;  32 -> 65: 4 k 20 / 14, 107 k 461 / 64
+//   outside  at 107 k rows 16 -> 32: 16 / 36, 16 -> 48: 17 / 47, 16 -> 136: 26 / 105, 64 -> 256: 38 / 164;
+//            at 1 k rows 7.8 / 8.5, 7.8 / 9.3, 7.8 / 11, 7.8 / 14
+// Inside, cuDNN has its TF32 GEMM too at 96 channels (32 -> 96 at 107 k: 23 / 67) and beyond about 1e9 products
+// (64 -> 64 at 440 k: 50 / 471, 64 -> 128 at 220 k: 42 / 236); its error is 3e-4 there, ours 2e-7, and these stay
+// in fp32 like their neighbours.
+bool own_pointwise_weight_grad(const Tensor& weight, const Tensor& data) {
+  return weight.size(0) >= 64 && weight.size(0) <= 128 && weight.scalar_type() == torch::kFloat32 &&
+         data.scalar_type() == torch::kFloat32 && data.is_cuda() && data.is_contiguous();
+}
+
 Tensor pointwise_conv_tc(Tensor data_in, Tensor packed, int num_output, c10::optional<Tensor> scale,
                          c10::optional<Tensor> bias, c10::optional<Tensor> residual, bool relu,
                          Tensor status) {
@@ -1322,7 +1337,7 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     res[4] = gbb;
     gz = gz.contiguous();
     if (kind == 2) {
-      const bool ours = own_weight_grad(weight, data);
+      const bool ours = own_pointwise_weight_grad(weight, data);
       if (need_data || need_bias || (need_weight && !ours)) {
         c10::optional<at::IntArrayRef> bias_sizes;
         vector<int64_t> bs = {weight.size(0)};
@@ -1345,13 +1360,6 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
       res[1] = gr[1];
     }
     return res;
-  }
-
-  // At 64 to 128 output channels cuDNN forms a 1x1 layer's weight gradient with a direct fp32 kernel (16 ->
-  // 64 at 107 k nodes: 395 us); ours is used there.  Elsewhere cuDNN takes a GEMM (about 55 us).
-  static bool own_weight_grad(const Tensor& weight, const Tensor& data) {
-    return weight.size(0) >= 64 && weight.size(0) <= 128 && weight.scalar_type() == torch::kFloat32 &&
-           data.scalar_type() == torch::kFloat32 && data.is_contiguous();
   }
 };
 
@@ -2737,6 +2745,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("scale") = py::none(), py::arg("bias") = py::none(),
         py::arg("residual") = py::none(), py::arg("relu") = false);
   m.def("pointwise_conv_weight_grad", &pointwise_conv_weight_grad);
+  m.def("own_pointwise_weight_grad", &own_pointwise_weight_grad, py::arg("weight"), py::arg("data"));
   m.def("pointwise_conv_tc", &pointwise_conv_tc, py::arg("data_in"), py::arg("packed"),
         py::arg("num_output"), py::arg("scale") = py::none(), py::arg("bias") = py::none(),
         py::arg("residual") = py::none(), py::arg("relu") = false, py::arg("status"));

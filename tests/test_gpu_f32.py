@@ -108,6 +108,27 @@ def test_pointwise_training_layer(ocnn):
       assert a.shape == b.shape and off(a, b.double()) < 2e-3     # (torch's own may run in TF32)
 
 
+@pytest.mark.parametrize('cout', [63, 64, 96, 128, 129])
+def test_weight_gradient_of_a_pointwise_training_layer(ocnn, cout):
+  """The layer alone and in its block follow one rule, and inside it the weight gradient is fp32 throughout."""
+  torch.manual_seed(cout)
+  x, g = torch.randn(1, 32, 3000, 1, device='cuda'), torch.randn(1, cout, 3000, 1, device='cuda')
+  layer, block = ocnn.OctreeConv1x1(32, cout).cuda().train(), ocnn.OctreeConv1x1Bn(32, cout).cuda().train()
+  own = ocnn.nn.own_pointwise_weight_grad(layer.conv1x1.weight, x)
+  assert own == (64 <= cout <= 128)
+  assert not ocnn.nn.own_pointwise_weight_grad(layer.conv1x1.weight, x.half())
+  assert not ocnn.nn.own_pointwise_weight_grad(layer.conv1x1.weight, x.contiguous(memory_format=torch.channels_last))
+  want = g.view(cout, -1).double() @ x.view(32, -1).double().t()
+  got, = torch.autograd.grad(layer(x), layer.conv1x1.weight, g)
+  assert off(got.view(cout, 32), want) < (1e-6 if own else 2e-3)
+  # the block's gradient reaches its 1x1 layer through the BatchNorm: the same through the modules one by one
+  weight, bn = block.conv1x1.conv1x1.weight, block.bn
+  y = torch.einsum('oc,nchw->nohw', weight.detach()[:, :, 0].double(), x.double()).float().requires_grad_()
+  gy, = torch.autograd.grad(bn(y), y, g)
+  got, = torch.autograd.grad(block(x), weight, g)
+  assert off(got.view(cout, 32), gy.view(cout, -1).double() @ x.view(32, -1).double().t()) < 5e-3
+
+
 class _Geometry(ctypes.Structure):
   _fields_ = [(n, ctypes.c_int32) for n in ('transposed', 'stride', 'nempty', 'h_in', 'h_out')] + \
       [(n, ctypes.c_void_p) for n in ('neigh', 'child', 'ichild')]
