@@ -559,16 +559,27 @@ bool use_conv_f32() {
 // tensor cores (three bf16 parts per value) where that kernel serves the layer, everything else on
 // the CUDA cores.  OCNN_CONV_F32=0 keeps fp32 on the CUDA cores.
 //
-// fma_chain: every output as one chain of rounded multiply-adds in the weights' order.  Training asks
-// for it, in both directions: its networks take maxima and ReLUs of these values and feed them to TF32
-// products, so a sum that differs in its last bit sends single nodes' gradients elsewhere (1e-7 in a
-// forward pass is 1e-2 in a weight gradient), and a run should not depend on the kernel.  It is kept
-// up to 4 GFLOP a layer, where it costs a tenth of a millisecond at most; beyond that the tensor
-// cores are four times faster (24 GFLOP, 32 -> 64 at 217 k nodes: 598 us against 176).
-// Few channels stay on the CUDA cores in any case: the tensor-core kernel's gather moves 16-byte
-// pieces whatever the channel count (3 -> 32 at 222 k nodes: 40 us against 77; 16 -> 16 at 217 k, where
-// the two meet: 88 against 91); for every kind of layer, so that few channels give the same bits in and
-// outside of training, on all nodes and on the non-empty ones.
+// fma_chain: what training asks for, in both directions: every output as one chain of rounded
+// multiply-adds in the weights' order, up to 4 GFLOP a layer.  Either kernel is fp32 (off 64 bits by 3e-7 to
+// 1.4e-6 of the norm, growing with the channels, the tensor cores by 2e-7 to 3.5e-7), but a network's gradient is not a
+// smooth function of such differences: its 1x1 layers run in TF32 inside cuDNN and its maxima have ties.
+// The weight gradients of a training step of ResNet, 16 x 10 k points at depth 5, differ by 7e-3 (median) to 2e-2 between the two kernels
+// (by 6e-7 to 2e-6 with TF32 off) and its time does not (2.7 to 2.9 ms).  With the chain, a network of which every
+// layer is below the line has the activations and data gradients of the CUDA-core kernels, bit for bit,
+// whatever the batch (its weight gradients are conv_f32_wgrad.cu's: nothing else is formed from them).  Above it
+// that is given up for time, and the last bits of a layer depend on which side of the line a batch puts it.  What
+// the chain costs, us chain / tensor cores: 32 -> 32 0.35 GF 30 / 24, 1.6 GF 57 / 32, 3.4 GF 111 / 54, 6.6 GF 190 / 98,
+// 13.5 GF 342 / 173; 64 -> 64 0.35 GF 51 / 23, 1.4 GF 76 / 31, 3.4 GF 124 / 47, 7 GF 209 / 61, 26 GF 651 / 211;
+// 128 -> 128 3.0 GF 207 / 40, 8 GF 245 / 62, 28 GF 741 / 160 (forward; data gradients up to 1.4 times the chain's).
+// Time alone would put the line at about 0.3 GFLOP; at 4 the chain costs up to 0.17 ms a layer.
+//
+// Few channels (cin * cout <= 256) stay on the CUDA cores in any case.  On all nodes, channel-major, stride 1
+// (conv_group.cu) they are as fast or faster: 3 -> 32 at 9 k / 119 k / 964 k nodes 5.5 / 26 / 155 us against 13 / 54 /
+// 289, 8 -> 8 6 / 31 / 186 against 14 / 50 / 272, 16 -> 16 12 / 61 / 368 against 17 / 61 / 395, 8 -> 32 11 / 54 / 353
+// against 14 / 55 / 295.  The other kinds of layer follow so that few channels give the same bits on all and
+// on the non-empty nodes, in either layout, in and outside of training; there it costs time (conv_simt.cu
+// against the tensor cores: 16 -> 16 on 317 k non-empty nodes 653 / 137 us, node-major 713 / 136, stride 2 at 121 k
+// groups 267 / 131; 3 -> 32 178 / 91, 260 / 101, 74 / 75).
 void run_conv(const DataRef& x, const Tensor& w, Tensor& y, const ocnn_conv_geometry& g, int cin, int cout,
               const vector<int>& ks, const ocnn_conv_epilogue* ep, bool fma_chain = false) {
   const int taps = ks[0] * ks[1] * ks[2];
@@ -1361,6 +1372,7 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     }
     return res;
   }
+
 };
 
 Tensor train_block(Tensor data, Tensor weight, c10::optional<Tensor> bias, Tensor bn_weight, Tensor bn_bias,

@@ -212,3 +212,31 @@ def test_infinities(ocnn, octree, cin, cout, depth, exact):
   same_kinds(ocnn.nn.octree_conv_grad(x, w, tree, g, depth, cout, [3, 3, 3], 1, False, False, True)[1], g.view(cout, h).double() @ col.t())
   same_kinds(ocnn.nn.octree_deconv(g, w, tree, depth, cin, [3, 3, 3], 1, False),
              ocnn.nn.octree_deconv(g, w, tree, depth, cin, [3, 3, 3], 1, False, True))
+
+
+@pytest.mark.parametrize('big', [False, True])
+def test_which_kernel_a_training_layer_takes(ocnn, octree, big_octree, big):
+  """Below 4 GFLOP forward and data gradient are the CUDA cores' chain bit for bit (ocnn_octree_conv_general), above
+  it the tensor-core kernel's values."""
+  tree, v = big_octree if big else octree
+  d, c = (6, 64) if big else (5, 32)
+  h = int(v.nnum[d])
+  assert (2 * 27 * c * c * h > 4e9) == big
+  layer = ocnn.OctreeConv(d, c, c).cuda().train()
+  w = layer.weights.detach()
+  x = torch.randn(1, c, h, 1, device='cuda', requires_grad=True)
+  g = torch.randn(1, c, h, 1, device='cuda')
+  y = layer(x, tree)
+  gx, = torch.autograd.grad(y, x, g)
+  if big:
+    want = (ocnn.nn.octree_conv(x.detach(), w, tree, d, c, [3, 3, 3], 1, False),
+            ocnn.nn.octree_deconv(g, w, tree, d, c, [3, 3, 3], 1, False))
+  else:
+    lib, neigh, want = ctypes.CDLL(ocnn.LIBRARY), ocnn.octree_property(tree, 'neigh', d).contiguous(), []
+    for transposed, data in ((0, x.detach()), (1, g)):
+      geo, out = _Geometry(transposed, 1, 0, h, h, neigh.data_ptr(), None, None), torch.empty_like(data)
+      assert lib.ocnn_octree_conv_general(*(ctypes.c_void_p(t.data_ptr()) for t in (data, w, out)), ctypes.byref(geo), c, c,
+                                          (ctypes.c_int * 3)(3, 3, 3), 0, 0, None,
+                                          ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+      want.append(out)
+  assert torch.equal(y.detach(), want[0]) and torch.equal(gx, want[1])
