@@ -12,6 +12,7 @@
 //    channels_last (node-major).  Outputs keep the dtype and layout of the input.
 //  * Errors raise Python exceptions; nothing aborts (pytorch/cpp uses CHECK -> abort()).
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime.h>
@@ -1190,19 +1191,36 @@ class ConvLayer {
 
  private:
   // The packed image of the module's parameter `weights` (`w`: its float32 values), made when it was
-  // not seen before (another tensor, or written to since); undefined for a shape the tensor-core
-  // kernel does not take.
+  // not seen before (another storage, or written to since); undefined for a shape the tensor-core
+  // kernel does not take.  The weak reference keeps the storage's address from being reused for another one
+  // (a parameter that went to the CPU and came back usually lies where it lay, at the same version).  Another
+  // stream than the one that packed waits for it, and the allocator learns of its use; what is packed under
+  // stream capture belongs to the graph and is not kept.
   Tensor packed_for(const Tensor& weights, const Tensor& w, bool half) {
     const bool versioned = !weights.is_inference();
-    const void* ptr = weights.data_ptr();
+    c10::StorageImpl* impl = weights.storage().unsafeGetStorageImpl();
     const int64_t version = versioned ? (int64_t)weights._version() : -1;
+    const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
     std::lock_guard<std::mutex> lock(mutex_);
-    if (versioned && ptr == ptr_ && version == version_ && half == half_) return packed_;
-    packed_ = Tensor();
+    if (versioned && storage_._unsafe_get_target() == impl && offset_ == weights.storage_offset() &&
+        version == version_ && half == half_) {
+      if (packed_.defined() && stream != *stream_) {
+        if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) ready_.block(stream);
+        packed_.record_stream(stream);
+      }
+      return packed_;
+    }
+    Tensor packed;
     if (ocnn_conv_packed_weight_bytes_general(cin_, cout_, ks_.data(), stride_, transposed_, nempty_) > 0)
-      packed_ = conv_pack_weights_general(w, cin_, cout_, ks_, stride_, transposed_, nempty_, half);
-    ptr_ = ptr; version_ = version; half_ = half;
-    return packed_;
+      packed = conv_pack_weights_general(w, cin_, cout_, ks_, stride_, transposed_, nempty_, half);
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return packed;
+    packed_ = packed;
+    ready_ = at::cuda::CUDAEvent();        // (one per packing: the module may have gone to another GPU)
+    if (packed.defined()) ready_.record(stream);
+    storage_ = c10::weak_intrusive_ptr<c10::StorageImpl>(
+        c10::intrusive_ptr<c10::StorageImpl>::reclaim_copy(impl));
+    offset_ = weights.storage_offset(); version_ = version; half_ = half; stream_ = stream;
+    return packed;
   }
   int cin_, cout_;
   vector<int> ks_;
@@ -1210,9 +1228,11 @@ class ConvLayer {
   bool nempty_, transposed_, point_;
   std::mutex mutex_;
   Tensor packed_;
-  const void* ptr_ = nullptr;
-  int64_t version_ = -1;
+  c10::weak_intrusive_ptr<c10::StorageImpl> storage_{c10::intrusive_ptr<c10::StorageImpl>()};
+  int64_t offset_ = 0, version_ = -1;
   bool half_ = false;
+  c10::optional<c10::cuda::CUDAStream> stream_;
+  at::cuda::CUDAEvent ready_;
 };
 
 // 1x1x1 convolution over the concatenated channels of two tensors of the same rows: the sum of a
@@ -1372,7 +1392,6 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     }
     return res;
   }
-
 };
 
 Tensor train_block(Tensor data, Tensor weight, c10::optional<Tensor> bias, Tensor bn_weight, Tensor bn_bias,

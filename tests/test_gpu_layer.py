@@ -205,3 +205,49 @@ def test_conv1d_of_another_width(ocnn):
         ref = torch.einsum('oc,ch->oh', layer.conv1x1.weight[:, :, 0].double(), x.squeeze(0).squeeze(-1).double())
         assert got.shape == (1, cout, 300, 1)
         assert float((got.double().squeeze(0).squeeze(-1) - ref).norm() / ref.norm()) < tol
+
+
+def test_another_parameter_at_the_same_place(ocnn, batch):
+  """A parameter that is dropped for a new one of the same size, which the allocator puts where it lay."""
+  octree, v = batch
+  x = torch.randn(1, 64, int(v.nnum[4]), 1, device='cuda').to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+  layer = ocnn.OctreeConv(4, 64, 64).cuda().eval()
+  layer.weights = torch.nn.Parameter(torch.randn(64, 64 * 27, device='cuda'))
+  same = 0
+  with torch.no_grad():
+    for _ in range(8):
+      before = layer.weights.data_ptr(), layer.weights._version
+      layer(x, octree)
+      del layer.weights
+      layer.weights = torch.nn.Parameter(torch.randn(64, 64 * 27, device='cuda'))
+      same += (layer.weights.data_ptr(), layer.weights._version) == before
+      assert torch.equal(layer(x, octree), copy.deepcopy(layer)(x, octree))
+  assert same > 0
+
+
+def test_packed_weights_on_another_stream(ocnn, batch):
+  """A second stream waits for the weights that the first one is still to pack."""
+  octree, v = batch
+  x = torch.randn(1, 64, int(v.nnum[4]), 1, device='cuda').to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+  layer = ocnn.OctreeConv(4, 64, 64).cuda().eval()
+  ocnn.octree_property(octree, 'child', 4)                 # (the octree's header is read)
+  side = torch.cuda.Stream()
+  torch.cuda.synchronize()
+  with torch.no_grad():
+    torch.cuda._sleep(20_000_000)                          # about 10 ms on the first stream
+    mine = layer(x, octree)
+    with torch.cuda.stream(side):
+      theirs = layer(x, octree)
+    torch.cuda.synchronize()
+    assert torch.equal(mine, theirs)
+    # packed inside a capture: the graph's own, not kept for later calls
+    fresh = copy.deepcopy(layer)
+    fresh.weights.mul_(2.0)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+      y = fresh(x, octree)
+    eager = fresh(x, octree)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, eager)
