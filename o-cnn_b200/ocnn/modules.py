@@ -30,13 +30,20 @@ def _trainable(data, weight, bn, residual):
           data.is_contiguous() and weight.dtype == torch.float32 and weight.is_cuda and bn.affine and
           bn.track_running_stats and bn.momentum is not None and bn.weight.dtype == torch.float32 and
           (residual is None or residual.dtype == torch.float32) and not torch.is_autocast_enabled() and
-          not hooked(bn))
+          not hooked(bn) and _only_backward())
 
 
 def hooked(module):
   """Whether someone asked to see this module's calls: a path that passes it by has to leave it alone."""
   return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or
               module._backward_pre_hooks or torch.nn.modules.module._has_any_global_hook())
+
+
+def _only_backward():
+  """Whether no more than reverse-mode autograd looks on: a functorch transform, a level of forward-mode
+  derivatives, a tracer or a compiler has to see torch's own operators."""
+  return (torch._C._functorch.peek_interpreter_stack() is None and torch.autograd.forward_ad._current_level < 0 and
+          torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
 
 
 def _stock_conv1x1(conv):
@@ -120,7 +127,8 @@ class FcBnRelu(_nn.Module):
 
 
 class _Conv1x1Function(torch.autograd.Function):
-  """torch's own 1x1 convolution with this library's kernel for the weight gradient."""
+  """torch's own 1x1 convolution with this library's kernel for the weight gradient (torch's where that is to be
+  differentiated again)."""
 
   @staticmethod
   def forward(ctx, data, weight, bias):
@@ -134,12 +142,13 @@ class _Conv1x1Function(torch.autograd.Function):
     need_x, need_w, need_b = ctx.needs_input_grad
     grad = grad.contiguous()
     gx = gw = gb = None
-    if need_x or need_b:
-      gx, _, gb = torch.ops.aten.convolution_backward(
+    own = need_w and not torch.is_grad_enabled()
+    if need_x or need_b or (need_w and not own):
+      gx, gw, gb = torch.ops.aten.convolution_backward(
           grad.squeeze(-1), data.squeeze(-1), weight, ctx.bias, [1], [0], [1], False, [0], 1,
-          [need_x, False, need_b])
+          [need_x, need_w and not own, need_b])
       gx = gx if gx is None else gx.unsqueeze(-1)
-    if need_w:
+    if own:
       gw = nn.pointwise_conv_weight_grad(data, grad).view_as(weight)
     return gx, gw, gb
 
@@ -161,7 +170,7 @@ class OctreeConv1x1(_nn.Module):
       # training: torch's own 1x1 convolution (as the reference), which autograd differentiates; for some
       # widths with this library's weight gradient
       if nn.own_pointwise_weight_grad(conv.weight, data_in) and not torch.is_autocast_enabled() and \
-          _stock_conv1x1(conv):
+          _stock_conv1x1(conv) and _only_backward():
         out = _Conv1x1Function.apply(data_in, conv.weight, conv.bias)
       else:
         out = conv(data_in.squeeze(-1)).unsqueeze(-1)

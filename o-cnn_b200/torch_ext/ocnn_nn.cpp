@@ -1302,6 +1302,37 @@ using torch::autograd::AutogradContext;
 using torch::autograd::Variable;
 using torch::autograd::variable_list;
 
+// A (de)convolution as autograd sees it in the modules one by one (TrainBlock::differentiable).
+struct TrainConv : public torch::autograd::Function<TrainConv> {
+  static Variable forward(AutogradContext* ctx, const Tensor& data, const Tensor& weight, const Tensor& octree,
+                          bool deconv, int64_t depth, int64_t num_output, const vector<int64_t>& kernel_size,
+                          int64_t stride, bool nempty) {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    ctx->save_for_backward({data, weight, octree});
+    ctx->saved_data["deconv"] = deconv;
+    ctx->saved_data["depth"] = depth;
+    ctx->saved_data["num_output"] = num_output;
+    ctx->saved_data["ks"] = kernel_size;
+    ctx->saved_data["stride"] = stride;
+    ctx->saved_data["nempty"] = nempty;
+    const vector<int> ks(kernel_size.begin(), kernel_size.end());
+    return (deconv ? octree_deconv : octree_conv)(data, weight, octree, (int)depth, (int)num_output, ks, (int)stride,
+                                                  nempty, true);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const auto k64 = ctx->saved_data["ks"].toIntVector();
+    auto gr = conv_grad_impl(saved[0], saved[1], saved[2], grads[0].contiguous(), (int)ctx->saved_data["depth"].toInt(),
+                             (int)ctx->saved_data["num_output"].toInt(), vector<int>(k64.begin(), k64.end()),
+                             (int)ctx->saved_data["stride"].toInt(), ctx->saved_data["nempty"].toBool(),
+                             ctx->saved_data["deconv"].toBool(), ctx->needs_input_grad(0), ctx->needs_input_grad(1));
+    variable_list res(9);
+    res[0] = gr[0];
+    res[1] = gr[1];
+    return res;
+  }
+};
+
 struct TrainBlock : public torch::autograd::Function<TrainBlock> {
   // kind: 0 convolution, 1 deconvolution, 2 1x1 layer
   static Variable forward(AutogradContext* ctx, const Tensor& data, const Tensor& weight,
@@ -1360,6 +1391,10 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     if (out.defined()) g = at::threshold_backward(g, out, 0);
     variable_list res(18);
     if (has_res) res[5] = g;
+    if (at::GradMode::is_enabled()) {
+      differentiable(ctx, data, weight, bn_weight, octree, g, need_data, need_weight, need_bias, res);
+      return res;
+    }
     Tensor gz, gbw, gbb;
     std::tie(gz, gbw, gbb) = at::_batch_norm_impl_index_backward(
         ctx->saved_data["impl"].toInt(), z, g, bn_weight, saved[9], saved[10], saved[4], saved[5], /*train=*/true,
@@ -1391,6 +1426,37 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
       res[1] = gr[1];
     }
     return res;
+  }
+
+  // The gradients where they are to be differentiated again (create_graph): those of the modules one by one,
+  // which are formed anew from the saved inputs.  (What the forward pass kept, z and its statistics, has no
+  // history: the derivatives of the gradients with respect to what z depends on would be missing.)
+  static void differentiable(AutogradContext* ctx, const Tensor& data, const Tensor& weight, const Tensor& bn_weight,
+                             const Tensor& octree, const Tensor& g, bool need_data, bool need_weight, bool need_bias,
+                             variable_list& res) {
+    const int64_t kind = ctx->saved_data["kind"].toInt();
+    Tensor z;
+    if (kind == 2) {
+      z = at::conv1d(data.squeeze(-1), weight).unsqueeze(-1);    // (a bias falls out of the batch's statistics)
+    } else {
+      z = TrainConv::apply(data, weight, octree, kind == 1, ctx->saved_data["depth"].toInt(),
+                           ctx->saved_data["num_output"].toInt(), ctx->saved_data["ks"].toIntVector(),
+                           ctx->saved_data["stride"].toInt(), ctx->saved_data["nempty"].toBool());
+    }
+    if (!z.requires_grad()) z.requires_grad_();
+    const Tensor scale = bn_weight.requires_grad() ? bn_weight : bn_weight.detach().requires_grad_();
+    const Tensor y = at::batch_norm(z, scale, at::zeros_like(scale), {}, {}, /*training=*/true, 0.0,
+                                    ctx->saved_data["eps"].toDouble(), at::globalContext().userEnabledCuDNN());
+    variable_list inputs = {z, scale};
+    if (need_data) inputs.push_back(data);
+    if (need_weight) inputs.push_back(weight);
+    const variable_list got = torch::autograd::grad({y}, inputs, {g}, /*retain_graph=*/true, /*create_graph=*/true);
+    size_t at_got = 2;
+    if (need_data) res[0] = got[at_got++];
+    if (need_weight) res[1] = got[at_got++];
+    if (need_bias) res[2] = got[0].sum({0, 2, 3});
+    res[3] = got[1];
+    res[4] = g.sum({0, 2, 3});
   }
 };
 
