@@ -33,10 +33,12 @@ def _trainable(data, weight, bn, residual):
           not hooked(bn) and _only_backward())
 
 
-def hooked(module):
-  """Whether someone asked to see this module's calls: a path that passes it by has to leave it alone."""
-  return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or
-              module._backward_pre_hooks or torch.nn.modules.module._has_any_global_hook())
+def hooked(*modules):
+  """Whether someone asked to see these modules' calls: a path that passes them by has to leave them alone."""
+  for m in modules:
+    if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks:
+      return True
+  return bool(torch.nn.modules.module._has_any_global_hook())
 
 
 def _only_backward():
@@ -156,7 +158,7 @@ class _Conv1x1Function(torch.autograd.Function):
 class OctreeConv1x1(_nn.Module):
   """A per-node linear map.  The parameters live in a torch Conv1d (as in the reference, so the
   state_dict keys match); the product runs on this library's pointwise kernels."""
-  _layer, _layer_shape = None, None
+  _layer = None
 
   def __init__(self, channel_in, channel_out, use_bias=False):
     super().__init__()
@@ -180,10 +182,9 @@ class OctreeConv1x1(_nn.Module):
       if residual is not None:
         out = out + residual
       return torch.relu(out) if relu else out
-    cout, cin = conv.weight.shape[:2]
-    if self._layer is None or self._layer_shape != (cin, cout):      # (the Conv1d can be replaced)
+    if self._layer is None:
+      cout, cin = conv.weight.shape[:2]
       self._layer = nn.ConvLayer(cin, cout, [1, 1, 1], 1, False, False, True)
-      self._layer_shape = (cin, cout)
     affine = bn_vectors(bn)
     if conv.bias is not None:
       with torch.no_grad():

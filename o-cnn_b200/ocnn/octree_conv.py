@@ -24,10 +24,11 @@ _STATUS = {}
 def tc_status(device):
   """The int32 status word the tensor-core kernels write on a bounded wait that ran out (one per
   device; 0 = no kernel ever gave up)."""
-  key = torch.device(device)
-  if key not in _STATUS:
-    _STATUS[key] = nn.tc_status(key)
-  return _STATUS[key]
+  status = _STATUS.get(device)
+  if status is None:
+    key = torch.device(device)
+    status = _STATUS[key] = nn.tc_status(key)
+  return status
 
 
 def resize_with_last_val(list_in, num=3):

@@ -42,13 +42,17 @@ class ResNet(_nn.Module):
     if self.training or data.dtype not in (torch.bfloat16, torch.float16) or torch.is_autocast_enabled():
       return False
     head = self.header
-    if type(head) is not _nn.Sequential or len(head) != 2:
+    if type(head) is not _nn.Sequential or len(head._modules) != 2:
       return False
-    pool, fc = head
-    if type(pool) is not FullOctreeGlobalPool or type(pool.octree2voxel) is not FullOctree2Voxel or \
-        type(fc) is not _nn.Linear or any(hooked(m) for m in (head, pool, pool.octree2voxel, fc)):
+    pool, fc = head._modules.values()
+    if type(pool) is not FullOctreeGlobalPool or type(fc) is not _nn.Linear:
       return False
-    params = [p for p in (fc.weight, fc.bias) if p is not None]
-    return (all(p.dtype == torch.float32 and p.device == data.device for p in params) and
-            data.is_contiguous(memory_format=torch.channels_last) and
-            not (torch.is_grad_enabled() and any(t.requires_grad for t in (data, *params))))
+    voxel = pool.octree2voxel
+    if type(voxel) is not FullOctree2Voxel or hooked(head, pool, voxel, fc):
+      return False
+    weight, bias = fc.weight, fc.bias
+    if weight.dtype != torch.float32 or (bias is not None and bias.dtype != torch.float32) or \
+        not data.is_contiguous(memory_format=torch.channels_last):
+      return False
+    return not (torch.is_grad_enabled() and (data.requires_grad or weight.requires_grad or
+                                             (bias is not None and bias.requires_grad)))

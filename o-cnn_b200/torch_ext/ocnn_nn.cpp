@@ -1138,7 +1138,10 @@ class ConvLayer {
     c10::cuda::CUDAGuard guard(data.device());
     DataRef x = get_data(data, what);
     const int K = ks_[0] * ks_[1] * ks_[2];
-    TORCH_CHECK(x.C == cin_, what, ": the data has ", x.C, " channels, the layer takes ", cin_);
+    // (a 1x1 layer's Conv1d can be replaced by one of another width)
+    TORCH_CHECK(!point_ || weights.dim() >= 2, what, ": the weights of a 1x1 layer are [Cout, Cin, 1]");
+    const int cin = point_ ? (int)weights.size(1) : cin_, cout = point_ ? (int)weights.size(0) : cout_;
+    TORCH_CHECK(x.C == cin, what, ": the data has ", x.C, " channels, the layer takes ", cin);
     Geometry geo;
     if (point_) {
       memset(&geo.g, 0, sizeof(geo.g));
@@ -1152,14 +1155,14 @@ class ConvLayer {
     Tensor keep[5];     // float32 copies of parameters that are held in another type
     auto f32 = [&](const c10::optional<Tensor>& t, int slot) -> const float* {
       if (!t.has_value() || !t->defined()) return nullptr;
-      TORCH_CHECK(t->is_cuda() && t->numel() == cout_, what, ": per-channel vectors must be CUDA tensors of ",
-                  cout_, " values");
+      TORCH_CHECK(t->is_cuda() && t->numel() == cout, what, ": per-channel vectors must be CUDA tensors of ",
+                  cout, " values");
       keep[slot] = t->to(torch::kFloat32).contiguous();
       return keep[slot].data_ptr<float>();
     };
     const bool has_bn = bn_var.has_value() && bn_var->defined();
-    Tensor y = new_data(cout_, geo.g.h_out, x);
-    ocnn_conv_epilogue ep = make_epilogue(c10::nullopt, c10::nullopt, residual, relu, cout_, y);
+    Tensor y = new_data(cout, geo.g.h_out, x);
+    ocnn_conv_epilogue ep = make_epilogue(c10::nullopt, c10::nullopt, residual, relu, cout, y);
     ep.scale_dev = f32(scale, 0);
     ep.bias_dev = f32(bias, 1);
     if (has_bn) {
@@ -1169,19 +1172,19 @@ class ConvLayer {
       ep.bn_eps = (float)bn_eps;
     }
     Tensor w = point_ ? weights.to(torch::kFloat32).contiguous() : weights;
-    check_weights(w, cin_, cout_, K);
-    const bool tc_layout = x.dtype != OCNN_F32 && cin_ % 8 == 0 && cout_ % 8 == 0 &&
+    check_weights(w, cin, cout, K);
+    const bool tc_layout = x.dtype != OCNN_F32 && cin % 8 == 0 && cout % 8 == 0 &&
                            data.is_contiguous(at::MemoryFormat::ChannelsLast);
     if (tc_layout) {
-      Tensor packed = packed_for(weights, w, x.dtype == OCNN_F16);
+      Tensor packed = packed_for(weights, w, cin, cout, x.dtype == OCNN_F16);
       if (packed.defined()) {
         TORCH_CHECK(status.is_cuda() && status.scalar_type() == torch::kInt32 && status.numel() >= 1,
                     "status must be an int32 CUDA tensor");
-        run_conv_tc(x.t.data_ptr(), packed, y, geo.g, cin_, cout_, ks_, x.dtype, &ep, status.data_ptr<int32_t>());
+        run_conv_tc(x.t.data_ptr(), packed, y, geo.g, cin, cout, ks_, x.dtype, &ep, status.data_ptr<int32_t>());
         return y;
       }
     }
-    run_conv(x, w.contiguous(), y, geo.g, cin_, cout_, ks_, &ep);
+    run_conv(x, w.contiguous(), y, geo.g, cin, cout, ks_, &ep);
     return y;
   }
 
@@ -1190,36 +1193,51 @@ class ConvLayer {
   }
 
  private:
+  static bool capturing(const c10::cuda::CUDAStream& stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (stream.stream() == nullptr) return false;         // the default stream cannot be captured
+    return cudaStreamIsCapturing(stream.stream(), &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+  }
+
   // The packed image of the module's parameter `weights` (`w`: its float32 values), made when it was
-  // not seen before (another storage, or written to since); undefined for a shape the tensor-core
+  // not seen before (another storage or view of it, or written to since); undefined for a shape the tensor-core
   // kernel does not take.  The weak reference keeps the storage's address from being reused for another one
   // (a parameter that went to the CPU and came back usually lies where it lay, at the same version).  Another
-  // stream than the one that packed waits for it, and the allocator learns of its use; what is packed under
-  // stream capture belongs to the graph and is not kept.
-  Tensor packed_for(const Tensor& weights, const Tensor& w, bool half) {
+  // stream than the one that packed waits for it once, and the allocator learns of its use.  A graph that is
+  // captured with an image keeps it alive (a later one, of changed weights, does not reach the graph); what is
+  // packed under capture belongs to the graph and is not kept for others.
+  Tensor packed_for(const Tensor& weights, const Tensor& w, int cin, int cout, bool half) {
     const bool versioned = !weights.is_inference();
     c10::StorageImpl* impl = weights.storage().unsafeGetStorageImpl();
     const int64_t version = versioned ? (int64_t)weights._version() : -1;
     const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
     std::lock_guard<std::mutex> lock(mutex_);
     if (versioned && storage_._unsafe_get_target() == impl && offset_ == weights.storage_offset() &&
-        version == version_ && half == half_) {
-      if (packed_.defined() && stream != *stream_) {
-        if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) ready_.block(stream);
+        version == version_ && half == half_ && weights.sizes() == at::IntArrayRef(sizes_) &&
+        weights.strides() == at::IntArrayRef(strides_)) {
+      if (packed_.defined() && capturing(stream)) {
+        if (captured_.empty() || !captured_.back().is_same(packed_)) captured_.push_back(packed_);
+      } else if (packed_.defined() && stream != *stream_) {
+        if (std::find(waited_.begin(), waited_.end(), stream.id()) == waited_.end() && !capturing(*stream_)) {
+          at::cuda::CUDAEvent done;
+          done.record(*stream_);
+          done.block(stream);
+          waited_.push_back(stream.id());
+        }
         packed_.record_stream(stream);
       }
       return packed_;
     }
     Tensor packed;
-    if (ocnn_conv_packed_weight_bytes_general(cin_, cout_, ks_.data(), stride_, transposed_, nempty_) > 0)
-      packed = conv_pack_weights_general(w, cin_, cout_, ks_, stride_, transposed_, nempty_, half);
-    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return packed;
+    if (ocnn_conv_packed_weight_bytes_general(cin, cout, ks_.data(), stride_, transposed_, nempty_) > 0)
+      packed = conv_pack_weights_general(w, cin, cout, ks_, stride_, transposed_, nempty_, half);
+    if (capturing(stream)) return packed;
     packed_ = packed;
-    ready_ = at::cuda::CUDAEvent();        // (one per packing: the module may have gone to another GPU)
-    if (packed.defined()) ready_.record(stream);
+    waited_.clear();
     storage_ = c10::weak_intrusive_ptr<c10::StorageImpl>(
         c10::intrusive_ptr<c10::StorageImpl>::reclaim_copy(impl));
     offset_ = weights.storage_offset(); version_ = version; half_ = half; stream_ = stream;
+    sizes_ = weights.sizes().vec(); strides_ = weights.strides().vec();
     return packed;
   }
   int cin_, cout_;
@@ -1230,9 +1248,11 @@ class ConvLayer {
   Tensor packed_;
   c10::weak_intrusive_ptr<c10::StorageImpl> storage_{c10::intrusive_ptr<c10::StorageImpl>()};
   int64_t offset_ = 0, version_ = -1;
+  vector<int64_t> sizes_, strides_;
   bool half_ = false;
-  c10::optional<c10::cuda::CUDAStream> stream_;
-  at::cuda::CUDAEvent ready_;
+  c10::optional<c10::cuda::CUDAStream> stream_;       // the one that packed
+  vector<c10::StreamId> waited_;
+  vector<Tensor> captured_;
 };
 
 // 1x1x1 convolution over the concatenated channels of two tensors of the same rows: the sum of a

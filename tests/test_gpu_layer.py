@@ -251,3 +251,31 @@ def test_packed_weights_on_another_stream(ocnn, batch):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, eager)
+    # captured with weights that were packed before, on this stream or another: the graph's image stays
+    for warm_up in (torch.cuda.current_stream(), side):
+      with torch.cuda.stream(warm_up):
+        eager = fresh(x, octree)
+      torch.cuda.synchronize()
+      later = torch.cuda.CUDAGraph()
+      with torch.cuda.graph(later, stream=side):
+        z = fresh(x, octree)
+      fresh.weights.mul_(2.0)
+      double = fresh(x, octree)
+      for _ in range(4):
+        torch.randn_like(layer.weights)    # (would take the place of an image that is given back)
+      later.replay()
+      torch.cuda.synchronize()
+      assert torch.equal(z, eager) and not torch.equal(double, eager)
+      fresh.weights.mul_(0.25)
+
+
+def test_parameter_read_as_another_view(ocnn, batch):
+  """The same storage, transposed, is another set of weights."""
+  octree, v = batch
+  x = torch.randn(1, 64, int(v.nnum[4]), 1, device='cuda').to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+  layer = ocnn.OctreeConv1x1(64, 64).cuda().eval()
+  weight = layer.conv1x1.weight.detach()
+  with torch.no_grad():
+    layer(x)
+    layer.conv1x1.weight.data = weight.transpose(0, 1)
+    assert torch.equal(layer(x), copy.deepcopy(layer)(x))
