@@ -12,6 +12,7 @@ by one.
 """
 import torch
 from torch import nn as _nn
+from torch.autograd import forward_ad
 
 from . import nn
 from .octree_conv import OctreeConv, OctreeDeconv, bn_vectors, tc_status
@@ -23,14 +24,15 @@ bn_momentum, bn_eps = 0.01, 0.001       # pytorch/ocnn/modules.py:5
 FUSE_EVAL_BN = True
 
 
-def _trainable(data, weight, bn, residual):
+def _trainable(data, weight, bn, residual, *passed_by):
   """Whether a block in training mode can run as the one native autograd node: plain fp32 on the GPU,
-  a BatchNorm with parameters and running statistics, no hooks that would have to see the modules inside."""
+  a BatchNorm with parameters and running statistics, no hooks that would have to see it or the other modules
+  passed by."""
   return (torch.is_grad_enabled() and bn.training and data.is_cuda and data.dtype == torch.float32 and
           data.is_contiguous() and weight.dtype == torch.float32 and weight.is_cuda and bn.affine and
           bn.track_running_stats and bn.momentum is not None and bn.weight.dtype == torch.float32 and
           (residual is None or residual.dtype == torch.float32) and not torch.is_autocast_enabled() and
-          not hooked(bn) and _only_backward())
+          not hooked(bn, *passed_by) and _only_backward())
 
 
 def hooked(*modules):
@@ -41,17 +43,21 @@ def hooked(*modules):
   return bool(torch.nn.modules.module._has_any_global_hook())
 
 
+_functorch_level = torch._C._functorch.peek_interpreter_stack
+_tracing_state, _compiling = torch._C._get_tracing_state, torch.compiler.is_compiling
+
+
 def _only_backward():
   """Whether no more than reverse-mode autograd looks on: a functorch transform, a level of forward-mode
   derivatives, a tracer or a compiler has to see torch's own operators."""
-  return (torch._C._functorch.peek_interpreter_stack() is None and torch.autograd.forward_ad._current_level < 0 and
-          torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
+  return (_functorch_level() is None and forward_ad._current_level < 0 and _tracing_state() is None and
+          not _compiling())
 
 
 def _stock_conv1x1(conv):
   """Whether a 1x1 layer's product may be formed from the weight and bias of `conv` without calling it."""
   return (type(conv) is _nn.Conv1d and conv.kernel_size == (1,) and conv.stride == (1,) and
-          conv.padding == (0,) and conv.groups == 1 and not hooked(conv))
+          conv.padding == (0,) and conv.groups == 1)
 
 
 def _train_block(data, weight, bias, bn, residual, octree, kind, depth, cout, kernel_size, stride, nempty, relu):
@@ -92,7 +98,7 @@ class _OctreeBlock(_nn.Module):
         data_in = nn.octree_depad(data_in, octree, op.depth)
       return op._run(data_in, octree, self.bn, residual, relu)
     if foldable and type(self.bn) is _nn.BatchNorm2d and type(op) in (OctreeConv, OctreeDeconv) and \
-        _trainable(data_in, op.weights, self.bn, residual) and not hooked(op):
+        _trainable(data_in, op.weights, self.bn, residual, op):
       assert data_in.size(1) == op.channel_in
       if not op.is_conv_layer() and op.stride == 2 and not op.nempty:
         data_in = octree_depad(data_in, octree, op.depth)
@@ -172,7 +178,7 @@ class OctreeConv1x1(_nn.Module):
       # training: torch's own 1x1 convolution (as the reference), which autograd differentiates; for some
       # widths with this library's weight gradient
       if nn.own_pointwise_weight_grad(conv.weight, data_in) and not torch.is_autocast_enabled() and \
-          _stock_conv1x1(conv) and _only_backward():
+          _stock_conv1x1(conv) and not hooked(conv) and _only_backward():
         out = _Conv1x1Function.apply(data_in, conv.weight, conv.bias)
       else:
         out = conv(data_in.squeeze(-1)).unsqueeze(-1)
@@ -217,7 +223,7 @@ class _Conv1x1Block(_nn.Module):
       return self.conv1x1.run(data_in, self.bn, residual, relu)
     conv = self.conv1x1.conv1x1
     if type(self.bn) is _nn.BatchNorm2d and type(self.conv1x1) is OctreeConv1x1 and \
-        _stock_conv1x1(conv) and _trainable(data_in, conv.weight, self.bn, residual) and not hooked(self.conv1x1):
+        _stock_conv1x1(conv) and _trainable(data_in, conv.weight, self.bn, residual, conv, self.conv1x1):
       return _train_block(data_in, conv.weight, conv.bias, self.bn, residual, None, 2, 0, conv.weight.shape[0],
                           [1], 1, False, relu)
     out = self.bn(self.conv1x1(data_in))
