@@ -97,14 +97,15 @@ class _OctreeBlock(_nn.Module):
       if not op.is_conv_layer() and op.stride == 2 and not op.nempty:
         data_in = nn.octree_depad(data_in, octree, op.depth)
       return op._run(data_in, octree, self.bn, residual, relu)
-    if foldable and type(self.bn) is _nn.BatchNorm2d and type(op) in (OctreeConv, OctreeDeconv) and \
-        _trainable(data_in, op.weights, self.bn, residual, op):
+    bn = self.bn
+    if foldable and type(bn) is _nn.BatchNorm2d and type(op) in (OctreeConv, OctreeDeconv) and \
+        _trainable(data_in, op.weights, bn, residual, op):
       assert data_in.size(1) == op.channel_in
       if not op.is_conv_layer() and op.stride == 2 and not op.nempty:
         data_in = octree_depad(data_in, octree, op.depth)
-      return _train_block(data_in, op.weights, None, self.bn, residual, octree, int(not op.is_conv_layer()),
+      return _train_block(data_in, op.weights, None, bn, residual, octree, int(not op.is_conv_layer()),
                           op.depth, op.channel_out, op.kernel_size, op.stride, op.nempty, relu)
-    out = self.bn(op(data_in, octree))
+    out = bn(op(data_in, octree))
     if residual is not None:
       out = out + residual
     return torch.relu_(out) if relu else out
@@ -221,12 +222,13 @@ class _Conv1x1Block(_nn.Module):
     relu = self.with_relu if relu is None else relu
     if FUSE_EVAL_BN and not self.training:
       return self.conv1x1.run(data_in, self.bn, residual, relu)
-    conv = self.conv1x1.conv1x1
-    if type(self.bn) is _nn.BatchNorm2d and type(self.conv1x1) is OctreeConv1x1 and \
-        _stock_conv1x1(conv) and _trainable(data_in, conv.weight, self.bn, residual, conv, self.conv1x1):
-      return _train_block(data_in, conv.weight, conv.bias, self.bn, residual, None, 2, 0, conv.weight.shape[0],
-                          [1], 1, False, relu)
-    out = self.bn(self.conv1x1(data_in))
+    layer, bn = self.conv1x1, self.bn
+    conv = layer.conv1x1
+    if type(bn) is _nn.BatchNorm2d and type(layer) is OctreeConv1x1 and _stock_conv1x1(conv):
+      weight = conv.weight
+      if _trainable(data_in, weight, bn, residual, conv, layer):
+        return _train_block(data_in, weight, conv.bias, bn, residual, None, 2, 0, weight.shape[0], [1], 1, False, relu)
+    out = bn(layer(data_in))
     if residual is not None:
       out = out + residual
     return torch.relu_(out) if relu else out
