@@ -274,7 +274,8 @@ int ocnn_octree_conv_f32(const float* x_dev, const float* weights_dev, float* y_
  * [Cout, h_out], x = layer input [Cin, h_in], dw = [Cout, Cin*K].  Deconvolution at depth d: a =
  * layer input [Cin, .], x = output gradient [Cout, .], geometry = that of the convolution from the
  * output level back to the input level, dw = [Cin, Cout*K].  fp32 data in either layout; dw is
- * cleared and then accumulated with atomic additions. */
+ * cleared and then accumulated with atomic additions.  Needs no workspace; where there is one to give,
+ * ocnn_octree_conv_weight_grad_f32 below is two to five times as fast. */
 int ocnn_octree_conv_weight_grad(const float* a_dev, const float* x_dev, float* dw_dev,
                                  const ocnn_conv_geometry* geometry, int m_channels, int x_channels,
                                  const int kernel_size[3], int layout, void* stream);

@@ -20,10 +20,10 @@
 // This file is compiled with --fmad=false: the signal must round exactly like the reference's
 // separate multiplies and adds (octree.cpp:330-348).
 //
-// A depth-6 batch is 16 launches: encode + first histogram, two sort passes of 9 bits, count and
-// compact for all levels at once, averages, emit, neighbour tables.  (A count and a compact launch
-// per level, a sort over the cloud bits too and separate header / table copies made it 33, most of
-// them shorter than their launch.)
+// A depth-6 batch is 15 launches and a memset: encode + first histogram, two sort passes of 9 bits (five
+// launches), count and compact for all levels at once, averages, emit, five for the neighbour tables.  (A
+// count and a compact launch per level, a sort over the cloud bits too and separate header / table copies
+// made it 29, most of them shorter than their launch.)
 #include <cstring>
 #include <vector>
 

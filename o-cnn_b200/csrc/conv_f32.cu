@@ -1,5 +1,7 @@
 // Octree convolution in fp32 on the tensor cores (tcgen05 + TMEM): every fp32 value is carried as the sum
-// of three bf16 values and the product as six bf16 products accumulated in fp32.
+// of three bf16 values and the product as six bf16 products accumulated in fp32 (a published method: G. Henry,
+// P. T. P. Tang, A. Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision
+// Computations", 2019).
 //
 //     x = xh + xm + xl,  w = wh + wm + wl       (each part the rounded rest of the ones before: 8 bits
 //                                                of significand each, together the 24 of an fp32)
@@ -9,9 +11,10 @@
 // large partial sum; the epilogue adds them smallest first.
 //
 // Two launches: conv_f32_prepare_kernel rewrites the input rows node-major and split (per row and
-// block of 32 channels the three parts side by side; Cin rounded up to 8) and packs the weights; conv_f32_kernel is the implicit GEMM of conv_tc.cu on K-blocks
-// of 32: the stage of a K-block holds three A tiles [128 rows x 64 bytes] (the gathered rows' high,
-// middle and low parts) and one B image of the weights' parts stacked, so that
+// block of 32 channels the three parts side by side; Cin rounded up to 8) and packs the weights;
+// conv_f32_kernel is the implicit GEMM of conv_tc.cu on K-blocks of 32: the stage of a K-block
+// holds three A tiles [128 rows x 64 bytes] (the gathered rows' high, middle and low parts) and one B image of the
+// weights' parts stacked, so that
 //     Ah x [Bh | Bm | Bl] -> [D0 | D1 | D2],   Am x [Bh | Bm] -> [D1 | D2],   Al x Bh -> D2
 // are three instructions per 16 K values (four where 3 N columns exceed an instruction's 256).
 //

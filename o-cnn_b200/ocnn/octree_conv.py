@@ -5,11 +5,13 @@ channel_in * K] for the convolution, [channel_in, channel_out * K] for the decon
 index c * K + tap — so a reference state_dict loads unchanged.  Every variant (stride 1 or 2, all
 nodes or non-empty nodes only) is one implicit-GEMM CUDA kernel; no column buffer is built.
 
-Data in bfloat16 / float16 with torch's channels_last memory format runs on the tensor-core
-kernel (weights are packed when they change, `nn.ConvLayer`); float32 data, or the
-reference's contiguous [1,C,H,1] layout, runs on the CUDA-core kernel.  float32 data that takes
-part in autograd (training) goes through `OctreeConvFunction` / `OctreeDeconvFunction`, whose
-backward is the transposed operator for the data and a node-reduction kernel for the weights.
+Data in bfloat16 / float16 with torch's channels_last memory format runs on the 16-bit
+tensor-core kernel (weights are packed when they change, `nn.ConvLayer`; 16-bit data in another
+layout on the CUDA cores).  float32 data, in either layout, runs on the tensor cores as three bf16
+parts per value, layers of few channels on the CUDA cores.  float32 data that takes part in autograd
+(training) goes through `OctreeConvFunction` / `OctreeDeconvFunction`: layers of up to 4 GFLOP on the
+CUDA cores' chain of multiply-adds, forward and data gradient (the transposed operator), and the
+weight gradient as a reduction over the nodes on the tensor cores.
 """
 import torch
 from torch import nn as _nn
