@@ -36,6 +36,7 @@ struct F32Args {
   const int* ichild;
   int h_in, h_out, cp, cout, npad, T, stride, identity, up;
   int tiles, slices, splits, nkb, kb_per_split, stages, tmem_cols, node_major;
+  int vec4;                // node-major rows of whole float4 on a 16-byte boundary
   long long y_elems;
   ChannelAffine aff;
   const float* residual;
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(kF32Threads, NG <= 4 ? 2 : 1) conv_f32_kernel(
       const int co_base = item_slice(item) * N;
       float* out = a.partial ? a.partial + item_split(item) * a.y_elems : a.y;
       const bool finish = a.partial == nullptr;
-      if (a.node_major && (a.cout & 3) == 0) {
+      if (a.vec4) {
         const long long at0 = (long long)h * a.cout + co_base;
 #pragma unroll
         for (int j = 0; j < N; j += 4) {
@@ -562,6 +563,7 @@ extern "C" int ocnn_octree_conv_f32(const float* x, const float* w, float* y, co
   a.tiles = s.tiles; a.slices = s.slices; a.splits = s.splits;
   a.nkb = s.nkb; a.kb_per_split = s.kb_per_split; a.stages = s.stages;
   a.tmem_cols = s.tmem_cols; a.node_major = layout == OCNN_NODE_MAJOR;
+  a.vec4 = a.node_major && cout % 4 == 0 && (uintptr_t)y % 16 == 0;
   a.y_elems = (long long)g->h_out * cout;
   a.aff = channel_affine_of(ep);
   a.residual = ep ? static_cast<const float*>(ep->residual_dev) : nullptr;

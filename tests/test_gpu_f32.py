@@ -240,3 +240,27 @@ def test_which_kernel_a_training_layer_takes(ocnn, octree, big_octree, big):
                                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
       want.append(out)
   assert torch.equal(y.detach(), want[0]) and torch.equal(gx, want[1])
+
+
+@pytest.mark.parametrize('shift', [0, 1, 2])
+@pytest.mark.parametrize('cout', [32, 96])
+def test_output_on_any_float_boundary(ocnn, octree, shift, cout):
+  """ocnn_octree_conv_f32 writes node-major rows of whole float4 also where they are not aligned as such."""
+  tree, v = octree
+  d, cin, h = 5, 40, int(v.nnum[5])
+  lib, ks = ctypes.CDLL(ocnn.LIBRARY), (ctypes.c_int * 3)(3, 3, 3)
+  lib.ocnn_octree_conv_f32_workspace_bytes.restype = ctypes.c_size_t
+  neigh = ocnn.octree_property(tree, 'neigh', d).contiguous()
+  x, w = torch.randn(1, cin, h, 1, device='cuda'), torch.randn(cout, cin * 27, device='cuda') * 0.1
+  rows = x.contiguous(memory_format=torch.channels_last)
+  geo = _Geometry(0, 1, 0, h, h, neigh.data_ptr(), None, None)
+  bytes_ = lib.ocnn_octree_conv_f32_workspace_bytes(ctypes.byref(geo), cin, cout, ks)
+  ws, status = torch.empty(bytes_, dtype=torch.uint8, device='cuda'), torch.zeros(1, dtype=torch.int32, device='cuda')
+  out = torch.full((h * cout + 8,), 5.0, device='cuda')
+  ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+  assert lib.ocnn_octree_conv_f32(ptr(rows), ptr(w), ptr(out[shift:]), ctypes.byref(geo), cin, cout, ks, 1, None, ptr(ws),
+                                  ctypes.c_size_t(bytes_), ptr(status),
+                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+  want = ocnn.octree_conv(rows, w, tree, d, cout, [3, 3, 3], 1)
+  assert torch.equal(out[shift:shift + h * cout].view(h, cout).t(), want.view(cout, h))
+  assert bool((out[:shift] == 5.0).all()) and bool((out[shift + h * cout:] == 5.0).all()) and int(status) == 0
