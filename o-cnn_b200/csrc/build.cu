@@ -518,6 +518,7 @@ struct UniqueArgs {
   const KeyT* keys;
   long long n;
   int depth, full, levels;
+  int wide;                 // 32-bit keys on a 16-byte boundary (the workspace may lie on 8)
   int* blockcnt;            // [levels][blocks]
   int* counts;              // by depth
   int* host_counts;         // the same in mapped host memory
@@ -546,12 +547,12 @@ __device__ __forceinline__ void scan_range(long long n, long long* beg, long lon
   *end = e < n ? e : n;
 }
 
-// Four consecutive keys per thread (16-byte reads of 32-bit keys) and the key before them.
+// Four consecutive keys per thread (one 16-byte read where `wide`) and the key before them.
 template <typename KeyT>
 __device__ __forceinline__ void load_items(const UniqueArgs<KeyT>& a, long long i0, long long end,
                                            KeyT (&key)[kScanItems], int (&lvl)[kScanItems]) {
   KeyT prev = (i0 > 0 && i0 < end) ? a.keys[i0 - 1] : 0;
-  if (sizeof(KeyT) == 4 && i0 + kScanItems <= end) {
+  if (sizeof(KeyT) == 4 && a.wide && i0 + kScanItems <= end) {
     const uint4 q = *reinterpret_cast<const uint4*>(a.keys + i0);
     key[0] = (KeyT)q.x; key[1] = (KeyT)q.y; key[2] = (KeyT)q.z; key[3] = (KeyT)q.w;
   } else {
@@ -1067,6 +1068,7 @@ int sort_and_unique(const EncodeArgs& ea, const Layout& L, int chunks, uint8_t* 
   UniqueArgs<KeyT> u;
   memset(&u, 0, sizeof(u));
   u.keys = reinterpret_cast<const KeyT*>(ws + L.off_keys[L.passes & 1]);
+  u.wide = sizeof(KeyT) == 4 && (uintptr_t)u.keys % 16 == 0;
   u.n = L.n; u.depth = L.depth; u.full = L.full; u.levels = L.depth - L.full + 1;
   u.blockcnt = reinterpret_cast<int*>(ws + L.off_blockcnt);
   u.counts = reinterpret_cast<int*>(ws + L.off_counts);

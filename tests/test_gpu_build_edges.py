@@ -1,6 +1,8 @@
 """Where the batch builder changes its path: clouds at the sizes of a sort chunk, more clouds than ride
 in the launch parameters, every digit width and key width, signals averaged into compact arrays (up
 to six channels) or per node, bit-identical to the CPU oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -8,6 +10,7 @@ import torch
 import gpu_util as gu
 from oracle import oracle as oc
 from ocnn_harness import synth
+from test_capi_host import Meta
 
 pytestmark = pytest.mark.gpu
 FLAGS = (False, False, False, False, 4, 0.1, 2.0, False, False, False)
@@ -73,3 +76,41 @@ def test_batches_sorted_over_their_cloud_bits(ocnn, depth, key_bits, sizes):
 @pytest.mark.parametrize('points', [6999, 7000])
 def test_average_size_at_which_clouds_are_sorted_one_by_one(ocnn, points):
   check(ocnn, clouds_of([points - 500, points + 500] * 33, 77, channels=2), 6, 2, 64)
+
+
+class _Params(ctypes.Structure):
+  _fields_ = [(n, ctypes.c_int32) for n in ('depth', 'full_depth', 'key_bits', 'merged', 'node_dis', 'split_label', 'save_pts',
+                                            'adp_depth')] + \
+      [('th_normal', ctypes.c_float), ('th_distance', ctypes.c_float), ('bbmin', ctypes.c_float * 3), ('bbmax', ctypes.c_float * 3)]
+
+
+class _Batch(ctypes.Structure):
+  _fields_ = [('batch', ctypes.c_int32), ('offsets', ctypes.c_void_p), ('xyz', ctypes.c_void_p), ('normal', ctypes.c_void_p),
+              ('feature', ctypes.c_void_p), ('channels', ctypes.c_int32), ('label', ctypes.c_void_p)]
+
+
+@pytest.mark.parametrize('shift', [0, 8, 16])
+@pytest.mark.parametrize('depth', [5, 9, 11])              # (two and three sort passes, 32- and 64-bit keys)
+def test_workspace_on_an_8_byte_boundary(ocnn, depth, shift):
+  ocnn.set_key_bits(64)
+  p, q = synth.primitive_union(7001, 5)
+  want = oc.points2octree(oc.points_new(p, q), depth, 2, key_bits=64)
+  xyz, nrm = torch.from_numpy(p).cuda(), torch.from_numpy(q).cuda()
+  lib, meta = ctypes.CDLL(ocnn.LIBRARY), Meta()
+  lib.ocnn_octree_build_workspace_bytes.restype = ctypes.c_size_t
+  lib.ocnn_last_error.restype = ctypes.c_char_p
+  size = lib.ocnn_octree_build_workspace_bytes(ctypes.c_int64(len(p)), 1, depth, 2)
+  ws = torch.empty(size + 64, dtype=torch.uint8, device='cuda')
+  offsets = (ctypes.c_int32 * 2)(0, len(p))
+  xs, ns = (ctypes.c_void_p * 1)(xyz.data_ptr()), (ctypes.c_void_p * 1)(nrm.data_ptr())
+  at = lambda a: ctypes.cast(a, ctypes.c_void_p)
+  batch = _Batch(1, at(offsets), at(xs), at(ns), None, 0, None)
+  params = _Params(depth, 2, 64, 0, 0, 0, 0, 4, 0.1, 2.0, (ctypes.c_float * 3)(-1, -1, -1), (ctypes.c_float * 3)(1, 1, 1))
+  work, stream = ctypes.c_void_p(ws.data_ptr() + shift), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+  assert lib.ocnn_octree_build_plan(ctypes.byref(batch), ctypes.byref(params), work, ctypes.c_size_t(size), ctypes.byref(meta),
+                                    stream) == 0, lib.ocnn_last_error()
+  out = torch.empty(meta.ptr_dis[6], dtype=torch.uint8, device='cuda')
+  assert lib.ocnn_octree_build_emit(ctypes.byref(batch), ctypes.byref(params), ctypes.byref(meta), work, ctypes.c_size_t(size),
+                                    ctypes.c_void_p(out.data_ptr()), ctypes.c_size_t(out.numel()), None, stream) == 0
+  torch.cuda.synchronize()
+  assert np.array_equal(out.cpu().numpy(), want)
