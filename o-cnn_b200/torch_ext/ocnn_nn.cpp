@@ -92,6 +92,12 @@ void drop_expired(std::vector<std::shared_ptr<OctreeTables>>* released) {
   }
 }
 
+// `t` itself, or a copy where it is CUDA memory that does not start on a multiple of `bytes` (a byte-wise view into
+// another tensor): the kernels read whole words.
+Tensor on_boundary(const Tensor& t, size_t bytes) {
+  return t.is_cuda() && reinterpret_cast<uintptr_t>(t.data_ptr()) % bytes != 0 ? t.clone() : t;
+}
+
 OctreeRef get_octree(const Tensor& octree) {
   TORCH_CHECK(octree.scalar_type() == torch::kUInt8 && octree.dim() == 1 && octree.is_contiguous(),
               "the octree must be a contiguous 1-D uint8 tensor");
@@ -99,6 +105,8 @@ OctreeRef get_octree(const Tensor& octree) {
   OctreeRef ref;
   ref.base = octree.data_ptr<uint8_t>();
   ref.cuda = octree.is_cuda();
+  TORCH_CHECK(!ref.cuda || reinterpret_cast<uintptr_t>(ref.base) % 4 == 0,
+              "the octree must start on a 4-byte boundary (clone() a byte-wise view)");
   if (!ref.cuda) {
     memset(ref.raw, 0, sizeof(ref.raw));
     memcpy(ref.raw, ref.base, 716);
@@ -1552,6 +1560,8 @@ const void* level_keys(const OctreeRef& o, const Tensor& octree, int depth, bool
   const void* keys = o.base + off;
   *n_key = o.meta.nnum[depth];
   const int kb = o.meta.key_bits / 8;
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(keys) % kb == 0, what, ": the octree's keys must lie on a ", kb,
+              "-byte boundary (clone() a view into another tensor)");
   auto opts = octree.options().dtype(torch::kUInt8);
   if (nempty) {
     const int nne = o.meta.nnum_nempty[depth];
@@ -1801,7 +1811,7 @@ Tensor normalize_points(Tensor data_in, float radius, vector<float> center) {
 vector<Tensor> clip_points(Tensor data_in, vector<float> bbmin, vector<float> bbmax) {
   TORCH_CHECK(bbmin.size() == 3 && bbmax.size() == 3, "clip_points: bbmin / bbmax must hold 3 values");
   PointsHeader h = read_points_header(data_in);
-  Tensor src = data_in.to(torch::kCUDA).contiguous();
+  Tensor src = on_boundary(data_in.to(torch::kCUDA).contiguous(), 4);
   c10::cuda::CUDAGuard guard(src.device());
   Tensor out = src.clone();      // header and (for an all-inside cloud) every block already in place
   const float* sp[4]; float* dp[4]; int ch[4];
@@ -1865,7 +1875,7 @@ vector<float> bounding_sphere(Tensor data_in, string method) {
   PointsHeader h = read_points_header(data_in);
   float box[6];
   if (data_in.is_cuda()) {
-    Tensor src = data_in.contiguous();
+    Tensor src = on_boundary(data_in.contiguous(), 4);
     c10::cuda::CUDAGuard guard(src.device());
     const size_t ws_bytes = ocnn_points_bbox_workspace_bytes();
     Tensor ws = torch::empty({(int64_t)ws_bytes}, src.options());
@@ -2163,7 +2173,7 @@ std::tuple<Tensor, Tensor, Tensor> prepare_cloud(
   PointsHeader h = read_points_header(points);
   const BuildFlags flags = make_flags(depth, full_depth, node_dis, node_feature, split_label, adaptive, adp_depth,
                                       th_normal, th_distance, extrapolate, save_pts, key2xyz);
-  Tensor host_pts = points.contiguous();
+  Tensor host_pts = on_boundary(points.contiguous(), 4);
   if (radius < 0) {
     vector<float> sphere = bounding_sphere(host_pts, "box");
     radius = sphere[0];
@@ -2225,11 +2235,11 @@ Tensor octree_batch(vector<Tensor> tensors_in) {
   vector<const void*> ptrs(B);
   uint8_t first[OCNN_HEADER_BYTES];
   for (int b = 0; b < B; ++b) {
-    OctreeRef o = get_octree(tensors_in[b].contiguous());
+    const Tensor in = on_boundary(tensors_in[b].contiguous(), 8);
+    OctreeRef o = get_octree(in);
     metas[b] = o.meta;
     if (b == 0) memcpy(first, o.raw, sizeof(first));
-    dev[b] = tensors_in[b].is_cuda() ? tensors_in[b].contiguous()
-                                     : tensors_in[b].contiguous().to(torch::kCUDA, /*non_blocking=*/false);
+    dev[b] = in.is_cuda() ? in : in.to(torch::kCUDA, /*non_blocking=*/false);
     ptrs[b] = dev[b].data_ptr();
   }
   c10::cuda::CUDAGuard guard(dev[0].device());
