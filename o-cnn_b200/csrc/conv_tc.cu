@@ -1465,7 +1465,7 @@ int tc_shape(int cin, int cout, const int ks[3], const LayerKind& kind, TcShape*
   // nodes: 66 CTAs of 108 K-blocks, 58 us).
   s->splits = 1;
   const long long whole = rows < 0 ? 0 : (rows + kTileM - 1) / kTileM * s->slices;
-  if (can_split && rows >= 0 && !s->group && !s->expand_out && s->nkb >= 32 && 2 * whole <= sms && split_mode() != 0) {
+  if (can_split && rows > 0 && !s->group && !s->expand_out && s->nkb >= 32 && 2 * whole <= sms && split_mode() != 0) {
     s->tile_rows = kTileM;
     const long long want = sms / whole, most = s->nkb / 8;
     s->splits = (int)(want < most ? want : most);

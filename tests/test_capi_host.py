@@ -195,3 +195,20 @@ def test_build_workspace_grows_with_the_points(lib, depth, batch):
   for tiles in (592, 1184, 1776):
     around = [size(tiles * 2048 + k) for k in (-5000, -1, 0, 1, 2, 100, 2047, 2048, 2049, 5000, 20000)]
     assert around == sorted(around)
+
+
+class Geometry(ctypes.Structure):
+  _fields_ = [(n, ctypes.c_int32) for n in ('transposed', 'stride', 'nempty', 'h_in', 'h_out')] + \
+      [(n, ctypes.c_void_p) for n in ('neigh', 'child', 'ichild')]
+
+
+@pytest.mark.parametrize('cin,cout,ks', [(128, 128, 3), (64, 512, 3), (4096, 64, 1), (8, 8, 3), (16, 40, 2)])
+@pytest.mark.parametrize('transposed,stride,nempty', [(0, 1, 0), (0, 1, 1), (1, 1, 1), (0, 2, 0), (1, 2, 1)])
+def test_empty_levels_need_no_workspace(lib, cin, cout, ks, transposed, stride, nempty):
+  """A level without rows: nothing to split, nothing to divide by."""
+  geo, kernel = Geometry(transposed, stride, nempty, 0, 0, None, None, None), (ctypes.c_int * 3)(ks, ks, ks)
+  for name in ('ocnn_octree_conv_tc_workspace_bytes', 'ocnn_octree_conv_f32_workspace_bytes',
+               'ocnn_octree_conv_weight_grad_f32_workspace_bytes'):
+    fn = getattr(lib, name)
+    fn.restype = ctypes.c_size_t
+    assert fn(ctypes.byref(geo), cin, cout, kernel) == 0, name

@@ -238,3 +238,14 @@ def test_fp16_pointwise_and_feature(ocnn, batch, shape):
   assert feat.dtype == torch.float16
   f = v.prop('feature', 6)
   assert np.array_equal(gu.to_np(feat)[:f.shape[0]], gu.half_round(f))
+
+
+@pytest.mark.parametrize('cin,cout', [(8, 8), (128, 128)])          # (the wide one has K to split)
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+def test_level_without_rows(cin, cout, dtype):
+  import ocnn
+  x = torch.empty(1, cin, 0, 1, device='cuda', dtype=dtype).contiguous(memory_format=torch.channels_last)
+  wide = torch.empty(1, 4096, 0, 1, device='cuda', dtype=dtype).contiguous(memory_format=torch.channels_last)
+  with torch.no_grad():
+    assert ocnn.OctreeConv1x1(cin, cout).cuda().eval()(x).shape == (1, cout, 0, 1)
+    assert ocnn.OctreeConv1x1(4096, cout).cuda().eval()(wide).shape == (1, cout, 0, 1)
