@@ -486,9 +486,10 @@ bool f32_shape(const ocnn_conv_geometry* g, int cin, int cout, const TapList& tl
   const long long items = ctas * s->splits;
   const bool share = pair && items > sms;
   const size_t budget = (share ? 112 : 220) * 1024;
+  // (scale and bias of all slices take 8 bytes a channel: beyond about 13 k output channels no ring is left)
+  if (fixed + 2 * stage > budget) return false;
   int st = (int)((budget - fixed) / stage);
   if (st > 6) st = 6;
-  if (st < 2) st = 2;
   s->stages = st;
   s->smem = fixed + st * stage;
   // the same number of items (within one) for every CTA

@@ -264,3 +264,13 @@ def test_output_on_any_float_boundary(ocnn, octree, shift, cout):
   want = ocnn.octree_conv(rows, w, tree, d, cout, [3, 3, 3], 1)
   assert torch.equal(out[shift:shift + h * cout].view(h, cout).t(), want.view(cout, h))
   assert bool((out[:shift] == 5.0).all()) and bool((out[shift + h * cout:] == 5.0).all()) and int(status) == 0
+
+
+@pytest.mark.parametrize('cout', [12800, 16000, 30000])
+def test_very_many_output_channels(ocnn, octree, cout):
+  """Where the epilogue's vectors leave no room for the ring the layer runs on the CUDA cores, as it did."""
+  tree, v = octree
+  h = int(v.nnum[2])
+  x, w = torch.randn(1, 8, h, 1, device='cuda'), torch.randn(cout, 8 * 27, device='cuda') * 0.1
+  want = (w.double() @ columns(ocnn, x, tree, 2, False)).view(1, cout, h, 1)
+  assert off(ocnn.octree_conv(x, w, tree, 2, cout, [3, 3, 3], 1), want) < 2e-6
