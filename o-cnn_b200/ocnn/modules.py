@@ -30,7 +30,7 @@ def _trainable(data, weight, bn, residual, *passed_by):
   passed by."""
   return (torch.is_grad_enabled() and bn.training and data.is_cuda and data.dtype == torch.float32 and
           data.is_contiguous() and weight.dtype == torch.float32 and weight.is_cuda and bn.affine and
-          bn.track_running_stats and bn.momentum is not None and bn.weight.dtype == torch.float32 and
+          bn.track_running_stats and bn.momentum is not None and bn._parameters['weight'].dtype == torch.float32 and
           (residual is None or residual.dtype == torch.float32) and not torch.is_autocast_enabled() and
           not hooked(bn, *passed_by) and _only_backward())
 
@@ -61,10 +61,12 @@ def _stock_conv1x1(conv):
 
 
 def _train_block(data, weight, bias, bn, residual, octree, kind, depth, cout, kernel_size, stride, nempty, relu):
-  if bn.num_batches_tracked is not None:
-    bn.num_batches_tracked.add_(1)
-  return nn.train_block(data, weight, bias, bn.weight, bn.bias, residual, bn.running_mean, bn.running_var,
-                        bn.momentum, bn.eps, octree, kind, depth, cout, kernel_size, stride, nempty, relu)
+  own, stats = bn._parameters, bn._buffers       # (Module's own look-up costs 0.4 us a name)
+  if stats['num_batches_tracked'] is not None:
+    stats['num_batches_tracked'].add_(1)
+  return nn.train_block(data, weight, bias, own['weight'], own['bias'], residual, stats['running_mean'],
+                        stats['running_var'], bn.momentum, bn.eps, octree, kind, depth, cout, kernel_size, stride,
+                        nempty, relu)
 
 
 def _folded(bn):
