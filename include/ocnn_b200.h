@@ -370,6 +370,29 @@ int ocnn_octree_conv_tc_general_ws(const void* x_dev, const void* packed_dev, vo
                                    int32_t* status_dev, void* workspace, size_t workspace_bytes, void* stream);
 
 
+/* Tap plan: the non-empty nodes of levels in the order in which tiles of 128 share few of the 27 taps, with the
+ * tables of their neighbours, for the 3x3x3 stride-1 convolutions on those nodes (OctreeConv(nempty=True),
+ * pytorch/ocnn/octree_conv.py): worth its four launches where several layers work on the same levels, as in a
+ * U-Net's forward.  neigh_dev / child_dev: the level's Neigh and Child blocks; nodes / rows: its nodes and
+ * non-empty nodes (neither 0); plan_dev: ocnn_tap_plan_bytes(rows) on a 32-byte boundary.  Up to 8 levels a call. */
+typedef struct ocnn_tap_level {
+  const int32_t* neigh_dev;
+  const int32_t* child_dev;
+  int32_t nodes, rows;
+  void* plan_dev;
+} ocnn_tap_level;
+size_t ocnn_tap_plan_bytes(int rows);
+size_t ocnn_tap_plan_workspace_bytes(const ocnn_tap_level* levels, int count);
+int ocnn_tap_plan(const ocnn_tap_level* levels, int count, void* workspace_dev, size_t workspace_bytes,
+                  void* stream);
+/* The convolution on a plan: x, y [rows, channels] 16-bit node-major; packed weights as for
+ * ocnn_octree_conv_tc_general with nempty, kernel 3x3x3, stride 1; cin a multiple of 16
+ * (OCNN_ERR_UNSUPPORTED otherwise). */
+size_t ocnn_octree_conv_tc_taps_workspace_bytes(int rows, int cin, int cout);
+int ocnn_octree_conv_tc_taps(const void* x_dev, const void* packed_dev, void* y_dev, const void* plan_dev,
+                             int rows, int cin, int cout, int dtype, const ocnn_conv_epilogue* epilogue,
+                             int32_t* status_dev, void* workspace_dev, size_t workspace_bytes, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Octree editing for the generative networks.  Replace octree_new / octree_grow / octree_update
  * (pytorch/cpp/octree_grow.cpp:108-148, 8-104, 150-177).  Headers are passed and returned as the

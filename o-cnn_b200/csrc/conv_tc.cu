@@ -33,6 +33,7 @@
 // returns, the gather threads wait for their own cp.async copies, the MMA thread commits what it
 // has issued and waits (bounded) for that commit, and the weight thread gives the bulk copies it
 // has in flight a bounded time to land — the launch never hangs the GPU.
+#include "conv_taps.cuh"
 #include "tc.cuh"
 
 namespace ocnn {
@@ -1244,19 +1245,25 @@ __device__ __forceinline__ float weight_at(const float* __restrict__ w, const We
                       : w[((long long)n * v.cin + ci) * v.T + t];
 }
 
-__device__ __forceinline__ void store_packed(uint16_t* __restrict__ packed, long long off, float v,
+// Returns whether the stored value is infinite or not a number.
+__device__ __forceinline__ bool store_packed(uint16_t* __restrict__ packed, long long off, float v,
                                              bool half) {
+  uint16_t bits;
   if (half) {
     const __half h = __float2half(v);
-    packed[off] = *reinterpret_cast<const uint16_t*>(&h);
+    bits = *reinterpret_cast<const uint16_t*>(&h);
   } else {
     const __nv_bfloat16 b = __float2bfloat16(v);
-    packed[off] = *reinterpret_cast<const uint16_t*>(&b);
+    bits = *reinterpret_cast<const uint16_t*>(&b);
   }
+  packed[off] = bits;
+  const uint16_t exponent = half ? 0x7c00 : 0x7f80;
+  return (bits & exponent) == exponent;
 }
 
 __global__ void pack_weights_kernel(const float* __restrict__ w, uint16_t* __restrict__ packed,
-                                    WeightView v, int ncols, int kdim, int npad, int nkb, bool half) {
+                                    WeightView v, int ncols, int kdim, int npad, int nkb, bool half,
+                                    int* __restrict__ nonfinite) {
   // ncols = output columns of this slice, kdim = K extent (taps * Cin, or 8*Cin when folded)
   const long long total = (long long)nkb * npad * kBlockK;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -1280,7 +1287,7 @@ __global__ void pack_weights_kernel(const float* __restrict__ w, uint16_t* __res
     }
     const long long off = (long long)kb * npad * 64 + (n >> 3) * 512 + (n & 7) * 64 +
                           (((kk >> 3) ^ (n & 7)) << 3) + (kk & 7);
-    store_packed(packed, off, val, half);
+    if (store_packed(packed, off, val, half) && nonfinite != nullptr) *nonfinite = 1;
   }
 }
 
@@ -1537,10 +1544,18 @@ PersistShape persist_shape(const TcShape& s, int R) {
   return p;
 }
 
+// Layers that a tap plan serves: 3x3x3 with stride 1 on non-empty nodes, whole 16-channel steps.
+bool takes_taps(const TcShape& s, const LayerKind& kind, int cin) {
+  return kind.nempty && !kind.transposed && kind.stride == 1 && s.T == 27 && cin % 16 == 0 && s.nkb <= kTapMaxBlocks;
+}
+
+size_t image_bytes(const TcShape& s) { return (size_t)s.slices * s.nkb * s.npad * 128; }
+constexpr size_t kFlagBytes = 128;       // behind the image of such a layer: whether a weight is not finite
+
 size_t packed_bytes_impl(int cin, int cout, const int kernel_size[3], const LayerKind& kind) {
   TcShape s;
   if (kernel_size == nullptr || tc_shape(cin, cout, kernel_size, kind, &s, -1) != OCNN_OK) return 0;
-  return (size_t)s.slices * s.nkb * s.npad * 128;
+  return image_bytes(s) + (takes_taps(s, kind, cin) ? kFlagBytes : 0);
 }
 
 int pack_weights_impl(const float* w, void* packed, int cin, int cout, const int kernel_size[3],
@@ -1561,6 +1576,11 @@ int pack_weights_impl(const float* w, void* packed, int cin, int cout, const int
     pack_weights_group_kernel<<<grid_for(total, 256), 256, 0, st>>>(
         w, static_cast<uint16_t*>(packed), cin, cout, tl.count, ta, s.npad, s.nkb, half);
   } else {
+    int* nonfinite = nullptr;
+    if (takes_taps(s, kind, cin)) {
+      nonfinite = reinterpret_cast<int*>(static_cast<uint8_t*>(packed) + image_bytes(s));
+      OCNN_CUDA_OK(cudaMemsetAsync(nonfinite, 0, kFlagBytes, st));
+    }
     // one packed image per slice of (at most) 256 output columns
     WeightView v;
     v.cin = cin; v.cout = cout; v.T = tl.count; v.transposed = kind.transposed ? 1 : 0;
@@ -1570,7 +1590,7 @@ int pack_weights_impl(const float* w, void* packed, int cin, int cout, const int
     for (int sl = 0; sl < s.slices; ++sl) {
       v.co_base = sl * cslice;
       pack_weights_kernel<<<grid_for(total, 256), 256, 0, st>>>(
-          w, static_cast<uint16_t*>(packed) + (size_t)sl * total, v, cslice, kdim, s.npad, s.nkb, half);
+          w, static_cast<uint16_t*>(packed) + (size_t)sl * total, v, cslice, kdim, s.npad, s.nkb, half, nonfinite);
       if (sl > 0) note_launches(1);
     }
   }
@@ -1819,10 +1839,124 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
   return OCNN_OK;
 }
 
+// Launch shape on a tap plan.  Two or three CTAs share an SM where two stages of each fit.  A level of few tiles
+// and a long K splits K over CTAs (a tile of 256 -> 256 still walks 76 of 108 K-blocks at 4.2 k nodes), at least
+// eight blocks of the full list a part.
+struct TapShape {
+  int stages, splits;
+  size_t smem;
+};
+TapShape tap_shape(const TcShape& s, long long rows) {
+  TapShape t;
+  const long long tiles = (rows + kTapTile - 1) / kTapTile * s.slices;
+  const int sms = sm_count();
+  t.splits = 1;
+  if (2 * tiles <= sms && s.nkb >= 32 && split_mode() != 0) {
+    const long long want = sms / tiles, most = s.nkb / 8;
+    t.splits = (int)(want < most ? want : most);
+  }
+  const size_t stage = (size_t)kTapTile * 128 + (size_t)s.npad * 128;
+  const size_t fixed = 1024 + 27 * kTapTile * 4 + (size_t)s.npad * 8 + 256 + 2 * kTapMaxBlocks;
+  int st = (int)((75 * 1024 - fixed) / stage);
+  if (st < 2 || 3 * s.tmem_cols > 512) st = (int)((113 * 1024 - fixed) / stage);
+  if (st < 2 || tiles * t.splits <= sms) st = (int)((200 * 1024 - fixed) / stage);
+  t.stages = st > 7 ? 7 : st;            // (three at 256 columns)
+  t.smem = fixed + (size_t)t.stages * stage;
+  return t;
+}
+
+size_t taps_workspace(const TcShape& s, const TapShape& t, long long rows) {
+  return t.splits > 1 ? (size_t)t.splits * rows * s.cout_eff * 4 : 0;
+}
+
+int conv_taps_impl(const void* x, const void* packed, void* y, const void* plan, int rows, int cin, int cout,
+                   int dtype, const ocnn_conv_epilogue* ep, int32_t* status, void* workspace,
+                   size_t workspace_bytes, cudaStream_t st) {
+  const char* who = "ocnn_octree_conv_tc_taps";
+  OCNN_REQUIRE(dtype == OCNN_BF16 || dtype == OCNN_F16, "%s: bf16 or fp16 data only (dtype %d)", who, dtype);
+  const int ks[3] = {3, 3, 3};
+  const LayerKind kind{1, false, true};
+  TcShape s;
+  if (int rc = tc_shape(cin, cout, ks, kind, &s, -1)) return rc;
+  if (!takes_taps(s, kind, cin))
+    return fail(OCNN_ERR_UNSUPPORTED, "%s: %d input channels (a multiple of 16, at most %d)", who, cin,
+                kTapMaxBlocks * 64 / 27);
+  if (rows == 0) return OCNN_OK;
+  OCNN_REQUIRE(x && packed && y && plan && status && rows > 0, "%s: null pointer", who);
+  OCNN_REQUIRE((uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)packed % 16 == 0 &&
+                   (uintptr_t)plan % 32 == 0,
+               "%s: data and weight pointers must be 16-byte aligned, the plan 32-byte", who);
+  const void* residual = ep ? ep->residual_dev : nullptr;
+  OCNN_REQUIRE((uintptr_t)residual % 16 == 0, "%s: residual must be 16-byte aligned", who);
+  OCNN_REQUIRE((long long)rows * cin * 2 < (1LL << 32), "%s: input tensor of %lld bytes exceeds the 4 GiB this kernel addresses",
+               who, (long long)rows * cin * 2);
+  TapShape t = tap_shape(s, rows);
+  OCNN_REQUIRE(taps_workspace(s, t, rows) <= workspace_bytes && (uintptr_t)workspace % 32 == 0,
+               "%s: the workspace needs %zu bytes on a 32-byte boundary", who, taps_workspace(s, t, rows));
+  TapConvArgs a = {};
+  a.x = static_cast<const uint8_t*>(x);
+  a.wpacked = static_cast<const uint8_t*>(packed);
+  a.nonfinite = reinterpret_cast<const int*>(a.wpacked + image_bytes(s));
+  a.y = static_cast<uint8_t*>(y);
+  a.plan = tap_plan_view(plan, rows);
+  a.rows = rows; a.cin = cin; a.npad = s.npad; a.nkb = s.nkb; a.stages = t.stages; a.tmem_cols = s.tmem_cols;
+  a.tap_magic = (uint32_t)(((1ull << 32) + cin / 8 - 1) / (cin / 8));
+  a.row_elems = s.slices > 1 ? 256 : s.cout_eff;
+  a.y_stride = s.cout_eff;
+  a.wide = (a.row_elems % 16 == 0 && (uintptr_t)y % 32 == 0 && (uintptr_t)residual % 32 == 0) ? 1 : 0;
+  a.aff = channel_affine_of(ep);
+  a.residual = t.splits > 1 ? nullptr : static_cast<const uint8_t*>(residual);
+  a.relu = epilogue_relu(ep);
+  a.partial = t.splits > 1 ? static_cast<float*>(workspace) : nullptr;
+  a.status = status;
+  static PerDeviceOnce attr_once;
+  int device = 0;
+  OCNN_CUDA_OK(cudaGetDevice(&device));
+  const bool half = dtype == OCNN_F16;
+  typedef void (*Fn)(const TapConvArgs);
+  static const Fn table[2] = {conv_taps_kernel<false>, conv_taps_kernel<true>};
+  {
+    std::lock_guard<std::mutex> lock(attr_once.mutex);
+    const bool known = device >= 0 && device < 64;
+    if (!known || !attr_once.done[device]) {
+      for (Fn f : table)
+        OCNN_CUDA_OK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+      if (known) attr_once.done[device] = true;
+    }
+  }
+  OCNN_CUDA_OK(launch_chained(table[half ? 1 : 0], dim3(a.plan.tiles, s.slices, t.splits), dim3(kTapThreads), t.smem,
+                              st, a));
+  OCNN_LAUNCH_OK("conv_taps_kernel");
+  if (t.splits > 1) {
+    const long long chunks = (long long)rows * a.y_stride / 8;
+    OCNN_CUDA_OK(launch_chained(half ? conv_tc_reduce_kernel<true> : conv_tc_reduce_kernel<false>,
+                                dim3(grid_for(chunks, 256)), dim3(256), 0, st, (const float*)a.partial,
+                                static_cast<uint4*>(y), chunks, t.splits, s.cout_eff, a.aff,
+                                static_cast<const uint4*>(residual), a.relu));
+    OCNN_LAUNCH_OK("conv_tc_reduce_kernel");
+  }
+  return OCNN_OK;
+}
+
 }  // namespace
 }  // namespace ocnn
 
 extern "C" {
+
+size_t ocnn_octree_conv_tc_taps_workspace_bytes(int rows, int cin, int cout) {
+  using namespace ocnn;
+  const int ks[3] = {3, 3, 3};
+  TcShape s;
+  if (rows <= 0 || tc_shape(cin, cout, ks, LayerKind{1, false, true}, &s, -1) != OCNN_OK) return 0;
+  return taps_workspace(s, tap_shape(s, rows), rows);
+}
+
+int ocnn_octree_conv_tc_taps(const void* x, const void* packed, void* y, const void* plan, int rows, int cin, int cout,
+                             int dtype, const ocnn_conv_epilogue* ep, int32_t* status, void* workspace,
+                             size_t workspace_bytes, void* stream) {
+  return ocnn::conv_taps_impl(x, packed, y, plan, rows, cin, cout, dtype, ep, status, workspace, workspace_bytes,
+                              static_cast<cudaStream_t>(stream));
+}
 
 size_t ocnn_conv_packed_weight_bytes(int cin, int cout, const int kernel_size[3], int stride) {
   return ocnn::packed_bytes_impl(cin, cout, kernel_size, ocnn::LayerKind{stride, false, false});

@@ -22,6 +22,16 @@ def _cat(skip, up):
   return torch.cat([skip, up], dim=1).contiguous(memory_format=fmt)
 
 
+def _with_tap_plan(octree, depths, data):
+  """The octree as one forward pass's layers are given it: a view that carries the tap plans of the levels that
+  they share (16-bit layers on the non-empty nodes).  It ends with the pass, and the plans with it."""
+  if not (octree.is_cuda and data.is_cuda and data.dtype in (torch.bfloat16, torch.float16)):
+    return octree
+  view = octree.view(-1)
+  view.tap_plan = nn.TapPlan(octree, depths, worthwhile=True)
+  return view
+
+
 class UNet(_nn.Module):
   def __init__(self, depth, channel_in, nout, nempty=False, interp='linear', use_checkpoint=False):
     super().__init__()
@@ -67,6 +77,8 @@ class UNet(_nn.Module):
     if data is None:
       data = octree_feature(octree, depth, self.nempty)
     assert data.size(1) == self.channel_in
+    if self.nempty:
+      octree = _with_tap_plan(octree, range(depth, depth - self.stages - 1, -1), data)
     level = {depth: self.conv1(data, octree)}
     for i in range(self.stages):
       d = depth - i - 1

@@ -1127,6 +1127,91 @@ Tensor pointwise_conv_tc(Tensor data_in, Tensor packed, int num_output, c10::opt
 // folded inside the kernel (ChannelAffine), so a layer is one call from Python and one launch.
 // (In Python, with the folded vectors computed by tensor operations, it was about 60 us of host time
 // and six launches per layer.)
+// Tap plans of an octree's levels (ocnn_tap_plan): made for one forward pass, whose layers on the non-empty nodes
+// of the same levels share them.  A layer takes the plan only for the octree, content and stream that it was
+// made for.
+class TapPlan {
+ public:
+  // `worthwhile`: only the levels of more tiles (128 rows) than SMs, and none if no level has twice as many.  With one
+  // tile per SM or less a layer is one wave of one chain of K-blocks either way, and the walk over all taps has shorter
+  // tiles and K split for it (256 -> 256 on 18.5 k rows 53 us against 58 on a plan; on 19.0 k rows, 149 tiles, 74
+  // against 59).  A plan costs 40 us and more, and its first 1.5 tiles per SM return less: a U-Net whose largest level
+  // has 37 k rows took 1286 us without and 1333 with one (50 k points, depth 7), with 49 k rows 1851 and 1810 (depth 9).
+  TapPlan(Tensor octree, const vector<int>& depths, bool worthwhile) : octree_(octree) {
+    OctreeRef o = get_octree(octree);
+    TORCH_CHECK(o.cuda, "TapPlan: the octree must be a CUDA tensor");
+    c10::cuda::CUDAGuard guard(octree.device());
+    version_ = octree._version();
+    stream_ = current_stream();
+    size_t bytes = 0;
+    vector<ocnn_tap_level> levels;
+    vector<size_t> at;
+    const int one_wave = worthwhile ? 128 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount : 0;
+    int most = 0;
+    for (int d : depths)
+      if (d >= 1 && d <= o.meta.depth) most = std::max(most, (int)o.meta.nnum_nempty[d]);
+    if (most <= 2 * one_wave) return;
+    for (int d : depths) {
+      if (d < 1 || d > o.meta.depth || depths_.size() == 8) continue;
+      if (o.meta.nnum_nempty[d] <= one_wave) continue;
+      const int64_t neigh = ocnn_prop_offset(&o.meta, OCNN_PROP_NEIGH, d);
+      const int64_t child = ocnn_prop_offset(&o.meta, OCNN_PROP_CHILD, d);
+      if (neigh < 0 || child < 0) continue;
+      depths_.push_back(d);
+      rows_.push_back(o.meta.nnum_nempty[d]);
+      ocnn_tap_level l;
+      l.neigh_dev = reinterpret_cast<const int32_t*>(o.base + neigh);
+      l.child_dev = reinterpret_cast<const int32_t*>(o.base + child);
+      l.nodes = o.meta.nnum[d];
+      l.rows = o.meta.nnum_nempty[d];
+      l.plan_dev = nullptr;
+      levels.push_back(l);
+      at.push_back(bytes);
+      bytes += (ocnn_tap_plan_bytes(l.rows) + 255) / 256 * 256;
+    }
+    if (levels.empty()) return;
+    const auto options = torch::dtype(torch::kUInt8).device(octree.device());
+    plan_ = torch::empty({(int64_t)bytes}, options);
+    for (size_t i = 0; i < levels.size(); ++i) {
+      levels[i].plan_dev = plan_.data_ptr<uint8_t>() + at[i];
+      plans_.push_back(levels[i].plan_dev);
+    }
+    const size_t need = ocnn_tap_plan_workspace_bytes(levels.data(), (int)levels.size());
+    Tensor ws = torch::empty({(int64_t)need}, options);
+    OCNN_CALL(ocnn_tap_plan(levels.data(), (int)levels.size(), ws.data_ptr(), need, stream_));
+  }
+
+  // The plan of a level, or NULL: not made, of another octree or content, or on another stream.
+  const void* find(const Tensor& octree, int depth, int rows) const {
+    if (!octree.storage().is_alias_of(octree_.storage()) || octree.storage_offset() != octree_.storage_offset() ||
+        octree._version() != version_ || current_stream() != stream_)
+      return nullptr;
+    for (size_t i = 0; i < depths_.size(); ++i)
+      if (depths_[i] == depth && rows_[i] == rows) return plans_[i];
+    return nullptr;
+  }
+
+  // (for tests) [tiles * 128] rows in the plan's order, and the taps of each tile
+  std::tuple<Tensor, Tensor> level(int depth) const {
+    for (size_t i = 0; i < depths_.size(); ++i) {
+      if (depths_[i] != depth) continue;
+      const int64_t tiles = (rows_[i] + 127) / 128;
+      const auto options = torch::dtype(torch::kInt32).device(plan_.device());
+      int* base = static_cast<int*>(const_cast<void*>(plans_[i]));
+      return {torch::from_blob(base, {tiles * 128}, options).clone(),
+              torch::from_blob(base + tiles * 128, {tiles}, options).clone()};
+    }
+    TORCH_CHECK(false, "TapPlan: no plan at depth ", depth);
+  }
+
+ private:
+  Tensor octree_, plan_;
+  uint32_t version_ = 0;
+  void* stream_ = nullptr;
+  vector<int> depths_, rows_;
+  vector<const void*> plans_;
+};
+
 class ConvLayer {
  public:
   ConvLayer(int cin, int cout, vector<int> ks, int stride, bool nempty, bool transposed, bool point)
@@ -1139,7 +1224,7 @@ class ConvLayer {
   Tensor run(Tensor data, Tensor weights, c10::optional<Tensor> octree, int depth,
              c10::optional<Tensor> scale, c10::optional<Tensor> bias, c10::optional<Tensor> bn_mean,
              c10::optional<Tensor> bn_var, double bn_eps, c10::optional<Tensor> residual, bool relu,
-             Tensor status) {
+             Tensor status, const TapPlan* taps) {
     torch::NoGradGuard no_grad;
     const char* what = transposed_ ? "octree_deconv" : "octree_conv";
     need_cuda(data, what);
@@ -1150,7 +1235,10 @@ class ConvLayer {
     TORCH_CHECK(!point_ || weights.dim() >= 2, what, ": the weights of a 1x1 layer are [Cout, Cin, 1]");
     const int cin = point_ ? (int)weights.size(1) : cin_, cout = point_ ? (int)weights.size(0) : cout_;
     TORCH_CHECK(x.C == cin, what, ": the data has ", x.C, " channels, the layer takes ", cin);
+    const bool tc_layout = x.dtype != OCNN_F32 && cin % 8 == 0 && cout % 8 == 0 &&
+                           data.is_contiguous(at::MemoryFormat::ChannelsLast);
     Geometry geo;
+    const void* plan = nullptr;
     if (point_) {
       memset(&geo.g, 0, sizeof(geo.g));
       geo.g.stride = 1; geo.g.h_in = x.H; geo.g.h_out = x.H;
@@ -1158,7 +1246,11 @@ class ConvLayer {
       TORCH_CHECK(octree.has_value(), what, ": octree required");
       OctreeRef o = get_octree(*octree);
       TORCH_CHECK(o.cuda, what, ": the octree must be a CUDA tensor");
-      geo = make_geometry(o, x, depth, ks_, stride_, nempty_, transposed_, what);
+      if (taps != nullptr && tc_layout && takes_taps(cin)) plan = taps->find(*octree, depth, x.H);
+      if (plan != nullptr) {
+        memset(&geo.g, 0, sizeof(geo.g));
+        geo.g.h_in = geo.g.h_out = x.H;
+      } else geo = make_geometry(o, x, depth, ks_, stride_, nempty_, transposed_, what);
     }
     Tensor keep[5];     // float32 copies of parameters that are held in another type
     auto f32 = [&](const c10::optional<Tensor>& t, int slot) -> const float* {
@@ -1181,13 +1273,20 @@ class ConvLayer {
     }
     Tensor w = point_ ? weights.to(torch::kFloat32).contiguous() : weights;
     check_weights(w, cin, cout, K);
-    const bool tc_layout = x.dtype != OCNN_F32 && cin % 8 == 0 && cout % 8 == 0 &&
-                           data.is_contiguous(at::MemoryFormat::ChannelsLast);
     if (tc_layout) {
       Tensor packed = packed_for(weights, w, cin, cout, x.dtype == OCNN_F16);
       if (packed.defined()) {
         TORCH_CHECK(status.is_cuda() && status.scalar_type() == torch::kInt32 && status.numel() >= 1,
                     "status must be an int32 CUDA tensor");
+        if (plan != nullptr) {
+          const size_t bytes = ocnn_octree_conv_tc_taps_workspace_bytes(x.H, cin, cout);
+          Tensor ws;
+          if (bytes > 0) ws = torch::empty({(int64_t)bytes}, torch::dtype(torch::kUInt8).device(y.device()));
+          OCNN_CALL(ocnn_octree_conv_tc_taps(x.t.data_ptr(), packed.data_ptr(), y.data_ptr(), plan, x.H, cin, cout,
+                                             x.dtype, &ep, status.data_ptr<int32_t>(),
+                                             bytes > 0 ? ws.data_ptr() : nullptr, bytes, current_stream()));
+          return y;
+        }
         run_conv_tc(x.t.data_ptr(), packed, y, geo.g, cin, cout, ks_, x.dtype, &ep, status.data_ptr<int32_t>());
         return y;
       }
@@ -1201,6 +1300,12 @@ class ConvLayer {
   }
 
  private:
+  // Layers for which a tap plan stands in for the geometry.
+  bool takes_taps(int cin) const {
+    return nempty_ && !transposed_ && stride_ == 1 && ks_[0] == 3 && ks_[1] == 3 && ks_[2] == 3 && cin % 16 == 0 &&
+           cin <= 512 && ocnn_conv_packed_weight_bytes_general(cin, cout_, ks_.data(), 1, 0, 1) > 0;
+  }
+
   static bool capturing(const c10::cuda::CUDAStream& stream) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     if (stream.stream() == nullptr) return false;         // the default stream cannot be captured
@@ -2917,6 +3022,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("bf16") = true, py::arg("half") = false);
   m.def("set_key_bits", &set_key_bits);
   m.def("get_key_bits", &get_key_bits);
+  py::class_<TapPlan>(m, "TapPlan")
+      .def(py::init<Tensor, const vector<int>&, bool>(), py::arg("octree"), py::arg("depths"),
+           py::arg("worthwhile") = false)
+      .def("level", &TapPlan::level);
   py::class_<ConvLayer>(m, "ConvLayer")
       .def(py::init<int, int, vector<int>, int, bool, bool, bool>(), py::arg("cin"), py::arg("cout"),
            py::arg("kernel_size"), py::arg("stride") = 1, py::arg("nempty") = false,

@@ -1,0 +1,133 @@
+"""Tap plans (`ocnn.nn.TapPlan`): the order and masks against numpy, and the convolution on a plan against the walk
+over all taps, which it equals bit for bit where neither splits K."""
+import numpy as np
+import pytest
+import torch
+
+import gpu_util as gu
+from oracle import oracle as oc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope='module')
+def ocnn():
+  import ocnn as mod
+  mod.set_key_bits(64)
+  return mod
+
+
+@pytest.fixture(scope='module')
+def small():
+  """Levels of 1 to about 3 k non-empty nodes."""
+  _, merged, _ = gu.oracle_batch(gu.small_clouds(3, 3000, 500), 5, 2, 64)
+  return gu.to_cuda_u8(merged), oc.OctreeView(merged)
+
+
+@pytest.fixture(scope='module')
+def large(ocnn):
+  """About 97 k non-empty nodes at depth 7, a slab among scattered points: from 1 to 27 neighbours."""
+  gen = torch.Generator().manual_seed(7)
+  p = 0.99 * (2 * torch.rand(100000, 3, generator=gen) - 1)
+  p[50000:] = p[50000:] * torch.tensor([1.0, 1.0, 0.02])
+  n = torch.nn.functional.normalize(torch.randn(100000, 3, generator=gen), dim=1)
+  return ocnn.octree_batch([ocnn.Points2Octree(7, 2)(ocnn.points_new(p, n, torch.zeros(0), torch.zeros(0)))]).cuda()
+
+
+def neighbour_sets(ocnn, octree, d):
+  """[rows, 27] which neighbours of a level's non-empty nodes are non-empty."""
+  child = ocnn.octree_property(octree, 'child', d).cpu().numpy()
+  neigh = ocnn.octree_property(octree, 'neigh', d).cpu().numpy().reshape(-1, 64)
+  t = np.arange(27)
+  h = np.nonzero(child >= 0)[0]
+  code = ((h & 4) << 2) | ((h & 2) << 1) | (h & 1)
+  at = neigh[h >> 3][np.arange(h.size)[:, None], ((t // 9 << 4) | (t // 3 % 3 << 2) | t % 3)[None] + code[:, None]]
+  return (at >= 0) & (child[np.maximum(at, 0)] >= 0)
+
+
+def check_plan(ocnn, octree, plan, d):
+  sets = neighbour_sets(ocnn, octree, d)
+  order, mask = (t.cpu().numpy() for t in plan.level(d))
+  live = order >= 0
+  assert np.array_equal(np.sort(order[live]), np.arange(len(sets))) and live[:len(sets)].all()
+  per_row = (sets.astype(np.int64) << np.arange(27)).sum(1)
+  want = np.where(live, per_row[np.maximum(order, 0)], 0).reshape(-1, 128)
+  assert np.array_equal(np.bitwise_or.reduce(want, axis=1), mask)
+  return sets, mask
+
+
+def test_plan_of_all_levels(ocnn, small, large):
+  octree, v = small
+  plan = ocnn.nn.TapPlan(octree, [5, 4, 3, 2, 1, 0, 9])      # (levels that are not there are left out)
+  for d in range(1, 6):
+    check_plan(ocnn, octree, plan, d)
+  with pytest.raises(RuntimeError):
+    plan.level(0)
+  plan = ocnn.nn.TapPlan(large, [7, 6, 5])
+  for d in (7, 6, 5):
+    sets, mask = check_plan(ocnn, large, plan, d)
+  sets, mask = check_plan(ocnn, large, plan, 7)
+  tile_taps = np.unpackbits(mask.view(np.uint8)).sum() / mask.size
+  assert sets.sum(1).mean() <= tile_taps < 17                 # (in Morton order it is 27)
+
+
+def both(ocnn, octree, d, cin, cout, dtype, with_res=False, edit=None):
+  h = int((ocnn.octree_property(octree, 'child', d) >= 0).sum())
+  torch.manual_seed(cin + cout + d)
+  fmt = dict(memory_format=torch.channels_last)
+  x = torch.randn(1, cin, h, 1, device='cuda').to(dtype).contiguous(**fmt)
+  res = torch.randn(1, cout, h, 1, device='cuda').to(dtype).contiguous(**fmt) if with_res else None
+  bn = torch.nn.BatchNorm2d(cout).cuda().eval() if with_res else None
+  layer = ocnn.OctreeConv(d, cin, cout, nempty=True).cuda().eval()
+  if edit is not None:
+    edit(layer.weights)
+  planned = octree.view(-1)
+  planned.tap_plan = ocnn.nn.TapPlan(octree, [d])
+  with torch.no_grad():
+    return [layer._run(x, o, bn, res, with_res) for o in (octree, planned)]
+
+
+# (channels that share K-blocks between taps, that leave a remainder, that fill 1 to 8 blocks; output columns of
+# one 16-column piece, with a remainder of 8, of one and of two slices)
+@pytest.mark.parametrize('cin,cout', [(16, 8), (32, 32), (48, 40), (96, 96), (128, 96), (192, 128), (64, 256), (32, 512),
+                                      (512, 16)])
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize('with_res', [False, True])
+def test_convolution_on_a_plan(ocnn, small, large, cin, cout, dtype, with_res):
+  for octree, d in ((large, 7), (small[0], 5), (small[0], 4), (small[0], 1)):
+    a, b = both(ocnn, octree, d, cin, cout, dtype, with_res)
+    if octree is large or cin <= 64:       # (fewer than 32 K-blocks, or tiles for every SM: K is not split)
+      assert torch.equal(a, b)
+    else:                                  # sums of parts: fp32 sums of up to 27 cin terms, rounded to 16 bits once
+      ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+      assert bool(((a.float() - b.float()).abs() <= 2 * ulp * a.float().abs() + 1e-5 * float(a.float().abs().max())).all())
+
+
+@pytest.mark.parametrize('value', [float('inf'), float('nan'), 1e6])     # (1e6: infinite as float16)
+def test_weights_that_are_not_finite(ocnn, small, value):
+  def edit(w):
+    with torch.no_grad():
+      w[3, 27 * 5 + 0] = value             # a corner tap: most tiles have none of it
+  a, b = both(ocnn, small[0], 5, 32, 32, torch.float16, edit=edit)
+  assert bool(torch.isnan(a).any())
+  torch.testing.assert_close(a, b, rtol=0, atol=0, equal_nan=True)
+
+
+def test_a_plan_serves_only_what_it_was_made_for(ocnn, small):
+  octree = small[0].clone()
+  h = int((ocnn.octree_property(octree, 'child', 5) >= 0).sum())
+  x = torch.randn(1, 32, h, 1, device='cuda').bfloat16().contiguous(memory_format=torch.channels_last)
+  layer = ocnn.OctreeConv(5, 32, 32, nempty=True).cuda().eval()
+  planned = octree.view(-1)
+  planned.tap_plan = ocnn.nn.TapPlan(octree, [5])
+  with torch.no_grad():
+    want = layer(x, octree)
+    assert torch.equal(layer(x, planned), want)
+    other = torch.cuda.Stream()
+    other.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(other):
+      got = layer(x, planned)              # not waited for there
+    torch.cuda.current_stream().wait_stream(other)
+    assert torch.equal(got, want)
+    planned.copy_(small[0])                # written to since
+    assert torch.equal(layer(x, planned), want)
