@@ -20,7 +20,7 @@
 // This file is compiled with --fmad=false: the signal must round exactly like the reference's
 // separate multiplies and adds (octree.cpp:330-348).
 //
-// A depth-6 batch is 15 launches and a memset: encode + first histogram, two sort passes of 9 bits (five
+// A small cloud's keys, sort and unique are one launch (small_build_kernel).  A depth-6 batch is 15 launches and a memset: encode + first histogram, two sort passes of 9 bits (five
 // launches), count and compact for all levels at once, averages, emit, five for the neighbour tables.  (A
 // count and a compact launch per level, a sort over the cloud bits too and separate header / table copies
 // made it 29, most of them shorter than their launch.)
@@ -226,7 +226,19 @@ struct EncodeArgs {
 };
 
 // normalize_pts + sort_keys' key computation (octree.cpp:155-170, 180-186): cell = trunc((p -
-// bbmin) * mul), only `depth` bits per axis enter the key.  One CTA per sort chunk, whose cloud is the
+// bbmin) * mul), only `depth` bits per axis enter the key.
+__device__ __forceinline__ uint64_t cell_key(const EncodeArgs& a, const float (&p)[3], uint64_t top) {
+  const uint32_t mask = (1u << a.depth) - 1u;
+  uint32_t cell[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const float s = (p[j] - a.bbmin[j]) * a.mul;
+    cell[j] = (uint32_t)s & mask;
+  }
+  return top | (spread3(cell[0]) << 2) | (spread3(cell[1]) << 1) | spread3(cell[2]);
+}
+
+// One CTA per sort chunk, whose cloud is the
 // CTA's (WHOLE: each of its points is looked up among the chunk's clouds); the first sort pass's digits are
 // counted on the way.
 template <typename KeyT, int RB, bool WHOLE>
@@ -247,7 +259,6 @@ __global__ void __launch_bounds__(kThreads) encode_kernel(const __grid_constant_
     range[threadIdx.x >> 5] = cloud_of_point(clouds, 0, a.batch - 1, threadIdx.x == 0 ? c.beg : c.end - 1);
   const float* xyz = WHOLE ? nullptr : clouds[c.segment].xyz - 3 * clouds[c.segment].offset;
   uint64_t top = (uint64_t)c.segment << (3 * a.depth);
-  const uint32_t mask = (1u << a.depth) - 1u;
   __syncthreads();
   for (long long i0 = c.beg; i0 < c.end; i0 += 4 * kThreads) {
     float p[4][3];
@@ -266,15 +277,9 @@ __global__ void __launch_bounds__(kThreads) encode_kernel(const __grid_constant_
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const long long i = i0 + u * kThreads + threadIdx.x;
-      uint32_t cell[3];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const float s = (p[u][j] - a.bbmin[j]) * a.mul;
-        cell[j] = (uint32_t)s & mask;
-      }
       if (WHOLE) top = i < c.end ? (uint64_t)cloud[u] << (3 * a.depth) : 0;
       // (with the cloud's bits: the top digit of a shallow tree reaches into them, here as in the scatter)
-      const uint64_t key = top | (spread3(cell[0]) << 2) | (spread3(cell[1]) << 1) | spread3(cell[2]);
+      const uint64_t key = cell_key(a, p[u], top);
       if (i < c.end) keys[i] = (KeyT)key;
       count_digit(sh[threadIdx.x >> 5], i < c.end ? (int)(key & ((1 << RB) - 1)) : (1 << RB), 1 << RB);
     }
@@ -675,6 +680,165 @@ __global__ void __launch_bounds__(kThreads) unique_compact_kernel(const __grid_c
   grid_dependency_trigger();    // at the end: the successor's blocks should not sit on SM slots early
 }
 
+// ---- a small cloud in one launch ----------------------------------------------------------------
+// Keys, sort and unique of a cloud that one CTA holds, in the workspace form that the launches above leave
+// (sorted indices, K and start of every level, counts, the table of clouds).  What bounds it: a chain of steps
+// that each run once, so latency and the fetching of code; the loops are rolled (unrolled over a thread's eight
+// keys and ten levels the kernel took 26 to 31 us at 5000 points, 20 us so; as nine launches, each 3 to 7 us for a
+// few blocks of work, it was 39 us of a data loader's 78 us a sample).
+//
+// Keys and indices lie in shared memory, twice.  A warp owns a run of rows of 32 keys; a pass counts its digits per
+// warp, prefixes the counts over the warps and the digits, and moves the keys row by row (ranks inside a row by
+// ballots: match_digit), which keeps equal digits in order.
+constexpr int kSmallThreads = 1024, kSmallWarps = 32, kSmallBins = 256, kSmallPoints = 6144;
+size_t small_smem(int64_t n) {
+  return (size_t)((n + 31) / 32 * 32) * 12 + (size_t)kSmallWarps * kSmallBins * 4 + (4 + 1) * kSmallBins * 4;
+}
+
+__global__ void __launch_bounds__(kSmallThreads) small_build_kernel(const __grid_constant__ EncodeArgs e,
+                                                                    const __grid_constant__ UniqueArgs<uint32_t> a,
+                                                                    uint32_t* __restrict__ idx_out, int passes) {
+  extern __shared__ __align__(16) uint8_t small_raw[];
+  const int n = (int)a.n, cap = (n + 31) & ~31;
+  uint32_t* key = reinterpret_cast<uint32_t*>(small_raw);            // [2][cap]
+  int* cnt = reinterpret_cast<int*>(key + 2 * cap);                  // [warp][digit]
+  int* part = cnt + kSmallWarps * kSmallBins;                        // [4][digit]
+  int* first = part + 4 * kSmallBins;                                // [digit]
+  uint16_t* idx = reinterpret_cast<uint16_t*>(first + kSmallBins);   // [2][cap]
+  __shared__ int s_scan[kSmallWarps], s_level[kSmallWarps][32], s_total[32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rows = (cap / 32 + kSmallWarps - 1) / kSmallWarps;       // rows a warp owns
+  const int run0 = min(warp * rows * 32, cap), run1 = min(run0 + rows * 32, cap);
+  const unsigned below = (1u << lane) - 1u;
+  grid_dependency_wait();       // launched as a programmatic dependent: see common.cuh
+  if (tid < 2) const_cast<CloudRef*>(e.table)[tid] = e.clouds[tid];
+#pragma unroll 4
+  for (int i = tid; i < n; i += kSmallThreads) {
+    const float* from = e.clouds[0].xyz + 3 * i;
+    const float p[3] = {from[0], from[1], from[2]};
+    key[i] = (uint32_t)cell_key(e, p, 0);
+    idx[i] = (uint16_t)i;
+  }
+  int from = 0;
+#pragma unroll 1
+  for (int pass = 0; pass < passes; ++pass, from ^= 1) {
+    const uint32_t* kin = key + from * cap;
+    const uint16_t* iin = idx + from * cap;
+    uint32_t* kout = key + (from ^ 1) * cap;
+    uint16_t* iout = idx + (from ^ 1) * cap;
+    int* mine = cnt + warp * kSmallBins;
+    for (int d = lane; d < kSmallBins; d += 32) mine[d] = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int i = run0 + lane; i < run1; i += 32) {
+      const int digit = i < n ? (int)((kin[i] >> (8 * pass)) & (kSmallBins - 1)) : kSmallBins;
+      count_digit(mine, digit, kSmallBins);
+    }
+    __syncthreads();
+    {                                    // a digit's counts over the warps: four threads a digit, eight warps each
+      const int digit = tid & (kSmallBins - 1), q = tid >> 8;
+      int* c = cnt + q * 8 * kSmallBins + digit;
+      int v[8], sum = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        v[w] = c[w * kSmallBins];
+        sum += v[w];
+      }
+      part[q * kSmallBins + digit] = sum;
+      __syncthreads();
+      int at = 0;
+      for (int p = 0; p < q; ++p) at += part[p * kSmallBins + digit];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        c[w * kSmallBins] = at;
+        at += v[w];
+      }
+      // the digits' totals, prefixed by the last quarter's warps
+      int inc = at;
+      if (q == 3) {
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += t;
+        }
+        if (lane == 31) s_scan[warp - 24] = inc;
+      }
+      __syncthreads();
+      if (q == 3) {
+        int base = inc - at;
+        for (int w = 0; w < warp - 24; ++w) base += s_scan[w];
+        first[digit] = base;
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int i = run0 + lane; i < run1; i += 32) {
+      const unsigned mask = __ballot_sync(0xffffffffu, i < n);
+      if (i < n) {
+        const uint32_t k = kin[i];
+        const int digit = (int)((k >> (8 * pass)) & (kSmallBins - 1));
+        const unsigned peers = match_digit<8>(mask, digit);
+        const int before = __popc(peers & below), at = mine[digit];
+        __syncwarp(mask);
+        if (before == 0) mine[digit] = at + __popc(peers);
+        kout[first[digit] + at + before] = k;
+        iout[first[digit] + at + before] = iin[i];
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+  }
+  const uint32_t* sorted = key + from * cap;
+  for (int i = tid; i < n; i += kSmallThreads) idx_out[i] = idx[from * cap + i];
+  // Nodes opened per level: a level's nodes of a row are its ballot; lane l keeps level l's count.
+  auto opened = [&](int i) { return i < n ? opened_level(a, sorted[i], i > 0 ? sorted[i - 1] : 0u, i == 0) : a.levels; };
+  int count = 0;
+#pragma unroll 1
+  for (int i = run0 + lane; i < run1; i += 32) {
+    const int lvl = opened(i);
+#pragma unroll 1
+    for (int l = 0; l < a.levels; ++l) {
+      const int c = __popc(__ballot_sync(0xffffffffu, lvl <= l));
+      if (lane == l) count += c;
+    }
+  }
+  s_level[warp][lane] = count;
+  __syncthreads();
+  if (warp < a.levels) {                 // warp l: the prefix of level l over the warps
+    const int v = s_level[lane][warp];
+    int t = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += u;
+    }
+    s_level[lane][warp] = t - v;
+    if (lane == 31) s_total[warp] = t;
+  }
+  __syncthreads();
+  count = s_level[warp][lane];
+#pragma unroll 1
+  for (int i = run0 + lane; i < run1; i += 32) {
+    const int lvl = opened(i);
+    int finer = i;                       // this node's first entry one level finer
+#pragma unroll 1
+    for (int l = a.levels - 1; l >= 0; --l) {
+      const unsigned opens = __ballot_sync(0xffffffffu, lvl <= l);
+      const int rank = __shfl_sync(0xffffffffu, count, l) + __popc(opens & below);
+      if (lvl <= l) {
+        a.K[l][rank] = sorted[i] >> (3 * (a.levels - 1 - l));
+        a.start[l][rank] = finer;
+      }
+      finer = rank;
+      if (lane == l) count += __popc(opens);
+    }
+  }
+  if (tid < a.levels) {
+    a.counts[a.full + tid] = s_total[tid];
+    a.host_counts[a.full + tid] = s_total[tid];
+    a.start[tid][s_total[tid]] = tid == a.levels - 1 ? n : s_total[tid + 1];
+  }
+  grid_dependency_trigger();
+}
+
 // ---- emit ------------------------------------------------------------------------------------
 struct EmitLevel {
   long long off_key, off_child, off_split;   // byte offsets of this level (split < 0: absent)
@@ -1061,10 +1225,7 @@ int sort_keys(const EncodeArgs& ea, const Layout& L, int chunks, uint8_t* ws, cu
 }
 
 template <typename KeyT>
-int sort_and_unique(const EncodeArgs& ea, const Layout& L, int chunks, uint8_t* ws, int* host_counts,
-                    cudaStream_t st) {
-  const int rc = L.radix_bits == 9 ? sort_keys<KeyT, 9>(ea, L, chunks, ws, st) : sort_keys<KeyT, 8>(ea, L, chunks, ws, st);
-  if (rc != OCNN_OK) return rc;
+UniqueArgs<KeyT> unique_args(const Layout& L, uint8_t* ws, int* host_counts) {
   UniqueArgs<KeyT> u;
   memset(&u, 0, sizeof(u));
   u.keys = reinterpret_cast<const KeyT*>(ws + L.off_keys[L.passes & 1]);
@@ -1077,6 +1238,42 @@ int sort_and_unique(const EncodeArgs& ea, const Layout& L, int chunks, uint8_t* 
     u.K[l] = reinterpret_cast<KeyT*>(ws + L.off_K[L.full + l]);
     u.start[l] = reinterpret_cast<int*>(ws + L.off_start[L.full + l]);
   }
+  return u;
+}
+
+// Whether one CTA sorts: one cloud with 32-bit keys, and as many points as it sorts in no more time than the launches
+// over the whole GPU.  A whole build in us, one CTA / several launches: 1000 points 37 / 53 at depth 5, 45 / 66 at
+// depth 8; 4000 points 46 / 57, 58 / 70; 8000 points 58 / 57, 76 / 73; 12288 points 71 / 58, 93 / 74.  (Several
+// clouds add a look-up per point: 32 of 380 points 90 / 66.)
+bool one_cta(const Layout& L) { return L.batch == 1 && L.key_bytes == 4 && L.n <= kSmallPoints; }
+
+int small_build(const EncodeArgs& ea, const Layout& L, uint8_t* ws, int* host_counts, cudaStream_t st) {
+  const UniqueArgs<uint32_t> u = unique_args<uint32_t>(L, ws, host_counts);
+  const int passes = (3 * L.depth + 7) / 8;
+  uint32_t* idx = reinterpret_cast<uint32_t*>(ws + L.off_idx[L.passes & 1]);      // where the emit looks for it
+  static PerDeviceOnce attr_once;
+  int device = 0;
+  OCNN_CUDA_OK(cudaGetDevice(&device));
+  {
+    std::lock_guard<std::mutex> lock(attr_once.mutex);
+    const bool known = device >= 0 && device < 64;
+    if (!known || !attr_once.done[device]) {
+      OCNN_CUDA_OK(cudaFuncSetAttribute(small_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)small_smem(kSmallPoints)));
+      if (known) attr_once.done[device] = true;
+    }
+  }
+  OCNN_CUDA_OK(launch_chained(small_build_kernel, dim3(1), dim3(kSmallThreads), small_smem(L.n), st, ea, u, idx, passes));
+  OCNN_LAUNCH_OK("small_build_kernel");
+  return OCNN_OK;
+}
+
+template <typename KeyT>
+int sort_and_unique(const EncodeArgs& ea, const Layout& L, int chunks, uint8_t* ws, int* host_counts,
+                    cudaStream_t st) {
+  const int rc = L.radix_bits == 9 ? sort_keys<KeyT, 9>(ea, L, chunks, ws, st) : sort_keys<KeyT, 8>(ea, L, chunks, ws, st);
+  if (rc != OCNN_OK) return rc;
+  const UniqueArgs<KeyT> u = unique_args<KeyT>(L, ws, host_counts);
   const int grid = grid_for(L.n, kScanTile, 4) < kMaxScanGrid ? grid_for(L.n, kScanTile, 4) : kMaxScanGrid;
   if (u.levels <= 8) {
     OCNN_CUDA_OK(launch_chained(unique_count_kernel<KeyT, 8>, dim3(grid), dim3(kThreads), 0, st, u));
@@ -1289,9 +1486,14 @@ int ocnn_octree_build_plan(const ocnn_points_batch* pts, const ocnn_build_params
   if (!ea.inline_clouds)
     OCNN_CUDA_OK(cudaMemcpyAsync(ws + L.off_clouds, big.data(), sizeof(CloudRef) * big.size(),
                                  cudaMemcpyHostToDevice, st));
-  OCNN_CUDA_OK(cudaMemsetAsync(ws + L.off_counts, 0, L.zero_bytes, st));
-  const int s = L.key_bytes == 4 ? sort_and_unique<uint32_t>(ea, L, chunks, ws, counts, st)
-                                 : sort_and_unique<uint64_t>(ea, L, chunks, ws, counts, st);
+  int s;
+  if (one_cta(L)) {
+    s = small_build(ea, L, ws, counts, st);
+  } else {
+    OCNN_CUDA_OK(cudaMemsetAsync(ws + L.off_counts, 0, L.zero_bytes, st));
+    s = L.key_bytes == 4 ? sort_and_unique<uint32_t>(ea, L, chunks, ws, counts, st)
+                         : sort_and_unique<uint64_t>(ea, L, chunks, ws, counts, st);
+  }
   if (s != OCNN_OK) return s;
   OCNN_CUDA_OK(cudaStreamSynchronize(st));
 

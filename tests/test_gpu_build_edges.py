@@ -114,3 +114,17 @@ def test_workspace_on_an_8_byte_boundary(ocnn, depth, shift):
                                     ctypes.c_void_p(out.data_ptr()), ctypes.c_size_t(out.numel()), None, stream) == 0
   torch.cuda.synchronize()
   assert np.array_equal(out.cpu().numpy(), want)
+
+
+# One cloud of up to 6144 points is sorted by one launch, others by several: the edges of each, a single point, rows that do not fill up, every
+# number of passes; and the chunk edges of the longer way.
+@pytest.mark.parametrize('sizes', [[1], [33], [1024], [1025], [6143], [6144], [6145], [1, 2047, 2048]])
+@pytest.mark.parametrize('depth,full,key_bits', [(1, 1, 64), (5, 2, 64), (6, 2, 32), (8, 2, 64), (9, 2, 64), (10, 1, 64)])
+def test_one_launch_or_several(ocnn, sizes, depth, full, key_bits):
+  check(ocnn, clouds_of(sizes, 300 + sum(sizes)), depth, full, key_bits)
+
+
+def test_points_in_one_cell(ocnn):
+  p = np.full((3000, 3), 0.123, np.float32)
+  q = np.tile(np.float32([0, 0, 1]), (3000, 1))
+  check(ocnn, [oc.points_new(p, q)], 6, 2, 64)
