@@ -65,9 +65,10 @@ __global__ void __launch_bounds__(256) conv_f32_wgrad_prepare_kernel(const WgPre
   }
   const long long i = (long long)(blockIdx.x - a.x_blocks) * 256 + threadIdx.x;
   if (i >= a.a_items) return;
-  const long long rows = (long long)a.steps * kWgStep;       // h fastest: coalesced channel-major reads
-  const int c8 = (int)(i / rows);
-  const long long h = i - (long long)c8 * rows;
+  const long long rows = (long long)a.steps * kWgStep;
+  int c8;
+  long long h;
+  chunk_of_block(i, rows, a.slices * a.npad / 8, c8, h);     // (a row of an image is four chunks)
   uint4 part[3];
   split_chunk(a.a, h, c8, a.h_a, a.m, a.node_major, part);
   const int slice = c8 / (a.npad / 8), n8 = c8 - slice * (a.npad / 8);

@@ -51,8 +51,9 @@ __device__ __forceinline__ void split3(float v, uint16_t& hi, uint16_t& mid, uin
 }
 
 // Chunk i of a [C, H] (or node-major [H, C]) fp32 tensor as parts: rows of 6 Cp bytes, per block of 32
-// channels [high | middle | low].  One thread per (8-channel chunk, node): eight reads that are
-// coalesced over the threads of a channel-major tensor (consecutive nodes), three 16-byte stores.
+// channels [high | middle | low].  One thread per (8-channel chunk, node): eight reads and three 16-byte stores.  Of a
+// channel-major tensor a warp takes 8 nodes by 4 chunks: whole 32-byte sectors on either side, 64 contiguous bytes per
+// part and node (32 nodes of one chunk wrote half sectors 6 Cp bytes apart: 64 channels x 218 k rows 77 us, 32 so).
 __device__ __forceinline__ void split_chunk(const float* __restrict__ x, long long h, int c8, long long rows,
                                             int channels, int node_major, uint4 (&part)[3]) {
   float v[8];
@@ -74,13 +75,22 @@ __device__ __forceinline__ void split_chunk(const float* __restrict__ x, long lo
   for (int q = 0; q < 3; ++q) part[q] = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
 }
 
+// (chunk, node) number i of a channel-major tensor: blocks of up to four chunks, nodes, chunks of the block.
+__device__ __forceinline__ void chunk_of_block(long long i, long long rows, int chunks, int& c8, long long& h) {
+  const int block = (int)(i / (4 * rows));
+  const uint32_t left = (uint32_t)min(4, chunks - 4 * block);
+  const long long rest = i - 4 * rows * block;
+  h = left == 4 ? rest >> 2 : rest / left;
+  c8 = 4 * block + (int)(rest - h * left);
+}
+
 __device__ __forceinline__ void split_rows(const float* __restrict__ x, uint8_t* __restrict__ xs, long long i,
                                            long long rows, int channels, int cp, int node_major) {
   const int chunks = cp >> 3;
   long long h;
   int c8;
   if (node_major) { h = i / chunks; c8 = (int)(i - h * chunks); }
-  else { c8 = (int)(i / rows); h = i - (long long)c8 * rows; }
+  else chunk_of_block(i, rows, chunks, c8, h);
   uint4 part[3];
   split_chunk(x, h, c8, rows, channels, node_major, part);
   const int block = c8 >> 2, width = min(4, chunks - 4 * block) * 16;
