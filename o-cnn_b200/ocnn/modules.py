@@ -204,7 +204,7 @@ class OctreeConv1x1(_nn.Module):
           scale, bias = _folded(bn)
           affine = (scale, bias + b * scale, None, None, 0.0)
     return self._layer.run(data_in, conv.weight, None, 0, *affine, residual, relu,
-                           tc_status(data_in.device), None)
+                           tc_status(data_in.device))
 
   def forward(self, data_in):
     return self.run(data_in)

@@ -148,10 +148,14 @@ class OctreeConvBase(_nn.Module):
     if layer is None:
       layer = self._layer = nn.ConvLayer(self.channel_in, self.channel_out, self.kernel_size,
                                          self.stride, self.nempty, not self.is_conv_layer())
-    # (a network that runs several layers on the same levels hands the octree on with a plan of them)
-    taps = getattr(octree, 'tap_plan', None) if self.nempty else None
+    if self.nempty:
+      # (a network that runs several layers on the same levels hands the octree on with a plan of them)
+      taps = getattr(octree, 'tap_plan', None)
+      if taps is not None:
+        return layer.run_on(data, self.weights, octree, self.depth, *bn_vectors(bn), residual, relu,
+                            tc_status(data.device), taps)
     return layer.run(data, self.weights, octree, self.depth, *bn_vectors(bn), residual, relu,
-                     tc_status(data.device), taps)
+                     tc_status(data.device))
 
   def extra_repr(self) -> str:
     return ('depth={}, channel_in={}, channel_out={}, kernel_size={}, stride={}, '
