@@ -124,6 +124,10 @@ int ocnn_cat_rows(const void* a_dev, const void* b_dev, void* out_dev, int64_t r
 int ocnn_octree_max_pool_pad(const void* btm_dev, void* top_dev, const int32_t* child_dev,
                              int channels, int btm_h, int top_h, int dtype, int layout,
                              void* stream);
+/* The same for fp32 channel-major data ([C, btm_h] -> [C, top_h], btm_dev on a 16-byte boundary), any C; mask_dev
+ * ([C, btm_h / 8] as ocnn_octree_max_pool writes it) may be NULL. */
+int ocnn_octree_max_pool_pad_f32(const float* btm_dev, float* top_dev, int32_t* mask_dev,
+                                 const int32_t* child_dev, int C, int btm_h, int top_h, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Neighbour table.  Replace calc_neigh_gpu (both overloads), octree/octree/octree_nn.cu:331-413,

@@ -85,6 +85,9 @@ class OctreeMaxPool(OctreePoolBase):
         return nn.octree_max_pool_pad(data, octree, self.depth)
     if not self.return_indices and data.dtype == torch.float32 and torch.is_grad_enabled() and data.requires_grad:
       return nn.train_max_pool(data, octree, self.depth)      # both steps as one autograd node
+    if not self.return_indices and data.dtype == torch.float32 and data.is_cuda and data.is_contiguous():
+      with torch.no_grad():
+        return nn.octree_max_pool_pad_f32(data, octree, self.depth)
     pool, mask = octree_max_pool(data, octree, self.depth)
     output = octree_pad(pool, octree, self.depth - 1)
     return output if not self.return_indices else (output, mask)

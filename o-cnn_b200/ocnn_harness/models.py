@@ -458,6 +458,9 @@ class GpuNet:
     if self.bf16 and x.shape[1] % 8 == 0:
       self.launches += 1
       return nn.octree_max_pool_pad(x, octree, d)          # pool + pad in one kernel
+    if x.dtype == self.torch.float32 and x.is_contiguous():
+      self.launches += 1
+      return nn.octree_max_pool_pad_f32(x, octree, d)
     top, _ = nn.octree_max_pool(x, octree, d)
     self.launches += 2
     return nn.octree_pad(top, octree, d - 1, 0.0)

@@ -333,6 +333,33 @@ Tensor octree_max_pool_pad(Tensor data_in, Tensor octree, int depth) {
   return top;
 }
 
+// OctreeMaxPool of fp32 channel-major data in one pass: {pooled and padded, argmax where asked for}.  Data off a 16-byte
+// boundary, and what the separate operators reject, goes to them.
+vector<Tensor> max_pool_pad_f32(const Tensor& data_in, const Tensor& octree, int depth, bool want_mask) {
+  OctreeRef o = get_octree(octree);
+  TORCH_CHECK(depth > 1, "Depth should be larger than 1");
+  TORCH_CHECK(depth <= o.meta.depth, "octree_max_pool: depth ", depth, " exceeds the octree depth");
+  need_cuda(data_in, "octree_max_pool");
+  c10::cuda::CUDAGuard guard(data_in.device());
+  const Tensor data = data_in.contiguous();
+  DataRef b = get_data(data, "octree_max_pool");
+  TORCH_CHECK(b.dtype == OCNN_F32, "octree_max_pool_pad_f32 takes float32 data");
+  const int top_h = o.meta.nnum[depth - 1];
+  if (!o.cuda || reinterpret_cast<uintptr_t>(data.data_ptr()) % 16 != 0 || b.H != o.meta.nnum[depth] ||
+      b.H != 8 * o.meta.nnum_nempty[depth - 1] || b.C > 65535) {
+    vector<Tensor> pooled = octree_max_pool(data, octree, depth);
+    return {octree_pad(pooled[0], octree, depth - 1, 0.f), pooled[1]};
+  }
+  b.layout = OCNN_CHANNEL_MAJOR;
+  Tensor top = new_data(b.C, top_h, b), mask;
+  if (want_mask) mask = torch::empty({1, b.C, b.H / 8, 1}, data.options().dtype(torch::kInt32));
+  OCNN_CALL(ocnn_octree_max_pool_pad_f32(data.data_ptr<float>(), top.data_ptr<float>(),
+                                         want_mask ? mask.data_ptr<int32_t>() : nullptr,
+                                         level_ptr(o, OCNN_PROP_CHILD, depth - 1, "octree_max_pool"), b.C, b.H, top_h,
+                                         current_stream()));
+  return {top, mask};
+}
+
 ocnn_conv_epilogue make_epilogue(const c10::optional<Tensor>& scale, const c10::optional<Tensor>& bias,
                                  const c10::optional<Tensor>& residual, bool relu, int cout,
                                  const Tensor& y);
@@ -1613,10 +1640,10 @@ Tensor train_block(Tensor data, Tensor weight, c10::optional<Tensor> bias, Tenso
 struct TrainPool : public torch::autograd::Function<TrainPool> {
   static Variable forward(AutogradContext* ctx, const Tensor& data, const Tensor& octree, int64_t depth) {
     at::AutoDispatchBelowADInplaceOrView guard;
-    auto pooled = octree_max_pool(data.contiguous(), octree, (int)depth);
+    auto pooled = max_pool_pad_f32(data, octree, (int)depth, true);
     ctx->save_for_backward({pooled[1], octree});
     ctx->saved_data["depth"] = depth;
-    return octree_pad(pooled[0], octree, (int)depth - 1, 0.f);
+    return pooled[0];
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
@@ -2934,6 +2961,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("octree_tile", &octree_tile, "nearest upsampling: depad + repeat each row for its 8 children");
   m.def("cat_channels", &cat_channels, "torch.cat over the channels of two channels_last tensors");
   m.def("octree_max_pool", &octree_max_pool, "octree max pooling");
+  m.def("octree_max_pool_pad_f32", [](const Tensor& data, const Tensor& octree, int depth) {
+    return max_pool_pad_f32(data, octree, depth, false)[0];
+  }, "octree max pooling + pad to depth - 1 (float32, channel-major)");
   m.def("octree_max_pool_pad", &octree_max_pool_pad, "octree max pooling + pad to depth - 1 (bf16 node-major)");
   m.def("points_new", &points_new, "create a point cloud");
   m.def("transform_points", &transform_points, "transform the point cloud");

@@ -123,6 +123,28 @@ def test_pad_depad_pool(ocnn, batch, layout, bf16):
       assert np.array_equal(m, wm)
 
 
+@pytest.mark.parametrize('C', [1, 3, 4, 5, 33])
+@pytest.mark.parametrize('shift', [0, 1])                  # (off a 16-byte boundary the two operators run)
+def test_max_pool_pad_f32_is_the_two_operators(ocnn, batch, C, shift):
+  octree, v = batch[3], batch[4]
+  for d in range(2, 7):
+    h = int(v.nnum[d])
+    x = torch.randn(C * h + shift, device='cuda')[shift:].view(1, C, h, 1)
+    x[0, 0, 3::11], x[0, C - 1, 5::13], x[0, 0, 8:16] = float('nan'), float('inf'), -float('inf')
+    top, mask = ocnn.nn.octree_max_pool(x, octree, d)
+    want = ocnn.nn.octree_pad(top, octree, d - 1, 0.0)
+    with torch.no_grad():
+      got = ocnn.OctreeMaxPool(d)(x, octree)
+    torch.testing.assert_close(got, want, rtol=0, atol=0, equal_nan=True)
+    y = x.clone().requires_grad_()                         # the argmax of the training form, through its gradient
+    out = ocnn.OctreeMaxPool(d)(y, octree)
+    torch.testing.assert_close(out.detach(), want, rtol=0, atol=0, equal_nan=True)
+    g = torch.randn_like(out)
+    grad, = torch.autograd.grad(out, y, g)
+    ref = ocnn.nn.octree_max_unpool(ocnn.nn.octree_depad(g, octree, d - 1), mask, octree, d)
+    assert torch.equal(grad, ref)
+
+
 @pytest.mark.parametrize('C', [8, 32, 40])
 def test_max_pool_pad_fused(ocnn, batch, C):
   """ocnn_octree_max_pool_pad == octree_max_pool followed by octree_pad(0), bit for bit, on every
