@@ -62,11 +62,9 @@ def _stock_conv1x1(conv):
 
 def _train_block(data, weight, bias, bn, residual, octree, kind, depth, cout, kernel_size, stride, nempty, relu):
   own, stats = bn._parameters, bn._buffers       # (Module's own look-up costs 0.4 us a name)
-  if stats['num_batches_tracked'] is not None:
-    stats['num_batches_tracked'].add_(1)
   return nn.train_block(data, weight, bias, own['weight'], own['bias'], residual, stats['running_mean'],
                         stats['running_var'], bn.momentum, bn.eps, octree, kind, depth, cout, kernel_size, stride,
-                        nempty, relu)
+                        nempty, relu, stats['num_batches_tracked'])
 
 
 def _folded(bn):

@@ -1463,8 +1463,9 @@ Tensor global_pool_fc(Tensor data_in, Tensor weights, c10::optional<Tensor> bias
 // ---- training blocks ----------------------------------------------------------------------------------
 // The autograd forms of a block as one node each: (de)convolution or 1x1 layer + BatchNorm (batch
 // statistics) + residual + ReLU, and pool + pad.  The arithmetic is that of the separate modules, call
-// by call (torch's BatchNorm, the same convolution kernels), so results are bit-identical; what goes
-// away is host time: six autograd nodes, two of them in Python, and the modules around them were about
+// by call (torch's BatchNorm, the same convolution kernels), so results are bit-identical (but for the last bits of a
+// first layer's gradients); what goes away is launches (residual, ReLU and the count of batches are one) and host time:
+// six autograd nodes, two of them in Python, and the modules around them were about
 // 150 us per block and direction, and a training step was bound by them.
 using torch::autograd::AutogradContext;
 using torch::autograd::Variable;
@@ -1509,7 +1510,7 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
                           const Tensor& running_var, double momentum, double eps,
                           const c10::optional<Tensor>& octree, int64_t kind, int64_t depth,
                           int64_t num_output, const vector<int64_t>& kernel_size, int64_t stride, bool nempty,
-                          bool relu) {
+                          bool relu, const c10::optional<Tensor>& num_batches) {
     at::AutoDispatchBelowADInplaceOrView guard;
     const vector<int> ks(kernel_size.begin(), kernel_size.end());
     Tensor z;
@@ -1527,8 +1528,25 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     std::tie(out, save_mean, save_var, reserve, impl) =
         at::_batch_norm_impl_index(z, bn_weight, bn_bias, running_mean, running_var, /*training=*/true, momentum,
                                    eps, at::globalContext().userEnabledCuDNN());
-    if (residual.has_value() && residual->defined()) out = at::add(out, *residual);
-    if (relu) at::relu_(out);
+    const bool has_res = residual.has_value() && residual->defined();
+    const bool counted = num_batches.has_value() && num_batches->defined();
+    const bool own_count = counted && num_batches->is_cuda() && num_batches->scalar_type() == torch::kInt64 &&
+                           num_batches->device() == out.device();
+    if (out.scalar_type() == torch::kFloat32 && out.is_contiguous() &&
+        (!has_res || (residual->sizes() == out.sizes() && residual->scalar_type() == torch::kFloat32 &&
+                      residual->is_contiguous() && residual->device() == out.device()))) {
+      // residual, ReLU and the count of batches in one launch
+      c10::cuda::CUDAGuard device(out.device());
+      OCNN_CALL(ocnn_batch_norm_finish(out.data_ptr<float>(), has_res ? residual->data_ptr<float>() : nullptr,
+                                       out.numel(), relu, own_count ? num_batches->data_ptr<int64_t>() : nullptr,
+                                       current_stream()));
+      if (own_count && !num_batches->is_inference()) num_batches->unsafeGetTensorImpl()->bump_version();
+      if (counted && !own_count) num_batches->add_(1);
+    } else {
+      if (has_res) out = at::add(out, *residual);
+      if (relu) at::relu_(out);
+      if (counted) num_batches->add_(1);
+    }
     ctx->save_for_backward({data, weight, z, bn_weight, save_mean, save_var, reserve, relu ? out : Tensor(),
                             octree.has_value() ? *octree : Tensor(), running_mean, running_var});
     ctx->saved_data["impl"] = impl;
@@ -1540,7 +1558,7 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     ctx->saved_data["stride"] = stride;
     ctx->saved_data["nempty"] = nempty;
     ctx->saved_data["bias"] = bias.has_value() && bias->defined();
-    ctx->saved_data["residual"] = residual.has_value() && residual->defined();
+    ctx->saved_data["residual"] = has_res;
     return out;
   }
 
@@ -1556,20 +1574,36 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     const bool need_bias = has_bias && ctx->needs_input_grad(at_input);
     at_input += has_bias ? 1 : 0;
     Tensor g = grads[0];
-    if (out.defined()) g = at::threshold_backward(g, out, 0);
-    variable_list res(18);
-    if (has_res) res[5] = g;
-    if (at::GradMode::is_enabled()) {
-      differentiable(ctx, data, weight, bn_weight, octree, g, need_data, need_weight, need_bias, res);
-      return res;
-    }
+    variable_list res(19);
     Tensor gz, gbw, gbb;
-    std::tie(gz, gbw, gbb) = at::_batch_norm_impl_index_backward(
-        ctx->saved_data["impl"].toInt(), z, g, bn_weight, saved[9], saved[10], saved[4], saved[5], /*train=*/true,
-        ctx->saved_data["eps"].toDouble(), {true, true, true}, saved[6]);
+    if (!need_data && !has_res && !at::GradMode::is_enabled() && z.dim() == 4 && z.size(0) == 1 && z.size(3) == 1 &&
+        z.scalar_type() == torch::kFloat32 && z.is_contiguous() && g.scalar_type() == torch::kFloat32 &&
+        (!out.defined() || out.is_contiguous()) && bn_weight.is_contiguous()) {
+      // the gradient ends here: mask and BatchNorm in one launch (see batch_norm.cu for why only here)
+      c10::cuda::CUDAGuard device(z.device());
+      g = g.contiguous();
+      gz = at::empty_like(z);
+      gbw = at::empty({z.size(1)}, z.options());
+      gbb = at::empty_like(gbw);
+      OCNN_CALL(ocnn_batch_norm_backward(z.data_ptr<float>(), g.data_ptr<float>(),
+                                         out.defined() ? out.data_ptr<float>() : nullptr, gz.data_ptr<float>(), nullptr,
+                                         (int)z.size(1), (int)z.size(2), bn_weight.data_ptr<float>(),
+                                         saved[4].data_ptr<float>(), saved[5].data_ptr<float>(), gbw.data_ptr<float>(),
+                                         gbb.data_ptr<float>(), current_stream()));
+    } else {
+      if (out.defined()) g = at::threshold_backward(g, out, 0);
+      if (has_res) res[5] = g;
+      if (at::GradMode::is_enabled()) {
+        differentiable(ctx, data, weight, bn_weight, octree, g, need_data, need_weight, need_bias, res);
+        return res;
+      }
+      std::tie(gz, gbw, gbb) = at::_batch_norm_impl_index_backward(
+          ctx->saved_data["impl"].toInt(), z, g, bn_weight, saved[9], saved[10], saved[4], saved[5], /*train=*/true,
+          ctx->saved_data["eps"].toDouble(), {true, true, true}, saved[6]);
+      gz = gz.contiguous();
+    }
     res[3] = gbw;
     res[4] = gbb;
-    gz = gz.contiguous();
     if (kind == 2) {
       const bool ours = own_pointwise_weight_grad(weight, data);
       if (need_data || need_bias || (need_weight && !ours)) {
@@ -1631,9 +1665,10 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
 Tensor train_block(Tensor data, Tensor weight, c10::optional<Tensor> bias, Tensor bn_weight, Tensor bn_bias,
                    c10::optional<Tensor> residual, Tensor running_mean, Tensor running_var, double momentum,
                    double eps, c10::optional<Tensor> octree, int64_t kind, int64_t depth, int64_t num_output,
-                   vector<int64_t> kernel_size, int64_t stride, bool nempty, bool relu) {
+                   vector<int64_t> kernel_size, int64_t stride, bool nempty, bool relu,
+                   c10::optional<Tensor> num_batches) {
   return TrainBlock::apply(data, weight, bias, bn_weight, bn_bias, residual, running_mean, running_var, momentum, eps,
-                           octree, kind, depth, num_output, kernel_size, stride, nempty, relu);
+                           octree, kind, depth, num_output, kernel_size, stride, nempty, relu, num_batches);
 }
 
 // OctreeMaxPool: pool level `depth`, pad to every node of the level above.
