@@ -1682,7 +1682,13 @@ Tensor train_block(Tensor data, Tensor weight, c10::optional<Tensor> bias, Tenso
 struct TrainPool : public torch::autograd::Function<TrainPool> {
   static Variable forward(AutogradContext* ctx, const Tensor& data, const Tensor& octree, int64_t depth) {
     at::AutoDispatchBelowADInplaceOrView guard;
-    auto pooled = max_pool_pad_f32(data, octree, (int)depth, true);
+    vector<Tensor> pooled;
+    if (data.scalar_type() == torch::kFloat32) {
+      pooled = max_pool_pad_f32(data, octree, (int)depth, true);
+    } else {
+      pooled = octree_max_pool(data.contiguous(), octree, (int)depth);
+      pooled[0] = octree_pad(pooled[0], octree, (int)depth - 1, 0.f);
+    }
     ctx->save_for_backward({pooled[1], octree});
     ctx->saved_data["depth"] = depth;
     return pooled[0];

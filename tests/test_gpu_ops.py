@@ -145,6 +145,26 @@ def test_max_pool_pad_f32_is_the_two_operators(ocnn, batch, C, shift):
     assert torch.equal(grad, ref)
 
 
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize('node_major', [False, True])
+def test_train_max_pool_of_16_bit_data(ocnn, batch, dtype, node_major):
+  """The autograd node takes every type that the two operators take."""
+  octree, v = batch[3], batch[4]
+  for d in (6, 2):
+    x = torch.randn(1, 24, int(v.nnum[d]), 1, device='cuda').to(dtype)
+    if node_major:
+      x = x.contiguous(memory_format=torch.channels_last)
+    x.requires_grad_()
+    with torch.no_grad():
+      top, mask = ocnn.nn.octree_max_pool(x.contiguous(), octree, d)
+      want = ocnn.nn.octree_pad(top, octree, d - 1, 0.0)
+    out = ocnn.nn.train_max_pool(x, octree, d)
+    assert out.dtype == dtype and torch.equal(out.detach(), want)
+    g = torch.randn(out.shape, device='cuda').to(dtype)
+    grad, = torch.autograd.grad(out, x, g)
+    assert torch.equal(grad, ocnn.nn.octree_max_unpool(ocnn.nn.octree_depad(g, octree, d - 1), mask, octree, d))
+
+
 @pytest.mark.parametrize('C', [8, 32, 40])
 def test_max_pool_pad_fused(ocnn, batch, C):
   """ocnn_octree_max_pool_pad == octree_max_pool followed by octree_pad(0), bit for bit, on every
