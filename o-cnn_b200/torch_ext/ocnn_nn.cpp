@@ -3094,7 +3094,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("tc_status", [](py::object device) {
     return tc_status(torch::python::detail::py_object_to_device(device));
   });
-  m.def("train_block", &train_block);
+  m.def("train_block", &train_block, py::arg("data"), py::arg("weight"), py::arg("bias"), py::arg("bn_weight"),
+        py::arg("bn_bias"), py::arg("residual"), py::arg("running_mean"), py::arg("running_var"), py::arg("momentum"),
+        py::arg("eps"), py::arg("octree"), py::arg("kind"), py::arg("depth"), py::arg("num_output"),
+        py::arg("kernel_size"), py::arg("stride"), py::arg("nempty"), py::arg("relu"), py::arg("num_batches") = py::none());
   m.def("train_max_pool", &train_max_pool);
   m.def("octree_info", &octree_info);
   // (pytorch/cpp/pybind.cpp:35-41)

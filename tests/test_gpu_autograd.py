@@ -130,3 +130,14 @@ def test_first_derivatives_of_an_octree_block_under_create_graph(ocnn, deconv):
     gw, = torch.autograd.grad(b(x, octree, residual=res), b.bn.weight, g, create_graph=True)
     second.append(torch.autograd.grad(gw.pow(2).sum(), g)[0])
   close(second[0], second[1])
+
+
+def test_a_block_is_called_without_a_count_of_batches(ocnn):
+  """The native block's count is an optional last argument: left out, the rest is as with it."""
+  block = make(ocnn, 'bnrelu', 24)
+  conv, bn = block.conv1x1.conv1x1, block.bn
+  x = torch.randn(1, 16, 200, 1, device='cuda')
+  args = lambda: (x, conv.weight, conv.bias, bn.weight, bn.bias, None, torch.zeros(24, device='cuda'),
+                  torch.ones(24, device='cuda'), 0.01, 1e-3, None, 2, 0, 24, [1], 1, False, True)
+  seen = torch.zeros((), dtype=torch.int64, device='cuda')
+  assert torch.equal(ocnn.nn.train_block(*args()), ocnn.nn.train_block(*args(), seen)) and int(seen) == 1
