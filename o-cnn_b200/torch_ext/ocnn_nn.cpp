@@ -1538,7 +1538,7 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     const bool has_res = residual.has_value() && residual->defined();
     const bool counted = num_batches.has_value() && num_batches->defined();
     const bool own_count = counted && num_batches->is_cuda() && num_batches->scalar_type() == torch::kInt64 &&
-                           num_batches->device() == out.device();
+                           num_batches->numel() == 1 && num_batches->device() == out.device();
     if (out.scalar_type() == torch::kFloat32 && out.is_contiguous() &&
         (!has_res || (residual->sizes() == out.sizes() && residual->scalar_type() == torch::kFloat32 &&
                       residual->is_contiguous() && residual->device() == out.device()))) {
@@ -1547,13 +1547,14 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
       OCNN_CALL(ocnn_batch_norm_finish(out.data_ptr<float>(), has_res ? residual->data_ptr<float>() : nullptr,
                                        out.numel(), relu, own_count ? num_batches->data_ptr<int64_t>() : nullptr,
                                        current_stream()));
-      if (own_count && !num_batches->is_inference()) num_batches->unsafeGetTensorImpl()->bump_version();
       if (counted && !own_count) num_batches->add_(1);
     } else {
       if (has_res) out = at::add(out, *residual);
       if (relu) at::relu_(out);
       if (counted) num_batches->add_(1);
     }
+    // (under the guard no operator counts its writes)
+    if (counted && !num_batches->is_inference()) num_batches->unsafeGetTensorImpl()->bump_version();
     ctx->save_for_backward({data, weight, z, bn_weight, save_mean, save_var, reserve, relu ? out : Tensor(),
                             octree.has_value() ? *octree : Tensor(), running_mean, running_var});
     ctx->saved_data["impl"] = impl;

@@ -141,3 +141,20 @@ def test_a_block_is_called_without_a_count_of_batches(ocnn):
                   torch.ones(24, device='cuda'), 0.01, 1e-3, None, 2, 0, 24, [1], 1, False, True)
   seen = torch.zeros((), dtype=torch.int64, device='cuda')
   assert torch.equal(ocnn.nn.train_block(*args()), ocnn.nn.train_block(*args(), seen)) and int(seen) == 1
+
+
+@pytest.mark.parametrize('count', ['gpu', 'cpu', 'int32', 'two'])
+@pytest.mark.parametrize('residual', ['none', 'rows', 'transposed'])       # (the last: added by torch's operator)
+def test_a_block_counts_batches_as_a_write(ocnn, count, residual):
+  """num_batches_tracked goes up by one and so does its version, wherever and however it is held."""
+  block = make(ocnn, 'bnrelu', 24)
+  seen = {'gpu': lambda: torch.tensor(5, device='cuda'), 'cpu': lambda: torch.tensor(5),
+          'int32': lambda: torch.tensor(5, dtype=torch.int32, device='cuda'),
+          'two': lambda: torch.tensor([5, 9], device='cuda')}[count]()
+  block.bn.num_batches_tracked = seen
+  x = torch.randn(1, 16, 200, 1, device='cuda')
+  res = {'none': None, 'rows': torch.randn(1, 24, 200, 1, device='cuda'),
+         'transposed': torch.randn(1, 200, 24, 1, device='cuda').transpose(1, 2)}[residual]
+  want, version = seen + 1, seen._version
+  block(x, residual=res)
+  assert torch.equal(seen, want) and seen._version == version + 1
