@@ -148,7 +148,7 @@ def test_max_pool_pad_f32_is_the_two_operators(ocnn, batch, C, shift):
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize('node_major', [False, True])
 def test_train_max_pool_of_16_bit_data(ocnn, batch, dtype, node_major):
-  """The autograd node takes every type that the two operators take."""
+  """The autograd node's forward takes every type that the two operators take (the gradient is float32's)."""
   octree, v = batch[3], batch[4]
   for d in (6, 2):
     x = torch.randn(1, 24, int(v.nnum[d]), 1, device='cuda').to(dtype)
@@ -156,13 +156,11 @@ def test_train_max_pool_of_16_bit_data(ocnn, batch, dtype, node_major):
       x = x.contiguous(memory_format=torch.channels_last)
     x.requires_grad_()
     with torch.no_grad():
-      top, mask = ocnn.nn.octree_max_pool(x.contiguous(), octree, d)
-      want = ocnn.nn.octree_pad(top, octree, d - 1, 0.0)
+      want = ocnn.nn.octree_pad(ocnn.nn.octree_max_pool(x.contiguous(), octree, d)[0], octree, d - 1, 0.0)
     out = ocnn.nn.train_max_pool(x, octree, d)
     assert out.dtype == dtype and torch.equal(out.detach(), want)
-    g = torch.randn(out.shape, device='cuda').to(dtype)
-    grad, = torch.autograd.grad(out, x, g)
-    assert torch.equal(grad, ocnn.nn.octree_max_unpool(ocnn.nn.octree_depad(g, octree, d - 1), mask, octree, d))
+    with pytest.raises(RuntimeError, match='float32 data only'):
+      out.sum().backward()
 
 
 @pytest.mark.parametrize('C', [8, 32, 40])
