@@ -305,7 +305,10 @@ int ocnn_octree_mask_pool(const float* btm_dev, const int32_t* mask_dev, float* 
 
 /* Tensor-core path: weights packed once per layer into bf16 K-major tiles.  The packed image
  * depends on the kernel shape AND the stride the layer will run with (stride-1 neighbourhood
- * convolutions with few channels use a per-sibling-group formulation with expanded weights). */
+ * convolutions with few channels use a per-sibling-group formulation with expanded weights).  The image of a
+ * 3x3x3 stride-1 layer on non-empty nodes whose cin is a multiple of 16 ends in OCNN_PACKED_FLAG_BYTES (an int32:
+ * whether a weight is not finite) that only ocnn_octree_conv_tc_taps reads; the rest is a multiple of 2048 bytes. */
+#define OCNN_PACKED_FLAG_BYTES 128
 size_t ocnn_conv_packed_weight_bytes_nempty(int cin, int cout, const int kernel_size[3]);
 int ocnn_conv_pack_weights_nempty(const float* weights_dev, void* packed_dev, int cin, int cout,
                                   const int kernel_size[3], void* stream);

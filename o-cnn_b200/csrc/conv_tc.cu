@@ -1550,7 +1550,7 @@ bool takes_taps(const TcShape& s, const LayerKind& kind, int cin) {
 }
 
 size_t image_bytes(const TcShape& s) { return (size_t)s.slices * s.nkb * s.npad * 128; }
-constexpr size_t kFlagBytes = 128;       // behind the image of such a layer: whether a weight is not finite
+constexpr size_t kFlagBytes = OCNN_PACKED_FLAG_BYTES;      // behind the image of such a layer: whether a weight is not finite
 
 size_t packed_bytes_impl(int cin, int cout, const int kernel_size[3], const LayerKind& kind) {
   TcShape s;

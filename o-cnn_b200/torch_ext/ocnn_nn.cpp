@@ -744,6 +744,13 @@ Tensor conv_pack_weights(Tensor weights, int cin, int cout, vector<int> kernel_s
   return packed;
 }
 
+// `packed` as an image of `bytes`, or the same without the flag behind it (an image that was saved before there was one;
+// only layers on a tap plan read it).
+bool is_packed_image(const Tensor& packed, size_t bytes) {
+  const size_t flag = bytes % 2048 == OCNN_PACKED_FLAG_BYTES ? OCNN_PACKED_FLAG_BYTES : 0, n = (size_t)packed.numel();
+  return packed.is_cuda() && packed.scalar_type() == torch::kUInt8 && (n == bytes || n + flag == bytes);
+}
+
 Tensor octree_conv_tc(Tensor data_in, Tensor packed, Tensor octree, int depth, int num_output,
                       vector<int> kernel_size, int stride, c10::optional<Tensor> scale,
                       c10::optional<Tensor> bias, c10::optional<Tensor> residual, bool relu,
@@ -815,8 +822,7 @@ Tensor octree_conv_tc_nempty(Tensor data_in, Tensor packed, Tensor octree, int d
   x.layout = OCNN_NODE_MAJOR;
   const int nne = o.meta.nnum_nempty[depth];
   TORCH_CHECK(x.H == nne, "octree_conv_tc_nempty: data height ", x.H, " != non-empty node number ", nne);
-  TORCH_CHECK(packed.is_cuda() && packed.scalar_type() == torch::kUInt8 &&
-                  (size_t)packed.numel() == ocnn_conv_packed_weight_bytes_nempty(x.C, num_output, ks.data()),
+  TORCH_CHECK(is_packed_image(packed, ocnn_conv_packed_weight_bytes_nempty(x.C, num_output, ks.data())),
               "packed weights do not match this convolution's shape");
   TORCH_CHECK(status.is_cuda() && status.scalar_type() == torch::kInt32 && status.numel() >= 1,
               "status must be an int32 CUDA tensor");
@@ -942,9 +948,8 @@ Tensor octree_conv_tc_general(Tensor data_in, Tensor packed, Tensor octree, int 
               " takes bfloat16 or float16 channels_last data");
   x.layout = OCNN_NODE_MAJOR;
   Geometry geo = make_geometry(o, x, depth, ks, stride, nempty, transposed, what);
-  TORCH_CHECK(packed.is_cuda() && packed.scalar_type() == torch::kUInt8 &&
-                  (size_t)packed.numel() == ocnn_conv_packed_weight_bytes_general(
-                                                x.C, num_output, ks.data(), stride, transposed, nempty),
+  TORCH_CHECK(is_packed_image(packed, ocnn_conv_packed_weight_bytes_general(x.C, num_output, ks.data(), stride,
+                                                                            transposed, nempty)),
               "packed weights do not match this convolution's shape");
   TORCH_CHECK(status.is_cuda() && status.scalar_type() == torch::kInt32 && status.numel() >= 1,
               "status must be an int32 CUDA tensor");

@@ -445,6 +445,24 @@ def test_conv_tensor_core_nempty(ocnn, batch, case):
   assert gu.rel_err(gu.to_np(got), full) < BF16_TOL
 
 
+@pytest.mark.parametrize('cin,cout', [(16, 8), (64, 64), (128, 512)])
+def test_packed_image_without_its_flag(ocnn, batch, cin, cout):
+  """An image of a non-empty 3x3x3 layer that was saved before it ended in a flag still serves the walk over all taps."""
+  _, octree, v = batch
+  x = gu.data_cuda(np.random.default_rng(3).normal(size=(cin, int(v.nnum_nempty[4]))), True, True)
+  packed = ocnn.nn.conv_pack_weights_nempty(torch.randn(cout, cin * 27, device='cuda'), cin, cout, [3, 3, 3])
+  status = torch.zeros(1, dtype=torch.int32, device='cuda')
+  image = packed[:-128].clone()
+  assert image.numel() % 2048 == 0
+  runs = [lambda p: ocnn.nn.octree_conv_tc_nempty(x, p, octree, 4, cout, [3, 3, 3], None, None, None, False, status),
+          lambda p: ocnn.nn.octree_conv_tc_general(x, p, octree, 4, cout, [3, 3, 3], 1, True, False, None, None, None,
+                                                   False, status)]
+  for run in runs:
+    assert torch.equal(run(image), run(packed))
+    with pytest.raises(RuntimeError, match='packed weights'):
+      run(packed[:-256].clone())
+
+
 @pytest.mark.parametrize('half', [False, True], ids=['bf16', 'fp16'])
 @pytest.mark.parametrize('triple', [(8, 32, 8), (16, 64, 16), (16, 32, 8), (8, 16, 8)])
 def test_conv1x1_chain_is_the_two_layers(ocnn, batch, triple, half):
