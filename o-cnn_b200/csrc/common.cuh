@@ -74,7 +74,8 @@ inline int grid_for(long long work, int threads, int blocks_per_sm = 8) {
 // wave: its CTAs do their private set-up (barrier init, TMEM allocation) and then block in
 // grid_dependency_wait() until the predecessor has completed and its writes are visible.  Every
 // kernel launched this way must call grid_dependency_wait() before its first access to global
-// memory, and calls grid_dependency_trigger() first thing so that its own successor can queue up.
+// memory, and calls grid_dependency_trigger() first thing so that its own successor can queue up
+// (a kernel with accumulators in TMEM as soon as it has them: tmem_alloc in tc.cuh).
 __device__ __forceinline__ void grid_dependency_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -102,7 +102,6 @@ __global__ void __launch_bounds__(kF32Threads, NB <= 2 ? 2 : 1) conv_f32_wgrad_k
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  grid_dependency_trigger();
   if (tid == 0) {
     for (int s = 0; s < a.stages; ++s) {
       mbar_init(smem_u32(&full[s]), 128 + 1);
@@ -116,12 +115,7 @@ __global__ void __launch_bounds__(kF32Threads, NB <= 2 ? 2 : 1) conv_f32_wgrad_k
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 8) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_holder)), "r"((uint32_t)a.tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 8) tmem_alloc(tmem_holder, a.tmem_cols);
   grid_dependency_wait();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

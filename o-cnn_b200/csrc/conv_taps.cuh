@@ -73,7 +73,6 @@ __global__ void __launch_bounds__(kTapThreads, 3) conv_taps_kernel(const TapConv
   const int tile = a.plan.tiles - 1 - (int)blockIdx.x;
   const int co_base = blockIdx.y * a.row_elems;
   const uint8_t* wpacked = a.wpacked + (size_t)blockIdx.y * a.nkb * stage_b;
-  grid_dependency_trigger();
   if (tid == 0) {
     for (int s = 0; s < a.stages; ++s) {
       mbar_init(smem_u32(&full[s]), kTapTile + 1);
@@ -89,12 +88,7 @@ __global__ void __launch_bounds__(kTapThreads, 3) conv_taps_kernel(const TapConv
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 4) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)),
-                 "r"((uint32_t)a.tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 4) tmem_alloc(tmem_holder, a.tmem_cols);
   grid_dependency_wait();
   const uint32_t present = a.plan.mask[tile];
   if (warp == 5) {

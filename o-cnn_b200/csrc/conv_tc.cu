@@ -203,7 +203,6 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
   const int kb_first = blockIdx.z * a.kb_per_split;
   const int kb_end = min(a.nkb, kb_first + a.kb_per_split);
   const uint8_t* wpacked = a.wpacked + (size_t)blockIdx.y * a.nkb * (a.npad * 128);
-  grid_dependency_trigger();     // the next layer's CTAs may queue up behind this grid's last wave
 
   if (tid == 0) {
     for (int s = 0; s < a.stages; ++s) {
@@ -214,12 +213,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const TcArgs a) {
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 4) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_holder)), "r"((uint32_t)a.tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 4) tmem_alloc(tmem_holder, a.tmem_cols);
   // everything above is private to the CTA; from here on global memory is read, so the previous
   // kernel of the stream must have completed
   grid_dependency_wait();
@@ -740,7 +734,6 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
   // A layer of one K-block (a 1x1x1 layer on 64 channels) uses the same weight tile for every
   // tile of rows: it is fetched once into slot 0 of the B ring and stays there.
   const bool b_resident = a.nkb == 1;
-  grid_dependency_trigger();
 
   if (tid == 0) {
     for (int s = 0; s < a.stages; ++s) {
@@ -755,12 +748,7 @@ __global__ void __launch_bounds__(32 * (4 * R + 6), 1) conv_tc_persist_kernel(co
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kGatherWarps) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_holder)), "r"((uint32_t)(acc_cols * acc_bufs))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == kGatherWarps) tmem_alloc(tmem_holder, acc_cols * acc_bufs);
   grid_dependency_wait();
   for (int n = tid; n < a.npad; n += kThreadsP) {
     const bool live = n < a.row_elems;

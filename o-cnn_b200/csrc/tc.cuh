@@ -73,6 +73,16 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
                : "memory");
 }
 
+// TMEM for a CTA (by one whole warp); its base goes to *holder.  Only a CTA that has its columns lets the stream's next
+// kernel in: an allocation waits until enough columns of its SM are free, and a CTA of the next kernel that took them first
+// would keep them until this grid has ended, each waiting for the other.
+__device__ __forceinline__ void tmem_alloc(uint32_t* holder, uint32_t columns) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)), "r"(columns)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  grid_dependency_trigger();
+}
+
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),

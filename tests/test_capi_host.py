@@ -50,6 +50,24 @@ def test_exports_every_declared_symbol(lib):
   assert lib.ocnn_compiled_arch() == 100
 
 
+def test_kernels_let_their_successor_in_once_they_hold_tmem():
+  """A kernel launched while its predecessor runs may allocate TMEM; where a CTA of the predecessor had still to do so,
+  each could wait for the other.  So the permission follows the allocation, in tmem_alloc, and is given nowhere else."""
+  csrc = os.path.join(ROOT, 'o-cnn_b200', 'csrc')
+  kernels = 0
+  for name in sorted(os.listdir(csrc)):
+    text = re.sub(r'//.*', '', open(os.path.join(csrc, name)).read())
+    for alloc in re.finditer(r'tcgen05\.alloc\.', text):
+      end = text.index('\n}', alloc.start())
+      assert name == 'tc.cuh' and 'grid_dependency_trigger();' in text[alloc.start():end]
+    for kernel in re.split(r'__global__', text)[1:]:
+      if 'tmem_alloc(' in kernel:
+        kernels += 1
+        body = kernel[:kernel.index('\n}')]
+        assert 'grid_dependency_trigger' not in body and body.index('tmem_alloc(') < body.index('grid_dependency_wait()')
+  assert kernels >= 5
+
+
 def parse(lib, buf):
   m = Meta()
   raw = np.ascontiguousarray(buf, np.uint8).tobytes()
