@@ -395,10 +395,9 @@ int ocnn_tap_plan(const ocnn_tap_level* levels, int count, void* workspace_dev, 
 /* The convolution on a plan: x, y [rows, channels] 16-bit node-major; packed weights as for
  * ocnn_octree_conv_tc_general with nempty, kernel 3x3x3, stride 1; cin a multiple of 16
  * (OCNN_ERR_UNSUPPORTED otherwise). */
-size_t ocnn_octree_conv_tc_taps_workspace_bytes(int rows, int cin, int cout);
 int ocnn_octree_conv_tc_taps(const void* x_dev, const void* packed_dev, void* y_dev, const void* plan_dev,
                              int rows, int cin, int cout, int dtype, const ocnn_conv_epilogue* epilogue,
-                             int32_t* status_dev, void* workspace_dev, size_t workspace_bytes, void* stream);
+                             int32_t* status_dev, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Octree editing for the generative networks.  Replace octree_new / octree_grow / octree_update

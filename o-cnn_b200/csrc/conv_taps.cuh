@@ -33,20 +33,19 @@ struct TapConvArgs {
   const int* nonfinite;
   uint8_t* y;
   TapPlanView plan;
-  int rows, cin, npad, nkb, stages, tmem_cols;
+  int cin, npad, nkb, stages, tmem_cols;
   int row_elems;                         // output columns of a slice
   int y_stride;                          // elements between output rows
   int wide;                              // output and residual rows lie on 32-byte boundaries
   int relu;
   ChannelAffine aff;
   const uint8_t* residual;
-  float* partial;                        // K split: fp32 sums [split][rows][y_stride]
   int* status;
   uint32_t tap_magic;                    // ceil(2^32 / (cin / 8)): a chunk's tap without a division
   __device__ __forceinline__ uint32_t tap_of(uint32_t chunk) const { return __umulhi(chunk, tap_magic); }
 };
 
-// grid: x = tiles, y = 256-column slices, z = parts of K
+// grid: x = tiles, y = 256-column slices
 template <bool HALF>
 __global__ void __launch_bounds__(kTapThreads, 3) conv_taps_kernel(const TapConvArgs a) {
   extern __shared__ uint8_t smem_raw[];
@@ -125,10 +124,7 @@ __global__ void __launch_bounds__(kTapThreads, 3) conv_taps_kernel(const TapConv
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_holder;
-  // this CTA's share of the list
   const int blocks = *s_blocks;
-  const int share = (blocks + (int)gridDim.z - 1) / (int)gridDim.z;
-  const int b0 = min(blocks, (int)blockIdx.z * share), b1 = min(blocks, b0 + share);
   bool alive = true;
 
   if (warp < 4) {
@@ -141,7 +137,7 @@ __global__ void __launch_bounds__(kTapThreads, 3) conv_taps_kernel(const TapConv
     uint32_t pe = 1;
     ZeroRows<8> zeros;
     alive = mbar_wait(smem_u32(table_in), 0, abort_flag, a.status, kErrFullWait);
-    for (int b = b0; b < b1; ++b) {
+    for (int b = 0; b < blocks; ++b) {
       const uint32_t entry = s_list[b];
       // (a chunk whose tap is not walked stays as it is: nobody multiplies it)
       const bool has = (entry >> (8 + (chunk >> 1))) & 1u;
@@ -153,7 +149,7 @@ __global__ void __launch_bounds__(kTapThreads, 3) conv_taps_kernel(const TapConv
         p[0] = lo.x; p[1] = lo.y; p[2] = lo.z; p[3] = lo.w;
         p[4] = hi.x; p[5] = hi.y; p[6] = hi.z; p[7] = hi.w;
       }
-      if (alive && b - b0 >= a.stages)
+      if (alive && b >= a.stages)
         alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrEmptyWait);
       if (alive && has) {
         const uint32_t stage_base = smem_u32(sA + s * kA);
@@ -212,17 +208,6 @@ __global__ void __launch_bounds__(kTapThreads, 3) conv_taps_kernel(const TapConv
         const int n0 = c0 + 16 * part;
         if (n0 >= a.npad || !row_ok || n0 >= a.row_elems) break;
         const uint32_t (&v)[16] = v2[part];
-        if (a.partial != nullptr) {
-          uint32_t* out = reinterpret_cast<uint32_t*>(a.partial) +
-                          ((long long)blockIdx.z * a.rows + row) * a.y_stride + co_base + n0;
-          const uint32_t keep = b0 < b1 ? 0xffffffffu : 0u;        // (no K-block fell to this part: nothing in TMEM)
-#pragma unroll
-          for (int j = 0; j < 16; j += 8)
-            if (n0 + j < a.row_elems)
-              st_global_32B(out + j, make_uint4(v[j] & keep, v[j + 1] & keep, v[j + 2] & keep, v[j + 3] & keep),
-                            make_uint4(v[j + 4] & keep, v[j + 5] & keep, v[j + 6] & keep, v[j + 7] & keep));
-          continue;
-        }
         uint4 ov[2];
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
@@ -271,7 +256,7 @@ __global__ void __launch_bounds__(kTapThreads, 3) conv_taps_kernel(const TapConv
                              ((uint32_t)(kTapTile >> 4) << 24);
       int s = 0;
       uint32_t pf = 0, sum = 0;
-      for (int b = b0; b < b1; ++b) {
+      for (int b = 0; b < blocks; ++b) {
         const uint32_t steps = (uint32_t)s_list[b] >> 8;
         alive = mbar_wait(smem_u32(&full[s]), pf, abort_flag, a.status, kErrFullWait);
         if (!alive) break;
@@ -300,8 +285,8 @@ __global__ void __launch_bounds__(kTapThreads, 3) conv_taps_kernel(const TapConv
     // ---------------- weight tiles: one bulk copy per K-block ----------------
     int s = 0;
     uint32_t pe = 1;
-    for (int b = b0; b < b1; ++b) {
-      if (b - b0 >= a.stages) alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrWeightWait);
+    for (int b = 0; b < blocks; ++b) {
+      if (b >= a.stages) alive = mbar_wait(smem_u32(&empty[s]), pe, abort_flag, a.status, kErrWeightWait);
       if (!alive) break;
       const uint32_t bar = smem_u32(&full[s]);
       mbar_arrive_expect_tx(bar, (uint32_t)stage_b);

@@ -1827,39 +1827,26 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
   return OCNN_OK;
 }
 
-// Launch shape on a tap plan.  Two or three CTAs share an SM where two stages of each fit.  A level of few tiles
-// and a long K splits K over CTAs (a tile of 256 -> 256 still walks 76 of 108 K-blocks at 4.2 k nodes), at least
-// eight blocks of the full list a part.
+// Launch shape on a tap plan.  Two or three CTAs share an SM where two stages of each fit.
 struct TapShape {
-  int stages, splits;
+  int stages;
   size_t smem;
 };
 TapShape tap_shape(const TcShape& s, long long rows) {
   TapShape t;
   const long long tiles = (rows + kTapTile - 1) / kTapTile * s.slices;
-  const int sms = sm_count();
-  t.splits = 1;
-  if (2 * tiles <= sms && s.nkb >= 32 && split_mode() != 0) {
-    const long long want = sms / tiles, most = s.nkb / 8;
-    t.splits = (int)(want < most ? want : most);
-  }
   const size_t stage = (size_t)kTapTile * 128 + (size_t)s.npad * 128;
   const size_t fixed = 1024 + 27 * kTapTile * 4 + (size_t)s.npad * 8 + 256 + 2 * kTapMaxBlocks;
   int st = (int)((75 * 1024 - fixed) / stage);
   if (st < 2 || 3 * s.tmem_cols > 512) st = (int)((113 * 1024 - fixed) / stage);
-  if (st < 2 || tiles * t.splits <= sms) st = (int)((200 * 1024 - fixed) / stage);
+  if (st < 2 || tiles <= sm_count()) st = (int)((200 * 1024 - fixed) / stage);
   t.stages = st > 7 ? 7 : st;            // (three at 256 columns)
   t.smem = fixed + (size_t)t.stages * stage;
   return t;
 }
 
-size_t taps_workspace(const TcShape& s, const TapShape& t, long long rows) {
-  return t.splits > 1 ? (size_t)t.splits * rows * s.cout_eff * 4 : 0;
-}
-
 int conv_taps_impl(const void* x, const void* packed, void* y, const void* plan, int rows, int cin, int cout,
-                   int dtype, const ocnn_conv_epilogue* ep, int32_t* status, void* workspace,
-                   size_t workspace_bytes, cudaStream_t st) {
+                   int dtype, const ocnn_conv_epilogue* ep, int32_t* status, cudaStream_t st) {
   const char* who = "ocnn_octree_conv_tc_taps";
   OCNN_REQUIRE(dtype == OCNN_BF16 || dtype == OCNN_F16, "%s: bf16 or fp16 data only (dtype %d)", who, dtype);
   const int ks[3] = {3, 3, 3};
@@ -1878,24 +1865,21 @@ int conv_taps_impl(const void* x, const void* packed, void* y, const void* plan,
   OCNN_REQUIRE((uintptr_t)residual % 16 == 0, "%s: residual must be 16-byte aligned", who);
   OCNN_REQUIRE((long long)rows * cin * 2 < (1LL << 32), "%s: input tensor of %lld bytes exceeds the 4 GiB this kernel addresses",
                who, (long long)rows * cin * 2);
-  TapShape t = tap_shape(s, rows);
-  OCNN_REQUIRE(taps_workspace(s, t, rows) <= workspace_bytes && (uintptr_t)workspace % 32 == 0,
-               "%s: the workspace needs %zu bytes on a 32-byte boundary", who, taps_workspace(s, t, rows));
+  const TapShape t = tap_shape(s, rows);
   TapConvArgs a = {};
   a.x = static_cast<const uint8_t*>(x);
   a.wpacked = static_cast<const uint8_t*>(packed);
   a.nonfinite = reinterpret_cast<const int*>(a.wpacked + image_bytes(s));
   a.y = static_cast<uint8_t*>(y);
   a.plan = tap_plan_view(plan, rows);
-  a.rows = rows; a.cin = cin; a.npad = s.npad; a.nkb = s.nkb; a.stages = t.stages; a.tmem_cols = s.tmem_cols;
+  a.cin = cin; a.npad = s.npad; a.nkb = s.nkb; a.stages = t.stages; a.tmem_cols = s.tmem_cols;
   a.tap_magic = (uint32_t)(((1ull << 32) + cin / 8 - 1) / (cin / 8));
   a.row_elems = s.slices > 1 ? 256 : s.cout_eff;
   a.y_stride = s.cout_eff;
   a.wide = (a.row_elems % 16 == 0 && (uintptr_t)y % 32 == 0 && (uintptr_t)residual % 32 == 0) ? 1 : 0;
   a.aff = channel_affine_of(ep);
-  a.residual = t.splits > 1 ? nullptr : static_cast<const uint8_t*>(residual);
+  a.residual = static_cast<const uint8_t*>(residual);
   a.relu = epilogue_relu(ep);
-  a.partial = t.splits > 1 ? static_cast<float*>(workspace) : nullptr;
   a.status = status;
   static PerDeviceOnce attr_once;
   int device = 0;
@@ -1912,17 +1896,8 @@ int conv_taps_impl(const void* x, const void* packed, void* y, const void* plan,
       if (known) attr_once.done[device] = true;
     }
   }
-  OCNN_CUDA_OK(launch_chained(table[half ? 1 : 0], dim3(a.plan.tiles, s.slices, t.splits), dim3(kTapThreads), t.smem,
-                              st, a));
+  OCNN_CUDA_OK(launch_chained(table[half ? 1 : 0], dim3(a.plan.tiles, s.slices), dim3(kTapThreads), t.smem, st, a));
   OCNN_LAUNCH_OK("conv_taps_kernel");
-  if (t.splits > 1) {
-    const long long chunks = (long long)rows * a.y_stride / 8;
-    OCNN_CUDA_OK(launch_chained(half ? conv_tc_reduce_kernel<true> : conv_tc_reduce_kernel<false>,
-                                dim3(grid_for(chunks, 256)), dim3(256), 0, st, (const float*)a.partial,
-                                static_cast<uint4*>(y), chunks, t.splits, s.cout_eff, a.aff,
-                                static_cast<const uint4*>(residual), a.relu));
-    OCNN_LAUNCH_OK("conv_tc_reduce_kernel");
-  }
   return OCNN_OK;
 }
 
@@ -1931,19 +1906,9 @@ int conv_taps_impl(const void* x, const void* packed, void* y, const void* plan,
 
 extern "C" {
 
-size_t ocnn_octree_conv_tc_taps_workspace_bytes(int rows, int cin, int cout) {
-  using namespace ocnn;
-  const int ks[3] = {3, 3, 3};
-  TcShape s;
-  if (rows <= 0 || tc_shape(cin, cout, ks, LayerKind{1, false, true}, &s, -1) != OCNN_OK) return 0;
-  return taps_workspace(s, tap_shape(s, rows), rows);
-}
-
 int ocnn_octree_conv_tc_taps(const void* x, const void* packed, void* y, const void* plan, int rows, int cin, int cout,
-                             int dtype, const ocnn_conv_epilogue* ep, int32_t* status, void* workspace,
-                             size_t workspace_bytes, void* stream) {
-  return ocnn::conv_taps_impl(x, packed, y, plan, rows, cin, cout, dtype, ep, status, workspace, workspace_bytes,
-                              static_cast<cudaStream_t>(stream));
+                             int dtype, const ocnn_conv_epilogue* ep, int32_t* status, void* stream) {
+  return ocnn::conv_taps_impl(x, packed, y, plan, rows, cin, cout, dtype, ep, status, static_cast<cudaStream_t>(stream));
 }
 
 size_t ocnn_conv_packed_weight_bytes(int cin, int cout, const int kernel_size[3], int stride) {

@@ -1331,12 +1331,8 @@ class ConvLayer {
         TORCH_CHECK(status.is_cuda() && status.scalar_type() == torch::kInt32 && status.numel() >= 1,
                     "status must be an int32 CUDA tensor");
         if (plan != nullptr) {
-          const size_t bytes = ocnn_octree_conv_tc_taps_workspace_bytes(x.H, cin, cout);
-          Tensor ws;
-          if (bytes > 0) ws = torch::empty({(int64_t)bytes}, torch::dtype(torch::kUInt8).device(y.device()));
           OCNN_CALL(ocnn_octree_conv_tc_taps(x.t.data_ptr(), packed.data_ptr(), y.data_ptr(), plan, x.H, cin, cout,
-                                             x.dtype, &ep, status.data_ptr<int32_t>(),
-                                             bytes > 0 ? ws.data_ptr() : nullptr, bytes, current_stream()));
+                                             x.dtype, &ep, status.data_ptr<int32_t>(), current_stream()));
           return y;
         }
         run_conv_tc(x.t.data_ptr(), packed, y, geo.g, cin, cout, ks_, x.dtype, &ep, status.data_ptr<int32_t>());

@@ -1,5 +1,5 @@
 """Tap plans (`ocnn.nn.TapPlan`): the order and masks against numpy, and the convolution on a plan against the walk
-over all taps, which it equals bit for bit where neither splits K."""
+over all taps, which it equals bit for bit where that one does not split K."""
 import numpy as np
 import pytest
 import torch
