@@ -642,14 +642,13 @@ int ocnn_global_pool_fc(const void* x_dev, const float* w_dev, const float* bias
  * finish: y = relu?(y + residual) in place over `count` values (residual_dev may be NULL), and one more in the
  * int64 at num_batches_dev unless NULL.
  * backward: data [channels][rows], rows > 1; save_mean / save_invstd [channels] of the forward pass; out_dev =
- * the block's output where it ended in a ReLU, else NULL; g = gy where not out <= 0; gx, the gradients of
- * weight and bias, and g itself to g_out_dev unless NULL (the residual's gradient). */
+ * the block's output where it ended in a ReLU, else NULL; g = gy where not out <= 0; gx and the gradients of
+ * weight and bias. */
 int ocnn_batch_norm_finish(float* y_dev, const float* residual_dev, int64_t count, int relu,
                            int64_t* num_batches_dev, void* stream);
 int ocnn_batch_norm_backward(const float* x_dev, const float* gy_dev, const float* out_dev, float* gx_dev,
-                             float* g_out_dev, int channels, int rows, const float* weight_dev,
-                             const float* save_mean_dev, const float* save_invstd_dev, float* g_weight_dev,
-                             float* g_bias_dev, void* stream);
+                             int channels, int rows, const float* weight_dev, const float* save_mean_dev,
+                             const float* save_invstd_dev, float* g_weight_dev, float* g_bias_dev, void* stream);
 
 #ifdef __cplusplus
 }

@@ -5,12 +5,12 @@
 // everywhere the training step of 16 x 10k points was 300 us shorter and its gradients 5e-7 off with TF32 off,
 // but 3e-4 with it on, where any other last bit moves roundings to TF32.
 //
-// What bounds the gradient: memory.  It reads x, gy and the output's sign and writes gx (and the residual's
-// gradient): three to five passes.  A channel's H values are split over a cluster of up to eight CTAs; each CTA
-// keeps x and g of its slice in shared memory between the two sums and the result (of a slice that does
-// not fit the rest is read again, from L2 mostly), the sums travel through distributed shared memory, and so
-// one launch reads every value once.  Sums are formed in 64 bits: their conversions and multiply-adds hide
-// under the loads, and the result is exact to fp32's rounding of its last few operations.
+// What bounds the gradient: memory.  It reads x, gy and the output's sign and writes gx: four passes.  A channel's
+// H values are split over a cluster of up to eight CTAs; each CTA keeps x and g of its slice in shared memory
+// between the two sums and the result (of a slice that does not fit the rest is read again, from L2 mostly), the
+// sums travel through distributed shared memory, and so one launch reads every value once.  Sums are formed in 64
+// bits: their conversions and multiply-adds hide under the loads, and the result is exact to fp32's rounding of its
+// last few operations.
 // 64 channels on depth 5 of 16 x 10k points: cuDNN 142 us and the mask 8, 51 us so.
 #include <cooperative_groups.h>
 
@@ -32,7 +32,6 @@ struct BnArgs {
   const float* mean;
   const float* invstd;
   float* gx;
-  float* g_out;              // gy behind the ReLU (the residual's gradient), or NULL
   float* g_weight;
   float* g_bias;
   int channels, rows, cluster;
@@ -161,7 +160,6 @@ __global__ void __launch_bounds__(kBnThreads) bn_backward_kernel(const BnArgs a)
         store_piece<V>(kept + i * V, p[u]);
         store_piece<V>(kept_g + i * V, g[u]);
       }
-      if (a.g_out != nullptr) store_piece<V>(a.g_out + base + (long long)i * V, g[u]);
     }
   }
   const double2 sum = cluster_sum(sg, sx, warps, &total);
@@ -264,19 +262,19 @@ int ocnn_batch_norm_finish(float* y, const float* residual, int64_t count, int r
   return OCNN_OK;
 }
 
-int ocnn_batch_norm_backward(const float* x, const float* gy, const float* out, float* gx, float* g_out,
-                             int channels, int rows, const float* weight, const float* save_mean,
-                             const float* save_invstd, float* g_weight, float* g_bias, void* stream) {
+int ocnn_batch_norm_backward(const float* x, const float* gy, const float* out, float* gx, int channels, int rows,
+                             const float* weight, const float* save_mean, const float* save_invstd, float* g_weight,
+                             float* g_bias, void* stream) {
   using namespace ocnn;
   OCNN_REQUIRE(channels > 0 && channels < (1 << 28) && rows > 1,
                "ocnn_batch_norm_backward: channels (%d) and more than one row (%d)", channels, rows);
   OCNN_REQUIRE(x && gy && gx && weight && save_mean && save_invstd && g_weight && g_bias,
                "ocnn_batch_norm_backward: null pointer");
   BnArgs a = {};
-  a.x = x; a.gy = gy; a.out = out; a.gx = gx; a.g_out = g_out; a.weight = weight;
+  a.x = x; a.gy = gy; a.out = out; a.gx = gx; a.weight = weight;
   a.mean = save_mean; a.invstd = save_invstd; a.g_weight = g_weight; a.g_bias = g_bias;
   a.channels = channels; a.rows = rows;
-  const bool vec = rows % 4 == 0 && aligned16(x) && aligned16(gy) && aligned16(out) && aligned16(gx) && aligned16(g_out);
+  const bool vec = rows % 4 == 0 && aligned16(x) && aligned16(gy) && aligned16(out) && aligned16(gx);
   return bn_backward(a, vec, static_cast<cudaStream_t>(stream));
 }
 

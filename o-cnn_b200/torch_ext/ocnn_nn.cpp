@@ -1595,7 +1595,7 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
       gbw = at::empty({z.size(1)}, z.options());
       gbb = at::empty_like(gbw);
       OCNN_CALL(ocnn_batch_norm_backward(z.data_ptr<float>(), g.data_ptr<float>(),
-                                         out.defined() ? out.data_ptr<float>() : nullptr, gz.data_ptr<float>(), nullptr,
+                                         out.defined() ? out.data_ptr<float>() : nullptr, gz.data_ptr<float>(),
                                          (int)z.size(1), (int)z.size(2), bn_weight.data_ptr<float>(),
                                          saved[4].data_ptr<float>(), saved[5].data_ptr<float>(), gbw.data_ptr<float>(),
                                          gbb.data_ptr<float>(), current_stream()));

@@ -28,8 +28,8 @@ def placed(t, shift):
 @pytest.mark.parametrize('channels,rows,shift', [
     (1, 2, 0), (3, 5, 0), (7, 1024, 1), (64, 4095, 0), (5, 4096, 0), (33, 16388, 2), (2, 40001, 0), (300, 8200, 0),
     (2, 500000, 0)])                       # the last: more than eight CTAs' shared memory holds
-@pytest.mark.parametrize('relu,with_res', [(False, False), (True, True), (True, False)])
-def test_gradient_against_64_bits(channels, rows, shift, relu, with_res):
+@pytest.mark.parametrize('relu', [False, True])
+def test_gradient_against_64_bits(channels, rows, shift, relu):
   gen = torch.Generator('cuda').manual_seed(rows + channels)
   rand = lambda *s: torch.randn(*s, device='cuda', generator=gen)
   x = placed(rand(channels, rows) + 30 * rand(channels, 1), shift)
@@ -42,10 +42,7 @@ def test_gradient_against_64_bits(channels, rows, shift, relu, with_res):
   want = (g64 - g64.mean(1, keepdim=True) - xhat * (g64 * xhat).mean(1, keepdim=True)) * \
       (w.double() * invstd.double())[:, None]
   gx, gw, gb = placed(torch.empty_like(x), shift), torch.empty_like(w), torch.empty_like(w)
-  g_out = placed(torch.empty_like(x), shift) if with_res else None
-  call('ocnn_batch_norm_backward', x, gy, out, gx, g_out, channels, rows, w, mean, invstd, gw, gb)
-  if g_out is not None:
-    assert torch.equal(g_out.double(), g64)
+  call('ocnn_batch_norm_backward', x, gy, out, gx, channels, rows, w, mean, invstd, gw, gb)
   # five operations, each rounded once, on terms no larger than |g| + |mean| + |xhat * mean(g xhat)|
   terms = g64.abs() + g64.mean(1, keepdim=True).abs() + (xhat * (g64 * xhat).mean(1, keepdim=True)).abs()
   assert bool(((gx.double() - want).abs() <= 8 * EPS32 * terms * (w.double() * invstd.double()).abs()[:, None]).all())
