@@ -3116,6 +3116,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   py::class_<TapPlan>(m, "TapPlan")
       .def(py::init<Tensor, const vector<int>&, bool>(), py::arg("octree"), py::arg("depths"),
            py::arg("worthwhile") = false)
+      .def("serves", [](const TapPlan& p, const Tensor& octree, int depth, int rows) {
+        return p.find(octree, depth, rows) != nullptr;
+      }, "whether a layer on `rows` nodes of this level of this octree would run on the plan now (for tests)")
       .def("level", &TapPlan::level);
   py::class_<ConvLayer>(m, "ConvLayer")
       .def(py::init<int, int, vector<int>, int, bool, bool, bool>(), py::arg("cin"), py::arg("cout"),

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import gpu_util as gu
+from ocnn_harness import synth
 from oracle import oracle as oc
 
 pytestmark = pytest.mark.gpu
@@ -131,3 +132,99 @@ def test_a_plan_serves_only_what_it_was_made_for(ocnn, small):
     assert torch.equal(got, want)
     planned.copy_(small[0])                # written to since
     assert torch.equal(layer(x, planned), want)
+
+
+# ---- the network on its plans --------------------------------------------------------------------------------
+@pytest.fixture(scope='module')
+def scene(ocnn):
+  """An octree whose levels 9 to 7 have more tiles than SMs and go on a plan, and whose levels 6 and 5 do not."""
+  xyz, nrm, rgb = (torch.from_numpy(t) for t in synth.indoor_scene(120000, 11))
+  octree = ocnn.Points2Octree(9, 2).batch([ocnn.points_new(xyz, nrm, rgb, torch.zeros(0))])
+  rows = {d: int((ocnn.octree_property(octree, 'child', d) >= 0).sum()) for d in range(5, 10)}
+  one_wave = 128 * torch.cuda.get_device_properties(0).multi_processor_count
+  planned = {d for d in rows if rows[d] > one_wave}
+  assert planned and set(rows) - planned and max(rows.values()) > 2 * one_wave, rows
+  pts = torch.cat([xyz[:5000], torch.zeros(5000, 1)], 1).cuda()
+  return octree, rows, planned, pts
+
+
+def make_unet(ocnn, seed):
+  torch.manual_seed(seed)
+  net = ocnn.UNet(9, 8, 20, nempty=True).cuda()
+  with torch.no_grad():
+    for m in net.modules():
+      if isinstance(m, (torch.nn.BatchNorm1d, torch.nn.BatchNorm2d)):
+        m.weight.uniform_(0.5, 1.5), m.bias.uniform_(-0.2, 0.2)
+        m.running_mean.uniform_(-0.2, 0.2), m.running_var.uniform_(0.5, 1.5)
+  return net.eval()
+
+
+def node_data(octree, ocnn, dtype):
+  half = dtype == torch.float16
+  return ocnn.octree_depad(ocnn.nn.feature_node_major(octree, 8, not half, half), octree, 9)
+
+
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
+def test_network_on_plans_is_the_network_without(ocnn, scene, dtype, monkeypatch):
+  """`UNet.forward` with the plans it makes: every 3x3x3 layer of a larger level runs on one and the others do not, down
+  and up again, and the scores are those of the walk over all taps bit for bit."""
+  octree, rows, planned, pts = scene
+  net, data = make_unet(ocnn, 5), node_data(octree, ocnn, dtype)
+  base, make, seen = ocnn.OctreeConv.__base__, ocnn.unet._with_tap_plan, []
+  run = base._run
+
+  def spy(layer, x, o, *args):
+    plan = getattr(o, 'tap_plan', None)
+    seen.append((layer, x.shape[2], plan is not None and plan.serves(o, layer.depth, x.shape[2])))
+    return run(layer, x, o, *args)
+
+  with torch.no_grad():
+    monkeypatch.setattr(ocnn.unet, '_with_tap_plan', lambda o, depths, x: o)
+    want, want_nodes = net(octree, pts, data), net(octree, None, data)
+    monkeypatch.setattr(ocnn.unet, '_with_tap_plan', make)
+    monkeypatch.setattr(base, '_run', spy)
+    got = net(octree, pts, data)
+    assert torch.equal(got, want)
+    assert torch.equal(net(octree, None, data), want_nodes)
+  layers = [(m.depth, n, on) for m, n, on in seen if type(m) is ocnn.OctreeConv and m.kernel_size == [3, 3, 3]]
+  assert len(layers) == 2 * 47               # (conv1, and two layers of each of 15 + 8 residual blocks)
+  for depth, n, on in layers:
+    assert n == rows[depth] and on == (depth in planned)
+  assert not hasattr(octree, 'tap_plan')
+  assert int(ocnn.tc_status(octree.device).item()) == 0
+
+
+def test_plans_end_with_the_pass(ocnn, scene):
+  octree, _, _, pts = scene
+  net, data = make_unet(ocnn, 6), node_data(octree, ocnn, torch.bfloat16)
+  with torch.no_grad():
+    net(octree, pts, data)                   # (weights packed, tables of the octree made)
+    before = torch.cuda.memory_allocated()
+    scores = net(octree, pts, data)
+    size = scores.untyped_storage().nbytes()
+    assert torch.cuda.memory_allocated() - before <= (size + 511) // 512 * 512
+
+
+def test_a_graph_of_the_whole_pass(ocnn, scene):
+  """Plans made under capture belong to the graph: a replay on other data makes them anew."""
+  octree, _, _, pts = scene
+  net, data = make_unet(ocnn, 7), node_data(octree, ocnn, torch.bfloat16)
+  other = torch.randn_like(data)
+  with torch.no_grad():
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+      want = [net(octree, pts, x) for x in (data, other)]
+    torch.cuda.current_stream().wait_stream(side)
+    x = data.clone(memory_format=torch.preserve_format)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+      scores = net(octree, pts, x)
+    junk = torch.full((1 << 26,), 255, dtype=torch.uint8, device='cuda')     # (memory between the replays)
+    for source, expected in zip((data, other, data), (want[0], want[1], want[0])):
+      x.copy_(source)
+      junk.fill_(255)
+      graph.replay()
+      assert torch.equal(scores, expected)
+  torch.cuda.synchronize()
+  del graph
