@@ -207,17 +207,12 @@ int bn_backward(BnArgs a, bool vec, cudaStream_t st) {
   typedef void (*Fn)(const BnArgs);
   static const Fn table[2] = {bn_backward_kernel<1>, bn_backward_kernel<4>};
   static PerDeviceOnce attr_once;
-  int device = 0;
-  OCNN_CUDA_OK(cudaGetDevice(&device));
-  {
-    std::lock_guard<std::mutex> lock(attr_once.mutex);
-    const bool known = device >= 0 && device < 64;
-    if (!known || !attr_once.done[device]) {
-      for (Fn f : table)
-        OCNN_CUDA_OK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBnSmem));
-      if (known) attr_once.done[device] = true;
-    }
-  }
+  const int limits = attr_once.run([&]() -> int {
+    for (Fn f : table)
+      OCNN_CUDA_OK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBnSmem));
+    return OCNN_OK;
+  });
+  if (limits != OCNN_OK) return limits;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)cluster * a.channels);
   cfg.blockDim = dim3(kBnThreads);

@@ -1252,17 +1252,12 @@ int small_build(const EncodeArgs& ea, const Layout& L, uint8_t* ws, int* host_co
   const int passes = (3 * L.depth + 7) / 8;
   uint32_t* idx = reinterpret_cast<uint32_t*>(ws + L.off_idx[L.passes & 1]);      // where the emit looks for it
   static PerDeviceOnce attr_once;
-  int device = 0;
-  OCNN_CUDA_OK(cudaGetDevice(&device));
-  {
-    std::lock_guard<std::mutex> lock(attr_once.mutex);
-    const bool known = device >= 0 && device < 64;
-    if (!known || !attr_once.done[device]) {
-      OCNN_CUDA_OK(cudaFuncSetAttribute(small_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)small_smem(kSmallPoints)));
-      if (known) attr_once.done[device] = true;
-    }
-  }
+  const int limits = attr_once.run([&]() -> int {
+    OCNN_CUDA_OK(cudaFuncSetAttribute(small_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)small_smem(kSmallPoints)));
+    return OCNN_OK;
+  });
+  if (limits != OCNN_OK) return limits;
   OCNN_CUDA_OK(launch_chained(small_build_kernel, dim3(1), dim3(kSmallThreads), small_smem(L.n), st, ea, u, idx, passes));
   OCNN_LAUNCH_OK("small_build_kernel");
   return OCNN_OK;

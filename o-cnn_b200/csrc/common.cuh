@@ -51,10 +51,23 @@ constexpr int kSMs = 148;  // B200: 2 dies x 74 SMs (compile-time sizing of fixe
 // fails); grid-size decisions taken at launch time use this.
 int sm_count();
 
-// "Done once per device" flags for per-function attributes (cudaFuncSetAttribute is per device).
+// What is set once per function and device (cudaFuncSetAttribute): `set` (which returns a status) runs under the lock,
+// on a device for the first time or again where it failed.
 struct PerDeviceOnce {
   std::mutex mutex;
   bool done[64] = {};
+
+  template <typename Set>
+  int run(Set set) {
+    int device = 0;
+    OCNN_CUDA_OK(cudaGetDevice(&device));
+    std::lock_guard<std::mutex> lock(mutex);
+    const bool known = device >= 0 && device < 64;
+    if (known && done[device]) return OCNN_OK;
+    const int status = set();
+    if (known && status == OCNN_OK) done[device] = true;
+    return status;
+  }
 };
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }

@@ -573,17 +573,12 @@ extern "C" int ocnn_octree_conv_f32(const float* x, const float* w, float* y, co
   static const KernelFn table[8] = {conv_f32_kernel<1>, conv_f32_kernel<2>, conv_f32_kernel<3>, conv_f32_kernel<4>,
                                     conv_f32_kernel<5>, conv_f32_kernel<6>, conv_f32_kernel<7>, conv_f32_kernel<8>};
   static PerDeviceOnce attr_once;
-  int device = 0;
-  OCNN_CUDA_OK(cudaGetDevice(&device));
-  {
-    std::lock_guard<std::mutex> lock(attr_once.mutex);
-    const bool known = device >= 0 && device < 64;
-    if (!known || !attr_once.done[device]) {
-      for (int k = 0; k < 8; ++k)
-        OCNN_CUDA_OK(cudaFuncSetAttribute(table[k], cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
-      if (known) attr_once.done[device] = true;
-    }
-  }
+  const int limits = attr_once.run([&]() -> int {
+    for (int k = 0; k < 8; ++k)
+      OCNN_CUDA_OK(cudaFuncSetAttribute(table[k], cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
+    return OCNN_OK;
+  });
+  if (limits != OCNN_OK) return limits;
   OCNN_CUDA_OK(launch_chained(table[s.npad / 16 - 1], dim3(s.ctas), dim3(kF32Threads), s.smem, st, a));
   OCNN_LAUNCH_OK("conv_f32_kernel");
   if (s.splits > 1) {

@@ -472,17 +472,12 @@ extern "C" int ocnn_octree_conv_weight_grad_f32(const float* a, const float* x, 
   static const KernelFn table[4] = {conv_f32_wgrad_kernel<1>, conv_f32_wgrad_kernel<2>, conv_f32_wgrad_kernel<3>,
                                     conv_f32_wgrad_kernel<4>};
   static PerDeviceOnce attr_once;
-  int device = 0;
-  OCNN_CUDA_OK(cudaGetDevice(&device));
-  {
-    std::lock_guard<std::mutex> lock(attr_once.mutex);
-    const bool known = device >= 0 && device < 64;
-    if (!known || !attr_once.done[device]) {
-      for (int k = 0; k < 4; ++k)
-        OCNN_CUDA_OK(cudaFuncSetAttribute(table[k], cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
-      if (known) attr_once.done[device] = true;
-    }
-  }
+  const int limits = attr_once.run([&]() -> int {
+    for (int k = 0; k < 4; ++k)
+      OCNN_CUDA_OK(cudaFuncSetAttribute(table[k], cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
+    return OCNN_OK;
+  });
+  if (limits != OCNN_OK) return limits;
   OCNN_CUDA_OK(launch_chained(table[s.npad / 32 - 1], dim3(s.ctas), dim3(kF32Threads), s.smem, st, w));
   OCNN_LAUNCH_OK("conv_f32_wgrad_kernel");
   OCNN_CUDA_OK(launch_chained(conv_f32_wgrad_reduce_kernel, dim3(grid_for((long long)s.groups * 4 * m_channels, 1)),

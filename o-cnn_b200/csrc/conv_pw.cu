@@ -194,16 +194,13 @@ template <int CIN, int COUT, int ROWS, bool HALF>
 int launch_pw_t(const PwArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)a.cin * COUT * sizeof(float);
   static PerDeviceOnce attr_once;      // one per template instance
-  int device = 0;
-  OCNN_CUDA_OK(cudaGetDevice(&device));
   if (smem > 48 * 1024) {
-    std::lock_guard<std::mutex> lock(attr_once.mutex);
-    const bool known = device >= 0 && device < 64;
-    if (!known || !attr_once.done[device]) {
+    const int rc = attr_once.run([]() -> int {
       OCNN_CUDA_OK(cudaFuncSetAttribute(conv_pw_kernel<CIN, COUT, ROWS, HALF>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-      if (known) attr_once.done[device] = true;
-    }
+      return OCNN_OK;
+    });
+    if (rc != OCNN_OK) return rc;
   }
   const int grid = grid_for(((long long)a.h + ROWS - 1) / ROWS, 256, 4);
   OCNN_CUDA_OK(launch_chained(conv_pw_kernel<CIN, COUT, ROWS, HALF>, dim3(grid), dim3(256), smem, st, a));

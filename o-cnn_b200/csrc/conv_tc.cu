@@ -1707,8 +1707,6 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
   }
   // raising the dynamic shared memory limit is per function and per device
   static PerDeviceOnce attr_once;
-  int device = 0;
-  OCNN_CUDA_OK(cudaGetDevice(&device));
   typedef void (*KernelFn)(const TcArgs);
   static const KernelFn table[2][8] = {
       {conv_tc_kernel<0, false, false>, conv_tc_kernel<1, false, false>, conv_tc_kernel<2, false, false>,
@@ -1745,26 +1743,23 @@ int conv_tc_impl(const void* x, const void* packed, void* y, const ocnn_conv_geo
   const bool needs_general = a.up || a.expand_cout > 0;
   if (x2 != nullptr) slot = 0;             // the variant with run-time channel counts
   KernelFn kernel = needs_general ? general[a.f16] : table[a.f16][slot];
-  {
-    std::lock_guard<std::mutex> lock(attr_once.mutex);
-    const bool known = device >= 0 && device < 64;
-    if (!known || !attr_once.done[device]) {
-      for (int h = 0; h < 2; ++h) {
-        for (int k = 0; k < 8; ++k)
-          OCNN_CUDA_OK(cudaFuncSetAttribute(table[h][k], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            220 * 1024));
-        for (int k = 0; k < 5; ++k)
-          OCNN_CUDA_OK(cudaFuncSetAttribute(persist[h][k], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            227 * 1024));
-        OCNN_CUDA_OK(cudaFuncSetAttribute(general[h], cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const int limits = attr_once.run([&]() -> int {
+    for (int h = 0; h < 2; ++h) {
+      for (int k = 0; k < 8; ++k)
+        OCNN_CUDA_OK(cudaFuncSetAttribute(table[h][k], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           220 * 1024));
-        for (int k = 0; k < 2; ++k)
-          OCNN_CUDA_OK(cudaFuncSetAttribute(persist_group[h][k],
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-      }
-      if (known) attr_once.done[device] = true;
+      for (int k = 0; k < 5; ++k)
+        OCNN_CUDA_OK(cudaFuncSetAttribute(persist[h][k], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          227 * 1024));
+      OCNN_CUDA_OK(cudaFuncSetAttribute(general[h], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        220 * 1024));
+      for (int k = 0; k < 2; ++k)
+        OCNN_CUDA_OK(cudaFuncSetAttribute(persist_group[h][k],
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     }
-  }
+    return OCNN_OK;
+  });
+  if (limits != OCNN_OK) return limits;
   OCNN_REQUIRE(x2 != nullptr || (long long)h_in * cin * 2 < (1LL << 32),
                "%s: input tensor of %lld bytes exceeds the 4 GiB this kernel addresses", who,
                (long long)h_in * cin * 2);
@@ -1882,20 +1877,15 @@ int conv_taps_impl(const void* x, const void* packed, void* y, const void* plan,
   a.relu = epilogue_relu(ep);
   a.status = status;
   static PerDeviceOnce attr_once;
-  int device = 0;
-  OCNN_CUDA_OK(cudaGetDevice(&device));
   const bool half = dtype == OCNN_F16;
   typedef void (*Fn)(const TapConvArgs);
   static const Fn table[2] = {conv_taps_kernel<false>, conv_taps_kernel<true>};
-  {
-    std::lock_guard<std::mutex> lock(attr_once.mutex);
-    const bool known = device >= 0 && device < 64;
-    if (!known || !attr_once.done[device]) {
-      for (Fn f : table)
-        OCNN_CUDA_OK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-      if (known) attr_once.done[device] = true;
-    }
-  }
+  const int limits = attr_once.run([&]() -> int {
+    for (Fn f : table)
+      OCNN_CUDA_OK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    return OCNN_OK;
+  });
+  if (limits != OCNN_OK) return limits;
   OCNN_CUDA_OK(launch_chained(table[half ? 1 : 0], dim3(a.plan.tiles, s.slices), dim3(kTapThreads), t.smem, st, a));
   OCNN_LAUNCH_OK("conv_taps_kernel");
   return OCNN_OK;

@@ -371,16 +371,11 @@ int ocnn_tap_plan(const ocnn_tap_level* levels, int count, void* workspace, size
   a.key2 = reinterpret_cast<uint32_t*>(a.node + w.slots);
   a.node2 = reinterpret_cast<int*>(a.key2 + w.slots);
   static PerDeviceOnce attr_once;
-  int device = 0;
-  OCNN_CUDA_OK(cudaGetDevice(&device));
-  {
-    std::lock_guard<std::mutex> lock(attr_once.mutex);
-    const bool known = device >= 0 && device < 64;
-    if (!known || !attr_once.done[device]) {
-      OCNN_CUDA_OK(cudaFuncSetAttribute(tap_bin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kBins));
-      if (known) attr_once.done[device] = true;
-    }
-  }
+  const int limits = attr_once.run([&]() -> int {
+    OCNN_CUDA_OK(cudaFuncSetAttribute(tap_bin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kBins));
+    return OCNN_OK;
+  });
+  if (limits != OCNN_OK) return limits;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   OCNN_CUDA_OK(cudaMemsetAsync(workspace, 0, (size_t)count * kBins * 8, st));
   OCNN_CUDA_OK(launch_chained(tap_key_kernel, dim3(key_blocks), dim3(kKeyThreads), 0, st, a));
