@@ -1540,7 +1540,7 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     const bool counted = num_batches.has_value() && num_batches->defined();
     const bool own_count = counted && num_batches->is_cuda() && num_batches->scalar_type() == torch::kInt64 &&
                            num_batches->numel() == 1 && num_batches->device() == out.device();
-    if (out.scalar_type() == torch::kFloat32 && out.is_contiguous() &&
+    if (out.is_cuda() && out.scalar_type() == torch::kFloat32 && out.is_contiguous() &&
         (!has_res || (residual->sizes() == out.sizes() && residual->scalar_type() == torch::kFloat32 &&
                       residual->is_contiguous() && residual->device() == out.device()))) {
       // residual, ReLU and the count of batches in one launch
@@ -1585,8 +1585,8 @@ struct TrainBlock : public torch::autograd::Function<TrainBlock> {
     Tensor g = grads[0];
     variable_list res(19);
     Tensor gz, gbw, gbb;
-    if (!need_data && !has_res && !at::GradMode::is_enabled() && z.dim() == 4 && z.size(0) == 1 && z.size(3) == 1 &&
-        z.scalar_type() == torch::kFloat32 && z.is_contiguous() && g.scalar_type() == torch::kFloat32 &&
+    if (z.is_cuda() && !need_data && !has_res && !at::GradMode::is_enabled() && z.dim() == 4 && z.size(0) == 1 &&
+        z.size(3) == 1 && z.scalar_type() == torch::kFloat32 && z.is_contiguous() && g.scalar_type() == torch::kFloat32 &&
         (!out.defined() || out.is_contiguous()) && bn_weight.is_contiguous()) {
       // the gradient ends here: mask and BatchNorm in one launch (see batch_norm.cu for why only here)
       c10::cuda::CUDAGuard device(z.device());
