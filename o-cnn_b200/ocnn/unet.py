@@ -24,8 +24,10 @@ def _cat(skip, up):
 
 def _with_tap_plan(octree, depths, data):
   """The octree as one forward pass's layers are given it: a view that carries the tap plans of the levels that
-  they share (16-bit layers on the non-empty nodes).  It ends with the pass, and the plans with it."""
-  if not (octree.is_cuda and data.is_cuda and data.dtype in (torch.bfloat16, torch.float16)):
+  they share (16-bit layers on the non-empty nodes, whose data is node-major: a plan serves no others).  It ends with
+  the pass, and the plans with it."""
+  if not (octree.is_cuda and data.is_cuda and data.dtype in (torch.bfloat16, torch.float16) and
+          data.is_contiguous(memory_format=torch.channels_last)):
     return octree
   view = octree.view(-1)
   view.tap_plan = nn.TapPlan(octree, depths, worthwhile=True)

@@ -194,6 +194,15 @@ def test_network_on_plans_is_the_network_without(ocnn, scene, dtype, monkeypatch
   assert int(ocnn.tc_status(octree.device).item()) == 0
 
 
+def test_no_plan_that_no_layer_takes(ocnn, scene):
+  """Plans serve node-major 16-bit data: for other data none is made."""
+  octree, data = scene[0], node_data(scene[0], ocnn, torch.bfloat16)
+  view = lambda x: ocnn.unet._with_tap_plan(octree, range(5, 10), x)
+  assert view(data).tap_plan.serves(octree, 9, data.shape[2])
+  for other in (data.contiguous(), data.float(), data.cpu()):
+    assert view(other) is octree
+
+
 def test_plans_end_with_the_pass(ocnn, scene):
   octree, _, _, pts = scene
   net, data = make_unet(ocnn, 6), node_data(octree, ocnn, torch.bfloat16)
