@@ -72,7 +72,16 @@ def test_plan_of_all_levels(ocnn, small, large):
   assert sets.sum(1).mean() <= tile_taps < 17                 # (in Morton order it is 27)
 
 
+def wipe_neighbours(octree, d):
+  """Neighbour table of a level set to "none", through memory that torch takes for another tensor's."""
+  v = oc.OctreeView(octree.cpu().numpy())
+  at = int(v.ptr_dis[oc.PROPS.index('neigh')]) + 32 * int(v.nnum_cum[d])
+  torch.from_dlpack(octree)[at:at + 32 * int(v.nnum[d])] = 255
+
+
 def both(ocnn, octree, d, cin, cout, dtype, with_res=False, edit=None):
+  """The layer over all taps and on a plan.  A plan has its own tables: the layer runs on it after the octree's were
+  wiped, which the walk over all taps does not survive."""
   h = int((ocnn.octree_property(octree, 'child', d) >= 0).sum())
   torch.manual_seed(cin + cout + d)
   fmt = dict(memory_format=torch.channels_last)
@@ -82,10 +91,15 @@ def both(ocnn, octree, d, cin, cout, dtype, with_res=False, edit=None):
   layer = ocnn.OctreeConv(d, cin, cout, nempty=True).cuda().eval()
   if edit is not None:
     edit(layer.weights)
-  planned = octree.view(-1)
-  planned.tap_plan = ocnn.nn.TapPlan(octree, [d])
+  base = octree.clone()
+  planned = base.view(-1)
+  planned.tap_plan = ocnn.nn.TapPlan(base, [d])
   with torch.no_grad():
-    return [layer._run(x, o, bn, res, with_res) for o in (octree, planned)]
+    want = layer._run(x, base, bn, res, with_res)
+    wipe_neighbours(base, d)
+    assert not torch.equal(layer._run(x, base, bn, res, with_res), want)
+    assert planned.tap_plan.serves(planned, d, h)
+    return want, layer._run(x, planned, bn, res, with_res)
 
 
 # (channels that share K-blocks between taps, that leave a remainder, that fill 1 to 8 blocks; output columns of
@@ -117,21 +131,33 @@ def test_weights_that_are_not_finite(ocnn, small, value):
 def test_a_plan_serves_only_what_it_was_made_for(ocnn, small):
   octree = small[0].clone()
   h = int((ocnn.octree_property(octree, 'child', 5) >= 0).sum())
+  # as many nodes on every level, others: the same clouds with x and y swapped
+  _, swapped, _ = gu.oracle_batch([[a[:, [1, 0, 2]] for a in c[:2]] for c in gu.small_clouds(3, 3000, 500)], 5, 2, 64)
+  swapped = gu.to_cuda_u8(swapped)
+  assert ocnn.nn.octree_info(swapped) == ocnn.nn.octree_info(octree) and swapped.numel() == octree.numel()
   x = torch.randn(1, 32, h, 1, device='cuda').bfloat16().contiguous(memory_format=torch.channels_last)
   layer = ocnn.OctreeConv(5, 32, 32, nempty=True).cuda().eval()
   planned = octree.view(-1)
-  planned.tap_plan = ocnn.nn.TapPlan(octree, [5])
+  plan = planned.tap_plan = ocnn.nn.TapPlan(octree, [5])
   with torch.no_grad():
-    want = layer(x, octree)
+    want, want_swapped = layer(x, octree), layer(x, swapped)
+    assert not torch.equal(want, want_swapped)
+    assert plan.serves(planned, 5, h) and plan.serves(octree, 5, h)
+    assert not (plan.serves(planned, 4, h) or plan.serves(planned, 5, h - 1) or plan.serves(small[0], 5, h))
     assert torch.equal(layer(x, planned), want)
     other = torch.cuda.Stream()
     other.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(other):
-      got = layer(x, planned)              # not waited for there
+      assert not plan.serves(planned, 5, h)                # made by work that this stream need not have waited for
+      got = layer(x, planned)
     torch.cuda.current_stream().wait_stream(other)
     assert torch.equal(got, want)
-    planned.copy_(small[0])                # written to since
-    assert torch.equal(layer(x, planned), want)
+    other_octree = swapped.view(-1)
+    other_octree.tap_plan = plan
+    assert torch.equal(layer(x, other_octree), want_swapped)
+    planned.copy_(swapped)                 # written to since
+    assert not plan.serves(planned, 5, h)
+    assert torch.equal(layer(x, planned), want_swapped)
 
 
 # ---- the network on its plans --------------------------------------------------------------------------------
