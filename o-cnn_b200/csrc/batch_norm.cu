@@ -192,7 +192,10 @@ __global__ void __launch_bounds__(kBnThreads) bn_backward_kernel(const BnArgs a)
 }
 
 // Cluster size: doubled while a CTA still has 4096 rows or more (eight a thread: less does not pay for the
-// exchange) and the GPU is not full (two CTAs an SM), or the slice does not fit into shared memory.
+// exchange) and the GPU is not full (four CTAs an SM), or the slice does not fit into shared memory.  In us with data
+// in L2, 1 / 2 / 4 / 8 CTAs a channel: 16 channels x 40 k rows 14.0 / 10.8 / 8.9 / 8.7 (the rule takes 8), 64 x 107 k
+// 65 / 33 / 35 / 34 (8), 256 x 107 k 169 / 137 / 136 / 123 (8), 256 x 16 k 14.5 / 13.5 / 14.2 / 22.8 (4), 256 x 4 k
+// 8.8 / 8.8 / 9.4 / 19.7 (2); it is off the best at 128 x 16 k, 8.7 / 8.9 / 8.8 / 12.5 (8).
 int bn_backward(BnArgs a, bool vec, cudaStream_t st) {
   constexpr size_t kRowBytes = 8;              // x and g
   int cluster = 1;

@@ -5,15 +5,16 @@
 // its mask, its table of rows and its first copies, a microsecond each, with the epilogue behind it; two or three
 // CTAs with a short ring share an SM to cover one another.  The gathered rows' indices come from the plan's table
 // in one bulk copy instead of 27 look-ups through neighbour and child arrays.  96 -> 96 at 192 k nodes of depth 9
-// (7 of 27 taps a tile): 146 us over all taps, 58 us so.  Slower: indices read from the plan by the gathering threads
-// (they queue behind their copies, 80 us), and one persistent CTA per SM with a ring of six stages, tables a tile
-// ahead and its own epilogue warps (91 us: a K-block is a chain of barriers, 0.3 us of it in the one thread that
-// issues the products, and one such chain per SM is too few); a warp that waits as a whole for the issuing lane
-// (73 us).
+// (7 of 27 taps a tile): 146 us over all taps, 52 us so.  Slower, when this form took 58: indices read from the plan
+// by the gathering threads (they queue behind their copies, 80 us), one persistent CTA per SM with a ring of six
+// stages, tables a tile ahead and its own epilogue warps (91 us at best: a K-block is a chain of barriers, and one
+// such chain per SM is too few), and a warp that waits as a whole for the issuing lane (73 us).  With K split over
+// CTAs as an option the same layers took 58 us in place of 52.
 //
 // K-blocks keep the packed weights' layout, in which a tap need not start on a block: of a block that is
 // shared by taps only the 16-channel steps of present ones are multiplied, and only their chunks gathered.
-// Results are those of the walk over all taps bit for bit: what is left out are additions of zero.  Weights
+// Results are those of the walk over all taps bit for bit, where that walk does not split K: what is left out are
+// additions of zero.  Weights
 // that are not finite are the exception (zero times infinity); the packed image says so, and then every tap
 // is walked.
 #pragma once

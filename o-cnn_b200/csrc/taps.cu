@@ -3,7 +3,7 @@
 // On the non-empty nodes of a scene a node has 2.4 (depth 9) to 12 (depth 5) of 27 neighbours, but 128 nodes
 // in Morton order have all 27 between them, so a convolution tile walks every tap: products of zeros and
 // weight tiles fetched for them.  Sorted by the set of taps they have, 128 nodes share 7 (depth 9), 12 (depth 8)
-// or 16 taps (200 k points), and the convolution (conv_taps.cu) walks only those.
+// or 16 taps (200 k points), and the convolution (conv_taps.cuh) walks only those.
 //
 // The sort key is the Gray rank of the 26-bit neighbour set with corners above edges above faces (neighbours in
 // that order differ by few taps: 4.8 / 10.6 taps a tile in full order, 5.1 / 11.3 without the Gray code, 5.2 /
@@ -12,7 +12,7 @@
 // takes is left to atomics: a node's result does not depend on it, only on the node's own rows.
 //
 // Four launches for all levels together (115 us for the five levels of a U-Net on 200 k points, 254 k sibling groups
-// and 443 k nodes; its 40 convolutions gain 0.8 ms), each bound by latency and scattered 4-byte reads of L2: keys and
+// and 443 k nodes; with 34 of its convolutions on the plan the pass is 0.85 ms shorter, plan included), each bound by latency and scattered 4-byte reads of L2: keys and
 // histogram (a sibling group's 64 neighbours are read once for its up to eight nodes), binning,
 // window sort, tables.  The tables hold the gathered rows' indices per tile and present tap, in the order in
 // which the convolution's threads read them.

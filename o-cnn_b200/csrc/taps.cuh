@@ -1,4 +1,4 @@
-// The tap plan of a level (taps.cu writes it, conv_taps.cu reads it).
+// The tap plan of a level (taps.cu writes it, conv_taps.cuh reads it).
 #pragma once
 
 #include "common.cuh"

@@ -1152,13 +1152,7 @@ Tensor pointwise_conv_tc(Tensor data_in, Tensor packed, int num_output, c10::opt
   return y;
 }
 
-// ---- a module's layer -------------------------------------------------------------------------------
-// What OctreeConv / OctreeDeconv (point = false) and OctreeConv1x1 (point = true) do for one call in
-// eval mode, with the BatchNorm, residual and ReLU that follow: choose the kernel, pack the weights when
-// they have changed, launch.  The module hands over its parameters as they are; the BatchNorm is
-// folded inside the kernel (ChannelAffine), so a layer is one call from Python and one launch.
-// (In Python, with the folded vectors computed by tensor operations, it was about 60 us of host time
-// and six launches per layer.)
+// ---- tap plans --------------------------------------------------------------------------------------
 // Tap plans of an octree's levels (ocnn_tap_plan): made for one forward pass, whose layers on the non-empty nodes
 // of the same levels share them.  A layer takes the plan only for the octree, content and stream that it was
 // made for.
@@ -1166,9 +1160,10 @@ class TapPlan {
  public:
   // `worthwhile`: only the levels of more tiles (128 rows) than SMs, and none if no level has twice as many.  With one
   // tile per SM or less a layer is one wave of one chain of K-blocks either way, and the walk over all taps has shorter
-  // tiles and K split for it (256 -> 256 on 18.5 k rows 53 us against 58 on a plan; on 19.0 k rows, 149 tiles, 74
-  // against 59).  A plan costs 40 us and more, and its first 1.5 tiles per SM return less: a U-Net whose largest level
-  // has 37 k rows took 1286 us without and 1333 with one (50 k points, depth 7), with 49 k rows 1851 and 1810 (depth 9).
+  // tiles and K split for it (256 -> 256 on 148 tiles 50 us against 55 on a plan; on 149 tiles 73 against 55).
+  // A plan costs 40 us and more, and its first 1.5 tiles per SM return less: a U-Net whose largest level has 37 k rows
+  // took 1287 us without and 1326 with one (50 k points, depth 7), with 42 k rows 1438 and 1416 (45 k, depth 8), with
+  // 49 k rows 1850 and 1747 (50 k, depth 9).
   TapPlan(Tensor octree, const vector<int>& depths, bool worthwhile) : octree_(octree) {
     OctreeRef o = get_octree(octree);
     TORCH_CHECK(o.cuda, "TapPlan: the octree must be a CUDA tensor");
@@ -1244,6 +1239,13 @@ class TapPlan {
   vector<const void*> plans_;
 };
 
+// ---- a module's layer -------------------------------------------------------------------------------
+// What OctreeConv / OctreeDeconv (point = false) and OctreeConv1x1 (point = true) do for one call in
+// eval mode, with the BatchNorm, residual and ReLU that follow: choose the kernel, pack the weights when
+// they have changed, launch.  The module hands over its parameters as they are; the BatchNorm is
+// folded inside the kernel (ChannelAffine), so a layer is one call from Python and one launch.
+// (In Python, with the folded vectors computed by tensor operations, it was about 60 us of host time
+// and six launches per layer.)
 class ConvLayer {
  public:
   ConvLayer(int cin, int cout, vector<int> ks, int stride, bool nempty, bool transposed, bool point)
