@@ -192,8 +192,8 @@ def node_data(octree, ocnn, dtype):
 
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
 def test_network_on_plans_is_the_network_without(ocnn, scene, dtype, monkeypatch):
-  """`UNet.forward` with the plans it makes: every 3x3x3 layer of a larger level runs on one and the others do not, down
-  and up again, and the scores are those of the walk over all taps bit for bit."""
+  """`UNet.forward` with the plans it makes: every 3x3x3 layer of a larger level finds one (conv1, of 8 channels, does
+  not take it) and the others do not, down and up again, and the scores are those of the walk over all taps bit for bit."""
   octree, rows, planned, pts = scene
   net, data = make_unet(ocnn, 5), node_data(octree, ocnn, dtype)
   base, make, seen = ocnn.OctreeConv.__base__, ocnn.unet._with_tap_plan, []
